@@ -10,10 +10,11 @@
 //    sin are the correctly rounded ones of st_crmath.cuh (equal to the host C
 //    library's wherever those are correctly rounded), or CUDA's with
 //    ST_TRAJ_CORRECTLY_ROUNDED 0 (st_fields.cuh).
-//  * The spin steppers are restated for the FP64 pipe: FMA-contracted stage
-//    sums, the field as a polynomial in segment time, reciprocal-form error
-//    weights and step controller.  Results agree with the reference to the
-//    integration tolerance, not bit for bit.
+//  * The spin steppers are restated: the field as a polynomial in segment time,
+//    reciprocal-form error weights and step controller.  DOP853 steps run in
+//    64-bit fixed point (st_fixed.cuh), the rest (and DOP853 steps outside the
+//    fixed-point range) in FMA-contracted FP64.  Results agree with the
+//    reference to the integration tolerance, not bit for bit.
 #pragma once
 
 #include <float.h>
@@ -22,6 +23,7 @@
 #include "st_fields.cuh"
 #include "st_tableau.h"
 #include "st_crmath.cuh"
+#include "st_fixed.cuh"
 
 namespace st {
 // The trajectory's transcendental functions (ST_TRAJ_CORRECTLY_ROUNDED, st_fields.cuh).
@@ -698,7 +700,9 @@ __device__ __forceinline__ bool traj_event(PState& p, const SetParams& P, double
 
 // ------------------------------------------------------------ field model
 // Integrator state of the current segment.  Omega(tau) = gamma*B at time
-// t0 + tau is the quadratic o0 + tau*(o1 + tau*o2) (plus the pulse).
+// t0 + tau is the quadratic o0 + tau*(o1 + tau*o2) (plus the pulse).  For
+// DOP853 in fixed point (fx) the same fields hold the Q63 words of st_fixed.cuh
+// (as bits): the scaled polynomial and pulse amplitude, and the spin in k.
 struct Seg {
   double o0x, o0y, o0z, o1x, o1y, o1z, o2x, o2y, o2z;
 #if !ST_GRAD_IS_LINEAR
@@ -706,13 +710,15 @@ struct Seg {
 #endif
   double gpa;          // gamma * pulse amplitude (0: no pulse)
   double t0, xf, x, h, posneg, facold;
-  double kx, ky, kz;   // DOP853: derivative at (x, y) (FSAL); RK45: last stage-6 state
+  double kx, ky, kz;   // DOP853: the spin (fx) or the derivative at (x, y) (FSAL); RK45: last stage-6 state
   double lastH, lnprev;
   double hu;           // step size of the last accepted attempt (read by the adjoint replay)
   unsigned int nstep;
   int turns;           // precession turns of the segment's accepted steps (count_turn)
   bool reject, last;
   bool acc;            // the last attempt was accepted
+  bool fx;             // DOP853 in fixed point, scaled by sc
+  fx::SegScale sc;
 };
 
 // Precession phase accumulation: the phase phi = atan2(Sz, Sy) about x jumps
@@ -733,6 +739,22 @@ __device__ __forceinline__ int count_turn(double y0, double z0, double y1, doubl
 __device__ inline void prepare_set(SetParams& P) {
   const double gm = P.gamma;
   const double g_ = P.gravity ? kGravity : 0.0;
+  // atol / rtol for the fixed-point step controller (-1: out of its range), and
+  // the pulse's turns per second |w| / 2 pi = wturn_m 2^(wturn_e - 64) to 64 bits
+  P.tol_ratio = P.beta == 0.0 && fx::bexp(P.rtol) > 0 && P.rtol > 0.0 && P.atol >= 0.0 ? P.atol / P.rtol : -1.0;
+  P.wturn_m = 0;
+  P.wturn_e = 0;
+  if (P.w != 0.0 && isfinite(P.w)) {
+    const double w = fabs(P.w), p = w * 0.15915494309189535;  // 1 / (2 pi) = 0.15915494309189535 -9.839338337591243e-18
+    const double e = fma(w, -9.839338337591243e-18, fma(w, 0.15915494309189535, -p));
+    const int x = fx::bexp(p) - 1022;  // p in [1/2, 1) 2^x
+    if (x > -900 && x < 900) {
+      const uint64_t m = (uint64_t)(fx::to_q63(p, x)) << 1;
+      const uint64_t de = (uint64_t)(long long)rint(ldexp(e, 64 - x));
+      P.wturn_m = (de >> 63) == 0 && m + de < m ? ~0ull : m + de;
+      P.wturn_e = x;
+    }
+  }
   P.gB0[0] = gm * P.B0x; P.gB0[1] = gm * P.B0y; P.gB0[2] = gm * P.B0z;
   const Vec3 ex = {1.0, 0.0, 0.0}, ey = {0.0, 1.0, 0.0}, ez = {0.0, 0.0, 1.0};
   const Vec3 c0 = st_grad(ex, P), c1 = st_grad(ey, P), c2 = st_grad(ez, P);
@@ -780,10 +802,57 @@ __device__ __forceinline__ void seg_begin(Seg& g, const SetParams& P, double t0,
   g.posneg = (t_end - t0 < 0.0) ? -1.0 : 1.0;
 }
 
-__device__ __forceinline__ void seg_setup(Seg& g, const SetParams& P, const SegStart& s0, double t_end) {
+// The fixed-point words of a segment's state, kept in its double fields.
+__device__ __forceinline__ double as_f64(fx::i64 m) { return __longlong_as_double(m); }
+__device__ __forceinline__ fx::i64 as_i64(double x) { return __double_as_longlong(x); }
+
+// The field of a segment as the trajectory side hands it to the spin side:
+// the polynomial's o0 and o1, for DOP853 sets scaled to fixed point where they
+// have a scale there (fx; then o0 and o1 hold Q63 words).
+struct SegPoly {
   double o0[3], o1[3];
-  seg_field(P, s0.px, s0.py, s0.pz, s0.vx, s0.vy, s0.vz, o0, o1);
-  seg_begin(g, P, s0.t, t_end, o0, o1);
+  fx::SegScale sc;
+  bool fx;
+};
+// Scale a polynomial given in doubles over a segment of length T.
+__device__ __forceinline__ void seg_scale(SegPoly& q, const SetParams& P, double T) {
+  q.fx = false;
+#if ST_GRAD_IS_LINEAR && ST_PULSE_IS_Z_COS
+  const double gpa = P.gamma * P.a;
+  if (P.integrator == 0 && P.tol_ratio >= 0.0 && (gpa == 0.0 || isfinite(P.w)))
+    q.fx = fx::field_scale(q.o0, q.o1, P.o2c, gpa, T, q.sc);
+  if (q.fx) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      q.o0[c] = as_f64(fx::to_q63(q.o0[c], q.sc.oe));
+      q.o1[c] = as_f64(fx::to_q63(q.o1[c], q.sc.oe - q.sc.te));
+    }
+  }
+#endif
+}
+__device__ __forceinline__ void seg_poly(SegPoly& q, const SetParams& P, const SegStart& s0, double t_end) {
+  seg_field(P, s0.px, s0.py, s0.pz, s0.vx, s0.vy, s0.vz, q.o0, q.o1);
+  seg_scale(q, P, t_end - s0.t);
+}
+
+// Fill the integrator's segment from the handed-over field.
+__device__ __forceinline__ void seg_open(Seg& g, const SetParams& P, const SegPoly& q, double t0, double t_end) {
+  seg_begin(g, P, t0, t_end, q.o0, q.o1);
+  g.fx = q.fx;
+  g.sc = q.sc;
+  if (q.fx) {
+    const int e2 = q.sc.oe - 2 * q.sc.te;
+    g.o2x = as_f64(fx::to_q63(g.o2x, e2));
+    g.o2y = as_f64(fx::to_q63(g.o2y, e2));
+    g.o2z = as_f64(fx::to_q63(g.o2z, e2));
+    g.gpa = as_f64(fx::to_q63(g.gpa, q.sc.oe));
+  }
+}
+
+__device__ __forceinline__ void seg_setup(Seg& g, const SetParams& P, const SegStart& s0, double t_end) {
+  SegPoly q;
+  seg_poly(q, P, s0, t_end);
+  seg_open(g, P, q, s0.t, t_end);
 #if !ST_GRAD_IS_LINEAR
   g.p0x = s0.px; g.p0y = s0.py; g.p0z = s0.pz;
   g.v0x = s0.vx; g.v0y = s0.vy; g.v0z = s0.vz;
@@ -875,6 +944,29 @@ __device__ __forceinline__ void homega_at(const HPoly& q, const Seg& g, const Se
 }
 
 // ------------------------------------------------------------ DOP853
+// A fixed-point segment's field back in doubles.
+__device__ __forceinline__ void seg_unscale(Seg& g) {
+  const int e0 = g.sc.oe, e1 = e0 - g.sc.te, e2 = e1 - g.sc.te;
+  g.o0x = fx::from_q63(as_i64(g.o0x), e0); g.o0y = fx::from_q63(as_i64(g.o0y), e0); g.o0z = fx::from_q63(as_i64(g.o0z), e0);
+  g.o1x = fx::from_q63(as_i64(g.o1x), e1); g.o1y = fx::from_q63(as_i64(g.o1y), e1); g.o1z = fx::from_q63(as_i64(g.o1z), e1);
+  g.o2x = fx::from_q63(as_i64(g.o2x), e2); g.o2y = fx::from_q63(as_i64(g.o2y), e2); g.o2z = fx::from_q63(as_i64(g.o2z), e2);
+  g.gpa = fx::from_q63(as_i64(g.gpa), e0);
+  g.fx = false;
+}
+
+// The spin of a fixed-point segment in progress as doubles.
+__device__ __forceinline__ void dop_spin(const Seg& g, double& Sx, double& Sy, double& Sz) {
+  Sx = fx::from_q63(as_i64(g.kx), g.sc.se);
+  Sy = fx::from_q63(as_i64(g.ky), g.sc.se);
+  Sz = fx::from_q63(as_i64(g.kz), g.sc.se);
+}
+
+// The derivative at the start of an FP64 segment, taking the segment out of fixed point first.
+static __device__ __noinline__ void dop_begin_f64(Seg& g, const SetParams& P, double Sx, double Sy, double Sz) {
+  if (g.fx) seg_unscale(g);
+  feval(g, P, 0.0, Sx, Sy, Sz, g.kx, g.ky, g.kz);
+}
+
 // Start a DOP853 call over the segment (src/integrator.cpp:102-119).
 __device__ __forceinline__ void dop_begin(Seg& g, const SetParams& P, double Sx, double Sy, double Sz, double h) {
   g.h = h;
@@ -883,127 +975,31 @@ __device__ __forceinline__ void dop_begin(Seg& g, const SetParams& P, double Sx,
   g.turns = 0;
   g.reject = false;
   g.last = false;
-  feval(g, P, 0.0, Sx, Sy, Sz, g.kx, g.ky, g.kz);
+  const double S[3] = {Sx, Sy, Sz};
+  if (g.fx && fx::spin_scale(S, g.sc.se) && fx::ratio_fits(P.tol_ratio, g.sc.se)) {
+    g.kx = as_f64(fx::to_q63(Sx, g.sc.se));
+    g.ky = as_f64(fx::to_q63(Sy, g.sc.se));
+    g.kz = as_f64(fx::to_q63(Sz, g.sc.se));
+  } else {
+    Seg t = g;  // the call takes its address: g itself stays in registers
+    dop_begin_f64(t, P, Sx, Sy, Sz);
+    g = t;
+  }
 }
 
-// DOP853 stage structure as constexpr functions of compile-time stage and
-// term indices (they fold to constants inside unrolled loops).
-namespace dopst {
-// earlier stages summed into stage s (2..12): stage 1, then 2 (s = 3),
-// 3.. (s = 4, 5) or 4.. (s >= 6)
-__device__ __forceinline__ constexpr int src(int s, int j) { return j == 0 ? 1 : (s == 3 ? 2 : (s <= 5 ? j + 2 : j + 3)); }
-__device__ __forceinline__ constexpr int cnt(int s) { return s <= 2 ? s - 1 : (s <= 4 ? 2 : (s == 5 ? 3 : s - 3)); }
-// coefficient of term j of stage s (the a_{s,src(s,j)} of the tableau)
-__device__ __forceinline__ constexpr double a(int s, int j) {
-  switch (s * 16 + j) {
-    case 32: return dop::A21;
-    case 48: return dop::A31;
-    case 49: return dop::A32;
-    case 64: return dop::A41;
-    case 65: return dop::A43;
-    case 80: return dop::A51;
-    case 81: return dop::A53;
-    case 82: return dop::A54;
-    case 96: return dop::A61;
-    case 97: return dop::A64;
-    case 98: return dop::A65;
-    case 112: return dop::A71;
-    case 113: return dop::A74;
-    case 114: return dop::A75;
-    case 115: return dop::A76;
-    case 128: return dop::A81;
-    case 129: return dop::A84;
-    case 130: return dop::A85;
-    case 131: return dop::A86;
-    case 132: return dop::A87;
-    case 144: return dop::A91;
-    case 145: return dop::A94;
-    case 146: return dop::A95;
-    case 147: return dop::A96;
-    case 148: return dop::A97;
-    case 149: return dop::A98;
-    case 160: return dop::A101;
-    case 161: return dop::A104;
-    case 162: return dop::A105;
-    case 163: return dop::A106;
-    case 164: return dop::A107;
-    case 165: return dop::A108;
-    case 166: return dop::A109;
-    case 176: return dop::A111;
-    case 177: return dop::A114;
-    case 178: return dop::A115;
-    case 179: return dop::A116;
-    case 180: return dop::A117;
-    case 181: return dop::A118;
-    case 182: return dop::A119;
-    case 183: return dop::A1110;
-    case 192: return dop::A121;
-    case 193: return dop::A124;
-    case 194: return dop::A125;
-    case 195: return dop::A126;
-    case 196: return dop::A127;
-    case 197: return dop::A128;
-    case 198: return dop::A129;
-    case 199: return dop::A1210;
-    case 200: return dop::A1211;
-    default: return 0.0;
-  }
-}
-// node of stage s (stage 12 at x + h)
-__device__ __forceinline__ constexpr double c(int s) {
-  switch (s) {
-    case 2: return dop::C2;
-    case 3: return dop::C3;
-    case 4: return dop::C4;
-    case 5: return dop::C5;
-    case 6: return dop::C6;
-    case 7: return dop::C7;
-    case 8: return dop::C8;
-    case 9: return dop::C9;
-    case 10: return dop::C10;
-    case 11: return dop::C11;
-    case 12: return 1.0;
-    default: return 0.0;
-  }
-}
-// 8th-order weight of stage s
-__device__ __forceinline__ constexpr double b(int s) {
-  switch (s) {
-    case 1: return dop::B1;
-    case 6: return dop::B6;
-    case 7: return dop::B7;
-    case 8: return dop::B8;
-    case 9: return dop::B9;
-    case 10: return dop::B10;
-    case 11: return dop::B11;
-    case 12: return dop::B12;
-    default: return 0.0;
-  }
-}
-}  // namespace dopst
-
-// Where an attempt keeps its stage derivatives k2..k11 (k1 and k12 stay in
-// registers): registers (a local array that the unrolled code indexes with
-// constants), or this thread's column of a [10][3][BLOCK] shared-memory
-// array, which frees ~30 registers per thread.
-struct StageRegs {
+// FP64 stage derivatives k2..k11.
+struct StageF64 {
   double v[12][3];
   __device__ __forceinline__ double& k(int s, int c) { return v[s][c]; }
 };
-struct StageSmem {
-  double* base;  // &array[0][0][thread]
-  int stride;    // BLOCK
-  __device__ __forceinline__ double& k(int s, int c) { return base[((s - 2) * 3 + c) * stride]; }
-};
 
-// One attempted DOP853 step (one pass of the loop at src/integrator.cpp:128-247),
-// stage derivatives in `ks`.  Returns 0 to continue, 1 when the segment's last
+// One attempted DOP853 step (one pass of the loop at src/integrator.cpp:128-247)
+// in FP64.  A call, not inlined: the fixed-point step takes all but a few.  Returns 0 to continue, 1 when the segment's last
 // step was accepted (g.h then holds that step, as the reference returns it),
 // -1 after more than nmax attempts.
-template <class KS>
-__device__ __forceinline__ int dop_attempt_ks(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz,
-                                              KS& ks) {
+static __device__ __noinline__ int dop_attempt_f64(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz) {
   using namespace dop;
+  StageF64 ks;
   if (g.nstep > P.nmax) return -1;
   double h = g.h;
   bool last = g.last;
@@ -1134,10 +1130,102 @@ __device__ __forceinline__ int dop_attempt_ks(Seg& g, const SetParams& P, double
 }
 
 
-// One attempted DOP853 step with the stage derivatives in registers.
+// The FP64 attempt for a segment in fixed point: on an accepted step the
+// segment goes on in FP64, a rejected one changes its step size only.
+__device__ __forceinline__ int dop_attempt_fallback(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz) {
+  Seg t = g;  // the call takes its address: g itself stays in registers
+  double S[3] = {Sx, Sy, Sz};
+  if (t.fx) {
+    seg_unscale(t);
+    dop_spin(g, S[0], S[1], S[2]);
+    feval(t, P, t.x - t.t0, S[0], S[1], S[2], t.kx, t.ky, t.kz);
+  }
+  const int r = dop_attempt_f64(t, P, S[0], S[1], S[2]);
+  if (g.fx && !t.acc) {
+    g.h = t.h;
+    g.reject = t.reject;
+    g.last = t.last;
+    g.nstep = t.nstep;
+    g.acc = false;
+  } else {
+    g = t;
+    Sx = S[0];
+    Sy = S[1];
+    Sz = S[2];
+  }
+  return r;
+}
+
+// One attempted DOP853 step (one pass of the loop at src/integrator.cpp:128-247),
+// spin components over the lanes of `view`, stage derivatives in `ks`.  While
+// the segment is in fixed point, Sx..Sz are brought up to date at its end.
+// Returns as dop_attempt_f64.
+//
+// What bounds it: issue.  ~3,500 instructions, a third of them IMAD.WIDE (2.1
+// cycles each per SM sub-partition), most others 1-2 cycles, against ~510 FP64
+// instructions of 76 cycles before.
+template <class V, class KS>
+__device__ __forceinline__ int dop_attempt_v(const V& view, KS& ks, Seg& g, const SetParams& P, double& Sx, double& Sy,
+                                             double& Sz) {
+  if (g.nstep > P.nmax) return -1;
+  if (!g.fx) return dop_attempt_fallback(g, P, Sx, Sy, Sz);
+  double h = g.h;
+  bool last = g.last;
+  if ((g.x + 1.01 * h - g.xf) * g.posneg > 0.0) {
+    h = g.xf - g.x;
+    last = true;
+  }
+  if (h < P.hmin && !last) h = P.hmin;
+  fx::i64 o0[V::N], o1[V::N], o2[V::N], S[V::N], Sn[V::N];
+  view.pick(as_i64(g.o0x), as_i64(g.o0y), as_i64(g.o0z), o0);
+  view.pick(as_i64(g.o1x), as_i64(g.o1y), as_i64(g.o1z), o1);
+  view.pick(as_i64(g.o2x), as_i64(g.o2y), as_i64(g.o2z), o2);
+  view.pick(as_i64(g.kx), as_i64(g.ky), as_i64(g.kz), S);
+  const fx::StepTol tol = {P.rtol, P.tol_ratio};
+  fx::StepOut out;
+  if (!fx::dop_step(view, ks, g.sc, o0, o1, o2, as_i64(g.gpa), (fx::u64)P.wturn_m, P.wturn_e, g.x, g.x - g.t0, h, tol, S,
+                    Sn, out))
+    return dop_attempt_fallback(g, P, Sx, Sy, Sz);
+  g.nstep++;
+  g.acc = false;
+  // step-size controller (clamped to [fac1, fac2]; beta = 0)
+  const double grow = max_d(P.fac1, P.safe * out.root8);
+  double hnew;
+  if (out.accept || P.fixed) {
+    hnew = h * min_d(P.fac2, grow);
+    g.acc = true;
+    g.hu = h;
+    fx::i64 N3[3];
+    view.gather(Sn, N3);
+    const fx::i64 y0 = as_i64(g.ky), z0 = as_i64(g.kz);
+    if (y0 < 0 && N3[1] < 0 && (z0 < 0) != (N3[2] < 0)) g.turns += z0 < 0 ? -1 : 1;  // count_turn
+    g.kx = as_f64(N3[0]);
+    g.ky = as_f64(N3[1]);
+    g.kz = as_f64(N3[2]);
+    g.x = g.x + h;
+    if (last) {
+      g.h = h;
+      g.last = true;
+      dop_spin(g, Sx, Sy, Sz);
+      return 1;
+    }
+    if (fabs(hnew) > P.hmax) hnew = g.posneg * P.hmax;
+    if (g.reject) hnew = g.posneg * min_d(fabs(hnew), fabs(h));
+    g.reject = false;
+  } else {
+    hnew = h * grow;
+    g.reject = true;
+    last = false;
+  }
+  g.last = last;
+  g.h = P.fixed ? h : hnew;
+  return 0;
+}
+
+// One attempted DOP853 step on one lane, stage derivatives in local memory.
 __device__ __forceinline__ int dop_attempt(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz) {
-  StageRegs ks;
-  return dop_attempt_ks(g, P, Sx, Sy, Sz, ks);
+  fx::StageLocal<3> ks;
+  return dop_attempt_v(fx::Lane3(), ks, g, P, Sx, Sy, Sz);
 }
 
 // ------------------------------------------------------------ RK45

@@ -302,8 +302,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_persistent(RunArgs a) {
 //
 // Record fields (field-major, conflict-free): qd[(slot * kRecF + f) * BLOCK + tid]
 //   f = 0 t_start, 1 t_end, 2..4 o0, 5..7 o1 (+ 8..13 p0, v0 when the grad hook is not linear)
+// (o0, o1 as Q63 words when the flags say so: SegPoly), the field's scale
+// qs[slot * BLOCK + tid] = (norm bits, exponents),
 // flags qf[slot * BLOCK + tid]: bit0 window end reached, bit1 stop, bit2 bounce, bit3 gas
-// collision, bits 8-15 sanity failure code.
+// collision, bit4 field in fixed point, bits 8-15 sanity failure code.
 constexpr int kRecF = ST_GRAD_IS_LINEAR ? 8 : 14;
 
 // ---- adjoint tape (TAPE instantiation only)
@@ -401,8 +403,21 @@ __device__ __forceinline__ DeviceState state_slot(const DeviceState& b, int64_t 
   return s;
 }
 
+// A record's field scale in two words.
+__device__ __forceinline__ int2 pack_scale(const fx::SegScale& s) {
+  return make_int2((int)fx::f32_bits(s.on), (s.oe << 16) | (s.te & 0xffff));
+}
+__device__ __forceinline__ fx::SegScale unpack_scale(int2 v) {
+  fx::SegScale s;
+  s.on = fx::bits_f32((uint32_t)v.x);
+  s.oe = v.y >> 16;
+  s.te = (int)(short)(v.y & 0xffff);
+  s.se = 0;
+  return s;
+}
+
 template <int BLOCK, bool TAPE, bool GAS, bool EXT>
-__device__ __forceinline__ void produce_record(PState& tp, const SetParams& P, double tf, double* qd, int* qf,
+__device__ __forceinline__ void produce_record(PState& tp, const SetParams& P, double tf, double* qd, int2* qs, int* qf,
                                                int slot, int tid, bool& blocked, EventDefer& dd, const TapeArgs& ta,
                                                TapeCursor& tc) {
   SegStart s0;
@@ -411,11 +426,16 @@ __device__ __forceinline__ void produce_record(PState& tp, const SetParams& P, d
   double* r = qd + (size_t)slot * kRecF * BLOCK + tid;
   r[0 * BLOCK] = s0.t;
   r[1 * BLOCK] = tp.t;
+  int fixed = 0;
   if (spin_on<EXT>(P.integrator)) {
-    double o0[3], o1[3];
-    seg_field(P, s0.px, s0.py, s0.pz, s0.vx, s0.vy, s0.vz, o0, o1);
-    r[2 * BLOCK] = o0[0]; r[3 * BLOCK] = o0[1]; r[4 * BLOCK] = o0[2];
-    r[5 * BLOCK] = o1[0]; r[6 * BLOCK] = o1[1]; r[7 * BLOCK] = o1[2];
+    SegPoly q;
+    seg_poly(q, P, s0, tp.t);
+    r[2 * BLOCK] = q.o0[0]; r[3 * BLOCK] = q.o0[1]; r[4 * BLOCK] = q.o0[2];
+    r[5 * BLOCK] = q.o1[0]; r[6 * BLOCK] = q.o1[1]; r[7 * BLOCK] = q.o1[2];
+    if (q.fx) {
+      qs[slot * BLOCK + tid] = pack_scale(q.sc);
+      fixed = 16;
+    }
 #if !ST_GRAD_IS_LINEAR
     r[8 * BLOCK] = s0.px; r[9 * BLOCK] = s0.py; r[10 * BLOCK] = s0.pz;
     r[11 * BLOCK] = s0.vx; r[12 * BLOCK] = s0.vy; r[13 * BLOCK] = s0.vz;
@@ -424,7 +444,7 @@ __device__ __forceinline__ void produce_record(PState& tp, const SetParams& P, d
   // the segments the spin side integrates, in order
   if (TAPE && !tp.stop && tp.fail == 0) tape_seg(ta, tc, s0);
   qf[slot * BLOCK + tid] = (fin ? 1 : 0) | (tp.stop ? 2 : 0) | (tp.n_bounce != nb ? 4 : 0) |
-                           (tp.n_coll != nc ? 8 : 0) | ((tp.fail & 0xff) << 8);
+                           (tp.n_coll != nc ? 8 : 0) | fixed | ((tp.fail & 0xff) << 8);
   if (fin || tp.stop) blocked = true;
 }
 
@@ -438,16 +458,18 @@ enum BatchedMode { B_FETCH = 0, B_NEED = 1, B_SEG = 2, B_WEND = 3, B_DONE = 4 };
 // TAPE: also write the adjoint tape (steps and segments of every particle)
 // and state checkpoints at every ta.ckpt_every-th window end.
 // GAS = false: the instantiation for launches without gas collisions.
-// STAGES = 1: DOP853 stage derivatives k2..k11 in shared memory (after the
-// rings), not in registers.
 // EXT: also integrator types 2-5.
-template <int BLOCK, int MINB, int QCAP, bool TAPE, bool GAS, int STAGES, bool EXT>
+template <int BLOCK, int MINB, int QCAP, bool TAPE, bool GAS, bool EXT>
 __global__ void __launch_bounds__(BLOCK, MINB)
     k_batched(RunArgs a, int topup_start, int topup_keep, int defer_k, TapeArgs ta) {
   extern __shared__ double st_smem[];
   double* qd = st_smem;
-  int* qf = reinterpret_cast<int*>(st_smem + (size_t)QCAP * kRecF * BLOCK);
-  double* stage_col = st_smem + (size_t)QCAP * kRecF * BLOCK + (size_t)(QCAP * BLOCK + 1) / 2 + threadIdx.x;
+  int2* qs = reinterpret_cast<int2*>(st_smem + (size_t)QCAP * kRecF * BLOCK);
+  int* qf = reinterpret_cast<int*>(qs + QCAP * BLOCK);
+  // DOP853 stage derivatives, after the rings
+  char* stages = reinterpret_cast<char*>(qf + (QCAP * BLOCK + 3) / 4 * 4);
+  fx::StageSmem ks{reinterpret_cast<fx::Limb2*>(stages) + threadIdx.x,
+                   reinterpret_cast<fx::Limb*>(stages + 12 * sizeof(fx::Limb2) * BLOCK) + threadIdx.x, BLOCK};
   const int tid = threadIdx.x;
   const unsigned FULL = 0xffffffffu;
   int mode = B_FETCH;
@@ -530,9 +552,12 @@ __global__ void __launch_bounds__(BLOCK, MINB)
           tp.n_steps += 1;
           mode = B_WEND;
         } else if (spin_on<EXT>(P->integrator)) {
-          const double o0[3] = {r[2 * BLOCK], r[3 * BLOCK], r[4 * BLOCK]};
-          const double o1[3] = {r[5 * BLOCK], r[6 * BLOCK], r[7 * BLOCK]};
-          seg_begin(g, *P, r[0], r[1 * BLOCK], o0, o1);
+          SegPoly q;
+          q.fx = (flags & 16) != 0;
+          if (q.fx) q.sc = unpack_scale(qs[slot * BLOCK + tid]);
+          q.o0[0] = r[2 * BLOCK]; q.o0[1] = r[3 * BLOCK]; q.o0[2] = r[4 * BLOCK];
+          q.o1[0] = r[5 * BLOCK]; q.o1[1] = r[6 * BLOCK]; q.o1[2] = r[7 * BLOCK];
+          seg_open(g, *P, q, r[0], r[1 * BLOCK]);
 #if !ST_GRAD_IS_LINEAR
           g.p0x = r[8 * BLOCK]; g.p0y = r[9 * BLOCK]; g.p0z = r[10 * BLOCK];
           g.v0x = r[11 * BLOCK]; g.v0y = r[12 * BLOCK]; g.v0z = r[13 * BLOCK];
@@ -590,7 +615,7 @@ __global__ void __launch_bounds__(BLOCK, MINB)
         if (prod) {
           int slot = qhead + qcount;
           if (slot >= QCAP) slot -= QCAP;
-          produce_record<BLOCK, TAPE, GAS, EXT>(tp, *P, tf, qd, qf, slot, tid, blocked, dd, ta, tc);
+          produce_record<BLOCK, TAPE, GAS, EXT>(tp, *P, tf, qd, qs, qf, slot, tid, blocked, dd, ta, tc);
           ++qcount;
           ++n_seg;
         }
@@ -615,13 +640,10 @@ __global__ void __launch_bounds__(BLOCK, MINB)
     if (mode == B_SEG) {
       int r;
       if (P->integrator == 0) {
-        const double y0x = tp.Sx, y0y = tp.Sy, y0z = tp.Sz, x0 = g.x;
-        if (STAGES) {
-          StageSmem ks{stage_col, BLOCK};
-          r = dop_attempt_ks(g, *P, tp.Sx, tp.Sy, tp.Sz, ks);
-        } else {
-          r = dop_attempt(g, *P, tp.Sx, tp.Sy, tp.Sz);
-        }
+        double y0x = tp.Sx, y0y = tp.Sy, y0z = tp.Sz;
+        if (TAPE && g.fx) dop_spin(g, y0x, y0y, y0z);
+        const double x0 = g.x;
+        r = dop_attempt_v(fx::Lane3(), ks, g, *P, tp.Sx, tp.Sy, tp.Sz);
         ++n_dop;
         if (TAPE && g.acc) tape_step(ta, tc, y0x, y0y, y0z, x0, g.hu);
       } else if (!EXT || P->integrator == 1) {

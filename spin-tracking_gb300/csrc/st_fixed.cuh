@@ -1,0 +1,723 @@
+// DOP853 step arithmetic in 64-bit fixed point on the integer pipes.
+//
+// GB300 issues one FP64 warp instruction per 64 or more cycles on each SM
+// sub-partition (measured: 76 cycles per DFMA, DADD, DMUL or DSETP), while a
+// 32 x 32 + 64 bit multiply-add (IMAD.WIDE) takes 2.1 cycles and a 32-bit add
+// about 1.  A spin step is a few hundred multiply-adds on values whose size is
+// known (the spin's norm is constant, the stage derivatives are h Omega times
+// it), so it runs in block fixed point: three IMAD.WIDE replace one DFMA, and
+// every value keeps 59 or more bits of its block's scale, six more than a
+// double's significand.
+//
+// Numbers are Q63: an int64 m stands for m 2^-63, |m 2^-63| < 1, times a power
+// of two kept beside it (one per block: spin, field, step).  A factor of a
+// product is split into limbs, m 2^-63 = (h 2^27 + l) 2^-58 with 0 <= l < 2^27
+// (|l| <= 2^26 for tableau entries), rounded to 58 fractional bits.  A sum of
+// products accumulates the h h terms (weight 2^-62) and the h l + l h terms
+// (weight 2^-89) in one int64 each; the l l terms (below 2^-62 each, 2^-64 on
+// average) are left out.  Up to 15 terms fit the second accumulator whatever their
+// size, and the first one while the sum of the products' magnitudes stays
+// below 2.
+//
+// The stages run as one rolled loop over tables in constant memory, with the
+// stage derivatives in shared (or local) memory: the hot code has to stay
+// within the ~16 KB of instructions that a sub-partition holds close by.
+// Beyond that, instructions arrive at 8 bytes per cycle and SM, one per 8
+// cycles and sub-partition; the same step fully unrolled (40 KB) spent 78% of its
+// time waiting for them and was slower than FP64.
+//
+// Steps whose rotation angle h |Omega| reaches 1, whose stage values leave the
+// checked range, or whose tolerances do not fit return false: the caller
+// takes them in FP64 (dop_attempt_f64 in st_device.cuh).  Also compiled for the
+// host, for tests.
+#pragma once
+
+#include <math.h>
+#include <stdint.h>
+
+#include "st_tableau.h"
+
+namespace st {
+
+// DOP853 stage structure as constexpr functions of compile-time stage and
+// term indices (they fold to constants inside unrolled loops).
+namespace dopst {
+// earlier stages summed into stage s (2..12): stage 1, then 2 (s = 3),
+// 3.. (s = 4, 5) or 4.. (s >= 6)
+__device__ __forceinline__ constexpr int src(int s, int j) { return j == 0 ? 1 : (s == 3 ? 2 : (s <= 5 ? j + 2 : j + 3)); }
+__device__ __forceinline__ constexpr int cnt(int s) { return s <= 2 ? s - 1 : (s <= 4 ? 2 : (s == 5 ? 3 : s - 3)); }
+// coefficient of term j of stage s (the a_{s,src(s,j)} of the tableau)
+__device__ __forceinline__ constexpr double a(int s, int j) {
+  switch (s * 16 + j) {
+    case 32: return dop::A21;
+    case 48: return dop::A31;
+    case 49: return dop::A32;
+    case 64: return dop::A41;
+    case 65: return dop::A43;
+    case 80: return dop::A51;
+    case 81: return dop::A53;
+    case 82: return dop::A54;
+    case 96: return dop::A61;
+    case 97: return dop::A64;
+    case 98: return dop::A65;
+    case 112: return dop::A71;
+    case 113: return dop::A74;
+    case 114: return dop::A75;
+    case 115: return dop::A76;
+    case 128: return dop::A81;
+    case 129: return dop::A84;
+    case 130: return dop::A85;
+    case 131: return dop::A86;
+    case 132: return dop::A87;
+    case 144: return dop::A91;
+    case 145: return dop::A94;
+    case 146: return dop::A95;
+    case 147: return dop::A96;
+    case 148: return dop::A97;
+    case 149: return dop::A98;
+    case 160: return dop::A101;
+    case 161: return dop::A104;
+    case 162: return dop::A105;
+    case 163: return dop::A106;
+    case 164: return dop::A107;
+    case 165: return dop::A108;
+    case 166: return dop::A109;
+    case 176: return dop::A111;
+    case 177: return dop::A114;
+    case 178: return dop::A115;
+    case 179: return dop::A116;
+    case 180: return dop::A117;
+    case 181: return dop::A118;
+    case 182: return dop::A119;
+    case 183: return dop::A1110;
+    case 192: return dop::A121;
+    case 193: return dop::A124;
+    case 194: return dop::A125;
+    case 195: return dop::A126;
+    case 196: return dop::A127;
+    case 197: return dop::A128;
+    case 198: return dop::A129;
+    case 199: return dop::A1210;
+    case 200: return dop::A1211;
+    default: return 0.0;
+  }
+}
+// node of stage s (stage 12 at x + h)
+__device__ __forceinline__ constexpr double c(int s) {
+  switch (s) {
+    case 2: return dop::C2;
+    case 3: return dop::C3;
+    case 4: return dop::C4;
+    case 5: return dop::C5;
+    case 6: return dop::C6;
+    case 7: return dop::C7;
+    case 8: return dop::C8;
+    case 9: return dop::C9;
+    case 10: return dop::C10;
+    case 11: return dop::C11;
+    case 12: return 1.0;
+    default: return 0.0;
+  }
+}
+// 8th-order weight of stage s
+__device__ __forceinline__ constexpr double b(int s) {
+  switch (s) {
+    case 1: return dop::B1;
+    case 6: return dop::B6;
+    case 7: return dop::B7;
+    case 8: return dop::B8;
+    case 9: return dop::B9;
+    case 10: return dop::B10;
+    case 11: return dop::B11;
+    case 12: return dop::B12;
+    default: return 0.0;
+  }
+}
+}  // namespace dopst
+
+namespace fx {
+
+typedef long long i64;
+typedef unsigned long long u64;
+
+#ifdef __CUDA_ARCH__
+__device__ __forceinline__ int clz64(u64 x) { return __clzll((long long)x); }
+__device__ __forceinline__ float lg2f_approx(float x) {
+  float r;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float ex2f_approx(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float rcpf_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ uint32_t f32_bits(float x) { return __float_as_uint(x); }
+__device__ __forceinline__ float bits_f32(uint32_t b) { return __uint_as_float(b); }
+// a * b + c in one IMAD.WIDE (left to the compiler, factors that it proves
+// non-negative turn into 64 x 64 bit products).
+__device__ __forceinline__ i64 madw(int a, int b, i64 c) {
+  i64 r;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ u64 f64_bits(double x) { return (u64)__double_as_longlong(x); }
+__device__ __forceinline__ double bits_f64(u64 b) { return __longlong_as_double((long long)b); }
+#else
+inline int clz64(u64 x) { return x ? __builtin_clzll(x) : 64; }
+inline float lg2f_approx(float x) { return log2f(x); }
+inline float ex2f_approx(float x) { return exp2f(x); }
+inline float rcpf_approx(float x) { return 1.0f / x; }
+inline i64 madw(int a, int b, i64 c) { return (i64)a * b + c; }
+inline uint32_t f32_bits(float x) {
+  uint32_t b;
+  __builtin_memcpy(&b, &x, 4);
+  return b;
+}
+inline float bits_f32(uint32_t b) {
+  float x;
+  __builtin_memcpy(&x, &b, 4);
+  return x;
+}
+inline u64 f64_bits(double x) {
+  u64 b;
+  __builtin_memcpy(&b, &x, 8);
+  return b;
+}
+inline double bits_f64(u64 b) {
+  double x;
+  __builtin_memcpy(&x, &b, 8);
+  return x;
+}
+#endif
+
+__device__ __forceinline__ i64 shl(i64 a, int k) { return (i64)((u64)a << k); }
+
+// ---------------------------------------------------------------- conversions
+// Biased exponent of x (0: zero or subnormal, 0x7ff: infinite or NaN).
+__device__ __forceinline__ int bexp(double x) { return (int)((f64_bits(x) >> 52) & 0x7ff); }
+
+// x 2^-E as Q63, for |x| < 2^E (and E within the exponents of normal doubles);
+// rounded to nearest, ties away from zero.  Subnormal x give 0.
+__device__ __forceinline__ i64 to_q63(double x, int E) {
+  const u64 b = f64_bits(x);
+  const int e = (int)((b >> 52) & 0x7ff);
+  const u64 m = ((b & 0x000fffffffffffffull) | 0x0010000000000000ull) << 11;  // x = m 2^(e - 1023 - 63)
+  int s = E + 1023 - e;  // x 2^-E 2^63 = m >> s
+  s = s > 63 ? 63 : s;
+  u64 q = (m >> s) + ((m >> (s > 0 ? s - 1 : 0)) & (s > 0 ? 1u : 0u));
+  if (e == 0) q = 0;
+  return (i64)b < 0 ? -(i64)q : (i64)q;
+}
+
+// m 2^(E - 63), rounded to nearest.
+__device__ __forceinline__ double from_q63(i64 m, int E) {
+  const double d = (double)m;  // correctly rounded
+  const u64 b = f64_bits(d);
+  return m == 0 ? 0.0 : bits_f64(b + ((u64)(i64)(E - 63) << 52));
+}
+
+// ---------------------------------------------------------------- products
+struct Limb {
+  int h, l;
+};
+// m to 58 fractional bits, rounded down (callers add 16 units first to round to nearest).
+__device__ __forceinline__ Limb limb(i64 m) { return {(int)(m >> 32), (int)((unsigned)m >> 5)}; }
+__device__ __forceinline__ Limb neg(Limb a) { return {-a.h, -a.l}; }
+
+struct Acc {
+  i64 hh, mid;
+};
+__device__ __forceinline__ void mac(Acc& a, Limb x, Limb y) {
+  a.hh = madw(x.h, y.h, a.hh);
+  a.mid = madw(x.h, y.l, a.mid);
+  a.mid = madw(x.l, y.h, a.mid);
+}
+// Start value of `mid` that makes a following limb split round to nearest.
+constexpr i64 kHalfLimb = 1ll << 30;
+// The sum as Q63 times 2^k.
+__device__ __forceinline__ i64 q63(const Acc& a, int k = 0) { return shl(a.hh, 1 + k) + (a.mid >> (26 - k)); }
+__device__ __forceinline__ i64 mulq(Limb x, Limb y, int k = 0) {
+  Acc a{0, kHalfLimb};
+  mac(a, x, y);
+  return q63(a, k);
+}
+// A tableau entry times 2^-p as limbs (folds to immediates).
+__device__ __forceinline__ constexpr Limb coef(double a, int p) {
+  const double s = a * (double)(1ull << (58 - p));
+  const i64 q = (i64)(s + (s < 0.0 ? -0.5 : 0.5));
+  const i64 h = (q + (1ll << 26)) >> 27;
+  return {(int)h, (int)(q - (i64)((u64)h << 27))};
+}
+// High 64 bits of the product of two 64-bit fractions, at most 3 units low.
+__device__ __forceinline__ u64 umul(u64 a, u64 b) {
+  const uint32_t ah = (uint32_t)(a >> 32), al = (uint32_t)a, bh = (uint32_t)(b >> 32), bl = (uint32_t)b;
+  return (u64)ah * bh + (((u64)ah * bl) >> 32) + (((u64)al * bh) >> 32);
+}
+
+// ---------------------------------------------------------------- lanes
+// All three spin components on one lane.
+struct Lane3 {
+  static constexpr int N = 3;
+  // kappa = y x w for the lane's components (w's limbs and their negatives)
+  __device__ __forceinline__ void cross(const Limb y[3], const Limb w[3], Acc k[3]) const {
+    const Limb n[3] = {neg(w[0]), neg(w[1]), neg(w[2])};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const int a = c == 2 ? 0 : c + 1, b = c == 0 ? 2 : c - 1;
+      k[c] = {0, kHalfLimb};
+      mac(k[c], y[a], w[b]);
+      mac(k[c], y[b], n[a]);
+    }
+  }
+  __device__ __forceinline__ void gather(const i64 v[3], i64 all[3]) const {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) all[c] = v[c];
+  }
+  __device__ __forceinline__ bool any(bool b) const { return b; }
+  __device__ __forceinline__ bool is_z(int c) const { return c == 2; }
+  __device__ __forceinline__ void pick(i64 x, i64 y, i64 z, i64 v[3]) const {
+    v[0] = x;
+    v[1] = y;
+    v[2] = z;
+  }
+};
+
+// Where an attempt keeps its stage derivatives kappa_1..kappa_12: this
+// thread's column of two shared-memory arrays, [12][BLOCK] x (16 + 8) bytes
+// (conflict-free), or a local array.
+struct alignas(16) Limb2 {
+  Limb a, b;
+};
+struct StageSmem {
+  Limb2* xy;  // &array[0][thread]
+  Limb* z;
+  int stride;  // BLOCK
+  __device__ __forceinline__ void load(int s, Limb k[3]) const {
+    const Limb2 v = xy[s * stride];
+    k[0] = v.a;
+    k[1] = v.b;
+    k[2] = z[s * stride];
+  }
+  __device__ __forceinline__ void store(int s, const Limb k[3]) {
+    xy[s * stride] = {k[0], k[1]};
+    z[s * stride] = k[2];
+  }
+};
+template <int N>
+struct StageLocal {
+  Limb v[12][N];
+  __device__ __forceinline__ void load(int s, Limb k[N]) const {
+#pragma unroll
+    for (int c = 0; c < N; ++c) k[c] = v[s][c];
+  }
+  __device__ __forceinline__ void store(int s, const Limb k[N]) {
+#pragma unroll
+    for (int c = 0; c < N; ++c) v[s][c] = k[c];
+  }
+};
+
+// ---------------------------------------------------------------- pulse
+// (pi/2)^2k / (2k)! / 4 with alternating sign as Q63, k = 0..7, and 2^32 times
+// it for k = 8..11.
+__device__ __forceinline__ constexpr i64 cos_coef(int k) {
+  switch (k) {
+    case 0: return 2305843009213693952ll;
+    case 1: return -2844719788994575541ll;
+    case 2: return 584922061444309466ll;
+    case 3: return -48107911266041808ll;
+    case 4: return 2119669878386351ll;
+    case 5: return -58111953223829ll;
+    case 6: return 1086253767602ll;
+    case 7: return -14726504073ll;
+    case 8: return 650261490920323669ll;
+    case 9: return -5243319993991956ll;
+    case 10: return 34045719795410ll;
+    default: return -181827806240ll;
+  }
+}
+
+// cos(2 pi phi) / 2 as Q63, phi in turns as a 64-bit fraction.  phi is brought
+// to a quarter turn either side of 0 (a half turn flips the sign); with
+// y = (4 phi)^2 <= 1 the series sum (-1)^k (pi/2)^2k / (2k)! y^k runs to k = 11
+// (the next term is below 2^-63).  The terms from k = 8 on sum to less than
+// 2^-33 and take one limb product each.  A double's cos costs some 25 FP64
+// instructions (1,900 cycles of the pipe); this takes 33 multiply-adds.
+__device__ __forceinline__ i64 half_cos_turns(u64 phi) {
+  const u64 flip = (phi + 0x4000000000000000ull) >> 63;  // phi in [1/4, 3/4)
+  const Limb z = limb((i64)(phi + (flip << 63)));        // 2 phi, in [-1/2, 1/2)
+  const Limb y = limb(mulq(z, z, 1));                    // y / 2
+  i64 t = cos_coef(11);
+#pragma unroll
+  for (int k = 2; k >= 0; --k) t = cos_coef(8 + k) + shl(madw((int)(t >> 32), y.h, 0), 2);
+  t >>= 32;
+#pragma unroll
+  for (int k = 7; k >= 0; --k) t = cos_coef(k) + mulq(y, limb(t), 1);
+  t = shl(t, 1);
+  return flip ? -t : t;
+}
+
+// frac(t turns_per_s) as a 64-bit fraction for t >= 0; turns_per_s = wm 2^(we - 64), wm normalised.
+__device__ __forceinline__ u64 turns_of(double t, u64 wm, int we) {
+  const u64 b = f64_bits(t);
+  const int e = (int)(b >> 52);
+  if (e == 0) return 0;
+  const u64 m = ((b & 0x000fffffffffffffull) | 0x0010000000000000ull) << 11;  // t = m 2^(e - 1022 - 64)
+#ifdef __CUDA_ARCH__
+  const u64 hi = __umul64hi(m, wm);
+#else
+  const u64 hi = (u64)(((unsigned __int128)m * wm) >> 64);
+#endif
+  const u64 lo = m * wm;
+  const int s = e - 1022 + we;  // the product's integer bits
+  if (s <= 0) return s > -64 ? hi >> -s : 0;
+  return s < 64 ? (hi << s) | (lo >> (64 - s)) : lo << (s < 128 ? s - 64 : 63);
+}
+
+// ---------------------------------------------------------------- segment
+// The field polynomial of a segment in block fixed point: with tau = u 2^te,
+// 0 <= u < 1/2 on the segment, Omega(tau) = 2^oe (o0 + u (o1 + u o2)) plus the
+// pulse's 2^oe ga cos on z, where the norm of the summed magnitudes lies in
+// [1/4, 1/2) (on: that norm).  The spin is 2^se times a vector of norm in
+// (1/8, 1/4], so that a spin of norm 1 sits at the top of its range.
+struct SegScale {
+  int oe, te, se;
+  float on;
+};
+
+// 31-bit magnitude of x 2^-E (|x| < 2^E), for norms.
+__device__ __forceinline__ uint32_t mag31(double x, int E) {
+  const u64 b = f64_bits(x);
+  const int e = (int)((b >> 52) & 0x7ff);
+  const uint32_t m = ((uint32_t)(b >> 32) & 0xfffffu | 0x100000u) << 11;
+  const int s = E + 1023 - e;
+  return e == 0 || s > 31 ? 0u : m >> s;
+}
+__device__ __forceinline__ int imax(int a, int b) { return a > b ? a : b; }
+__device__ __forceinline__ u64 sq32(uint32_t a) { return (u64)a * a; }
+
+// Scale of the spin: false when a component is infinite or NaN, or all are zero.
+__device__ __forceinline__ bool spin_scale(const double S[3], int& se) {
+  const int e = imax(imax(bexp(S[0]), bexp(S[1])), bexp(S[2]));
+  if (e == 0x7ff || e < 64) return false;
+  se = e - 1021;  // the largest component is in [1/4, 1/2), the norm in [1/4, 0.87)
+  const u64 n2 = sq32(mag31(S[0], se)) + sq32(mag31(S[1], se)) + sq32(mag31(S[2], se));  // norm^2 2^62
+  if (n2 > 0x0405400000000000ull) ++se;  // 0.2506^2: a norm within 0.2% of a power of two rounds down to it
+  if (n2 > 0x1015000000000000ull) ++se;  // 0.5012^2
+  return true;
+}
+
+// Scale of the field over a segment of length T: false when a coefficient is
+// infinite or NaN, T is not positive, or an exponent leaves the usual range.
+__device__ __forceinline__ bool field_scale(const double o0[3], const double o1[3], const double o2[3], double ga,
+                                            double T, SegScale& q) {
+  if (!(T > 0.0)) return false;
+  const int t = bexp(T) - 1021;  // T < 2^(te - 1)
+  int e0 = bexp(ga), e1 = 0, e2 = 0;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    e0 = imax(e0, bexp(o0[c]));
+    e1 = imax(e1, bexp(o1[c]));
+    e2 = imax(e2, bexp(o2[c]));
+  }
+  if (e0 == 0x7ff || e1 == 0x7ff || e2 == 0x7ff || t < -900 || t > 900) return false;
+  int e = e0;
+  if (e1) e = imax(e, e1 + t);
+  if (e2) e = imax(e, e2 + 1 + 2 * t);
+  if (e < 64) e = 64;  // no field to speak of: every coefficient rounds to zero
+  if (e > 1900) return false;
+  const int E = e - 1023 + 3;  // each term below 1/4, the sum of a component's below 1
+  u64 n2 = 0;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const u64 m = (u64)mag31(o0[c], E) + mag31(o1[c], E - t) + 2ull * mag31(o2[c], E - 2 * t) +
+                  (c == 2 ? mag31(ga, E) : 0u) + 4u;  // units of 2^-31, rounded up
+    n2 += (m * m) >> 2;
+  }
+  const float n = sqrtf((float)n2) * 0x1p-30f;  // norm of 2^-E Omega, below 1.8
+  const uint32_t nb = f32_bits(n);
+  const int ne = (int)(nb >> 23) - 125;  // n 2^-ne in [1/4, 1/2)
+  q.oe = E + ne;
+  q.te = t;
+  q.on = bits_f32(nb - ((uint32_t)ne << 23)) * 1.00001f;
+  return true;
+}
+
+// ---------------------------------------------------------------- step
+// Tolerances of a set: sk = atol + rtol |S| = rtol (atol / rtol + |S|).
+struct StepTol {
+  double rtol, ratio;  // ratio = atol / rtol
+};
+// Whether a spin of scale se can be stepped with this ratio.  A component near
+// zero is weighted by atol alone, while its error estimate carries the rounding
+// of the whole spin (2^-58 of its norm): up to norm / ratio = 16 the estimate was
+// better than the FP64 step's on every case tried, at 64 it spoiled the growth of
+// tiny steps (14 of 20,000).
+__device__ __forceinline__ bool ratio_fits(double ratio, int se) {
+  const int e = bexp(ratio) - 1023;  // ratio >= 2^e
+  return ratio > 0.0 && e >= se - 6 && e < se + 40;
+}
+
+// Result of an attempt.
+struct StepOut {
+  bool accept;   // err <= 1
+  double root8;  // err^(-1/8); infinite when err = 0
+};
+
+// Powers of two p >= the sums of the magnitudes of a stage's coefficients.
+__device__ __forceinline__ constexpr int stage_p(int s) { return s <= 4 || s == 6 || s == 7 || s == 8 ? -1 : (s == 5 ? 2 : 7); }
+
+// Row s of the stage loop: its terms' first coefficient in kStageCoef, their
+// number, the first source after kappa_1, p, and the halves of its node and of
+// the node's square.
+struct StageRow {
+  int off, n, src, p;
+  Limb c, c2;
+};
+#define ST_ROW(s, off) {off, dopst::cnt(s), (s) == 3 ? 1 : ((s) <= 5 ? 2 : 3), stage_p(s), \
+                        coef(dopst::c(s), 1), coef(dopst::c(s) * dopst::c(s), 1)}
+static __constant__ StageRow kStageRows[12] = {ST_ROW(1, 0),  ST_ROW(2, 0),  ST_ROW(3, 1),  ST_ROW(4, 3),
+                                               ST_ROW(5, 5),  ST_ROW(6, 8),  ST_ROW(7, 11), ST_ROW(8, 15),
+                                               ST_ROW(9, 20), ST_ROW(10, 26), ST_ROW(11, 33), ST_ROW(12, 41)};
+#undef ST_ROW
+#define ST_A(s, j) coef(dopst::a(s, j), stage_p(s))
+static __constant__ Limb kStageCoef[50] = {
+    ST_A(2, 0),  ST_A(3, 0),  ST_A(3, 1),  ST_A(4, 0),  ST_A(4, 1),  ST_A(5, 0),  ST_A(5, 1),  ST_A(5, 2),
+    ST_A(6, 0),  ST_A(6, 1),  ST_A(6, 2),  ST_A(7, 0),  ST_A(7, 1),  ST_A(7, 2),  ST_A(7, 3),  ST_A(8, 0),
+    ST_A(8, 1),  ST_A(8, 2),  ST_A(8, 3),  ST_A(8, 4),  ST_A(9, 0),  ST_A(9, 1),  ST_A(9, 2),  ST_A(9, 3),
+    ST_A(9, 4),  ST_A(9, 5),  ST_A(10, 0), ST_A(10, 1), ST_A(10, 2), ST_A(10, 3), ST_A(10, 4), ST_A(10, 5),
+    ST_A(10, 6), ST_A(11, 0), ST_A(11, 1), ST_A(11, 2), ST_A(11, 3), ST_A(11, 4), ST_A(11, 5), ST_A(11, 6),
+    ST_A(11, 7), ST_A(12, 0), ST_A(12, 1), ST_A(12, 2), ST_A(12, 3), ST_A(12, 4), ST_A(12, 5), ST_A(12, 6),
+    ST_A(12, 7), ST_A(12, 8)};
+#undef ST_A
+// The 8th-order weights b / 16, the third-order error row (b - bhh) / 16 and the
+// fifth-order one er / 8 of kappa_1, kappa_6..kappa_12.
+static __constant__ Limb kSumCoef[8][3] = {
+    {coef(dop::B1, 4), coef(dop::B1 - dop::BHH1, 4), coef(dop::ER1, 3)},
+    {coef(dop::B6, 4), coef(dop::B6, 4), coef(dop::ER6, 3)},
+    {coef(dop::B7, 4), coef(dop::B7, 4), coef(dop::ER7, 3)},
+    {coef(dop::B8, 4), coef(dop::B8, 4), coef(dop::ER8, 3)},
+    {coef(dop::B9, 4), coef(dop::B9 - dop::BHH2, 4), coef(dop::ER9, 3)},
+    {coef(dop::B10, 4), coef(dop::B10, 4), coef(dop::ER10, 3)},
+    {coef(dop::B11, 4), coef(dop::B11, 4), coef(dop::ER11, 3)},
+    {coef(dop::B12, 4), coef(dop::B12 - dop::BHH3, 4), coef(dop::ER12, 3)}};
+
+// y^(1/16) of y = b / (a 2^k) for a, b in (0, 1) as 64-bit fractions with a >= b
+// and k >= 0, in two factors 2^-j r / 2: Newton's iteration for r^16 a 2^i = b
+// (k = 16 j + i), the powers of two of i fed in between the squarings so that
+// every intermediate stays in [1/4, 1].  From a seed good to 2^-20 two steps
+// reach 2^-60.  Returns r / 2 as a 64-bit fraction.
+__device__ __forceinline__ u64 root16(u64 a, u64 b, int i) {
+  const float af = (float)(uint32_t)(a >> 32), bf = (float)(uint32_t)(b >> 32);
+  const float lg = lg2f_approx(bf) - lg2f_approx(af) - (float)i;
+  u64 r = (u64)(ex2f_approx(0.0625f * lg) * 0x1.fffff8p62f);
+  const float ib = rcpf_approx(bf) * 0x1p-35f;  // 2 / (16 b), b in units of 2^-64
+#pragma unroll
+  for (int it = 0; it < 2; ++it) {
+    u64 v = umul(r, r) << 1 << ((i >> 3) & 1);  // half of r^2 2^b3
+    v = umul(v, v) << 1 << ((i >> 2) & 1);
+    v = umul(v, v) << 1 << ((i >> 1) & 1);
+    v = umul(v, v) << 1 << (i & 1);
+    const i64 d = (i64)((b >> 1) - umul(v, a));  // (b - r^16 2^i a) / 2
+    const float f = (float)d * ib * (float)(uint32_t)(r >> 32);  // the correction of r / 2 in units of 2^-32
+    r += (u64)(i64)(f * 0x1p32f);
+  }
+  return r;
+}
+
+// One attempted DOP853 step of size h at tau = tx (t = x) over a scaled
+// segment: new spin in S (on any outcome the caller decides whether to keep
+// it: Sn), the error's verdict in out.  False: outside the fixed-point range.
+template <class V, class KS>
+__device__ __forceinline__ bool dop_step(const V& view, KS& ks, const SegScale& q, const i64* o0, const i64* o1, const i64* o2,
+                                         i64 ga, u64 wm, int we, double x, double tx, double h, const StepTol& tol,
+                                         const i64* S, i64* Sn, StepOut& out) {
+  using namespace dop;
+  constexpr int N = V::N;
+  // ---- the step in segment units
+  if (!(h > 0.0) || !(tx >= 0.0)) return false;
+  const int eh = bexp(h) - 1021;  // h = hm 2^eh, hm in [1/4, 1/2)
+  if (bexp(tx) - 1022 >= q.te || eh - 1 > q.te || bexp(h) < 64) return false;
+  const i64 u = to_q63(tx, q.te);
+  const i64 hm = to_q63(h, eh);
+  const int sh = q.te - eh + 1;  // eta = h 2^-te = 2 hm 2^-sh
+  if ((u64)u + ((u64)hm << 1 >> (sh > 63 ? 63 : sh)) > 0x4010000000000000ull) return false;  // past the segment's end
+  // ---- h Omega = 2^ez omega, |omega| in [1/4, 1/2)
+  const bool small = (float)(uint32_t)(hm >> 32) * q.on < 0x1.ff8p-4f * 0x1p31f;
+  const i64 hs = small ? hm << 1 : hm;
+  const int ez = eh + q.oe - 1 - (small ? 1 : 0);
+  if (ez > 1) return false;  // the step turns the spin by up to 1 rad or more
+  const int r = 1 - ez > 63 ? 63 : 1 - ez;
+  const Limb hsl = limb(hs), hml = limb(hm), ul = limb(u);
+  const int s63 = sh > 63 ? 63 : sh;
+  const i64 g1 = mulq(hsl, hml, 1) >> s63;  // hs eta
+  const Limb g1l = limb(g1);
+  const i64 g2 = mulq(g1l, hml, 1) >> s63;  // hs eta^2
+  const Limb g2l = limb(g2);
+  i64 w0[N];
+  Limb w1[N], w2[N];
+#pragma unroll
+  for (int c = 0; c < N; ++c) {
+    const Limb o2l = limb(o2[c]);
+    const i64 t1 = mulq(ul, o2l);
+    w0[c] = mulq(hsl, limb(o0[c] + mulq(ul, limb(o1[c] + t1))), 1);
+    w1[c] = limb(mulq(g1l, limb(o1[c] + shl(t1, 1)), 1));
+    w2[c] = limb(mulq(g2l, o2l, 1));
+  }
+  const bool pulse = ga != 0;
+  Limb hgl{0, 0}, dphi{0, 0};
+  u64 phi0 = 0;
+  if (pulse) {
+    hgl = limb(mulq(hsl, limb(ga), 1));
+    const u64 dp = turns_of(h, wm, we);
+    if (dp >= 0x4000000000000000ull || bexp(h) - 1022 + we > 0) return false;  // a quarter turn or more
+    dphi = limb((i64)dp);
+    const u64 p = turns_of(fabs(x), wm, we);
+    phi0 = x < 0.0 ? 0ull - p : p;
+  }
+  // ---- stages: kappa_s = Y_s x omega_s, Y_s = S + 2^ez sum a_sj kappa_j
+  unsigned bad = 0;  // set where a sum leaves the range in which nothing overflows
+#pragma unroll 1
+  for (int s = 0; s < 12; ++s) {
+    const StageRow& row = kStageRows[s];
+    Acc a[N];
+#pragma unroll
+    for (int c = 0; c < N; ++c) a[c] = {0, 0};
+    Limb k[N];
+    ks.load(0, k);
+    int src = row.src;
+#pragma unroll 1
+    for (int j = 0; j < row.n; ++j) {
+      const Limb f = kStageCoef[row.off + j];
+      Limb next[N];
+      ks.load(src, next);  // one ahead (the last one unused, within the array)
+      ++src;
+#pragma unroll
+      for (int c = 0; c < N; ++c) {
+        mac(a[c], f, k[c]);
+        k[c] = next[c];
+      }
+    }
+    Limb Y[N], W[N];
+#pragma unroll
+    for (int c = 0; c < N; ++c) {
+      const int p = row.p;
+      // |2 sum a kappa| < 1/2: neither the shift below nor Y can overflow
+      bad |= ((unsigned)(int)(a[c].hh >> 32) + (1u << (28 - p))) & ~((1u << (29 - p)) - 1u);
+      Y[c] = limb(S[c] + (q63(a[c], 1 + p) >> r) + 16);
+      Acc o{0, 0};
+      mac(o, row.c, w1[c]);
+      mac(o, row.c2, w2[c]);
+      i64 w = w0[c] + q63(o, 1);
+      if (pulse && view.is_z(c))
+        w += mulq(hgl, limb(half_cos_turns(phi0 + (u64)mulq(row.c, dphi, 1)) + 16), 1);
+      W[c] = limb(w + 16);
+    }
+    view.cross(Y, W, a);
+#pragma unroll
+    for (int c = 0; c < N; ++c) k[c] = limb(q63(a[c]));
+    ks.store(s, k);
+  }
+  // ---- 8th-order sum, new spin, the two error rows
+  Acc sb[N], s3[N], s5[N];
+#pragma unroll
+  for (int c = 0; c < N; ++c) sb[c] = s3[c] = s5[c] = {0, 0};
+  {
+    Limb k[N];
+    ks.load(0, k);
+#pragma unroll 1
+    for (int j = 0; j < 8; ++j) {
+      const Limb fb = kSumCoef[j][0], f3 = kSumCoef[j][1], f5 = kSumCoef[j][2];
+      Limb next[N];
+      ks.load(j < 7 ? 5 + j : 11, next);
+#pragma unroll
+      for (int c = 0; c < N; ++c) {
+        mac(sb[c], fb, k[c]);
+        mac(s3[c], f3, k[c]);
+        mac(s5[c], f5, k[c]);
+        k[c] = next[c];
+      }
+    }
+  }
+  i64 e3[N], e5[N], big[N];
+  const i64 half = (i64)((1ull << r) >> 1);
+#pragma unroll
+  for (int c = 0; c < N; ++c) {
+    bad |= ((unsigned)(int)(sb[c].hh >> 32) + (1u << 24)) & ~((1u << 25) - 1u);
+    Sn[c] = S[c] + ((q63(sb[c], 5) + half) >> r);
+    e3[c] = q63(s3[c]);  // 2^-4 of the row
+    e5[c] = q63(s5[c]);  // 2^-3 of the row
+    const i64 m0 = S[c] < 0 ? -S[c] : S[c], m1 = Sn[c] < 0 ? -Sn[c] : Sn[c];
+    big[c] = m0 > m1 ? m0 : m1;
+  }
+  if (view.any(bad != 0)) return false;
+  // ---- err^2 = 2^2(ez - sa) N5^2 / (3 rtol^2 D^2 (N5 + N3 / 100)) with
+  // G_c = |S_c| + atol / rtol in units of 2^(se + sa), D = Gx Gy Gz and
+  // N = sum (e_c D / G_c)^2: the weighted norms over their common denominator.
+  i64 E5[3], E3[3], Mx[3];
+  view.gather(e5, E5);
+  view.gather(e3, E3);
+  view.gather(big, Mx);
+  if (((u64)(Mx[0] | Mx[1] | Mx[2]) >> 62) != 0) return false;  // a spin twice its norm: a step far too long
+  const int be = bexp(tol.ratio);
+  int sa = be ? be - 1022 - q.se + 1 : 0;  // atol / rtol < 2^(se + sa - 1)
+  sa = sa < 0 ? 0 : sa;
+  const i64 ar = to_q63(tol.ratio, q.se + sa);
+  u64 Gx = (u64)((Mx[0] >> sa) + ar) << 1, Gy = (u64)((Mx[1] >> sa) + ar) << 1, Gz = (u64)((Mx[2] >> sa) + ar) << 1;
+  const u64 Px = umul(Gy, Gz), Py = umul(Gx, Gz), Pz = umul(Gx, Gy);
+  u64 D = umul(Pz, Gz);
+  u64 m5[3], m3[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    m5[c] = (u64)(E5[c] < 0 ? -E5[c] : E5[c]);
+    m3[c] = (u64)(E3[c] < 0 ? -E3[c] : E3[c]);
+  }
+  u64 all5 = m5[0] | m5[1] | m5[2];
+  const u64 all3 = m3[0] | m3[1] | m3[2];
+  out.accept = true;
+  out.root8 = bits_f64(0x7ff0000000000000ull);
+  if (all5 == 0) return true;
+  const int l5 = clz64(all5), l3 = all3 ? clz64(all3) : 63;
+  auto sumsq = [&](const u64* m, int l) {
+    const u64 a = umul(m[0] << l, Px), b = umul(m[1] << l, Py), c = umul(m[2] << l, Pz);
+    return (umul(a, a) >> 1) + (umul(b, b) >> 1) + (umul(c, c) >> 1);  // halved against overflow
+  };
+  u64 n5 = sumsq(m5, l5);
+  const u64 n3 = umul(sumsq(m3, l3), 184467440737095516ull);  // N3 / 100
+  const int d2 = 2 * ((l5 - 3) - (l3 - 4));  // N3's block is 2^d2 of N5's
+  u64 t;
+  int et;  // N5 + N3 / 100 = t 2^(et - 64) in units of N5's block
+  if (d2 >= 0) {
+    t = n3 + (d2 > 63 ? 0 : n5 >> d2);
+    et = d2;
+  } else {
+    t = n5 + (d2 < -63 ? 0 : n3 >> -d2);
+    et = 0;
+  }
+  if (n5 == 0 || t == 0 || D == 0) return false;
+  const int z5 = clz64(n5), zt = clz64(t), zd = clz64(D);
+  n5 <<= z5;
+  t <<= zt;
+  const u64 rb = f64_bits(tol.rtol);
+  const u64 rt = ((rb & 0x000fffffffffffffull) | 0x0010000000000000ull) << 11;  // rtol = rt 2^(bexp - 1022 - 64)
+  const u64 dr = umul(D << zd, rt);
+  const u64 A = umul(n5, n5);                                             // in [1/4, 1)
+  const u64 B = umul(umul(dr, dr), t);                                    // times 3 / 16: in [2^-8, 1/4)
+  const u64 b = (B >> 3) + (B >> 4);
+  // (9 - 2 l5: the sum's halving, 2^3 of the row, Q63 against a 64-bit fraction, the normalising shift)
+  const int k = 2 * (ez - sa) - 2 * z5 - (et - zt) + 2 * zd - 2 * (bexp(tol.rtol) - 1022) + 9 - 2 * l5 - 4;
+  // X = err^2 = 2^k A / b, A >= b
+  out.accept = k <= 0 && (k < -10 || (A >> -k) <= b);
+  const int i = k & 15, j = k >> 4;  // k = 16 j + i
+  const u64 rr = root16(A, b, i);
+  out.root8 = from_q63((i64)(rr >> 1), 1 - j);
+  return true;
+}
+
+}  // namespace fx
+}  // namespace st

@@ -36,6 +36,9 @@ struct SetParams {
   // ---- stepper (src/integrator.cpp:90-337)
   double rtol, atol, hmin, hmax, h0, safe, fac1, fac2, beta;
   double facc1, facc2, expo1, inv_safe;
+  double tol_ratio;               // atol / rtol, filled by launch_prepare_sets (-1: FP64 steps only)
+  uint64_t wturn_m;               // |w| / (2 pi) = wturn_m 2^(wturn_e - 64), likewise
+  int wturn_e;
   // ---- windows (src/simulation.cpp:43-49)
   double t0, tf, ioutInt;
   double yi_x, yi_y, yi_z;

@@ -236,10 +236,10 @@ static const void* variant_fn_g(int v) {
     case 4: return reinterpret_cast<const void*>(&k_persistent<256, 1, false>);
     case 5:
     case 6:
-    case 19: return reinterpret_cast<const void*>(&k_batched<128, 1, 6, false, GAS, 0, false>);
-    case 7: return reinterpret_cast<const void*>(&k_batched<128, 2, 4, false, GAS, 0, false>);
-    case 12: return reinterpret_cast<const void*>(&k_batched<64, 2, 8, false, GAS, 1, false>);
-    case 13: return reinterpret_cast<const void*>(&k_batched<64, 5, 6, false, GAS, 1, false>);
+    case 19: return reinterpret_cast<const void*>(&k_batched<128, 1, 6, false, GAS, false>);
+    case 7: return reinterpret_cast<const void*>(&k_batched<128, 2, 4, false, GAS, false>);
+    case 12: return reinterpret_cast<const void*>(&k_batched<64, 2, 8, false, GAS, false>);
+    case 13: return reinterpret_cast<const void*>(&k_batched<64, 5, 6, false, GAS, false>);
     case 14: return reinterpret_cast<const void*>(&k_split<3, 1, 2, 8, GAS, 0, 0>);
     case 15: return reinterpret_cast<const void*>(&k_split<6, 2, 1, 8, GAS, 0, 0>);
 #if ST_TRAJ_CORRECTLY_ROUNDED
@@ -257,8 +257,8 @@ static const void* variant_fn_g(int v) {
     case 21:
     case 22:
     case 23:
-    case 24: return reinterpret_cast<const void*>(&k_batched<64, 2, 12, false, GAS, 0, false>);
-    default: return reinterpret_cast<const void*>(&k_batched<64, 2, 8, false, GAS, 0, false>);  // 8 to 11, 20
+    case 24: return reinterpret_cast<const void*>(&k_batched<64, 2, 12, false, GAS, false>);
+    default: return reinterpret_cast<const void*>(&k_batched<64, 2, 8, false, GAS, false>);  // 8 to 11, 20
   }
 }
 // The kernel of variant v: with gas collisions or without, and with
@@ -270,11 +270,11 @@ static const void* variant_fn(int v, bool gas, int kind) {
   return gas ? variant_fn_g<true>(v) : variant_fn_g<false>(v);
 }
 
-// Rings (records and flags), then the stage derivatives when they live in
-// shared memory (10 stages x 3 components x block).
-static size_t batched_smem(int block, int qcap, int stages) {
-  const size_t ring = (size_t)qcap * block * kRecF * sizeof(double) + (size_t)(qcap * block + 1) / 2 * sizeof(double);
-  return ring + (stages ? (size_t)30 * block * sizeof(double) : 0);
+// Rings (records, scales and flags), then the DOP853 stage derivatives (12
+// stages x 3 components x block).
+static size_t batched_smem(int block, int qcap) {
+  const size_t ring = (size_t)qcap * block * (kRecF * sizeof(double) + sizeof(int2)) + (size_t)(qcap * block + 3) / 4 * 16;
+  return ring + (size_t)12 * block * (sizeof(fx::Limb2) + sizeof(fx::Limb));
 }
 
 static int split_consumer_warps(int v) { return kVariants[v].cw; }
@@ -297,7 +297,7 @@ static size_t variant_smem(int v) {
   const Variant& x = kVariants[v];
   if (x.family == 0 || x.family == 3) return 0;
   if (x.family == 2) return split_smem_bytes(split_consumer_warps(v), x.qcap);
-  return batched_smem(x.block, x.qcap, x.stages);
+  return batched_smem(x.block, x.qcap);
 }
 
 // Function attributes are set per device: remember which devices have them
@@ -369,10 +369,10 @@ int launch_persistent(const RunArgs& a, int v, int blocks, int block, void* stre
 // 16 lanes); the EXT instantiation (st_kernels_ext.cu) records Magnus steps.
 static const void* tape_fn(bool gas, bool ext) {
   if (ext) return tape_fn_ext();
-  return gas ? reinterpret_cast<const void*>(&k_batched<kTapeBlock, 1, kTapeQcap, true, true, 0, false>)
-             : reinterpret_cast<const void*>(&k_batched<kTapeBlock, 1, kTapeQcap, true, false, 0, false>);
+  return gas ? reinterpret_cast<const void*>(&k_batched<kTapeBlock, 1, kTapeQcap, true, true, false>)
+             : reinterpret_cast<const void*>(&k_batched<kTapeBlock, 1, kTapeQcap, true, false, false>);
 }
-static size_t tape_smem() { return batched_smem(kTapeBlock, kTapeQcap, 0); }
+static size_t tape_smem() { return batched_smem(kTapeBlock, kTapeQcap); }
 
 static cudaError_t tape_ensure_smem(bool gas, bool ext) {
   static bool done[kAttrDevices][3] = {};

@@ -18,20 +18,20 @@ const void* variant_fn_ext(int v) {
     case 4: return reinterpret_cast<const void*>(&k_persistent<256, 1, true>);
     case 5:
     case 6:
-    case 19: return reinterpret_cast<const void*>(&k_batched<128, 1, 6, false, true, 0, true>);
-    case 7: return reinterpret_cast<const void*>(&k_batched<128, 2, 4, false, true, 0, true>);
-    case 12: return reinterpret_cast<const void*>(&k_batched<64, 2, 8, false, true, 1, true>);
-    case 13: return reinterpret_cast<const void*>(&k_batched<64, 5, 6, false, true, 1, true>);
+    case 19: return reinterpret_cast<const void*>(&k_batched<128, 1, 6, false, true, true>);
+    case 7: return reinterpret_cast<const void*>(&k_batched<128, 2, 4, false, true, true>);
+    case 12: return reinterpret_cast<const void*>(&k_batched<64, 2, 8, false, true, true>);
+    case 13: return reinterpret_cast<const void*>(&k_batched<64, 5, 6, false, true, true>);
     case 21:
     case 22:
     case 23:
-    case 24: return reinterpret_cast<const void*>(&k_batched<64, 2, 12, false, true, 0, true>);
-    default: return reinterpret_cast<const void*>(&k_batched<64, 2, 8, false, true, 0, true>);  // 8 to 11, 20
+    case 24: return reinterpret_cast<const void*>(&k_batched<64, 2, 12, false, true, true>);
+    default: return reinterpret_cast<const void*>(&k_batched<64, 2, 8, false, true, true>);  // 8 to 11, 20
   }
 }
 
 const void* tape_fn_ext() {
-  return reinterpret_cast<const void*>(&k_batched<kTapeBlock, 1, kTapeQcap, true, true, 0, true>);
+  return reinterpret_cast<const void*>(&k_batched<kTapeBlock, 1, kTapeQcap, true, true, true>);
 }
 
 template <int B>

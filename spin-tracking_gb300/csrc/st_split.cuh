@@ -299,7 +299,13 @@ __global__ void __launch_bounds__((CW + PW) * 32, MINB) k_split(RunArgs a) {
           tp.n_steps += 1;
           mode = B_WEND;
         } else if (spin_on<false>(P->integrator)) {
-          seg_begin(g, *P, r0, r1, o0, o1);
+          SegPoly q;
+          for (int c = 0; c < 3; ++c) {
+            q.o0[c] = o0[c];
+            q.o1[c] = o1[c];
+          }
+          seg_scale(q, *P, r1 - r0);
+          seg_open(g, *P, q, r0, r1);
 #if !ST_GRAD_IS_LINEAR
           g.p0x = pv[0]; g.p0y = pv[1]; g.p0z = pv[2];
           g.v0x = pv[3]; g.v0y = pv[4]; g.v0z = pv[5];
