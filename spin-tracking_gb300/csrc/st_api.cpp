@@ -104,6 +104,8 @@ int build_params(const st_options& o, int64_t first, SetParams* P) {
   if (!(o.ioutInt > 0.0)) return fail(ST_ERR_ARG, "ioutInt must be > 0");
   std::memset(P, 0, sizeof(*P));
   P->Lx = o.L.x; P->Ly = o.L.y; P->Lz = o.L.z;
+  P->hLx = P->Lx / 2.0; P->hLy = P->Ly / 2.0; P->hLz = P->Lz / 2.0;
+  P->limx = P->hLx + 1.0e-15; P->limy = P->hLy + 1.0e-15; P->limz = P->hLz + 1.0e-15;
   P->maxPosStep = o.maxPosStep;
   P->tc = o.tc;
   P->sqrtKT_m = o.sqrtKT_m;
@@ -180,6 +182,8 @@ struct st_ctx {
     int launches;
   };
   std::vector<RunGraph> graphs;
+  char* ahead = nullptr;     // trajectory-ahead kernel: scratch of its launched lanes (ensure_ahead)
+  size_t ahead_bytes = 0;
   void* ens_buf = nullptr;   // ensemble statistics: control slots, block partials, histogram
   // integratorType 6 (every set of the context): the noise-spectrum aggregators
   bool spectrum = false;
@@ -373,6 +377,8 @@ st::RunArgs make_args(st_ctx* c, int w_begin, int w_end, void* snap) {
   a.any_gas = 0;
   a.any_ext = ctx_any_ext(c) ? 1 : 0;
   a.any_rk45 = ctx_any_rk45(c) ? 1 : 0;
+  a.ahead = c->ahead;
+  a.ahead_q = 0;
   for (const auto& P : c->sets_h) a.any_gas |= P.gas ? 1 : 0;
   return a;
 }
@@ -418,12 +424,51 @@ int arm_deadline(st_ctx* c, st::RunArgs& a) {
 // fastest.
 int autotune(st_ctx* c);
 
+// Blocks of a persistent launch: the resident ones, no more than the work items fill.
+int persistent_blocks(const st_ctx* c, int variant, int per_sm) {
+  const int64_t block = std::max(1, st::persistent_variant_block(variant));
+  const int64_t lanes_per_item = st::persistent_variant_family(variant) == 3 ? 4 : 1;  // three of every 3.2 lanes
+  const int64_t need = (c->n * lanes_per_item + block - 1) / block;
+  return (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)c->sm_count * per_sm, need));
+}
+
+// Scratch of the trajectory-ahead kernel (its lanes' rings), kept with the context.  A larger one takes the place of the old: run graphs that hold its
+// address go too.
+int ensure_ahead(st_ctx* c, size_t need) {
+  if (need <= c->ahead_bytes) return ST_OK;
+  ST_CUDA(cudaStreamSynchronize(c->stream));
+  for (auto& g : c->graphs) cudaGraphExecDestroy(g.exec);
+  c->graphs.clear();
+  cudaFree(c->ahead);
+  c->ahead = nullptr;
+  c->ahead_bytes = 0;
+  cudaError_t e = cudaMalloc(&c->ahead, need);
+  if (e != cudaSuccess) return fail(ST_ERR_NOMEM, std::string("trajectory rings: ") + cudaGetErrorString(e));
+  c->ahead_bytes = need;
+  return ST_OK;
+}
+// The same for the context's launch configuration, at once large enough for every variant
+// at its highest occupancy, so that a change of configuration keeps the graphs.
+int ensure_ahead_variant(st_ctx* c) {
+  auto bytes = [&](int v, int per_sm) {
+    return st::ahead_scratch_bytes(st::persistent_variant_ring(v),
+                                   (int64_t)persistent_blocks(c, v, per_sm) * st::persistent_variant_block(v));
+  };
+  size_t need = bytes(c->lc.variant, c->lc.blocks_per_sm);
+  if (need <= c->ahead_bytes) return ST_OK;
+  for (int v = 0; v < st::persistent_variant_count(); ++v)
+    if (st::persistent_variant_ring(v) > 0)
+      need = std::max(need, bytes(v, st::persistent_max_blocks_per_sm(v, ctx_kind(c))));
+  return ensure_ahead(c, need);
+}
+
 int run_persistent(st_ctx* c, int w_begin, int w_end, void* snap) {
   ST_TRY(ctx_build_order(c));
   if (c->lc.variant < 0 || c->lc.blocks_per_sm <= 0) ST_TRY(autotune(c));
+  ST_TRY(ensure_ahead_variant(c));
   st::RunArgs a = make_args(c, w_begin, w_end, snap);
   ST_TRY(arm_deadline(c, a));
-  const int blocks = c->sm_count * c->lc.blocks_per_sm;
+  const int blocks = persistent_blocks(c, c->lc.variant, c->lc.blocks_per_sm);
   int e = st::launch_persistent(a, c->lc.variant, blocks, c->lc.block_threads, c->stream);
   if (e) return fail(ST_ERR_CUDA, std::string("persistent launch: ") + cudaGetErrorString((cudaError_t)e));
   return ST_OK;
@@ -659,6 +704,7 @@ void st_destroy(st_ctx* c) {
   cudaFree(c->status_d);
   cudaFree(c->order_d);
   for (auto& g : c->graphs) cudaGraphExecDestroy(g.exec);
+  cudaFree(c->ahead);
   cudaFree(c->ens_buf);
   cudaFree(c->spec_sets_d);
   cudaFree(c->spec_pp);
@@ -746,6 +792,7 @@ int st_run_windows(st_ctx* c, int kernel, int w_begin, int w_end, void* snap) {
     if (c->lc.variant < 0 || c->lc.blocks_per_sm <= 0) ST_TRY(autotune(c));
     if (int e = st::persistent_prepare(c->lc.variant))
       return fail(ST_ERR_CUDA, std::string("kernel attributes: ") + cudaGetErrorString((cudaError_t)e));
+    ST_TRY(ensure_ahead_variant(c));
   }
   c->fresh = false;
   c->adj_recorded = false;
@@ -1028,7 +1075,12 @@ int adj_reset_replay_tape(st_ctx* c) { return adj_reset_tape(c, c->tape); }
 
 int adj_tape_launch(st_ctx* c, const st::RunArgs& a, const st::TapeArgs& t) {
   const int per_sm = std::max(1, st::tape_record_max_blocks_per_sm(ctx_any_ext(c) ? 1 : 0));
-  int e = st::launch_tape_record(a, t, c->sm_count * per_sm, c->stream);
+  const int64_t block = st::tape_record_block();
+  const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)c->sm_count * per_sm, (a.nitems + block - 1) / block));
+  ST_TRY(ensure_ahead(c, st::ahead_scratch_bytes(st::tape_record_ring(), blocks * block)));
+  st::RunArgs r = a;
+  r.ahead = c->ahead;
+  int e = st::launch_tape_record(r, t, blocks, c->stream);
   if (e) return fail(ST_ERR_CUDA, std::string("adjoint tape launch: ") + cudaGetErrorString((cudaError_t)e));
   return ST_OK;
 }

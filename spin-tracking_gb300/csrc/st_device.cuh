@@ -4,8 +4,9 @@
 //
 // Two arithmetic regimes:
 //  * Trajectory and RNG code reproduces the reference's doubles bit for bit
-//    (same operation order, no FMA contraction: every add/mul/div/sqrt is an
-//    explicit round-to-nearest intrinsic), so event times, bounce/collision
+//    (same operation order, no FMA contraction: every add and mul is an
+//    explicit round-to-nearest intrinsic, every division and square root the
+//    correctly rounded one of st_softfp.cuh), so event times, bounce/collision
 //    counts and RNG draws match the CPU build exactly.  Its log, acos, cos and
 //    sin are the correctly rounded ones of st_crmath.cuh (equal to the host C
 //    library's wherever those are correctly rounded), or CUDA's with
@@ -24,6 +25,7 @@
 #include "st_tableau.h"
 #include "st_crmath.cuh"
 #include "st_fixed.cuh"
+#include "st_softfp.cuh"
 
 namespace st {
 // The trajectory's transcendental functions (ST_TRAJ_CORRECTLY_ROUNDED, st_fields.cuh).
@@ -134,18 +136,18 @@ __device__ __forceinline__ uint64_t rng_next(Rng& r) {
   return out;
 }
 // top 53 bits scaled by 2^-53 (exact), src/particle.cpp:72-83
-__device__ __forceinline__ double rng_uniform(Rng& r) { return xmul((double)(rng_next(r) >> 11), 0x1.0p-53); }
+__device__ __forceinline__ double rng_uniform(Rng& r) { return sfp::unit_53(rng_next(r)); }
 
 // The uniform pairs of the Marsaglia polar method until 0 < s = u^2 + v^2 < 1,
 // and the factor sqrt(-2 log s / s) from log s.
 __device__ __forceinline__ void marsaglia_draw(Rng& r, double& u, double& v, double& s) {
   do {
-    u = xadd(xmul(rng_uniform(r), 2.0), -1.0);
-    v = xadd(xmul(rng_uniform(r), 2.0), -1.0);
+    u = sfp::signed_unit_53(rng_next(r));
+    v = sfp::signed_unit_53(rng_next(r));
     s = xadd(xmul(u, u), xmul(v, v));
-  } while (s >= 1.0 || s == 0.0);
+  } while (sfp::f64_bits(s) >= 0x3ff0000000000000ull || s == 0.0);  // s >= 1 or s = 0
 }
-__device__ __forceinline__ double marsaglia_factor(double s, double log_s) { return xsqrt(xdiv(xmul(-2.0, log_s), s)); }
+__device__ __forceinline__ double marsaglia_factor(double s, double log_s) { return sfp::sqrt_rn(sfp::div_rn(xmul(-2.0, log_s), s)); }
 
 // Marsaglia polar normal with cached spare (src/particle.cpp:89-107).
 __device__ __forceinline__ double rng_normal(Rng& r, double mean, double sd) {
@@ -159,6 +161,15 @@ __device__ __forceinline__ double rng_normal(Rng& r, double mean, double sd) {
   r.spare = xmul(v, f);
   r.has = true;
   return xadd(mean, xmul(xmul(sd, u), f));
+}
+// Three standard normals, in a rolled loop (one copy of the draw's code).
+__device__ __forceinline__ void rng_normals(Rng& r, double& n0, double& n1, double& n2) {
+#pragma unroll 1
+  for (int k = 0; k < 3; ++k) {
+    n0 = n1;
+    n1 = n2;
+    n2 = rng_normal(r, 0.0, 1.0);
+  }
 }
 __device__ __forceinline__ double rng_exponential(Rng& r, double tc) {
   return xmul(-tc, traj_log(xsub(1.0, rng_uniform(r))));
@@ -282,8 +293,8 @@ struct SegStart {
 
 // A trajectory event whose draws were taken but whose logarithms, sines and
 // cosines are not yet computed (traj_event<true>): a cosine-law diffuse
-// reflection, or a gas collision with a Maxwell-Boltzmann velocity redraw.
-//   reflection: x[0] = sqrt(u1), x[1] = theta = 2 pi u2, x[2] = |v| at the wall
+// reflection, or a gas collision.
+//   reflection: x[0] = u1, x[1] = u2 (their sqrt and 2 pi, and |v|, are taken later too)
 //   gas:        x[0] = 1 - u of the gas clock's exponential draw, then the
 //               Marsaglia pairs drawn for the three velocity normals, (u, v, s)
 //               in x[1..3] and x[4..6]: one pair when the first normal is the
@@ -313,8 +324,15 @@ __device__ __forceinline__ void diffuse_apply(PState& p, double sp, double cp, d
   }
 }
 
+// A reflection's arguments from its draws: sqrt(u1), theta = 2 pi u2 and |v|.
+__device__ __forceinline__ double norm3(double x, double y, double z) {
+  return sfp::sqrt_rn(xadd(xadd(xmul(x, x), xmul(y, y)), xmul(z, z)));
+}
+__device__ __forceinline__ double theta_of(double u2) { return xmul(xmul(u2, 2.0), 3.141592653589793); }
+
 // New velocity of a cosine-law diffuse reflection off wall w (src/particle.cpp:309-328).
-__device__ __forceinline__ void diffuse_velocity(PState& p, double su, double theta, double speed, char w) {
+__device__ __forceinline__ void diffuse_velocity(PState& p, double u1, double u2, char w) {
+  const double su = sfp::sqrt_rn(u1), theta = theta_of(u2), speed = norm3(p.vx, p.vy, p.vz);
   double phi, cp, sp, ct, stt;
   traj_acos_sincos(su, phi, sp, cp);
   traj_sincos(theta, stt, ct);
@@ -336,11 +354,26 @@ __device__ __forceinline__ int nth_set_bit(unsigned m, int k) {
   return p;
 }
 
+// The velocity after a gas collision from its three normals: Maxwell-Boltzmann
+// ('M'), or the old speed in their direction ('C') (src/particle.cpp:373-391).
+__device__ __forceinline__ void gas_velocity(PState& p, const SetParams& P, double n1, double n2, double n3) {
+  if (P.dist == 'M') {
+    p.vx = xmul(n1, P.sqrtKT_m);
+    p.vy = xmul(n2, P.sqrtKT_m);
+    p.vz = xmul(n3, P.sqrtKT_m);
+  } else {
+    const double speed = norm3(p.vx, p.vy, p.vz), nrm = norm3(n1, n2, n3);
+    p.vx = sfp::div_rn(xmul(n1, speed), nrm);
+    p.vy = sfp::div_rn(xmul(n2, speed), nrm);
+    p.vz = sfp::div_rn(xmul(n3, speed), nrm);
+  }
+}
+
 // The rest of a deferred gas collision from the logarithms of its draws
 // (log_a of the gas clock's 1 - u, log_s0 and log_s1 of the Marsaglia pairs):
 // the gas clock as rng_exponential advances it, the three normals and the
-// cached spare as three rng_normal calls leave them, the Maxwell-Boltzmann
-// velocity (src/particle.cpp:117-119, 89-111, 373-380).
+// cached spare as three rng_normal calls leave them, and the new velocity
+// (src/particle.cpp:117-119, 89-111, 373-391).
 __device__ __forceinline__ void gas_finish(PState& p, const SetParams& P, const EventDefer& dd, double log_a,
                                            double log_s0, double log_s1) {
   p.next_gas = xadd(p.next_gas, xmul(-P.tc, log_a));
@@ -360,9 +393,7 @@ __device__ __forceinline__ void gas_finish(PState& p, const SetParams& P, const 
     n3 = xadd(0.0, xmul(xmul(1.0, dd.x[4]), f1));
     p.rng.spare = xmul(dd.x[5], f1);
   }
-  p.vx = xmul(n1, P.sqrtKT_m);
-  p.vy = xmul(n2, P.sqrtKT_m);
-  p.vz = xmul(n3, P.sqrtKT_m);
+  gas_velocity(p, P, n1, n2, n3);
 }
 
 // The deferred events of a warp, lanes `pend`, computed by all 32 lanes
@@ -385,9 +416,10 @@ __device__ __forceinline__ void deferred_events_warp(PState& p, const SetParams&
   if (refl) {
     const int np = __popc(refl);
     const bool mine = dd.pending && !dd.gas;
-    const double x = dd.x[0];
-    double y0 = 0.0, arg_a = 0.0;
+    double x = 0.0, theta = 0.0, y0 = 0.0, arg_a = 0.0;
     if (mine) {
+      x = sfp::sqrt_rn(dd.x[0]);
+      theta = theta_of(dd.x[1]);
       y0 = acos(x);
       arg_a = x < 1.0 ? crm::acos_newton_arg(x, y0) : 0.0;  // NaN and 1 use none
     }
@@ -398,7 +430,7 @@ __device__ __forceinline__ void deferred_events_warp(PState& p, const SetParams&
       // the theta of reflection j - np
       const int j = base + lane;
       const int src = nth_set_bit(refl, min(j < np ? j : j - np, np - 1));
-      const double a1 = __shfl_sync(FULL, arg_a, src), a2 = __shfl_sync(FULL, dd.x[1], src);
+      const double a1 = __shfl_sync(FULL, arg_a, src), a2 = __shfl_sync(FULL, theta, src);
       crm::DD sn, cs;
       crm::sincos_dd(j < np ? a1 : a2, sn, cs);
       // the reflection of rank r takes jobs r and np + r
@@ -420,8 +452,8 @@ __device__ __forceinline__ void deferred_events_warp(PState& p, const SetParams&
       double phi, sp, cp;
       if (!crm::acos_sincos_given(x, y0, sa, ca, phi, sp, cp)) crm::cr_acos_sincos(x, phi, sp, cp);
       double stt = st.hi, ctt = ct.hi;
-      if (!(crm::trig_sure(st) && crm::trig_sure(ct))) crm::sincos_accurate(dd.x[1], stt, ctt);
-      diffuse_apply(p, sp, cp, stt, ctt, dd.x[2], dd.wall);
+      if (!(crm::trig_sure(st) && crm::trig_sure(ct))) crm::sincos_accurate(theta, stt, ctt);
+      diffuse_apply(p, sp, cp, stt, ctt, norm3(p.vx, p.vy, p.vz), dd.wall);
       dd.pending = false;
     }
   }
@@ -464,11 +496,54 @@ __device__ __forceinline__ void deferred_events_warp(PState& p, const SetParams&
     if (GAS && dd.gas)
       gas_finish(p, P, dd, traj_log(dd.x[0]), traj_log(dd.x[3]), dd.spare_first ? 0.0 : traj_log(dd.x[6]));
     else
-      diffuse_velocity(p, dd.x[0], dd.x[1], dd.x[2], dd.wall);
+      diffuse_velocity(p, dd.x[0], dd.x[1], dd.wall);
     dd.pending = false;
     dd.gas = false;
   }
 #endif
+}
+
+// The ballistic move in the reference's own operations, for a dt that is not finite.
+static __device__ __noinline__ void move_any(double* x, double dt, double ay) {
+  const double hax = xmul(xmul(0.5 * 0.0, dt), dt), hay = xmul(xmul(0.5 * ay, dt), dt);
+  x[0] = xadd(xadd(x[0], xmul(x[3], dt)), hax);
+  x[1] = xadd(xadd(x[1], xmul(x[4], dt)), hay);
+  x[2] = xadd(xadd(x[2], xmul(x[5], dt)), hax);
+  x[3] = xadd(x[3], xmul(0.0, dt));
+  x[4] = xadd(x[4], xmul(ay, dt));
+  x[5] = xadd(x[5], xmul(0.0, dt));
+}
+
+// The nearest wall and its time; NaN when every comparison fails.
+__device__ __forceinline__ double first_wall(double dtx, double dty, double dtz, char& wall) {
+  double tb = __longlong_as_double(0x7ff8000000000000ll);
+  if (sfp::is_nan(dtx) || sfp::is_nan(dty) || sfp::is_nan(dtz)) {  // a NaN loses every comparison
+    if (dtx == dty) {
+      tb = dtx; wall = 'b';  // x-y edge
+    } else if (dtx == dtz) {
+      tb = dtx; wall = 'c';  // x-z edge
+    } else if (dty == dtz) {
+      tb = dty; wall = 'd';  // y-z edge
+    }
+    return tb;
+  }
+  const fx::i64 x = sfp::key(dtx), y = sfp::key(dty), z = sfp::key(dtz);
+  if (x < y && x < z) {
+    tb = dtx; wall = 'x';
+  } else if (y < x && y < z) {
+    tb = dty; wall = 'y';
+  } else if (z < x && z < y) {
+    tb = dtz; wall = 'z';
+  } else if (x == y && x == z) {
+    tb = dtx; wall = 'a';  // corner
+  } else if (x == y) {
+    tb = dtx; wall = 'b';  // x-y edge
+  } else if (x == z) {
+    tb = dtx; wall = 'c';  // x-z edge
+  } else if (y == z) {
+    tb = dty; wall = 'd';  // y-z edge
+  }
+  return tb;
 }
 
 // One trajectory event: calc_next_collision_time, update_position_and_velocity
@@ -483,29 +558,33 @@ __device__ __forceinline__ void deferred_events_warp(PState& p, const SetParams&
 // the draws possible here, non-zero except cos(phi) at u1 = 0, so it is NaN
 // or infinite only when the velocity before it already was, which fails the
 // same check (NaN) or the position check before it (infinite).  A gas
-// collision with a Maxwell-Boltzmann redraw is deferred the same way: its
-// uniform draws are taken here in the reference's order, the logarithms (of
-// the gas clock and of the Marsaglia pairs) later.  Its new velocity is the
-// product of finite normals and a finite sqrt(kT/m), so the NaN check gives the
-// outcome it gives on the velocity before the collision (which it also tests).
+// collision is deferred the same way: its uniform draws are taken here in the
+// reference's order, the logarithms (of the gas clock and of the Marsaglia
+// pairs) later.  Its new velocity is the product of finite normals and a finite
+// sqrt(kT/m), or the old speed in the direction of the normals, so the NaN check
+// gives the outcome it gives on the velocity before the collision (which it
+// also tests).
 //
 // GAS = false: compiled for launches in which no parameter set has gas
 // collisions.  Their gas clock is DBL_MAX and never moves, so the gas
 // collision is never the next event: either the wall time is finite and
 // smaller, or it is infinite and the step ends at the maxPosStep / window
 // limit either way.
+//
+// What bounds it: latency and issue of the integer code.  Divisions, square roots,
+// comparisons and draws run on the integer pipes (st_softfp.cuh), and the
+// reference's additions of a zero acceleration's terms are left out where they
+// change nothing (finite dt; -0 becomes 0 as they make it): some 35 FP64
+// instructions remain of about 180.
 template <bool DEFER = false, bool GAS = true>
 __device__ __forceinline__ bool traj_event(PState& p, const SetParams& P, double tf, SegStart& s0,
                                            EventDefer* dd = nullptr) {
   const double G = kGravity;
-  const double hLx = P.Lx / 2.0, hLy = P.Ly / 2.0, hLz = P.Lz / 2.0;
   double dtx, dty, dtz;
   // ---- time to the next wall (calc_next_collision_time)
+  dtx = sfp::div_rn(xsub(sfp::negative(p.vx) ? -P.hLx : P.hLx, p.px), p.vx);
+  dtz = sfp::div_rn(xsub(sfp::negative(p.vz) ? -P.hLz : P.hLz, p.pz), p.vz);
   if (P.gravity) {
-    const double dx = xsub(sgn1(p.vx) < 0.0 ? -hLx : hLx, p.px);
-    const double dz = xsub(sgn1(p.vz) < 0.0 ? -hLz : hLz, p.pz);
-    dtx = xdiv(dx, p.vx);
-    dtz = xdiv(dz, p.vz);
     const double y2 = xmul(p.vy, p.vy);
     // Moving down meets the floor; moving up meets the ceiling unless the apex
     // is below it (then rise and fall to the floor).  Floor and ceiling share
@@ -513,89 +592,71 @@ __device__ __forceinline__ bool traj_event(PState& p, const SetParams& P, double
     // are bit for bit its floor roots (sq - vy)/G, -(sq + vy)/G in swapped
     // order (IEEE addition commutes, negation is exact), and min(|r1|, |r2|)
     // does not depend on the order (both roots are NaN together), so both
-    // branches run the same sqrt and divisions, once.
+    // branches run the same sqrt and divisions, once.  The apex branch shares
+    // them too: its sqrt argument and its one division are chosen first.
     bool apex = false;
-    double arg = 0.0;
-    if (sgn1(p.vy) <= 0.0) {
-      const double dy = xadd(p.py, xmul(P.Ly, 0.5));
+    double arg, t1 = 0.0;
+    if (sfp::negative(p.vy)) {
+      const double dy = xadd(p.py, P.hLy);
       arg = xadd(xmul(-2.0 * G, dy), y2);
     } else {
-      const double top = xadd(xdiv(xmul(-0.5, y2), G), p.py);
-      apex = top < xmul(0.5, P.Ly);
-      arg = xsub(y2, xmul(2.0 * G, xsub(p.py, xmul(0.5, P.Ly))));
+      const double top = xadd(sfp::div_g(xmul(-0.5, y2)), p.py);
+      apex = sfp::lt(top, P.hLy);
+      if (apex) {
+        t1 = sfp::div_g(-p.vy);
+        const double ap = xadd(xadd(p.py, xmul(p.vy, t1)), xmul(xmul(0.5 * G, t1), t1));
+        arg = sfp::div_g(xmul(xsub(-P.hLy, ap), 2.0));
+      } else {
+        arg = xsub(y2, xmul(2.0 * G, xsub(p.py, P.hLy)));
+      }
     }
-    if (!apex) {
-      const double sq = xsqrt(arg);
-      const double r1 = xdiv(-xadd(sq, p.vy), G);
-      const double r2 = xdiv(xsub(sq, p.vy), G);
-      dty = std_min(fabs(r1), fabs(r2));
+    const double sq = sfp::sqrt_rn(arg);
+    if (apex) {
+      dty = xadd(t1, sq);
     } else {
-      const double t1 = xdiv(-p.vy, G);
-      const double ap = xadd(xadd(p.py, xmul(p.vy, t1)), xmul(xmul(0.5 * G, t1), t1));
-      const double t2 = xsqrt(xdiv(xmul(xsub(xmul(-0.5, P.Ly), ap), 2.0), G));
-      dty = xadd(t1, t2);
+      const double a1 = fabs(sfp::div_g(xadd(sq, p.vy))), a2 = fabs(sfp::div_g(xsub(sq, p.vy)));
+      dty = sfp::f64_bits(a2) < sfp::f64_bits(a1) ? a2 : a1;
     }
-    if (dtx < 1e-16 || isnan(dtx))  // only the first offending axis is replaced
+    if (!sfp::le(1e-16, dtx))  // only the first offending axis is replaced (below 1e-16, or NaN)
       dtx = 1e6;
-    else if (dty < 1e-16 || isnan(dty))
+    else if (!sfp::le(1e-16, dty))
       dty = 1e6;
-    else if (dtz < 1e-16 || isnan(dtz))
+    else if (!sfp::le(1e-16, dtz))
       dtz = 1e6;
   } else {
-    dtx = xdiv(xsub(sgn1(p.vx) < 0.0 ? -hLx : hLx, p.px), p.vx);
-    dty = xdiv(xsub(sgn1(p.vy) < 0.0 ? -hLy : hLy, p.py), p.vy);
-    dtz = xdiv(xsub(sgn1(p.vz) < 0.0 ? -hLz : hLz, p.pz), p.vz);
-    if (dtx < 1e-16)
+    dty = sfp::div_rn(xsub(sfp::negative(p.vy) ? -P.hLy : P.hLy, p.py), p.vy);
+    if (sfp::lt(dtx, 1e-16))
       dtx = 1e6;
-    else if (dty < 1e-16)
+    else if (sfp::lt(dty, 1e-16))
       dty = 1e6;
-    else if (dtz < 1e-16)
+    else if (sfp::lt(dtz, 1e-16))
       dtz = 1e6;
   }
-  double tb = __longlong_as_double(0x7ff8000000000000ll);  // unset when every comparison fails (NaN input)
-  if (dtx < dty && dtx < dtz) {
-    tb = dtx; p.wall = 'x';
-  } else if (dty < dtx && dty < dtz) {
-    tb = dty; p.wall = 'y';
-  } else if (dtz < dtx && dtz < dty) {
-    tb = dtz; p.wall = 'z';
-  } else if (dtx == dty && dtx == dtz) {
-    tb = dtx; p.wall = 'a';  // corner
-  } else if (dtx == dty) {
-    tb = dtx; p.wall = 'b';  // x-y edge
-  } else if (dtx == dtz) {
-    tb = dtx; p.wall = 'c';  // x-z edge
-  } else if (dty == dtz) {
-    tb = dty; p.wall = 'd';  // y-z edge
-  }
+  const double tb = first_wall(dtx, dty, dtz, p.wall);
   // ---- gas collision, wall, window end or maxPosStep
   bool gas_next = false;
   double to_col = tb;
   const double to_gas = GAS ? xsub(p.next_gas, p.t) : 0.0;
   if (!GAS) {
     // no gas collisions in this launch
-  } else if (to_gas < tb) {
+  } else if (sfp::lt(to_gas, tb)) {
     gas_next = true;
     to_col = to_gas;
-  } else if (to_gas == tb) {  // tie: the wall wins and the gas clock is redrawn
+  } else if (sfp::eq(to_gas, tb)) {  // tie: the wall wins and the gas clock is redrawn
     p.next_gas = xadd(p.next_gas, rng_exponential(p.rng, P.tc));
     to_col = to_gas;
-    gas_next = false;
-  } else {
-    gas_next = false;
-    to_col = tb;
   }
   const double left = xsub(tf, p.t);
-  const bool window_end = left <= P.maxPosStep;
+  const bool window_end = sfp::le(left, P.maxPosStep);
   const double to_free = window_end ? left : P.maxPosStep;
   bool finished = false;
   double dt;
-  if (to_col <= to_free) {
+  if (sfp::le(to_col, to_free)) {
     dt = to_col;
     if (gas_next) {
       p.coll = 'G';
       p.n_coll += 1;
-      if (DEFER && P.dist == 'M' && isfinite(P.sqrtKT_m)) {
+      if (DEFER && (P.dist != 'M' || sfp::is_finite(P.sqrtKT_m))) {
         dd->x[0] = xsub(1.0, rng_uniform(p.rng));  // rng_exponential's draw; its log later
         dd->gas = true;
       } else {
@@ -605,7 +666,7 @@ __device__ __forceinline__ bool traj_event(PState& p, const SetParams& P, double
       p.n_bounce += 1;
       p.coll = 'W';
     }
-    if (to_col == to_free && window_end) finished = true;
+    if (window_end && sfp::eq(to_col, to_free)) finished = true;
   } else {
     p.coll = 'N';
     dt = to_free;
@@ -616,41 +677,48 @@ __device__ __forceinline__ bool traj_event(PState& p, const SetParams& P, double
   s0.px = p.px; s0.py = p.py; s0.pz = p.pz;
   s0.vx = p.vx; s0.vy = p.vy; s0.vz = p.vz;
   p.t = xadd(p.t, dt);
-  const double ay = P.gravity ? G : 0.0;
-  const double hax = xmul(xmul(0.5 * 0.0, dt), dt);
-  const double hay = xmul(xmul(0.5 * ay, dt), dt);
-  p.px = xadd(xadd(s0.px, xmul(s0.vx, dt)), hax);
-  p.py = xadd(xadd(s0.py, xmul(s0.vy, dt)), hay);
-  p.pz = xadd(xadd(s0.pz, xmul(s0.vz, dt)), hax);
-  p.vx = xadd(p.vx, xmul(0.0, dt));
-  p.vy = xadd(p.vy, xmul(ay, dt));
-  p.vz = xadd(p.vz, xmul(0.0, dt));
-  const double speed = xsqrt(xadd(xadd(xmul(p.vx, p.vx), xmul(p.vy, p.vy)), xmul(p.vz, p.vz)));
+  if (sfp::is_finite(dt)) {
+    p.px = sfp::plus0(xadd(s0.px, xmul(s0.vx, dt)));
+    p.py = xadd(s0.py, xmul(s0.vy, dt));
+    p.pz = sfp::plus0(xadd(s0.pz, xmul(s0.vz, dt)));
+    p.vx = sfp::plus0(p.vx);
+    p.vz = sfp::plus0(p.vz);
+    if (P.gravity) {
+      p.py = xadd(p.py, xmul(xmul(0.5 * G, dt), dt));
+      p.vy = xadd(p.vy, xmul(G, dt));
+    } else {
+      p.py = sfp::plus0(p.py);
+      p.vy = sfp::plus0(p.vy);
+    }
+  } else {
+    double x[6] = {p.px, p.py, p.pz, p.vx, p.vy, p.vz};
+    move_any(x, dt, P.gravity ? G : 0.0);
+    p.px = x[0]; p.py = x[1]; p.pz = x[2];
+    p.vx = x[3]; p.vy = x[4]; p.vz = x[5];
+  }
   if (p.coll == 'W') {
     const char w = p.wall;
     const bool sx = (w == 'x' || w == 'a' || w == 'b' || w == 'c');
     const bool sy = (w == 'y' || w == 'a' || w == 'b' || w == 'd');
     const bool sz = (w == 'z' || w == 'a' || w == 'c' || w == 'd');
-    if (sx) p.px = p.px < 0.0 ? -xmul(P.Lx, 0.5) : xmul(P.Lx, 0.5);
-    if (sy) p.py = p.py < 0.0 ? -xmul(P.Ly, 0.5) : xmul(P.Ly, 0.5);
-    if (sz) p.pz = p.pz < 0.0 ? -xmul(P.Lz, 0.5) : xmul(P.Lz, 0.5);
+    if (sx) p.px = sfp::negative(p.px) ? -P.hLx : P.hLx;
+    if (sy) p.py = sfp::negative(p.py) ? -P.hLy : P.hLy;
+    if (sz) p.pz = sfp::negative(p.pz) ? -P.hLz : P.hLz;
     bool diffuse = false;
-    if (P.diffuse > (double)FLT_MIN) diffuse = rng_uniform(p.rng) < P.diffuse;
+    if (sfp::lt((double)FLT_MIN, P.diffuse)) diffuse = sfp::lt(rng_uniform(p.rng), P.diffuse);
     if (diffuse) {
       // cosine-law diffuse reflection (src/particle.cpp:309-328): both draws
-      // now, the trigonometry now or (DEFER) batched later
-      const double su = xsqrt(rng_uniform(p.rng));
-      const double theta = xmul(xmul(rng_uniform(p.rng), 2.0), 3.141592653589793);
+      // now, the roots and the trigonometry now or (DEFER) batched later
+      const double u1 = rng_uniform(p.rng), u2 = rng_uniform(p.rng);
       if (w == 'x' || w == 'y' || w == 'z') {
         if (DEFER) {
-          dd->x[0] = su;
-          dd->x[1] = theta;
-          dd->x[2] = speed;
+          dd->x[0] = u1;
+          dd->x[1] = u2;
           dd->wall = w;
           dd->gas = false;
           dd->pending = true;
         } else {
-          diffuse_velocity(p, su, theta, speed, w);
+          diffuse_velocity(p, u1, u2, w);
         }
       } else {
         p.stop = true;  // a diffuse hit on an edge or corner stops the particle
@@ -666,33 +734,33 @@ __device__ __forceinline__ bool traj_event(PState& p, const SetParams& P, double
       // normal is the cached spare or opens pair 0, whose spare is the second;
       // the third opens pair 1 (its spare stays cached) or is pair 0's spare
       dd->spare_first = p.rng.has;
-      marsaglia_draw(p.rng, dd->x[1], dd->x[2], dd->x[3]);
-      if (!dd->spare_first) marsaglia_draw(p.rng, dd->x[4], dd->x[5], dd->x[6]);
+#pragma unroll 1
+      for (int k = dd->spare_first ? 1 : 0; k < 2; ++k) {
+        double u, v, s;
+        marsaglia_draw(p.rng, u, v, s);
+        const bool first = k == 0 || dd->spare_first;
+        dd->x[first ? 1 : 4] = u;
+        dd->x[first ? 2 : 5] = v;
+        dd->x[first ? 3 : 6] = s;
+      }
       p.rng.has = !dd->spare_first;
       dd->pending = true;
-    } else if (P.dist == 'M') {
-      p.vx = xmul(rng_normal(p.rng, 0.0, 1.0), P.sqrtKT_m);
-      p.vy = xmul(rng_normal(p.rng, 0.0, 1.0), P.sqrtKT_m);
-      p.vz = xmul(rng_normal(p.rng, 0.0, 1.0), P.sqrtKT_m);
-    } else if (P.dist == 'C') {
-      const double dx = rng_normal(p.rng, 0.0, 1.0);
-      const double dy = rng_normal(p.rng, 0.0, 1.0);
-      const double dz = rng_normal(p.rng, 0.0, 1.0);
-      const double nrm = xsqrt(xadd(xadd(xmul(dx, dx), xmul(dy, dy)), xmul(dz, dz)));
-      p.vx = xdiv(xmul(dx, speed), nrm);
-      p.vy = xdiv(xmul(dy, speed), nrm);
-      p.vz = xdiv(xmul(dz, speed), nrm);
+    } else {
+      double n0 = 0.0, n1 = 0.0, n2 = 0.0;
+      rng_normals(p.rng, n0, n1, n2);
+      gas_velocity(p, P, n0, n1, n2);
     }
   }
-  // ---- sanity_check
-  const double tol = 1.0e-15;
-  if (fabs(p.px) > xadd(hLx, tol) || fabs(p.py) > xadd(hLy, tol) || fabs(p.pz) > xadd(hLz, tol)) {
+  // ---- sanity_check (limits: the half edges plus 1e-15)
+  if (sfp::abs_gt(p.px, P.limx) || sfp::abs_gt(p.py, P.limy) || sfp::abs_gt(p.pz, P.limz)) {
     p.stop = true; p.fail = 1;  // out of bounds
-  } else if (isinf(s0.t) || isinf(p.t)) {
+  } else if (sfp::is_inf(s0.t) || sfp::is_inf(p.t)) {
     p.stop = true; p.fail = 2;  // infinite time
-  } else if (isnan(s0.px) || isnan(s0.py) || isnan(s0.pz) || isnan(p.px) || isnan(p.py) || isnan(p.pz)) {
+  } else if (sfp::is_nan(s0.px) || sfp::is_nan(s0.py) || sfp::is_nan(s0.pz) || sfp::is_nan(p.px) ||
+             sfp::is_nan(p.py) || sfp::is_nan(p.pz)) {
     p.stop = true; p.fail = 3;  // NaN position
-  } else if (isnan(p.vx) || isnan(p.vy) || isnan(p.vz) || isnan(s0.vx) || isnan(s0.vy) || isnan(s0.vz)) {
+  } else if (sfp::is_nan(p.vx) || sfp::is_nan(p.vy) || sfp::is_nan(p.vz) || sfp::is_nan(s0.vx) ||
+             sfp::is_nan(s0.vy) || sfp::is_nan(s0.vz)) {
     p.stop = true; p.fail = 4;  // NaN velocity
   }
   return finished;
@@ -718,6 +786,7 @@ struct Seg {
   bool reject, last;
   bool acc;            // the last attempt was accepted
   bool fx;             // DOP853 in fixed point, scaled by sc
+  bool carry;          // k holds the spin in fixed point (kept from segment to segment; false at a window's start)
   fx::SegScale sc;
 };
 
@@ -810,7 +879,7 @@ __device__ __forceinline__ fx::i64 as_i64(double x) { return __double_as_longlon
 // the polynomial's o0 and o1, for DOP853 sets scaled to fixed point where they
 // have a scale there (fx; then o0 and o1 hold Q63 words).
 struct SegPoly {
-  double o0[3], o1[3];
+  double o0[3], o1[3], o2[3];
   fx::SegScale sc;
   bool fx;
 };
@@ -822,10 +891,12 @@ __device__ __forceinline__ void seg_scale(SegPoly& q, const SetParams& P, double
   if (P.integrator == 0 && P.tol_ratio >= 0.0 && (gpa == 0.0 || isfinite(P.w)))
     q.fx = fx::field_scale(q.o0, q.o1, P.o2c, gpa, T, q.sc);
   if (q.fx) {
-#pragma unroll
+    const int e0 = q.sc.oe, e1 = e0 - q.sc.te, e2 = e1 - q.sc.te;
+#pragma unroll 1  // rolled: less code
     for (int c = 0; c < 3; ++c) {
-      q.o0[c] = as_f64(fx::to_q63(q.o0[c], q.sc.oe));
-      q.o1[c] = as_f64(fx::to_q63(q.o1[c], q.sc.oe - q.sc.te));
+      q.o0[c] = as_f64(fx::to_q63(q.o0[c], e0));
+      q.o1[c] = as_f64(fx::to_q63(q.o1[c], e1));
+      q.o2[c] = as_f64(fx::to_q63(P.o2c[c], e2));
     }
   }
 #endif
@@ -839,12 +910,11 @@ __device__ __forceinline__ void seg_poly(SegPoly& q, const SetParams& P, const S
 __device__ __forceinline__ void seg_open(Seg& g, const SetParams& P, const SegPoly& q, double t0, double t_end) {
   seg_begin(g, P, t0, t_end, q.o0, q.o1);
   g.fx = q.fx;
+  const int se = g.sc.se;  // the spin's own scale goes on
   g.sc = q.sc;
+  g.sc.se = se;
   if (q.fx) {
-    const int e2 = q.sc.oe - 2 * q.sc.te;
-    g.o2x = as_f64(fx::to_q63(g.o2x, e2));
-    g.o2y = as_f64(fx::to_q63(g.o2y, e2));
-    g.o2z = as_f64(fx::to_q63(g.o2z, e2));
+    g.o2x = q.o2[0]; g.o2y = q.o2[1]; g.o2z = q.o2[2];
     g.gpa = as_f64(fx::to_q63(g.gpa, q.sc.oe));
   }
 }
@@ -961,6 +1031,13 @@ __device__ __forceinline__ void dop_spin(const Seg& g, double& Sx, double& Sy, d
   Sz = fx::from_q63(as_i64(g.kz), g.sc.se);
 }
 
+// A spin in fixed point stays there from segment to segment (g.carry): it becomes
+// doubles again at a window end, or where a segment runs in FP64.
+__device__ __forceinline__ void spin_settle(Seg& g, double& Sx, double& Sy, double& Sz) {
+  if (g.carry) dop_spin(g, Sx, Sy, Sz);
+  g.carry = false;
+}
+
 // The derivative at the start of an FP64 segment, taking the segment out of fixed point first.
 static __device__ __noinline__ void dop_begin_f64(Seg& g, const SetParams& P, double Sx, double Sy, double Sz) {
   if (g.fx) seg_unscale(g);
@@ -968,19 +1045,24 @@ static __device__ __noinline__ void dop_begin_f64(Seg& g, const SetParams& P, do
 }
 
 // Start a DOP853 call over the segment (src/integrator.cpp:102-119).
-__device__ __forceinline__ void dop_begin(Seg& g, const SetParams& P, double Sx, double Sy, double Sz, double h) {
+__device__ __forceinline__ void dop_begin(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz, double h) {
   g.h = h;
   g.facold = 1.0e-4;
   g.nstep = 0;
   g.turns = 0;
   g.reject = false;
   g.last = false;
-  const double S[3] = {Sx, Sy, Sz};
-  if (g.fx && fx::spin_scale(S, g.sc.se) && fx::ratio_fits(P.tol_ratio, g.sc.se)) {
-    g.kx = as_f64(fx::to_q63(Sx, g.sc.se));
-    g.ky = as_f64(fx::to_q63(Sy, g.sc.se));
-    g.kz = as_f64(fx::to_q63(Sz, g.sc.se));
-  } else {
+  if (g.fx && !g.carry) {
+    const double S[3] = {Sx, Sy, Sz};
+    if (fx::spin_scale(S, g.sc.se) && fx::ratio_fits(P.tol_ratio, g.sc.se)) {
+      g.kx = as_f64(fx::to_q63(Sx, g.sc.se));
+      g.ky = as_f64(fx::to_q63(Sy, g.sc.se));
+      g.kz = as_f64(fx::to_q63(Sz, g.sc.se));
+      g.carry = true;
+    }
+  }
+  if (!(g.fx && g.carry)) {
+    spin_settle(g, Sx, Sy, Sz);
     Seg t = g;  // the call takes its address: g itself stays in registers
     dop_begin_f64(t, P, Sx, Sy, Sz);
     g = t;
@@ -1130,35 +1212,35 @@ static __device__ __noinline__ int dop_attempt_f64(Seg& g, const SetParams& P, d
 }
 
 
-// The FP64 attempt for a segment in fixed point: on an accepted step the
-// segment goes on in FP64, a rejected one changes its step size only.
-__device__ __forceinline__ int dop_attempt_fallback(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz) {
-  Seg t = g;  // the call takes its address: g itself stays in registers
-  double S[3] = {Sx, Sy, Sz};
-  if (t.fx) {
-    seg_unscale(t);
-    dop_spin(g, S[0], S[1], S[2]);
-    feval(t, P, t.x - t.t0, S[0], S[1], S[2], t.kx, t.ky, t.kz);
-  }
-  const int r = dop_attempt_f64(t, P, S[0], S[1], S[2]);
-  if (g.fx && !t.acc) {
+// The FP64 attempt for any segment.  One in fixed point goes on in FP64 after an
+// accepted step; a rejected one changes its step size only.
+static __device__ __noinline__ int dop_attempt_slow(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz) {
+  if (!g.fx) return dop_attempt_f64(g, P, Sx, Sy, Sz);
+  Seg t = g;
+  double x, y, z;
+  dop_spin(g, x, y, z);
+  seg_unscale(t);
+  feval(t, P, t.x - t.t0, x, y, z, t.kx, t.ky, t.kz);
+  const int r = dop_attempt_f64(t, P, x, y, z);
+  if (t.acc) {
+    t.carry = false;
+    g = t;
+    Sx = x;
+    Sy = y;
+    Sz = z;
+  } else {
     g.h = t.h;
     g.reject = t.reject;
     g.last = t.last;
     g.nstep = t.nstep;
     g.acc = false;
-  } else {
-    g = t;
-    Sx = S[0];
-    Sy = S[1];
-    Sz = S[2];
   }
   return r;
 }
 
 // One attempted DOP853 step (one pass of the loop at src/integrator.cpp:128-247),
 // spin components over the lanes of `view`, stage derivatives in `ks`.  While
-// the segment is in fixed point, Sx..Sz are brought up to date at its end.
+// the segment is in fixed point Sx..Sz stay behind (spin_settle).
 // Returns as dop_attempt_f64.
 //
 // What bounds it: issue.  ~3,500 instructions, a third of them IMAD.WIDE (2.1
@@ -1168,31 +1250,46 @@ template <class V, class KS>
 __device__ __forceinline__ int dop_attempt_v(const V& view, KS& ks, Seg& g, const SetParams& P, double& Sx, double& Sy,
                                              double& Sz) {
   if (g.nstep > P.nmax) return -1;
-  if (!g.fx) return dop_attempt_fallback(g, P, Sx, Sy, Sz);
   double h = g.h;
   bool last = g.last;
-  if ((g.x + 1.01 * h - g.xf) * g.posneg > 0.0) {
+  const double over = g.x + 1.01 * h - g.xf;
+  if (g.posneg < 0.0 ? sfp::negative(over) : sfp::lt(0.0, over)) {
     h = g.xf - g.x;
     last = true;
   }
-  if (h < P.hmin && !last) h = P.hmin;
-  fx::i64 o0[V::N], o1[V::N], o2[V::N], S[V::N], Sn[V::N];
-  view.pick(as_i64(g.o0x), as_i64(g.o0y), as_i64(g.o0z), o0);
-  view.pick(as_i64(g.o1x), as_i64(g.o1y), as_i64(g.o1z), o1);
-  view.pick(as_i64(g.o2x), as_i64(g.o2y), as_i64(g.o2z), o2);
-  view.pick(as_i64(g.kx), as_i64(g.ky), as_i64(g.kz), S);
-  const fx::StepTol tol = {P.rtol, P.tol_ratio};
+  if (!last && sfp::lt(h, P.hmin)) h = P.hmin;
+  fx::i64 Sn[V::N];
   fx::StepOut out;
-  if (!fx::dop_step(view, ks, g.sc, o0, o1, o2, as_i64(g.gpa), (fx::u64)P.wturn_m, P.wturn_e, g.x, g.x - g.t0, h, tol, S,
-                    Sn, out))
-    return dop_attempt_fallback(g, P, Sx, Sy, Sz);
+  bool fixed = g.fx;
+  if (fixed) {
+    fx::i64 o0[V::N], o1[V::N], o2[V::N], S[V::N];
+    view.pick(as_i64(g.o0x), as_i64(g.o0y), as_i64(g.o0z), o0);
+    view.pick(as_i64(g.o1x), as_i64(g.o1y), as_i64(g.o1z), o1);
+    view.pick(as_i64(g.o2x), as_i64(g.o2y), as_i64(g.o2z), o2);
+    view.pick(as_i64(g.kx), as_i64(g.ky), as_i64(g.kz), S);
+    const fx::StepTol tol = {P.rtol, P.tol_ratio};
+    fixed = fx::dop_step(view, ks, g.sc, o0, o1, o2, as_i64(g.gpa), (fx::u64)P.wturn_m, P.wturn_e, g.x, g.x - g.t0, h,
+                         tol, S, Sn, out);
+  }
+  if (!fixed) {  // rare: on copies, so that g itself stays in registers
+    Seg t = g;
+    double x = Sx, y = Sy, z = Sz;
+    const int r = dop_attempt_slow(t, P, x, y, z);
+    g = t;
+    Sx = x;
+    Sy = y;
+    Sz = z;
+    return r;
+  }
   g.nstep++;
   g.acc = false;
   // step-size controller (clamped to [fac1, fac2]; beta = 0)
-  const double grow = max_d(P.fac1, P.safe * out.root8);
-  double hnew;
+  // (comparisons on the integer pipes; fac1 and fac2 are numbers)
+  const double raw = P.safe * out.root8;
+  double grow = sfp::lt(raw, P.fac1) ? P.fac1 : raw;
+  if ((out.accept || P.fixed) && sfp::lt(P.fac2, grow)) grow = P.fac2;
+  double hnew = h * grow;
   if (out.accept || P.fixed) {
-    hnew = h * min_d(P.fac2, grow);
     g.acc = true;
     g.hu = h;
     fx::i64 N3[3];
@@ -1206,14 +1303,12 @@ __device__ __forceinline__ int dop_attempt_v(const V& view, KS& ks, Seg& g, cons
     if (last) {
       g.h = h;
       g.last = true;
-      dop_spin(g, Sx, Sy, Sz);
       return 1;
     }
-    if (fabs(hnew) > P.hmax) hnew = g.posneg * P.hmax;
-    if (g.reject) hnew = g.posneg * min_d(fabs(hnew), fabs(h));
+    if (sfp::lt(P.hmax, fabs(hnew))) hnew = g.posneg * P.hmax;
+    if (g.reject) hnew = g.posneg * (sfp::lt(fabs(hnew), fabs(h)) ? fabs(hnew) : fabs(h));
     g.reject = false;
   } else {
-    hnew = h * grow;
     g.reject = true;
     last = false;
   }
@@ -1244,7 +1339,7 @@ __device__ __forceinline__ void rk45_begin(Seg& g, double h) {
 // state (zero on the first attempt of a call).  Returns 0 to continue, 1 when
 // the segment end was reached (g.h then holds the carried step), -1 when
 // h < hmin, -2 after more than nmax attempts.
-__device__ __forceinline__ int rk45_attempt(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz) {
+static __device__ __noinline__ int rk45_attempt_call(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz) {
   using namespace rk45;
   g.nstep++;
   if (g.nstep > P.nmax) return -2;
@@ -1325,6 +1420,18 @@ __device__ __forceinline__ int rk45_attempt(Seg& g, const SetParams& P, double& 
   g.h = P.fixed ? h : h * q;
   g.lnprev = lnr;
   return 0;
+}
+
+// The call on copies: the caller's segment and spin stay in registers.
+__device__ __forceinline__ int rk45_attempt(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz) {
+  Seg t = g;
+  double x = Sx, y = Sy, z = Sz;
+  const int r = rk45_attempt_call(t, P, x, y, z);
+  g = t;
+  Sx = x;
+  Sy = y;
+  Sz = z;
+  return r;
 }
 
 // ------------------------------------------------------------ integrator types 2-5

@@ -33,7 +33,7 @@ __device__ __forceinline__ bool spin_on(int it) {
 
 // Start the integrator of the set's type over a segment.
 template <bool EXT>
-__device__ __forceinline__ void spin_begin(Seg& g, const SetParams& P, double Sx, double Sy, double Sz, double h) {
+__device__ __forceinline__ void spin_begin(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz, double h) {
   if (P.integrator == 0)
     dop_begin(g, P, Sx, Sy, Sz, h);
   else if (!EXT || P.integrator == 1)
@@ -87,6 +87,8 @@ __device__ __forceinline__ bool window_nested(PState& p, const SetParams& P, dou
   double tempH = p.h;
   bool finished = false;
   unsigned int guard = 0;
+  Seg g;
+  g.carry = false;
   while (!finished && !p.stop) {
     SegStart s0;
     finished = traj_event(p, P, tf, s0);
@@ -94,7 +96,6 @@ __device__ __forceinline__ bool window_nested(PState& p, const SetParams& P, dou
     if (p.fail == 0) {
       int res = 0;
       if (spin_on<EXT>(P.integrator)) {
-        Seg g;
         seg_setup(g, P, s0, p.t);
         if (P.integrator == 0) {
           dop_begin(g, P, p.Sx, p.Sy, p.Sz, tempH);
@@ -128,10 +129,14 @@ __device__ __forceinline__ bool window_nested(PState& p, const SetParams& P, dou
         p.fail = res;
       }
     }
-    if (p.stop) nan_fill(p);
+    if (p.stop) {
+      nan_fill(p);
+      g.carry = false;
+    }
     p.n_steps += 1;
     if (((++guard) & 255u) == 0u && past_deadline(dl)) return false;
   }
+  spin_settle(g, p.Sx, p.Sy, p.Sz);
   return true;
 }
 
@@ -182,6 +187,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_persistent(RunArgs a) {
   const SetParams* P = a.sets;
   PState p;
   Seg g;
+  g.carry = false;
   int w = 0, wlast = 0;
   double tf = 0.0, tempH = 0.0;
   bool finished = false, hit = false;
@@ -222,7 +228,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_persistent(RunArgs a) {
             mode = M_SEG;
           } else {
             if (p.fail == 0 && P->keep) p.h = tempH;
-            if (p.stop) nan_fill(p);
+            if (p.stop) {
+              nan_fill(p);
+              g.carry = false;
+            }
             p.n_steps += 1;
             mode = (finished || p.stop) ? M_WEND : M_EVENT;
           }
@@ -234,6 +243,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_persistent(RunArgs a) {
         }
       }
       if (mode == M_WEND) {
+        spin_settle(g, p.Sx, p.Sy, p.Sz);
         write_snap(a, i, w, p);
         ++w;
         store_state(a.s, i, p);  // every window end is a resumable checkpoint
@@ -269,7 +279,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_persistent(RunArgs a) {
         p.stop = true;
         p.fail = r;
       }
-      if (p.stop) nan_fill(p);
+      if (p.stop) {
+        nan_fill(p);
+        g.carry = false;
+      }
       p.n_steps += 1;
       mode = (finished || p.stop) ? M_WEND : M_EVENT;
     }
@@ -290,23 +303,68 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_persistent(RunArgs a) {
 
 // ------------------------------------------------------------------ batched (trajectory ahead)
 // The trajectory of a particle does not depend on its spin, so each lane runs
-// its particle's trajectory ahead of the spin integration into a small ring of
-// segment records in shared memory.  Rings are topped up warp-synchronously,
-// only when many lanes have room (or one lane has run dry), so the long and
-// branchy trajectory code runs with most lanes of the warp active instead of
-// the few lanes whose segment just ended.  A record carries the segment's time
-// span and field polynomial (o0, o1), so starting a segment on the spin side
-// is a ring pop and one Bloch evaluation.  The trajectory stops at every
-// window end until the spin side has finished the window, so checkpoints and
-// snapshots at window ends are exact.
+// its particles' trajectories ahead of the spin integration, into a ring of
+// segment records in device memory.  A warp alternates two phases: the
+// trajectory phase fills the rings of all its lanes (one event per lane and
+// round), the spin phase integrates (one step attempt per lane and iteration)
+// until lanes run dry.  A record carries the segment's time span and field
+// polynomial (o0, o1), so starting a segment on the spin side is a ring pop.
 //
-// Record fields (field-major, conflict-free): qd[(slot * kRecF + f) * BLOCK + tid]
-//   f = 0 t_start, 1 t_end, 2..4 o0, 5..7 o1 (+ 8..13 p0, v0 when the grad hook is not linear)
-// (o0, o1 as Q63 words when the flags say so: SegPoly), the field's scale
-// qs[slot * BLOCK + tid] = (norm bits, exponents),
-// flags qf[slot * BLOCK + tid]: bit0 window end reached, bit1 stop, bit2 bounce, bit3 gas
-// collision, bit4 field in fixed point, bits 8-15 sanity failure code.
-constexpr int kRecF = ST_GRAD_IS_LINEAR ? 8 : 14;
+// Why phases this long, and rings in memory: the instructions of either phase
+// about fill what a sub-partition holds close by (~16 KB), and beyond that they
+// arrive at 8 bytes per cycle and SM.  With 8-record rings in shared memory the
+// two phases alternated every other attempt and half the time went into
+// instruction supply (1,048,576 particles x 0.1 s: 398 ms with the trajectory
+// in FP64, 463 ms with its faster but larger integer code).  A ring of 64 records is
+// about 190 attempts; its 5 KB per lane live in L2 and cost ~160 bytes of traffic per
+// segment.
+//
+// The trajectory side crosses window ends and goes on to its next particle, so
+// rings never block there: at a window end it saves its state in one of
+// kAheadSlots slots, from which the spin side writes the window's checkpoint
+// and snapshot when it gets there.  So every window end is an exact, resumable
+// checkpoint, and the main state holds nothing newer than the spin side's last
+// finished window.
+constexpr int kAheadSlots = 4;
+
+struct alignas(16) SegRec {
+  double t0, t1, o0[3], o1[3], o2[3];  // o2 only in fixed point (in doubles it is the set's)
+#if !ST_GRAD_IS_LINEAR
+  double p0[3], v0[3];
+#endif
+  int on, scale;  // the fixed-point field scale (SegScale), packed
+  int flags, pad;
+};
+// SegRec::flags: window end reached, particle stopped, bounce, gas collision, field in fixed
+// point, start of a new particle (its index in t0); bits 8-15 sanity failure code.
+enum { R_FIN = 1, R_STOP = 2, R_WALL = 4, R_GAS = 8, R_FX = 16, R_FETCH = 32 };
+
+// Trajectory fields of a particle's state.
+struct alignas(16) TrajState {
+  double t, px, py, pz, vx, vy, vz, next_gas, spare;
+  uint64_t rx, ry, rz, rw;
+  int marks, pad;  // last collision | wall << 8 | spare valid << 16
+};
+__device__ __forceinline__ TrajState traj_of(const PState& p) {
+  return {p.t, p.px, p.py, p.pz, p.vx, p.vy, p.vz, p.next_gas, p.rng.spare, p.rng.x, p.rng.y, p.rng.z, p.rng.w,
+          (int)(uint8_t)p.coll | (int)(uint8_t)p.wall << 8 | (p.rng.has ? 1 << 16 : 0), 0};
+}
+__device__ __forceinline__ void traj_into(PState& p, const TrajState& s) {
+  p.t = s.t;
+  p.px = s.px; p.py = s.py; p.pz = s.pz;
+  p.vx = s.vx; p.vy = s.vy; p.vz = s.vz;
+  p.next_gas = s.next_gas;
+  p.rng.spare = s.spare;
+  p.rng.x = s.rx; p.rng.y = s.ry; p.rng.z = s.rz; p.rng.w = s.rw;
+  p.coll = (char)(s.marks & 0xff);
+  p.wall = (char)((s.marks >> 8) & 0xff);
+  p.rng.has = (s.marks >> 16) != 0;
+}
+
+// A lane's scratch: the trajectory side's state between phases, the window-end slots, the ring.
+__host__ __device__ constexpr size_t ahead_lane_bytes(int q) {
+  return (size_t)(1 + kAheadSlots) * sizeof(TrajState) + (size_t)q * sizeof(SegRec);
+}
 
 // ---- adjoint tape (TAPE instantiation only)
 // Cursor of one particle's two tape chains.
@@ -363,30 +421,38 @@ __device__ __forceinline__ void tape_seg(const TapeArgs& t, TapeCursor& c, const
   }
 }
 
-// A particle's cursor at fetch: fresh chains, or (append) the chains the
-// previous launch closed, continued.
-__device__ __forceinline__ void tape_resume(const TapeArgs& t, TapeCursor& c, int64_t i) {
-  if (!t.append) {
-    tape_open(c);
-    return;
-  }
-  c.sp = t.step_page[i];
-  c.sf = c.sp < 0 ? kTapeStepsPerPage : t.step_fill[i];
+// A particle's segment (trajectory side) or step (spin side) cursor at its
+// fetch: a fresh chain, or (append) the chain the previous launch closed,
+// continued.
+__device__ __forceinline__ void tape_resume_segs(const TapeArgs& t, TapeCursor& c, int64_t i) {
+  tape_open(c);
+  if (!t.append) return;
   c.gp = t.seg_page[i];
   c.gf = c.gp < 0 ? kTapeSegsPerPage : t.seg_fill[i];
-  c.ns = t.nsteps[i];
   c.ng = t.nsegs[i];
   c.ok = t.complete[i] != 0;
 }
+__device__ __forceinline__ void tape_resume_steps(const TapeArgs& t, TapeCursor& c, int64_t i) {
+  tape_open(c);
+  if (!t.append) return;
+  c.sp = t.step_page[i];
+  c.sf = c.sp < 0 ? kTapeStepsPerPage : t.step_fill[i];
+  c.ns = t.nsteps[i];
+}
 
-__device__ __forceinline__ void tape_close(const TapeArgs& t, const TapeCursor& c, int64_t i) {
-  t.step_page[i] = c.sp;
-  t.step_fill[i] = c.sp < 0 ? 0 : c.sf;
+// Close a chain.  The trajectory side runs ahead, so it closes a particle's
+// segments first; the particle's tape is complete when both sides stored everything.
+__device__ __forceinline__ void tape_close_segs(const TapeArgs& t, const TapeCursor& c, int64_t i) {
   t.seg_page[i] = c.gp;
   t.seg_fill[i] = c.gp < 0 ? 0 : c.gf;
-  t.nsteps[i] = c.ns;
   t.nsegs[i] = c.ng;
   t.complete[i] = c.ok ? 1 : 0;
+}
+__device__ __forceinline__ void tape_close_steps(const TapeArgs& t, const TapeCursor& c, int64_t i) {
+  t.step_page[i] = c.sp;
+  t.step_fill[i] = c.sp < 0 ? 0 : c.sf;
+  t.nsteps[i] = c.ns;
+  if (!c.ok) t.complete[i] = 0;
 }
 
 // View of state checkpoint k (same field layout as checkpoint 0, k * stride
@@ -404,48 +470,50 @@ __device__ __forceinline__ DeviceState state_slot(const DeviceState& b, int64_t 
 }
 
 // A record's field scale in two words.
-__device__ __forceinline__ int2 pack_scale(const fx::SegScale& s) {
-  return make_int2((int)fx::f32_bits(s.on), (s.oe << 16) | (s.te & 0xffff));
-}
-__device__ __forceinline__ fx::SegScale unpack_scale(int2 v) {
+__device__ __forceinline__ int pack_exps(const fx::SegScale& s) { return (int)((unsigned)s.oe << 16) | (s.te & 0xffff); }
+__device__ __forceinline__ fx::SegScale unpack_scale(int on, int exps) {
   fx::SegScale s;
-  s.on = fx::bits_f32((uint32_t)v.x);
-  s.oe = v.y >> 16;
-  s.te = (int)(short)(v.y & 0xffff);
+  s.on = fx::bits_f32((uint32_t)on);
+  s.oe = exps >> 16;
+  s.te = (int)(short)(exps & 0xffff);
   s.se = 0;
   return s;
 }
 
-template <int BLOCK, bool TAPE, bool GAS, bool EXT>
-__device__ __forceinline__ void produce_record(PState& tp, const SetParams& P, double tf, double* qd, int2* qs, int* qf,
-                                               int slot, int tid, bool& blocked, EventDefer& dd, const TapeArgs& ta,
-                                               TapeCursor& tc) {
+// One trajectory event of a lane into ring record r.  Returns its flags.
+template <bool TAPE, bool GAS, bool EXT>
+__device__ __forceinline__ int produce_record(PState& tp, const SetParams& P, double tf, SegRec* r, EventDefer& dd,
+                                              const TapeArgs& ta, TapeCursor& tc) {
   SegStart s0;
-  const uint64_t nb = tp.n_bounce, nc = tp.n_coll;
+  tp.n_bounce = tp.n_coll = 0;
   const bool fin = traj_event<true, GAS>(tp, P, tf, s0, &dd);
-  double* r = qd + (size_t)slot * kRecF * BLOCK + tid;
-  r[0 * BLOCK] = s0.t;
-  r[1 * BLOCK] = tp.t;
-  int fixed = 0;
+  int flags = (fin ? R_FIN : 0) | (tp.stop ? R_STOP : 0) | (tp.n_bounce != 0 ? R_WALL : 0) | (tp.n_coll != 0 ? R_GAS : 0) |
+              ((tp.fail & 0xff) << 8);
+  r->t0 = s0.t;
+  r->t1 = tp.t;
   if (spin_on<EXT>(P.integrator)) {
     SegPoly q;
     seg_poly(q, P, s0, tp.t);
-    r[2 * BLOCK] = q.o0[0]; r[3 * BLOCK] = q.o0[1]; r[4 * BLOCK] = q.o0[2];
-    r[5 * BLOCK] = q.o1[0]; r[6 * BLOCK] = q.o1[1]; r[7 * BLOCK] = q.o1[2];
-    if (q.fx) {
-      qs[slot * BLOCK + tid] = pack_scale(q.sc);
-      fixed = 16;
+#pragma unroll 1
+    for (int c = 0; c < 3; ++c) {
+      r->o0[c] = q.o0[c];
+      r->o1[c] = q.o1[c];
+      r->o2[c] = q.o2[c];
     }
 #if !ST_GRAD_IS_LINEAR
-    r[8 * BLOCK] = s0.px; r[9 * BLOCK] = s0.py; r[10 * BLOCK] = s0.pz;
-    r[11 * BLOCK] = s0.vx; r[12 * BLOCK] = s0.vy; r[13 * BLOCK] = s0.vz;
+    r->p0[0] = s0.px; r->p0[1] = s0.py; r->p0[2] = s0.pz;
+    r->v0[0] = s0.vx; r->v0[1] = s0.vy; r->v0[2] = s0.vz;
 #endif
+    if (q.fx) {
+      r->on = (int)fx::f32_bits(q.sc.on);
+      r->scale = pack_exps(q.sc);
+      flags |= R_FX;
+    }
   }
   // the segments the spin side integrates, in order
   if (TAPE && !tp.stop && tp.fail == 0) tape_seg(ta, tc, s0);
-  qf[slot * BLOCK + tid] = (fin ? 1 : 0) | (tp.stop ? 2 : 0) | (tp.n_bounce != nb ? 4 : 0) |
-                           (tp.n_coll != nc ? 8 : 0) | fixed | ((tp.fail & 0xff) << 8);
-  if (fin || tp.stop) blocked = true;
+  r->flags = flags;
+  return flags;
 }
 
 enum BatchedMode { B_FETCH = 0, B_NEED = 1, B_SEG = 2, B_WEND = 3, B_DONE = 4 };
@@ -453,225 +521,344 @@ enum BatchedMode { B_FETCH = 0, B_NEED = 1, B_SEG = 2, B_WEND = 3, B_DONE = 4 };
 // Diffuse reflections and Maxwell-Boltzmann gas collisions are deferred
 // (traj_event<true>): a lane with one pending produces no further records
 // until the warp computes the pending events together (deferred_events_warp),
-// when defer_k lanes have one, or one of them is about to run dry or has
-// reached its window end.
+// when defer_k lanes have one or nothing else can go on.
+// starve: the spin phase ends when this many lanes have run dry (or every lane
+// that could go on has).  keep: the trajectory phase goes on while this many
+// lanes have room (or one is dry).
 // TAPE: also write the adjoint tape (steps and segments of every particle)
 // and state checkpoints at every ta.ckpt_every-th window end.
 // GAS = false: the instantiation for launches without gas collisions.
 // EXT: also integrator types 2-5.
-template <int BLOCK, int MINB, int QCAP, bool TAPE, bool GAS, bool EXT>
-__global__ void __launch_bounds__(BLOCK, MINB)
-    k_batched(RunArgs a, int topup_start, int topup_keep, int defer_k, TapeArgs ta) {
+template <int BLOCK, int MINB, bool TAPE, bool GAS, bool EXT>
+__global__ void __launch_bounds__(BLOCK, MINB) k_batched(RunArgs a, int starve, int keep, int defer_k, TapeArgs ta) {
   extern __shared__ double st_smem[];
-  double* qd = st_smem;
-  int2* qs = reinterpret_cast<int2*>(st_smem + (size_t)QCAP * kRecF * BLOCK);
-  int* qf = reinterpret_cast<int*>(qs + QCAP * BLOCK);
-  // DOP853 stage derivatives, after the rings
-  char* stages = reinterpret_cast<char*>(qf + (QCAP * BLOCK + 3) / 4 * 4);
+  // DOP853 stage derivatives
+  char* stages = reinterpret_cast<char*>(st_smem);
   fx::StageSmem ks{reinterpret_cast<fx::Limb2*>(stages) + threadIdx.x,
                    reinterpret_cast<fx::Limb*>(stages + 12 * sizeof(fx::Limb2) * BLOCK) + threadIdx.x, BLOCK};
-  const int tid = threadIdx.x;
   const unsigned FULL = 0xffffffffu;
-  int mode = B_FETCH;
+  const int QCAP = a.ahead_q;
+  char* const mine = a.ahead + ((size_t)blockIdx.x * BLOCK + threadIdx.x) * ahead_lane_bytes(QCAP);
+  TrajState* const slots = reinterpret_cast<TrajState*>(mine);  // [0]: between phases, [1 + k]: window ends
+  SegRec* const ring = reinterpret_cast<SegRec*>(slots + 1 + kAheadSlots);
+  // ---- trajectory side
+  int64_t ti = 0;
+  int tw = 0, twl = 0;
+  bool t_run = false, t_done = false, t_wend = false, t_stop = false;
+  // ---- ring and window slots (records and slots in use)
+  int qhead = 0, qcount = 0, whead = 0, wcount = 0;
+  // ---- spin side
+  int mode = B_NEED;
   int64_t i = 0;
   const SetParams* P = a.sets;
-  PState tp;  // trajectory fields run ahead; S, h, n_steps belong to the spin side
   Seg g;
-  uint64_t s_ncoll = 0, s_nbounce = 0;
-  int s_fail = 0;
-  bool s_stop = false, cur_fin = false, blocked = true;
-  int w = 0, wlast = 0, qhead = 0, qcount = 0;
-  double tf = 0.0, tempH = 0.0;
+  g.carry = false;
+  double Sx = 0.0, Sy = 0.0, Sz = 0.0, ph = 0.0, tempH = 0.0;
+  uint64_t n_steps = 0, s_ncoll = 0, s_nbounce = 0;
+  int s_fail = 0, turns = 0, w = 0, wlast = 0;
+  bool s_stop = false, s_slot = false, cur_fin = false, skip = false;
   unsigned long long n_dop = 0, n_rk = 0, n_ext = 0, n_seg = 0;
   unsigned int tick = 0, dry = 0;
   bool hit = false;
   const unsigned long long dl = run_deadline(a);
   const double nan = __longlong_as_double(0x7ff8000000000000ll);
-  TapeCursor tc;
-  tape_open(tc);
-  EventDefer dd;  // every field set: the warp's flush shuffles them from every lane
-#pragma unroll
-  for (int k = 0; k < 7; ++k) dd.x[k] = 0.0;
-  dd.wall = 'x';
-  dd.pending = false;
-  dd.gas = false;
-  dd.spare_first = false;
+  TapeCursor tcg, tcs;  // segment chain (trajectory side), step chain (spin side)
+  tape_open(tcg);
+  tape_open(tcs);
   while (true) {
-    // ---- A: spin-side boundaries of this lane (pop records, window ends, fetch)
-    bool starved = false;
+    // ================================================================ trajectory phase
+    {
+      PState tp;
+      tp.stop = false;
+      tp.fail = 0;
+      tp.Sx = tp.Sy = tp.Sz = tp.h = 0.0;
+      tp.turns = 0;
+      tp.n_coll = tp.n_bounce = tp.n_steps = 0;
+      traj_into(tp, slots[0]);
+      const SetParams* tP = a.sets;
+      double tf = 0.0;
+      if (t_run) {
+        tP = &a.sets[a.s.set[ti]];
+        tf = ((double)tw + 1.0) * tP->ioutInt;
+      }
+      EventDefer dd;  // every field set: the warp's flush shuffles them from every lane
+#pragma unroll
+      for (int k = 0; k < 7; ++k) dd.x[k] = 0.0;
+      dd.wall = 'x';
+      dd.pending = false;
+      dd.gas = false;
+      dd.spare_first = false;
 #pragma unroll 1
-    for (int guard = 0; guard < 8; ++guard) {
-      if (mode == B_FETCH) {
-        const unsigned long long item = atomicAdd(&a.status->queue_head, 1ull);
-        if (item >= (unsigned long long)a.nitems) {
-          mode = B_DONE;
-          break;
+      for (int round = 0; round < (1 << 20); ++round) {
+        // a finished window (or a stopped particle): its state into a slot, once the
+        // last reflection's velocity is known
+        if (t_wend && !dd.pending && wcount < kAheadSlots) {
+          int k = whead + wcount;
+          if (k >= kAheadSlots) k -= kAheadSlots;
+          slots[1 + k] = traj_of(tp);
+          ++wcount;
+          t_wend = false;
+          ++tw;
+          if (t_stop || tw >= twl) {
+            t_run = false;
+            if (TAPE) tape_close_segs(ta, tcg, ti);
+          } else {
+            tf = ((double)tw + 1.0) * tP->ioutInt;
+          }
+          t_stop = false;
         }
-        i = a.order ? a.order[item] : (int64_t)item;
-        P = &a.sets[a.s.set[i]];
-        w = a.s.w_done[i];
-        wlast = min(a.w_end, P->nwin);
-        if (TAPE) tape_resume(ta, tc, i);
-        dd.pending = false;
-        if (w >= wlast) {
-          if (TAPE) tape_close(ta, tc, i);
+        // the next particle
+        if (!t_run && !t_done && qcount < QCAP) {
+          const unsigned long long item = atomicAdd(&a.status->queue_head, 1ull);
+          if (item >= (unsigned long long)a.nitems) {
+            t_done = true;
+          } else {
+            ti = a.order ? a.order[item] : (int64_t)item;
+            tP = &a.sets[a.s.set[ti]];
+            tw = a.s.w_done[ti];
+            twl = min(a.w_end, tP->nwin);
+            if (TAPE) tape_resume_segs(ta, tcg, ti);
+            if (tw < twl) {
+              int k = qhead + qcount;
+              if (k >= QCAP) k -= QCAP;
+              ring[k].t0 = __longlong_as_double((long long)ti);
+              ring[k].flags = R_FETCH;
+              ++qcount;
+              tp = load_state(a.s, ti);
+              t_run = !tp.stop;  // a particle that stopped before: the spin side carries it to the end
+              tp.stop = false;
+              tp.fail = 0;
+              tf = ((double)tw + 1.0) * tP->ioutInt;
+            }
+            if (TAPE && !t_run) {
+              tape_close_segs(ta, tcg, ti);
+              if (tw >= twl) {  // nothing to run: its step chain as it was
+                TapeCursor same;
+                tape_resume_steps(ta, same, ti);
+                tape_close_steps(ta, same, ti);
+              }
+            }
+          }
+        }
+        const bool prod = t_run && !t_wend && !dd.pending && qcount < QCAP;
+        const unsigned pm = __ballot_sync(FULL, prod);
+        const unsigned defer_m = __ballot_sync(FULL, dd.pending);
+        const bool more = prod || (!t_run && !t_done && qcount < QCAP) || (t_wend && wcount < kAheadSlots);
+        const unsigned mm = __ballot_sync(FULL, more);
+        const bool leave = mm == 0u || (__popc(mm) < keep && !__any_sync(FULL, more && qcount == 0));
+        if (defer_m != 0u && (__popc(defer_m) >= defer_k || pm == 0u || leave)) {
+          deferred_events_warp<GAS>(tp, *tP, dd, defer_m, threadIdx.x & 31);
           continue;
         }
-        tp = load_state(a.s, i);
-        s_fail = tp.fail;
-        s_stop = tp.stop;
-        s_ncoll = tp.n_coll;
-        s_nbounce = tp.n_bounce;
-        qhead = qcount = 0;
-        tf = ((double)w + 1.0) * P->ioutInt;
-        tempH = tp.h;
-        blocked = s_stop;
-        mode = s_stop ? B_WEND : B_NEED;
-      } else if (mode == B_NEED) {
-        if (qcount == 0) {
-          starved = true;
-          break;
-        }
-        const int slot = qhead;
-        qhead = (qhead + 1 == QCAP) ? 0 : qhead + 1;
-        --qcount;
-        const double* r = qd + (size_t)slot * kRecF * BLOCK + tid;
-        const int flags = qf[slot * BLOCK + tid];
-        if (flags & 4) ++s_nbounce;
-        if (flags & 8) ++s_ncoll;
-        cur_fin = (flags & 1) != 0;
-        const int code = (int)(signed char)((flags >> 8) & 0xff);
-        if (code != 0) {
-          s_fail = code;
-          s_stop = true;
-        } else if (flags & 2) {
-          s_stop = true;  // diffuse hit on an edge or corner
-        }
-        if (s_stop) {
-          tp.Sx = tp.Sy = tp.Sz = nan;
-          tp.n_steps += 1;
-          mode = B_WEND;
-        } else if (spin_on<EXT>(P->integrator)) {
-          SegPoly q;
-          q.fx = (flags & 16) != 0;
-          if (q.fx) q.sc = unpack_scale(qs[slot * BLOCK + tid]);
-          q.o0[0] = r[2 * BLOCK]; q.o0[1] = r[3 * BLOCK]; q.o0[2] = r[4 * BLOCK];
-          q.o1[0] = r[5 * BLOCK]; q.o1[1] = r[6 * BLOCK]; q.o1[2] = r[7 * BLOCK];
-          seg_open(g, *P, q, r[0], r[1 * BLOCK]);
-#if !ST_GRAD_IS_LINEAR
-          g.p0x = r[8 * BLOCK]; g.p0y = r[9 * BLOCK]; g.p0z = r[10 * BLOCK];
-          g.v0x = r[11 * BLOCK]; g.v0y = r[12 * BLOCK]; g.v0z = r[13 * BLOCK];
-#endif
-          spin_begin<EXT>(g, *P, tp.Sx, tp.Sy, tp.Sz, tempH);
-          mode = B_SEG;
-          break;
-        } else {  // trajectory only: the segment completes at once
-          tp.n_steps += 1;
-          if (cur_fin) mode = B_WEND;
-        }
-      } else if (mode == B_WEND) {
-        // the window's last event reflected diffusely: its velocity is part of
-        // the state, computed in phase B first (one copy of that code)
-        if (dd.pending) break;
-        PState out = tp;
-        out.n_coll = s_ncoll;
-        out.n_bounce = s_nbounce;
-        out.fail = s_fail;
-        out.stop = s_stop;
-        if (s_stop) nan_fill(out);
-        write_snap(a, i, w, out);
-        ++w;
-        store_state(a.s, i, out);  // every window end is a resumable checkpoint
-        a.s.w_done[i] = w;
-        if (TAPE && ta.ckpt_every > 0 && w % ta.ckpt_every == 0 && w / ta.ckpt_every < ta.ckpt_count) {
-          const DeviceState ck = state_slot(ta.ckpt, ta.ckpt_stride, w / ta.ckpt_every);
-          store_state(ck, i, out);
-          ck.w_done[i] = w;
-        }
-        if (TAPE && w >= wlast) tape_close(ta, tc, i);
-        if (w < wlast) {
-          tf = ((double)w + 1.0) * P->ioutInt;
-          tempH = tp.h;
-          blocked = s_stop;
-          mode = s_stop ? B_WEND : B_NEED;
-        } else {
-          mode = B_FETCH;
-        }
-      } else {
-        break;  // B_SEG or B_DONE
-      }
-    }
-    // ---- B: warp-synchronous trajectory top-up
-    const unsigned starved_m = __ballot_sync(FULL, starved);
-    const unsigned defer_m = __ballot_sync(FULL, dd.pending);
-    if (defer_m != 0u &&
-        (__popc(defer_m) >= defer_k || __any_sync(FULL, dd.pending && (starved || qcount <= 1 || mode == B_WEND))))
-      deferred_events_warp<GAS>(tp, *P, dd, defer_m, tid & 31);
-    bool prod = (mode == B_NEED || mode == B_SEG) && !blocked && qcount < QCAP && !dd.pending;
-    unsigned pm = __ballot_sync(FULL, prod);
-    if (starved_m != 0u || __popc(pm) >= topup_start) {
-#pragma unroll 1
-      for (int round = 0; round < QCAP; ++round) {
+        if (leave) break;
         if (prod) {
-          int slot = qhead + qcount;
-          if (slot >= QCAP) slot -= QCAP;
-          produce_record<BLOCK, TAPE, GAS, EXT>(tp, *P, tf, qd, qs, qf, slot, tid, blocked, dd, ta, tc);
+          int k = qhead + qcount;
+          if (k >= QCAP) k -= QCAP;
+          const int flags = produce_record<TAPE, GAS, EXT>(tp, *tP, tf, ring + k, dd, ta, tcg);
           ++qcount;
           ++n_seg;
+          t_stop = (flags & R_STOP) != 0;
+          t_wend = t_stop || (flags & R_FIN) != 0;
         }
-        prod = (mode == B_NEED || mode == B_SEG) && !blocked && qcount < QCAP && !dd.pending;
-        pm = __ballot_sync(FULL, prod);
-        if (pm == 0u || __popc(pm) < topup_keep) break;
-      }
-      if (starved_m != 0u) {
-        // a starved lane always gets a record in the first top-up pass; this bound only
-        // protects the device from a logic error
-        if (++dry > 1000000u) {
+        if (((++tick) & 255u) == 0u && __any_sync(FULL, past_deadline(dl))) {
           hit = true;
-          atomicExch(&a.status->pad, 1);
           break;
         }
-        continue;
       }
+      slots[0] = traj_of(tp);
+      if (hit) break;
     }
-    dry = 0;
-    if (__all_sync(FULL, mode == B_DONE)) break;
-    // ---- C: one step attempt for every lane with an open segment
-    if (mode == B_SEG) {
-      int r;
-      if (P->integrator == 0) {
-        double y0x = tp.Sx, y0y = tp.Sy, y0z = tp.Sz;
-        if (TAPE && g.fx) dop_spin(g, y0x, y0y, y0z);
-        const double x0 = g.x;
-        r = dop_attempt_v(fx::Lane3(), ks, g, *P, tp.Sx, tp.Sy, tp.Sz);
-        ++n_dop;
-        if (TAPE && g.acc) tape_step(ta, tc, y0x, y0y, y0z, x0, g.hu);
-      } else if (!EXT || P->integrator == 1) {
-        r = rk45_attempt(g, *P, tp.Sx, tp.Sy, tp.Sz);
-        ++n_rk;
-      } else {
-        const double y0x = tp.Sx, y0y = tp.Sy, y0z = tp.Sz, x0 = g.x;
-        r = ext_attempt(g, *P, tp.Sx, tp.Sy, tp.Sz);
-        ++n_ext;
-        if (TAPE && g.acc) tape_step(ta, tc, y0x, y0y, y0z, x0, g.hu);
-      }
-      if (r != 0) {
-        tempH = g.h;
-        tp.turns += g.turns;
-        if (P->keep) tp.h = tempH;
-        if (r < 0) {
-          s_fail = r;
-          s_stop = true;
-          qcount = 0;  // records computed past the failure are dropped
-          blocked = true;
+    // ================================================================ spin phase
+    bool moved = false;
+#pragma unroll 1
+    while (true) {
+      // ---- boundaries of this lane: pop records, window ends, particles
+      bool starved = false;
+#pragma unroll 1
+      for (int guard = 0; guard < 8; ++guard) {
+        if (mode == B_NEED) {
+          if (qcount == 0) {
+            if (t_done && !t_run)
+              mode = B_DONE;
+            else
+              starved = true;
+            break;
+          }
+          const SegRec* r = ring + qhead;
+          qhead = (qhead + 1 == QCAP) ? 0 : qhead + 1;
+          --qcount;
+          moved = true;
+          const int flags = r->flags;
+          if (flags & R_FETCH) {
+            skip = false;
+            i = (int64_t)__double_as_longlong(r->t0);
+            P = &a.sets[a.s.set[i]];
+            w = a.s.w_done[i];
+            wlast = min(a.w_end, P->nwin);
+            Sx = a.s.Sx[i]; Sy = a.s.Sy[i]; Sz = a.s.Sz[i];
+            ph = tempH = a.s.h[i];
+            n_steps = a.s.n_steps[i];
+            s_ncoll = a.s.n_coll[i];
+            s_nbounce = a.s.n_bounce[i];
+            s_fail = a.s.fail[i];
+            turns = a.s.turns[i];
+            s_stop = a.s.stop[i] != 0;
+            s_slot = false;
+            if (TAPE) tape_resume_steps(ta, tcs, i);
+            if (s_stop) mode = B_WEND;
+            continue;
+          }
+          if (skip) {  // records past a stepper failure
+            if (flags & (R_FIN | R_STOP)) {
+              whead = (whead + 1 == kAheadSlots) ? 0 : whead + 1;
+              --wcount;
+            }
+            continue;
+          }
+          if (flags & R_WALL) ++s_nbounce;
+          if (flags & R_GAS) ++s_ncoll;
+          cur_fin = (flags & R_FIN) != 0;
+          const int code = (int)(signed char)((flags >> 8) & 0xff);
+          if (code != 0 || (flags & R_STOP)) {  // without a code: a diffuse hit on an edge or corner
+            if (code != 0) s_fail = code;
+            s_stop = s_slot = true;
+            Sx = Sy = Sz = nan;
+            g.carry = false;
+            n_steps += 1;
+            mode = B_WEND;
+          } else if (spin_on<EXT>(P->integrator)) {
+            SegPoly q;
+            q.fx = (flags & R_FX) != 0;
+            q.sc = unpack_scale(r->on, r->scale);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+              q.o0[c] = r->o0[c];
+              q.o1[c] = r->o1[c];
+              q.o2[c] = r->o2[c];
+            }
+            seg_open(g, *P, q, r->t0, r->t1);
+#if !ST_GRAD_IS_LINEAR
+            g.p0x = r->p0[0]; g.p0y = r->p0[1]; g.p0z = r->p0[2];
+            g.v0x = r->v0[0]; g.v0y = r->v0[1]; g.v0z = r->v0[2];
+#endif
+            spin_begin<EXT>(g, *P, Sx, Sy, Sz, tempH);
+            mode = B_SEG;
+            break;
+          } else {  // trajectory only: the segment completes at once
+            n_steps += 1;
+            if (cur_fin) {
+              s_slot = true;
+              mode = B_WEND;
+            }
+          }
+        } else if (mode == B_WEND) {
+          PState out;
+          if (s_slot) {
+            if (wcount == 0) {  // the trajectory side has not got round to it (slots were full)
+              starved = true;
+              break;
+            }
+            traj_into(out, slots[1 + whead]);
+            whead = (whead + 1 == kAheadSlots) ? 0 : whead + 1;
+            --wcount;
+          } else {
+            out = load_state(a.s, i);  // stopped: the trajectory fields stay (or become NaN)
+          }
+          spin_settle(g, Sx, Sy, Sz);
+          out.Sx = Sx; out.Sy = Sy; out.Sz = Sz;
+          out.h = ph;
+          out.turns = turns;
+          out.n_steps = n_steps;
+          out.n_coll = s_ncoll;
+          out.n_bounce = s_nbounce;
+          out.fail = s_fail;
+          out.stop = s_stop;
+          if (s_stop) nan_fill(out);
+          s_slot = false;
+          moved = true;
+          write_snap(a, i, w, out);
+          ++w;
+          store_state(a.s, i, out);  // every window end is a resumable checkpoint
+          a.s.w_done[i] = w;
+          if (TAPE && ta.ckpt_every > 0 && w % ta.ckpt_every == 0 && w / ta.ckpt_every < ta.ckpt_count) {
+            const DeviceState ck = state_slot(ta.ckpt, ta.ckpt_stride, w / ta.ckpt_every);
+            store_state(ck, i, out);
+            ck.w_done[i] = w;
+          }
+          if (TAPE && w >= wlast) tape_close_steps(ta, tcs, i);
+          tempH = ph;
+          mode = (w < wlast && s_stop) ? B_WEND : B_NEED;
+        } else {
+          break;  // B_SEG or B_DONE
         }
-        if (s_stop) tp.Sx = tp.Sy = tp.Sz = nan;
-        tp.n_steps += 1;
-        mode = (cur_fin || s_stop) ? B_WEND : B_NEED;
+      }
+      const unsigned seg_m = __ballot_sync(FULL, mode == B_SEG);
+      const unsigned starved_m = __ballot_sync(FULL, starved);
+      const unsigned busy_m = __ballot_sync(FULL, mode == B_NEED || mode == B_WEND);
+      if (starved_m != 0u && (__popc(starved_m) >= starve || seg_m == 0u)) break;
+      if (seg_m == 0u) {
+        if (busy_m == 0u) break;  // every lane done
+        continue;                 // lanes with more boundaries than one pass takes
+      }
+      moved = true;
+      // ---- one step attempt for every lane with an open segment
+      if (mode == B_SEG) {
+        int r;
+        if (P->integrator == 0) {
+          double y0x = Sx, y0y = Sy, y0z = Sz;
+          if (TAPE && g.fx) dop_spin(g, y0x, y0y, y0z);
+          const double x0 = g.x;
+          r = dop_attempt_v(fx::Lane3(), ks, g, *P, Sx, Sy, Sz);
+          ++n_dop;
+          if (TAPE && g.acc) tape_step(ta, tcs, y0x, y0y, y0z, x0, g.hu);
+        } else if (!EXT || P->integrator == 1) {
+          r = rk45_attempt(g, *P, Sx, Sy, Sz);
+          ++n_rk;
+        } else {
+          const double y0x = Sx, y0y = Sy, y0z = Sz, x0 = g.x;
+          r = ext_attempt(g, *P, Sx, Sy, Sz);
+          ++n_ext;
+          if (TAPE && g.acc) tape_step(ta, tcs, y0x, y0y, y0z, x0, g.hu);
+        }
+        if (r != 0) {
+          tempH = g.h;
+          turns += g.turns;
+          if (P->keep) ph = tempH;
+          if (r < 0) {
+            s_fail = r;
+            s_stop = true;
+            Sx = Sy = Sz = nan;
+            g.carry = false;
+            if (t_run && ti == i) {  // the trajectory side is still on this particle: it goes to the next
+              t_run = t_wend = t_stop = false;
+              qcount = wcount = 0;
+              if (TAPE) tape_close_segs(ta, tcg, i);
+            } else {
+              skip = true;
+              if (cur_fin) {
+                whead = (whead + 1 == kAheadSlots) ? 0 : whead + 1;
+                --wcount;
+              }
+            }
+          }
+          n_steps += 1;
+          s_slot = cur_fin && !s_stop;
+          mode = (cur_fin || s_stop) ? B_WEND : B_NEED;
+        }
+      }
+      if (((++tick) & 255u) == 0u && __any_sync(FULL, past_deadline(dl))) {
+        hit = true;
+        break;
       }
     }
-    if (((++tick) & 255u) == 0u && __any_sync(FULL, past_deadline(dl))) {
+    if (hit) break;
+    if (__all_sync(FULL, mode == B_DONE)) break;
+    // a starved lane always gets a record in the next trajectory phase; this bound only
+    // protects the device from a logic error
+    dry = __any_sync(FULL, moved) ? 0u : dry + 1u;
+    if (dry > 1000000u) {
       hit = true;
+      atomicExch(&a.status->pad, 1);
       break;
     }
   }
@@ -687,7 +874,7 @@ __global__ void __launch_bounds__(BLOCK, MINB)
 // ------------------------------------------------------------------ EXT instantiations
 // The adjoint's record pass: the trajectory-ahead kernel with its tape on, in
 // one configuration.
-constexpr int kTapeBlock = 128, kTapeQcap = 6;
+constexpr int kTapeBlock = 64, kTapeQcap = 64;
 
 // Defined in st_kernels_ext.cu: the kernel of persistent variant v with
 // integrator types 2-5, the record pass with them (gas-capable), and the plain

@@ -152,6 +152,12 @@ __device__ __forceinline__ float ex2f_approx(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
+// Leading bits of 1/x, relative error below 2^-20.
+__device__ __forceinline__ uint32_t rcp_hi(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  return (uint32_t)((unsigned long long)__double_as_longlong(r) >> 32);
+}
 __device__ __forceinline__ float rcpf_approx(float x) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -166,6 +172,11 @@ __device__ __forceinline__ i64 madw(int a, int b, i64 c) {
   asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
   return r;
 }
+__device__ __forceinline__ i64 mulw(int a, int b) {
+  i64 r;
+  asm("mul.wide.s32 %0, %1, %2;" : "=l"(r) : "r"(a), "r"(b));
+  return r;
+}
 __device__ __forceinline__ u64 f64_bits(double x) { return (u64)__double_as_longlong(x); }
 __device__ __forceinline__ double bits_f64(u64 b) { return __longlong_as_double((long long)b); }
 #else
@@ -174,6 +185,7 @@ inline float lg2f_approx(float x) { return log2f(x); }
 inline float ex2f_approx(float x) { return exp2f(x); }
 inline float rcpf_approx(float x) { return 1.0f / x; }
 inline i64 madw(int a, int b, i64 c) { return (i64)a * b + c; }
+inline i64 mulw(int a, int b) { return (i64)a * b; }
 inline uint32_t f32_bits(float x) {
   uint32_t b;
   __builtin_memcpy(&b, &x, 4);
@@ -194,6 +206,9 @@ inline double bits_f64(u64 b) {
   __builtin_memcpy(&x, &b, 8);
   return x;
 }
+// (for tests: seeds off by up to 1.5 x 2^-21)
+inline double seed_error(double x) { return 1.0 + ((int)(f64_bits(x) >> 20 & 3) - 1.5) * 0x1p-21; }
+inline uint32_t rcp_hi(double x) { return (uint32_t)(f64_bits(1.0 / x * seed_error(x)) >> 32); }
 #endif
 
 __device__ __forceinline__ i64 shl(i64 a, int k) { return (i64)((u64)a << k); }
@@ -238,14 +253,19 @@ __device__ __forceinline__ void mac(Acc& a, Limb x, Limb y) {
   a.mid = madw(x.h, y.l, a.mid);
   a.mid = madw(x.l, y.h, a.mid);
 }
+__device__ __forceinline__ Acc mac0(Limb x, Limb y, i64 mid = 0) {  // the first of a sum
+  Acc a;
+  a.hh = mulw(x.h, y.h);
+  a.mid = mid == 0 ? mulw(x.h, y.l) : madw(x.h, y.l, mid);
+  a.mid = madw(x.l, y.h, a.mid);
+  return a;
+}
 // Start value of `mid` that makes a following limb split round to nearest.
 constexpr i64 kHalfLimb = 1ll << 30;
 // The sum as Q63 times 2^k.
 __device__ __forceinline__ i64 q63(const Acc& a, int k = 0) { return shl(a.hh, 1 + k) + (a.mid >> (26 - k)); }
 __device__ __forceinline__ i64 mulq(Limb x, Limb y, int k = 0) {
-  Acc a{0, kHalfLimb};
-  mac(a, x, y);
-  return q63(a, k);
+  return q63(mac0(x, y, kHalfLimb), k);
 }
 // A tableau entry times 2^-p as limbs (folds to immediates).
 __device__ __forceinline__ constexpr Limb coef(double a, int p) {
@@ -260,6 +280,23 @@ __device__ __forceinline__ u64 umul(u64 a, u64 b) {
   return (u64)ah * bh + (((u64)ah * bl) >> 32) + (((u64)al * bh) >> 32);
 }
 
+constexpr u64 kFrac = 0x000fffffffffffffull, kOne = 0x0010000000000000ull;
+
+// 2^62 / b to a relative 2^-57 for b in [1/2, 1) as a 64-bit fraction (top bit set).
+__device__ __forceinline__ u64 recip(u64 b) {
+  // 1/x of the double with b's leading bits lies in (1, 2]: 31 bits, 2^30 = 1
+  const double x = bits_f64(((b >> 11) & kFrac) | 0x3fe0000000000000ull);
+  const uint32_t s = rcp_hi(x);
+  const uint32_t y0 = s >= 0x40000000u ? 0x7fffffffu : (s < 0x3ff00000u ? 0x40000000u : ((s & 0xfffffu) | 0x100000u) << 10);
+  // e = 1 - b y0 in units of 2^-62, |e| < 2^43; y1 = y0 + y0 e
+  const u64 t = (u64)(uint32_t)(b >> 32) * y0 + (((u64)(uint32_t)b * y0) >> 32);
+  const i64 e = (i64)(0x4000000000000000ull - t);
+  const u64 y1 = ((u64)y0 << 32) + (u64)(madw((int)y0, (int)(e >> 14), 0) >> 16);
+  // once more: |e| < 2^24 now
+  const i64 f = (i64)(0x4000000000000000ull - umul(b, y1));
+  return y1 + (u64)(madw((int)(y1 >> 32), (int)f, 0) >> 30);
+}
+
 // ---------------------------------------------------------------- lanes
 // All three spin components on one lane.
 struct Lane3 {
@@ -270,8 +307,7 @@ struct Lane3 {
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const int a = c == 2 ? 0 : c + 1, b = c == 0 ? 2 : c - 1;
-      k[c] = {0, kHalfLimb};
-      mac(k[c], y[a], w[b]);
+      k[c] = mac0(y[a], w[b], kHalfLimb);
       mac(k[c], y[b], n[a]);
     }
   }
@@ -308,6 +344,9 @@ struct StageSmem {
     xy[s * stride] = {k[0], k[1]};
     z[s * stride] = k[2];
   }
+  // a scratch array of 12 words over the same memory
+  __device__ __forceinline__ i64 word(int k) const { return *reinterpret_cast<const i64*>(&xy[k * stride]); }
+  __device__ __forceinline__ void set_word(int k, i64 v) { *reinterpret_cast<i64*>(&xy[k * stride]) = v; }
 };
 template <int N>
 struct StageLocal {
@@ -320,6 +359,8 @@ struct StageLocal {
 #pragma unroll
     for (int c = 0; c < N; ++c) v[s][c] = k[c];
   }
+  __device__ __forceinline__ i64 word(int k) const { return ((i64)v[k][0].h << 32) | (uint32_t)v[k][0].l; }
+  __device__ __forceinline__ void set_word(int k, i64 x) { v[k][0] = {(int)(x >> 32), (int)x}; }
 };
 
 // ---------------------------------------------------------------- pulse
@@ -419,7 +460,7 @@ __device__ __forceinline__ bool field_scale(const double o0[3], const double o1[
   if (!(T > 0.0)) return false;
   const int t = bexp(T) - 1021;  // T < 2^(te - 1)
   int e0 = bexp(ga), e1 = 0, e2 = 0;
-#pragma unroll
+#pragma unroll 1
   for (int c = 0; c < 3; ++c) {
     e0 = imax(e0, bexp(o0[c]));
     e1 = imax(e1, bexp(o1[c]));
@@ -433,7 +474,7 @@ __device__ __forceinline__ bool field_scale(const double o0[3], const double o1[
   if (e > 1900) return false;
   const int E = e - 1023 + 3;  // each term below 1/4, the sum of a component's below 1
   u64 n2 = 0;
-#pragma unroll
+#pragma unroll 1
   for (int c = 0; c < 3; ++c) {
     const u64 m = (u64)mag31(o0[c], E) + mag31(o1[c], E - t) + 2ull * mag31(o2[c], E - 2 * t) +
                   (c == 2 ? mag31(ga, E) : 0u) + 4u;  // units of 2^-31, rounded up
@@ -507,22 +548,20 @@ static __constant__ Limb kSumCoef[8][3] = {
     {coef(dop::B11, 4), coef(dop::B11, 4), coef(dop::ER11, 3)},
     {coef(dop::B12, 4), coef(dop::B12 - dop::BHH3, 4), coef(dop::ER12, 3)}};
 
-// y^(1/16) of y = b / (a 2^k) for a, b in (0, 1) as 64-bit fractions with a >= b
-// and k >= 0, in two factors 2^-j r / 2: Newton's iteration for r^16 a 2^i = b
-// (k = 16 j + i), the powers of two of i fed in between the squarings so that
-// every intermediate stays in [1/4, 1].  From a seed good to 2^-20 two steps
-// reach 2^-60.  Returns r / 2 as a 64-bit fraction.
+// (b / (a 2^i))^(1/16) / 2 as a 64-bit fraction, for fractions a >= b and 0 <= i < 16:
+// Newton's iteration for r^16 a 2^i = b, the powers of two of i fed in between the
+// squarings so that every intermediate stays in [1/4, 1].  From a seed good to
+// 2^-20 two steps reach 2^-60.
 __device__ __forceinline__ u64 root16(u64 a, u64 b, int i) {
   const float af = (float)(uint32_t)(a >> 32), bf = (float)(uint32_t)(b >> 32);
   const float lg = lg2f_approx(bf) - lg2f_approx(af) - (float)i;
   u64 r = (u64)(ex2f_approx(0.0625f * lg) * 0x1.fffff8p62f);
   const float ib = rcpf_approx(bf) * 0x1p-35f;  // 2 / (16 b), b in units of 2^-64
-#pragma unroll
+#pragma unroll 1
   for (int it = 0; it < 2; ++it) {
-    u64 v = umul(r, r) << 1 << ((i >> 3) & 1);  // half of r^2 2^b3
-    v = umul(v, v) << 1 << ((i >> 2) & 1);
-    v = umul(v, v) << 1 << ((i >> 1) & 1);
-    v = umul(v, v) << 1 << (i & 1);
+    u64 v = r;
+#pragma unroll 1
+    for (int q = 3; q >= 0; --q) v = umul(v, v) << 1 << ((i >> q) & 1);  // half of the square times a bit of 2^i
     const i64 d = (i64)((b >> 1) - umul(v, a));  // (b - r^16 2^i a) / 2
     const float f = (float)d * ib * (float)(uint32_t)(r >> 32);  // the correction of r / 2 in units of 2^-32
     r += (u64)(i64)(f * 0x1p32f);
@@ -540,7 +579,7 @@ __device__ __forceinline__ bool dop_step(const V& view, KS& ks, const SegScale& 
   using namespace dop;
   constexpr int N = V::N;
   // ---- the step in segment units
-  if (!(h > 0.0) || !(tx >= 0.0)) return false;
+  if ((i64)f64_bits(h) <= 0 || (i64)f64_bits(tx) < 0) return false;  // (a NaN is out of range below)
   const int eh = bexp(h) - 1021;  // h = hm 2^eh, hm in [1/4, 1/2)
   if (bexp(tx) - 1022 >= q.te || eh - 1 > q.te || bexp(h) < 64) return false;
   const i64 u = to_q63(tx, q.te);
@@ -565,7 +604,7 @@ __device__ __forceinline__ bool dop_step(const V& view, KS& ks, const SegScale& 
   for (int c = 0; c < N; ++c) {
     const Limb o2l = limb(o2[c]);
     const i64 t1 = mulq(ul, o2l);
-    w0[c] = mulq(hsl, limb(o0[c] + mulq(ul, limb(o1[c] + t1))), 1);
+    w0[c] = mulq(hsl, limb(o0[c] + mulq(ul, limb(o1[c] + t1))), -1);  // a quarter of it
     w1[c] = limb(mulq(g1l, limb(o1[c] + shl(t1, 1)), 1));
     w2[c] = limb(mulq(g2l, o2l, 1));
   }
@@ -581,6 +620,9 @@ __device__ __forceinline__ bool dop_step(const V& view, KS& ks, const SegScale& 
     phi0 = x < 0.0 ? 0ull - p : p;
   }
   // ---- stages: kappa_s = Y_s x omega_s, Y_s = S + 2^ez sum a_sj kappa_j
+  i64 Sr[N];
+#pragma unroll
+  for (int c = 0; c < N; ++c) Sr[c] = S[c] + 16;  // rounds the limb split
   unsigned bad = 0;  // set where a sum leaves the range in which nothing overflows
 #pragma unroll 1
   for (int s = 0; s < 12; ++s) {
@@ -588,20 +630,25 @@ __device__ __forceinline__ bool dop_step(const V& view, KS& ks, const SegScale& 
     Acc a[N];
 #pragma unroll
     for (int c = 0; c < N; ++c) a[c] = {0, 0};
-    Limb k[N];
+    // two terms a pass, each loaded one ahead (the last load unused, within the array)
+    Limb k[N], k2[N];
     ks.load(0, k);
-    int src = row.src;
+    int src = row.src, j = 0;
 #pragma unroll 1
-    for (int j = 0; j < row.n; ++j) {
-      const Limb f = kStageCoef[row.off + j];
-      Limb next[N];
-      ks.load(src, next);  // one ahead (the last one unused, within the array)
-      ++src;
+    for (; j + 1 < row.n; j += 2) {
+      const Limb f = kStageCoef[row.off + j], f2 = kStageCoef[row.off + j + 1];
+      ks.load(src, k2);
 #pragma unroll
-      for (int c = 0; c < N; ++c) {
-        mac(a[c], f, k[c]);
-        k[c] = next[c];
-      }
+      for (int c = 0; c < N; ++c) mac(a[c], f, k[c]);
+      ks.load(src + 1, k);
+      src += 2;
+#pragma unroll
+      for (int c = 0; c < N; ++c) mac(a[c], f2, k2[c]);
+    }
+    if (j < row.n) {
+      const Limb f = kStageCoef[row.off + j];
+#pragma unroll
+      for (int c = 0; c < N; ++c) mac(a[c], f, k[c]);
     }
     Limb Y[N], W[N];
 #pragma unroll
@@ -609,14 +656,16 @@ __device__ __forceinline__ bool dop_step(const V& view, KS& ks, const SegScale& 
       const int p = row.p;
       // |2 sum a kappa| < 1/2: neither the shift below nor Y can overflow
       bad |= ((unsigned)(int)(a[c].hh >> 32) + (1u << (28 - p))) & ~((1u << (29 - p)) - 1u);
-      Y[c] = limb(S[c] + (q63(a[c], 1 + p) >> r) + 16);
-      Acc o{0, 0};
-      mac(o, row.c, w1[c]);
+      Y[c] = limb(Sr[c] + (q63(a[c], 1 + p) >> r));
+      Acc o;
+      o.hh = madw(row.c.h, w1[c].h, w0[c]);
+      o.mid = madw(row.c.h, w1[c].l, kHalfLimb >> 1);
+      o.mid = madw(row.c.l, w1[c].h, o.mid);
       mac(o, row.c2, w2[c]);
-      i64 w = w0[c] + q63(o, 1);
+      i64 w = q63(o, 1);
       if (pulse && view.is_z(c))
         w += mulq(hgl, limb(half_cos_turns(phi0 + (u64)mulq(row.c, dphi, 1)) + 16), 1);
-      W[c] = limb(w + 16);
+      W[c] = limb(w);
     }
     view.cross(Y, W, a);
 #pragma unroll
@@ -631,16 +680,21 @@ __device__ __forceinline__ bool dop_step(const V& view, KS& ks, const SegScale& 
     Limb k[N];
     ks.load(0, k);
 #pragma unroll 1
-    for (int j = 0; j < 8; ++j) {
-      const Limb fb = kSumCoef[j][0], f3 = kSumCoef[j][1], f5 = kSumCoef[j][2];
-      Limb next[N];
-      ks.load(j < 7 ? 5 + j : 11, next);
+    for (int j = 0; j < 8; j += 2) {
+      Limb k2[N];
+      ks.load(5 + j, k2);
 #pragma unroll
       for (int c = 0; c < N; ++c) {
-        mac(sb[c], fb, k[c]);
-        mac(s3[c], f3, k[c]);
-        mac(s5[c], f5, k[c]);
-        k[c] = next[c];
+        mac(sb[c], kSumCoef[j][0], k[c]);
+        mac(s3[c], kSumCoef[j][1], k[c]);
+        mac(s5[c], kSumCoef[j][2], k[c]);
+      }
+      ks.load(j < 6 ? 6 + j : 11, k);
+#pragma unroll
+      for (int c = 0; c < N; ++c) {
+        mac(sb[c], kSumCoef[j + 1][0], k2[c]);
+        mac(s3[c], kSumCoef[j + 1][1], k2[c]);
+        mac(s5[c], kSumCoef[j + 1][2], k2[c]);
       }
     }
   }
@@ -656,40 +710,46 @@ __device__ __forceinline__ bool dop_step(const V& view, KS& ks, const SegScale& 
     big[c] = m0 > m1 ? m0 : m1;
   }
   if (view.any(bad != 0)) return false;
-  // ---- err^2 = 2^2(ez - sa) N5^2 / (3 rtol^2 D^2 (N5 + N3 / 100)) with
-  // G_c = |S_c| + atol / rtol in units of 2^(se + sa), D = Gx Gy Gz and
-  // N = sum (e_c D / G_c)^2: the weighted norms over their common denominator.
+  // ---- err^2 = 2^2(ez - sa) N5^2 / (3 rtol^2 (N5 + N3 / 100)), N = sum (e_c / G_c)^2 with
+  // G_c = |S_c| + atol / rtol in units of 2^(se + sa); one component after another in a
+  // rolled loop, their words in the stage array
   i64 E5[3], E3[3], Mx[3];
   view.gather(e5, E5);
   view.gather(e3, E3);
   view.gather(big, Mx);
   if (((u64)(Mx[0] | Mx[1] | Mx[2]) >> 62) != 0) return false;  // a spin twice its norm: a step far too long
-  const int be = bexp(tol.ratio);
-  int sa = be ? be - 1022 - q.se + 1 : 0;  // atol / rtol < 2^(se + sa - 1)
-  sa = sa < 0 ? 0 : sa;
-  const i64 ar = to_q63(tol.ratio, q.se + sa);
-  u64 Gx = (u64)((Mx[0] >> sa) + ar) << 1, Gy = (u64)((Mx[1] >> sa) + ar) << 1, Gz = (u64)((Mx[2] >> sa) + ar) << 1;
-  const u64 Px = umul(Gy, Gz), Py = umul(Gx, Gz), Pz = umul(Gx, Gy);
-  u64 D = umul(Pz, Gz);
-  u64 m5[3], m3[3];
+  u64 all5 = 0, all3 = 0;
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    m5[c] = (u64)(E5[c] < 0 ? -E5[c] : E5[c]);
-    m3[c] = (u64)(E3[c] < 0 ? -E3[c] : E3[c]);
+    const u64 m5 = (u64)(E5[c] < 0 ? -E5[c] : E5[c]), m3 = (u64)(E3[c] < 0 ? -E3[c] : E3[c]);
+    all5 |= m5;
+    all3 |= m3;
+    ks.set_word(c, (i64)m5);
+    ks.set_word(3 + c, (i64)m3);
+    ks.set_word(6 + c, Mx[c]);
   }
-  u64 all5 = m5[0] | m5[1] | m5[2];
-  const u64 all3 = m3[0] | m3[1] | m3[2];
+  const int be = bexp(tol.ratio);
+  int sa = be - 1021 - q.se;  // atol / rtol < 2^(se + sa - 1)
+  sa = sa < 0 ? 0 : sa;
+  const i64 ar = to_q63(tol.ratio, q.se + sa);
   out.accept = true;
   out.root8 = bits_f64(0x7ff0000000000000ull);
   if (all5 == 0) return true;
   const int l5 = clz64(all5), l3 = all3 ? clz64(all3) : 63;
-  auto sumsq = [&](const u64* m, int l) {
-    const u64 a = umul(m[0] << l, Px), b = umul(m[1] << l, Py), c = umul(m[2] << l, Pz);
-    return (umul(a, a) >> 1) + (umul(b, b) >> 1) + (umul(c, c) >> 1);  // halved against overflow
-  };
-  u64 n5 = sumsq(m5, l5);
-  const u64 n3 = umul(sumsq(m3, l3), 184467440737095516ull);  // N3 / 100
-  const int d2 = 2 * ((l5 - 3) - (l3 - 4));  // N3's block is 2^d2 of N5's
+  u64 n5 = 0, n3 = 0;
+#pragma unroll 1
+  for (int c = 0; c < 3; ++c) {
+    // 2^-8 / G, G in [2^-7, 1): 2^62 / (G 2^z) shifted by z
+    const u64 G = (u64)((ks.word(6 + c) >> sa) + ar) << 1;
+    const int z = clz64(G);
+    const u64 y = recip(G << z) >> (6 - z);
+    const u64 t5 = umul((u64)ks.word(c) << l5, y), t3 = umul((u64)ks.word(3 + c) << l3, y);
+    n5 += umul(t5, t5);
+    n3 += umul(t3, t3);
+  }
+  n3 = umul(n3, 184467440737095516ull);  // N3 / 100
+  // e5 = n 2^(1 - l5) 2^3, e3 = n 2^(1 - l3) 2^4, and 2^8 from 1 / G: the two blocks' scales
+  const int d2 = 2 * (l5 - l3 + 1);  // N3's block is 2^d2 of N5's
   u64 t;
   int et;  // N5 + N3 / 100 = t 2^(et - 64) in units of N5's block
   if (d2 >= 0) {
@@ -699,23 +759,22 @@ __device__ __forceinline__ bool dop_step(const V& view, KS& ks, const SegScale& 
     t = n5 + (d2 < -63 ? 0 : n3 >> -d2);
     et = 0;
   }
-  if (n5 == 0 || t == 0 || D == 0) return false;
-  const int z5 = clz64(n5), zt = clz64(t), zd = clz64(D);
+  if (n5 == 0 || t == 0) return false;
+  const int z5 = clz64(n5), zt = clz64(t);
   n5 <<= z5;
   t <<= zt;
   const u64 rb = f64_bits(tol.rtol);
-  const u64 rt = ((rb & 0x000fffffffffffffull) | 0x0010000000000000ull) << 11;  // rtol = rt 2^(bexp - 1022 - 64)
-  const u64 dr = umul(D << zd, rt);
-  const u64 A = umul(n5, n5);                                             // in [1/4, 1)
-  const u64 B = umul(umul(dr, dr), t);                                    // times 3 / 16: in [2^-8, 1/4)
+  const u64 rt = ((rb & kFrac) | kOne) << 11;  // rtol = rt 2^(bexp - 1022 - 64)
+  const u64 A = umul(n5, n5);                  // in [1/4, 1)
+  const u64 B = umul(umul(rt, rt), t);         // times 3 / 16: in [2^-7, 1/4)
   const u64 b = (B >> 3) + (B >> 4);
-  // (9 - 2 l5: the sum's halving, 2^3 of the row, Q63 against a 64-bit fraction, the normalising shift)
-  const int k = 2 * (ez - sa) - 2 * z5 - (et - zt) + 2 * zd - 2 * (bexp(tol.rtol) - 1022) + 9 - 2 * l5 - 4;
   // X = err^2 = 2^k A / b, A >= b
+  const int k = 2 * (ez - sa) + 24 - 2 * l5 - 2 * z5 - et + zt - 2 * (bexp(tol.rtol) - 1022) - 4;
   out.accept = k <= 0 && (k < -10 || (A >> -k) <= b);
   const int i = k & 15, j = k >> 4;  // k = 16 j + i
   const u64 rr = root16(A, b, i);
-  out.root8 = from_q63((i64)(rr >> 1), 1 - j);
+  const int zr = clz64(rr);  // rr / 2^64 = r / 2, to the nearest double
+  out.root8 = bits_f64(((u64)(1022 + 1 - zr - j) << 52) + ((rr << zr) >> 11) + (((rr << zr) >> 10) & 1) - kOne);
   return true;
 }
 

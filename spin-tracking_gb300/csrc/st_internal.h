@@ -17,6 +17,8 @@ constexpr double kC2 = 299792458.0 * 299792458.0;
 struct SetParams {
   // ---- trajectory (src/particle.cpp:121-444)
   double Lx, Ly, Lz;              // box edges
+  double hLx, hLy, hLz;           // half of them
+  double limx, limy, limz;        // the same plus 1e-15: the sanity check's limits
   double maxPosStep, tc, sqrtKT_m, diffuse, V;
   // ---- spin field (src/integrator.cpp:40-88)
   double gamma;
@@ -104,6 +106,8 @@ struct RunArgs {
   int any_gas;                    // some set has gas collisions (else gas-free kernels may run)
   int any_ext;                    // some set integrates with type 2-5 (the EXT kernels must run)
   int any_rk45;                   // some set integrates with RK45 (type 1)
+  char* ahead;                    // trajectory-ahead kernel: scratch of ahead_lane_bytes(ahead_q) per launched lane
+  int ahead_q;                    // its ring depth (records per lane)
 };
 
 // Discrete adjoint (st_adjoint.cu): gradient of L(S_final) with respect to
@@ -212,6 +216,10 @@ int persistent_prepare(int variant);
 int persistent_variant_block(int variant);
 // 0 flattened, 1 trajectory-ahead, 2 warp-specialised, 3 three lanes per particle
 int persistent_variant_family(int variant);
+// Ring depth of a trajectory-ahead variant (0: not one) and the scratch its launch needs.
+int persistent_variant_ring(int variant);
+size_t ahead_scratch_bytes(int ring, int64_t lanes);
+int tape_record_ring();
 const char* persistent_variant_name(int variant);
 
 }  // namespace st

@@ -189,41 +189,43 @@ int launch_pack_snapshot(const RunArgs& a, int slot, void* stream) {
 }
 
 // Persistent-kernel variants.  Family 0: the flattened kernel (k_persistent);
-// family 1: the trajectory-ahead kernel (k_batched) with its ring capacity
-// and top-up thresholds (start when this many lanes have room, keep filling
-// while this many still have room); family 2: the warp-specialised
+// family 1: the trajectory-ahead kernel (k_batched) with its ring depth, the
+// number of dry lanes that ends a spin phase and the number of lanes with room
+// that keeps a trajectory phase going; family 2: the warp-specialised
 // trajectory-ahead kernel (k_split, block = consumer warps + one producer
 // warp, ring capacity per particle; integrator types 0 and 1 only); family 3:
 // three lanes per particle (k_tpp3, the flattened loop shape; types 0 and 1,
 // the linear grad hook and the z cosine pulse).  Block threads and the minimum
 // resident blocks per SM set the register budget.
 struct Variant {
-  int family, block, minb, qcap, tstart, tkeep, defer, stages;
+  int family, block, minb, qcap, starve, keep, defer;
   const char* name;
   int cw, pw, creg, preg;  // family 2: consumer and producer warps, their register shares (0: no split)
 };
 static const Variant kVariants[] = {
-    {0, 128, 1, 0, 0, 0, 0, 0, "flat_b128_m1"},  {0, 128, 2, 0, 0, 0, 0, 0, "flat_b128_m2"},
-    {0, 128, 3, 0, 0, 0, 0, 0, "flat_b128_m3"},  {0, 64, 4, 0, 0, 0, 0, 0, "flat_b64_m4"},
-    {0, 256, 1, 0, 0, 0, 0, 0, "flat_b256_m1"},  {1, 128, 1, 6, 24, 16, 12, 0, "ahead_b128_q6_t24_d12"},
-    {1, 128, 1, 6, 16, 12, 12, 0, "ahead_b128_q6_t16_d12"}, {1, 128, 2, 4, 24, 16, 12, 0, "ahead_b128_q4_t24_d12"},
-    {1, 64, 2, 8, 24, 16, 12, 0, "ahead_b64_q8_t24_d12"},   {1, 64, 2, 8, 24, 16, 6, 0, "ahead_b64_q8_t24_d6"},
-    {1, 64, 2, 8, 24, 16, 18, 0, "ahead_b64_q8_t24_d18"},   {1, 64, 2, 8, 28, 20, 12, 0, "ahead_b64_q8_t28_d12"},
-    {1, 64, 2, 8, 28, 20, 12, 1, "ahead_b64_q8_t28_d12_ksmem"},
-    {1, 64, 5, 6, 28, 20, 12, 1, "ahead_b64_m5_q6_t28_d12_ksmem"},
-    {2, 128, 2, 8, 0, 0, 0, 0, "split_c3p1_q8", 3, 1, 0, 0},
-    {2, 256, 1, 8, 0, 0, 0, 0, "split_c6p2_q8", 6, 2, 0, 0},
-    {2, 384, 1, 8, 0, 0, 0, 0, "split_c8p4_q8_r184_136", 8, 4, 184, 136},
-    {3, 128, 2, 0, 0, 0, 0, 0, "tpp3_b128_m2"},    {3, 128, 3, 0, 0, 0, 0, 0, "tpp3_b128_m3"},
-    {1, 128, 1, 6, 16, 12, 16, 0, "ahead_b128_q6_t16_d16"}, {1, 64, 2, 8, 24, 16, 16, 0, "ahead_b64_q8_t24_d16"},
-    {1, 64, 2, 12, 24, 16, 12, 0, "ahead_b64_q12_t24_d12"}, {1, 64, 2, 12, 28, 20, 16, 0, "ahead_b64_q12_t28_d16"},
-    {1, 64, 2, 12, 20, 12, 12, 0, "ahead_b64_q12_t20_d12"}, {1, 64, 2, 12, 16, 8, 12, 0, "ahead_b64_q12_t16_d12"},
+    {0, 128, 1, 0, 0, 0, 0, "flat_b128_m1"}, {0, 128, 2, 0, 0, 0, 0, "flat_b128_m2"},
+    {0, 128, 3, 0, 0, 0, 0, "flat_b128_m3"}, {0, 64, 4, 0, 0, 0, 0, "flat_b64_m4"},
+    {0, 256, 1, 0, 0, 0, 0, "flat_b256_m1"}, {1, 64, 4, 64, 1, 8, 12, "ahead_b64_m4_q64_s1"},
+    {1, 64, 4, 64, 4, 8, 12, "ahead_b64_m4_q64_s4"}, {1, 64, 4, 128, 4, 8, 12, "ahead_b64_m4_q128_s4"},
+    {1, 64, 4, 32, 4, 8, 12, "ahead_b64_m4_q32_s4"}, {1, 64, 6, 64, 4, 8, 12, "ahead_b64_m6_q64_s4"},
+    {1, 64, 6, 64, 1, 8, 12, "ahead_b64_m6_q64_s1"}, {1, 64, 6, 64, 8, 8, 12, "ahead_b64_m6_q64_s8"},
+    {1, 64, 6, 128, 4, 8, 12, "ahead_b64_m6_q128_s4"}, {1, 64, 8, 64, 4, 8, 12, "ahead_b64_m8_q64_s4"},
+    {2, 128, 2, 8, 0, 0, 0, "split_c3p1_q8", 3, 1, 0, 0},
+    {2, 256, 1, 8, 0, 0, 0, "split_c6p2_q8", 6, 2, 0, 0},
+    {2, 384, 1, 8, 0, 0, 0, "split_c8p4_q8_r184_136", 8, 4, 184, 136},
+    {3, 128, 2, 0, 0, 0, 0, "tpp3_b128_m2"}, {3, 128, 3, 0, 0, 0, 0, "tpp3_b128_m3"},
+    {1, 256, 1, 64, 4, 8, 12, "ahead_b256_m1_q64_s4"}, {1, 64, 6, 32, 2, 8, 12, "ahead_b64_m6_q32_s2"},
 };
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 
 int persistent_variant_count() { return kNumVariants; }
 int persistent_variant_block(int v) { return (v >= 0 && v < kNumVariants) ? kVariants[v].block : 0; }
 int persistent_variant_family(int v) { return (v >= 0 && v < kNumVariants) ? kVariants[v].family : -1; }
+int persistent_variant_ring(int v) {
+  return (v >= 0 && v < kNumVariants && kVariants[v].family == 1) ? kVariants[v].qcap : 0;
+}
+size_t ahead_scratch_bytes(int ring, int64_t lanes) { return ring > 0 ? ahead_lane_bytes(ring) * (size_t)lanes : 0; }
+int tape_record_ring() { return kTapeQcap; }
 const char* persistent_variant_name(int v) { return (v >= 0 && v < kNumVariants) ? kVariants[v].name : "?"; }
 
 template <bool GAS>
@@ -234,12 +236,13 @@ static const void* variant_fn_g(int v) {
     case 2: return reinterpret_cast<const void*>(&k_persistent<128, 3, false>);
     case 3: return reinterpret_cast<const void*>(&k_persistent<64, 4, false>);
     case 4: return reinterpret_cast<const void*>(&k_persistent<256, 1, false>);
-    case 5:
-    case 6:
-    case 19: return reinterpret_cast<const void*>(&k_batched<128, 1, 6, false, GAS, false>);
-    case 7: return reinterpret_cast<const void*>(&k_batched<128, 2, 4, false, GAS, false>);
-    case 12: return reinterpret_cast<const void*>(&k_batched<64, 2, 8, false, GAS, false>);
-    case 13: return reinterpret_cast<const void*>(&k_batched<64, 5, 6, false, GAS, false>);
+    case 9:
+    case 10:
+    case 11:
+    case 12:
+    case 20: return reinterpret_cast<const void*>(&k_batched<64, 6, false, GAS, false>);
+    case 13: return reinterpret_cast<const void*>(&k_batched<64, 8, false, GAS, false>);
+    case 19: return reinterpret_cast<const void*>(&k_batched<256, 1, false, GAS, false>);
     case 14: return reinterpret_cast<const void*>(&k_split<3, 1, 2, 8, GAS, 0, 0>);
     case 15: return reinterpret_cast<const void*>(&k_split<6, 2, 1, 8, GAS, 0, 0>);
 #if ST_TRAJ_CORRECTLY_ROUNDED
@@ -254,11 +257,7 @@ static const void* variant_fn_g(int v) {
     case 17:
     case 18: return nullptr;  // the three-lane step assumes the default field hooks
 #endif
-    case 21:
-    case 22:
-    case 23:
-    case 24: return reinterpret_cast<const void*>(&k_batched<64, 2, 12, false, GAS, false>);
-    default: return reinterpret_cast<const void*>(&k_batched<64, 2, 8, false, GAS, false>);  // 8 to 11, 20
+    default: return reinterpret_cast<const void*>(&k_batched<64, 4, false, GAS, false>);  // 5 to 8
   }
 }
 // The kernel of variant v: with gas collisions or without, and with
@@ -270,12 +269,8 @@ static const void* variant_fn(int v, bool gas, int kind) {
   return gas ? variant_fn_g<true>(v) : variant_fn_g<false>(v);
 }
 
-// Rings (records, scales and flags), then the DOP853 stage derivatives (12
-// stages x 3 components x block).
-static size_t batched_smem(int block, int qcap) {
-  const size_t ring = (size_t)qcap * block * (kRecF * sizeof(double) + sizeof(int2)) + (size_t)(qcap * block + 3) / 4 * 16;
-  return ring + (size_t)12 * block * (sizeof(fx::Limb2) + sizeof(fx::Limb));
-}
+// The DOP853 stage derivatives (12 stages x 3 components x block).
+static size_t batched_smem(int block) { return (size_t)12 * block * (sizeof(fx::Limb2) + sizeof(fx::Limb)); }
 
 static int split_consumer_warps(int v) { return kVariants[v].cw; }
 
@@ -297,7 +292,7 @@ static size_t variant_smem(int v) {
   const Variant& x = kVariants[v];
   if (x.family == 0 || x.family == 3) return 0;
   if (x.family == 2) return split_smem_bytes(split_consumer_warps(v), x.qcap);
-  return batched_smem(x.block, x.qcap);
+  return batched_smem(x.block);
 }
 
 // Function attributes are set per device: remember which devices have them
@@ -352,7 +347,8 @@ int launch_persistent(const RunArgs& a, int v, int blocks, int block, void* stre
   cudaError_t e = ensure_smem(v, gas, kind);
   if (e != cudaSuccess) return (int)e;
   RunArgs args = a;
-  int t0 = x.tstart, t1 = x.tkeep, dk = x.defer;
+  int t0 = x.starve, t1 = x.keep, dk = x.defer;
+  if (x.family == 1) args.ahead_q = x.qcap;
   TapeArgs none{};
   void* params_flat[] = {&args};
   void* params_ahead[] = {&args, &t0, &t1, &dk, &none};
@@ -365,14 +361,13 @@ int launch_persistent(const RunArgs& a, int v, int blocks, int block, void* stre
 }
 
 // The record pass of the adjoint: the trajectory-ahead kernel with its tape on
-// (one configuration: kTapeBlock lanes, kTapeQcap-record rings, top-up at 24 /
-// 16 lanes); the EXT instantiation (st_kernels_ext.cu) records Magnus steps.
+// (one configuration: kTapeBlock lanes, kTapeQcap-record rings); the EXT instantiation (st_kernels_ext.cu) records Magnus steps.
 static const void* tape_fn(bool gas, bool ext) {
   if (ext) return tape_fn_ext();
-  return gas ? reinterpret_cast<const void*>(&k_batched<kTapeBlock, 1, kTapeQcap, true, true, false>)
-             : reinterpret_cast<const void*>(&k_batched<kTapeBlock, 1, kTapeQcap, true, false, false>);
+  return gas ? reinterpret_cast<const void*>(&k_batched<kTapeBlock, 4, true, true, false>)
+             : reinterpret_cast<const void*>(&k_batched<kTapeBlock, 4, true, false, false>);
 }
-static size_t tape_smem() { return batched_smem(kTapeBlock, kTapeQcap); }
+static size_t tape_smem() { return batched_smem(kTapeBlock); }
 
 static cudaError_t tape_ensure_smem(bool gas, bool ext) {
   static bool done[kAttrDevices][3] = {};
@@ -400,7 +395,8 @@ int launch_tape_record(const RunArgs& a, const TapeArgs& t, int blocks, void* st
   if (e != cudaSuccess) return (int)e;
   RunArgs args = a;
   TapeArgs tape = t;
-  int t0 = 24, t1 = 16, dk = 12;
+  int t0 = 4, t1 = 8, dk = 12;
+  args.ahead_q = kTapeQcap;
   void* params[] = {&args, &t0, &t1, &dk, &tape};
   return (int)cudaLaunchKernel(tape_fn(gas, ext), dim3(blocks), dim3(kTapeBlock), params, tape_smem(),
                                (cudaStream_t)stream);

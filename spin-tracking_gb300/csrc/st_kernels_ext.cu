@@ -16,22 +16,19 @@ const void* variant_fn_ext(int v) {
     case 2: return reinterpret_cast<const void*>(&k_persistent<128, 3, true>);
     case 3: return reinterpret_cast<const void*>(&k_persistent<64, 4, true>);
     case 4: return reinterpret_cast<const void*>(&k_persistent<256, 1, true>);
-    case 5:
-    case 6:
-    case 19: return reinterpret_cast<const void*>(&k_batched<128, 1, 6, false, true, true>);
-    case 7: return reinterpret_cast<const void*>(&k_batched<128, 2, 4, false, true, true>);
-    case 12: return reinterpret_cast<const void*>(&k_batched<64, 2, 8, false, true, true>);
-    case 13: return reinterpret_cast<const void*>(&k_batched<64, 5, 6, false, true, true>);
-    case 21:
-    case 22:
-    case 23:
-    case 24: return reinterpret_cast<const void*>(&k_batched<64, 2, 12, false, true, true>);
-    default: return reinterpret_cast<const void*>(&k_batched<64, 2, 8, false, true, true>);  // 8 to 11, 20
+    case 9:
+    case 10:
+    case 11:
+    case 12:
+    case 20: return reinterpret_cast<const void*>(&k_batched<64, 6, false, true, true>);
+    case 13: return reinterpret_cast<const void*>(&k_batched<64, 8, false, true, true>);
+    case 19: return reinterpret_cast<const void*>(&k_batched<256, 1, false, true, true>);
+    default: return reinterpret_cast<const void*>(&k_batched<64, 4, false, true, true>);  // 5 to 8
   }
 }
 
 const void* tape_fn_ext() {
-  return reinterpret_cast<const void*>(&k_batched<kTapeBlock, 1, kTapeQcap, true, true, true>);
+  return reinterpret_cast<const void*>(&k_batched<kTapeBlock, 4, true, true, true>);
 }
 
 template <int B>

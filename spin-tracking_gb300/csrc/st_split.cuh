@@ -52,6 +52,9 @@ enum { SD_T = 0, SD_PX, SD_PY, SD_PZ, SD_VX, SD_VY, SD_VZ, SD_NG, SD_SPARE, SD_T
 enum { SU_RX = 0, SU_RY, SU_RZ, SU_RW, SU_NCOLL, SU_NBOUNCE, SU_N };
 enum { SI_CTL = 0, SI_HEAD, SI_TAIL, SI_FAIL, SI_SET, SI_FLAGS, SI_N };
 
+// Record fields, field-major: t_start, t_end, o0, o1 (+ p0, v0 when the grad hook is not linear).
+constexpr int kRecF = ST_GRAD_IS_LINEAR ? 8 : 14;
+
 __host__ __device__ constexpr size_t split_smem_bytes(int cw, int qcap) {
   return (size_t)cw * 32 * (8 * ((size_t)qcap * kRecF + SD_N + SU_N) + 4 * ((size_t)qcap + SI_N));
 }
@@ -60,7 +63,7 @@ struct SplitSmem {
   double* qd;    // [q][field][slot] segment records
   double* sd;    // [field][slot] trajectory doubles
   uint64_t* su;  // [field][slot] RNG words and event counters
-  int* qf;       // [q][slot] record flags (as k_batched's)
+  int* qf;       // [q][slot] record flags (as SegRec::flags)
   int* si;       // [field][slot] control, head, tail, failure, set, packed flags
   int ns;        // slots of the block
 };
@@ -112,7 +115,7 @@ __device__ __forceinline__ void slot_load(const SplitSmem& m, int j, PState& p) 
 __device__ __forceinline__ int vload(const int* p) { return *reinterpret_cast<const volatile int*>(p); }
 __device__ __forceinline__ void vstore(int* p, int v) { *reinterpret_cast<volatile int*>(p) = v; }
 
-// One trajectory event of slot j into ring entry q (k_batched's record format).
+// One trajectory event of slot j into ring entry q (flags as SegRec::flags).
 template <bool GAS, bool EXT>
 __device__ __forceinline__ void split_produce(const SplitSmem& m, int j, int q, const SetParams& P, double tf) {
   PState tp;
@@ -221,6 +224,7 @@ __global__ void __launch_bounds__((CW + PW) * 32, MINB) k_split(RunArgs a) {
   const SetParams* P = a.sets;
   PState tp;  // the spin side's fields (S, h, n_steps, turns) and, at window ends, the slot's trajectory
   Seg g;
+  g.carry = false;
   uint64_t s_ncoll = 0, s_nbounce = 0;
   int s_fail = 0, head = 0;
   bool s_stop = false, cur_fin = false;
@@ -296,6 +300,7 @@ __global__ void __launch_bounds__((CW + PW) * 32, MINB) k_split(RunArgs a) {
         }
         if (s_stop) {
           tp.Sx = tp.Sy = tp.Sz = nan;
+          g.carry = false;
           tp.n_steps += 1;
           mode = B_WEND;
         } else if (spin_on<false>(P->integrator)) {
@@ -320,6 +325,7 @@ __global__ void __launch_bounds__((CW + PW) * 32, MINB) k_split(RunArgs a) {
       } else if (mode == B_WEND) {
         // the window's last record is in: the producer has parked the slot,
         // whose trajectory fields are the state at the window end
+        spin_settle(g, tp.Sx, tp.Sy, tp.Sz);
         PState out = tp;
         slot_load(m, j, out);
         out.Sx = tp.Sx; out.Sy = tp.Sy; out.Sz = tp.Sz;
@@ -382,7 +388,10 @@ __global__ void __launch_bounds__((CW + PW) * 32, MINB) k_split(RunArgs a) {
           s_stop = true;
           park = atomicCAS(&m.si[SI_CTL * NS + j], kSplitActive, kSplitStopReq) == kSplitActive;
         }
-        if (s_stop) tp.Sx = tp.Sy = tp.Sz = nan;
+        if (s_stop) {
+          tp.Sx = tp.Sy = tp.Sz = nan;
+          g.carry = false;
+        }
         tp.n_steps += 1;
         mode = park ? B_PARK : ((cur_fin || s_stop) ? B_WEND : B_NEED);
       }

@@ -55,6 +55,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tpp3(RunArgs a) {
   const SetParams* P = a.sets;
   PState p;
   Seg g;
+  g.carry = false;
   int w = 0, wlast = 0;
   double tf = 0.0, tempH = 0.0;
   bool finished = false, hit = false;
@@ -96,7 +97,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tpp3(RunArgs a) {
             mode = M_SEG;
           } else {
             if (p.fail == 0 && P->keep) p.h = tempH;
-            if (p.stop) nan_fill(p);
+            if (p.stop) {
+              nan_fill(p);
+              g.carry = false;
+            }
             p.n_steps += 1;
             mode = (finished || p.stop) ? M_WEND : M_EVENT;
           }
@@ -110,6 +114,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tpp3(RunArgs a) {
         }
       }
       if (mode == M_WEND) {
+        spin_settle(g, p.Sx, p.Sy, p.Sz);
         if (lead) {
           write_snap(a, i, w, p);
           store_state(a.s, i, p);  // every window end is a resumable checkpoint
@@ -147,7 +152,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tpp3(RunArgs a) {
         p.stop = true;
         p.fail = r;
       }
-      if (p.stop) nan_fill(p);
+      if (p.stop) {
+        nan_fill(p);
+        g.carry = false;
+      }
       p.n_steps += 1;
       mode = (finished || p.stop) ? M_WEND : M_EVENT;
     }
