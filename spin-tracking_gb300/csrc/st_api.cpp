@@ -880,10 +880,8 @@ int st_gather_spins(st_ctx* c, double* dst) {
   if (!c || !dst) return fail(ST_ERR_ARG, "null argument");
   ST_CUDA(cudaSetDevice(c->device));
   if (c->n == 0) return ST_OK;
-  const double* src[3] = {c->s.Sx, c->s.Sy, c->s.Sz};
-  for (int k = 0; k < 3; ++k)
-    ST_CUDA(cudaMemcpy2DAsync(dst + k, 3 * sizeof(double), src[k], sizeof(double), sizeof(double), (size_t)c->n,
-                              cudaMemcpyDeviceToDevice, c->stream));
+  if (int e = st::launch_gather_spins(c->s.Sx, c->s.Sy, c->s.Sz, c->n, dst, c->stream))
+    return fail(ST_ERR_CUDA, std::string("spin gather launch: ") + cudaGetErrorString((cudaError_t)e));
   ST_CUDA(cudaStreamSynchronize(c->stream));
   return ST_OK;
 }
@@ -1498,13 +1496,17 @@ int st_ensemble_stats(st_ctx* c, const void* snap, int set, st_ensemble* out) {
   if (set < 0 || set >= (int)c->sets_h.size()) return fail(ST_ERR_ARG, "no such parameter set");
   ST_CUDA(cudaSetDevice(c->device));
   const size_t ctl_b = 256, part_b = sizeof(double) * 8 * st::kEnsMaxBlocks;
-  if (!c->ens_buf) {
-    cudaError_t e = cudaMalloc(&c->ens_buf, ctl_b + part_b + sizeof(unsigned int) * st::kEnsHistBins);
+  const size_t hist_b = align256(sizeof(unsigned int) * (st::kEnsHistBins + st::kEnsPasses));
+  if (!c->ens_buf) {  // the phases of the largest set follow
+    int64_t most = 1;
+    for (const auto& q : c->sets_h) most = std::max(most, q.n);
+    cudaError_t e = cudaMalloc(&c->ens_buf, ctl_b + part_b + hist_b + sizeof(double) * (size_t)most);
     if (e != cudaSuccess) return fail(ST_ERR_NOMEM, std::string("ensemble scratch: ") + cudaGetErrorString(e));
   }
   double* ctl = (double*)c->ens_buf;
   double* part = (double*)((char*)c->ens_buf + ctl_b);
   unsigned int* hist = (unsigned int*)((char*)c->ens_buf + ctl_b + part_b);
+  double* phis = (double*)((char*)hist + hist_b);
   const double *t, *sx, *sy, *sz;
   const int32_t *fl, *tn;
   if (snap) {
@@ -1524,7 +1526,7 @@ int st_ensemble_stats(st_ctx* c, const void* snap, int set, st_ensemble* out) {
     tn = c->s.turns;
   }
   const SetParams& P = c->sets_h[(size_t)set];
-  int e = st::ensemble_device(t, sx, sy, sz, fl, tn, P.first, P.n, ctl, part, hist, st::kEnsMaxBlocks, c->stream);
+  int e = st::ensemble_device(t, sx, sy, sz, fl, tn, P.first, P.n, ctl, part, hist, phis, st::kEnsMaxBlocks, c->stream);
   if (e) return fail(ST_ERR_CUDA, std::string("ensemble launch: ") + cudaGetErrorString((cudaError_t)e));
   double h[32];
   ST_CUDA(cudaMemcpyAsync(h, ctl, sizeof(double) * st::ensemble_ctl_count(), cudaMemcpyDeviceToHost, c->stream));

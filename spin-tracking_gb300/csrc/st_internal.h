@@ -165,12 +165,14 @@ int adj_backward_max_blocks_per_sm(int magnus);
 // Ensemble statistics (st_ensemble.cu).
 int ensemble_device(const double* t, const double* Sx, const double* Sy, const double* Sz, const int32_t* fail,
                     const int32_t* turns, int64_t first, int64_t n, double* ctl, double* part, unsigned int* hist,
-                    int max_blocks, void* stream);
+                    double* phis, int max_blocks, void* stream);
 int ensemble_ctl_count();
-constexpr int kEnsMaxBlocks = 1024, kEnsHistBins = 1000;
+constexpr int kEnsMaxBlocks = 1024, kEnsHistBins = 1000, kEnsPasses = 6;
 enum { ENS_COUNT = 0, ENS_SX, ENS_SY, ENS_SZ, ENS_MIN, ENS_MAX, ENS_T, ENS_EDGE0, ENS_EDGE1, ENS_LOC, ENS_MEAN1,
        ENS_STD1, ENS_MEAN2, ENS_STD2, ENS_KEPT, ENS_UMEAN, ENS_USTD };
 // Unwrapped precession phase atan2(Sz, Sy) + 2 pi turns of n particles into dst.
+// Spins of n particles, three doubles each, into dst.
+int launch_gather_spins(const double* Sx, const double* Sy, const double* Sz, int64_t n, double* dst, void* stream);
 int launch_gather_phase(const double* Sy, const double* Sz, const int32_t* turns, int64_t n, double* dst,
                         void* stream);
 
