@@ -188,6 +188,7 @@ struct st_ctx {
   // integratorType 6 (every set of the context): the noise-spectrum aggregators
   bool spectrum = false;
   st::SpecSet* spec_sets_d = nullptr;
+  double* spec_tmp = nullptr;
   void* spec_pp = nullptr;        // s1, s2, im (17 x 3 per particle each), samples per particle
   st::SpecArgs spec{};
   // adjoint (allocated by st_adjoint_record)
@@ -289,6 +290,10 @@ int ctx_alloc(st_ctx* c) {
                             c->stream));
     const size_t acc = align256(sizeof(double) * 3 * st::kSpecFreqs * m);
     ST_CUDA(cudaMalloc(&c->spec_pp, 3 * acc + align256(8 * m)));
+    // one aggregator array per particle on its way to the host; the covariance sum's few values
+    ST_CUDA(cudaMalloc(&c->spec_tmp, std::max<size_t>(acc, sizeof(double) * 512)));
+    if (int e = st::spectrum_prepare())
+      return fail(ST_ERR_CUDA, std::string("spectrum kernel attributes: ") + cudaGetErrorString((cudaError_t)e));
     ST_CUDA(cudaMemsetAsync(c->spec_pp, 0, 3 * acc + align256(8 * m), c->stream));
     char* b = (char*)c->spec_pp;
     c->spec.sets = c->spec_sets_d;
@@ -708,6 +713,7 @@ void st_destroy(st_ctx* c) {
   cudaFree(c->ens_buf);
   cudaFree(c->spec_sets_d);
   cudaFree(c->spec_pp);
+  cudaFree(c->spec_tmp);
   cudaFree(c->adj_lam_buf);
   cudaFree(c->tape_pool);
   cudaFree(c->tape_prev);
@@ -1577,14 +1583,12 @@ int st_spectrum_state(st_ctx* c, double* s1, double* s2, double* imag, int64_t* 
   const size_t n = (size_t)c->n, f3 = 3 * (size_t)st::kSpecFreqs;
   if (n == 0) return ST_OK;
   // device arrays are field-major ([(k * 3 + c) * n + i]); the caller's are per particle ([i][k][c])
-  std::vector<double> buf(f3 * n);
   double* dst[3] = {s1, s2, imag};
   const double* src[3] = {c->spec.s1, c->spec.s2, c->spec.im};
   for (int a = 0; a < 3; ++a) {
-    ST_CUDA(cudaMemcpyAsync(buf.data(), src[a], sizeof(double) * f3 * n, cudaMemcpyDeviceToHost, c->stream));
-    ST_CUDA(cudaStreamSynchronize(c->stream));
-    for (size_t i = 0; i < n; ++i)
-      for (size_t j = 0; j < f3; ++j) dst[a][i * f3 + j] = buf[j * n + i];
+    if (int e = st::launch_spec_gather(src[a], c->spec_tmp, c->n, c->stream))
+      return fail(ST_ERR_CUDA, std::string("spectrum gather: ") + cudaGetErrorString((cudaError_t)e));
+    ST_CUDA(cudaMemcpyAsync(dst[a], c->spec_tmp, sizeof(double) * f3 * n, cudaMemcpyDeviceToHost, c->stream));
   }
   ST_CUDA(cudaMemcpyAsync(n_samples, c->spec.nsamp, 8 * n, cudaMemcpyDeviceToHost, c->stream));
   ST_CUDA(cudaStreamSynchronize(c->stream));
@@ -1595,38 +1599,26 @@ int st_covariance_spectrum(st_ctx* c, int set, double* variance, int64_t* n_samp
   if (!c || !variance || !n_samples) return fail(ST_ERR_ARG, "null argument");
   if (!c->spectrum) return fail(ST_ERR_STATE, "st_covariance_spectrum: the context's sets are not integratorType 6");
   if (set < 0 || set >= (int)c->sets_h.size()) return fail(ST_ERR_ARG, "no such parameter set");
-  const size_t n = (size_t)c->n, F = st::kSpecFreqs;
-  std::vector<double> s1(3 * F * n), s2(3 * F * n), im(3 * F * n);
-  std::vector<int64_t> ns(std::max<size_t>(n, 1));
-  ST_TRY(st_spectrum_state(c, s1.data(), s2.data(), im.data(), ns.data()));
+  ST_CUDA(cudaSetDevice(c->device));
   double fr[st::kSpecFreqs], dt = 0.0;
   if (st::floquet_frequencies(c->opts[(size_t)set], fr, &dt) != 0) return fail(ST_ERR_ARG, "no Floquet period");
-  std::memset(variance, 0, sizeof(double) * F * 18);
-  int64_t total = 0;
-  const int64_t lo = c->sets_h[(size_t)set].first, hi = lo + c->sets_h[(size_t)set].n;
-  for (int64_t i = lo; i < hi; ++i) {  // particle order, so the sum does not depend on the launch
-    if (c->opts[(size_t)set].numParticles == 0) break;
-    total += ns[(size_t)i];
-    for (size_t k = 0; k < F; ++k) {
-      // goertzel_stage_2 (src/floquet.cpp:40-47): c = a + i b, variance = c c^dag,
-      // a = s1 - cos(w dt) s2, b = sin(w dt) s2; then the Laplace term on the
-      // diagonal (SpectrumAggregator::get_covariance_spectrum, :130-145)
-      const double angle = fr[k] * dt, ca = cos(angle), sa = sin(angle);
-      double re[3], imc[3];
-      for (int q = 0; q < 3; ++q) {
-        const double x1 = s1[((size_t)i * F + k) * 3 + q], x2 = s2[((size_t)i * F + k) * 3 + q];
-        re[q] = x1 - ca * x2;
-        imc[q] = sa * x2;
-      }
-      double* m = variance + k * 18;
-      for (int r = 0; r < 3; ++r)
-        for (int q = 0; q < 3; ++q) {  // c_r conj(c_q)
-          m[(r * 3 + q) * 2 + 0] += re[r] * re[q] + imc[r] * imc[q];
-          m[(r * 3 + q) * 2 + 1] += imc[r] * re[q] - re[r] * imc[q];
-        }
-      for (int r = 0; r < 3; ++r) m[(r * 3 + r) * 2 + 1] += -im[((size_t)i * F + k) * 3 + r];
-    }
+  const int64_t first = c->sets_h[(size_t)set].first, cnt = c->sets_h[(size_t)set].n;
+  // the scratch's head: cos and sin of every frequency's phase per sample, then the result
+  double cs[2 * st::kSpecFreqs];
+  for (int k = 0; k < st::kSpecFreqs; ++k) {
+    cs[2 * k] = cos(fr[k] * dt);
+    cs[2 * k + 1] = sin(fr[k] * dt);
   }
+  double* out = c->spec_tmp + 64;
+  ST_CUDA(cudaMemcpyAsync(c->spec_tmp, cs, sizeof(cs), cudaMemcpyHostToDevice, c->stream));
+  if (int e = st::launch_covariance(c->spec, c->n, first, cnt, c->spec_tmp, out, c->stream))
+    return fail(ST_ERR_CUDA, std::string("covariance: ") + cudaGetErrorString((cudaError_t)e));
+  std::vector<int64_t> ns((size_t)std::max<int64_t>(cnt, 1), 0);
+  ST_CUDA(cudaMemcpyAsync(variance, out, sizeof(double) * st::kSpecFreqs * 18, cudaMemcpyDeviceToHost, c->stream));
+  ST_CUDA(cudaMemcpyAsync(ns.data(), c->spec.nsamp + first, 8 * (size_t)cnt, cudaMemcpyDeviceToHost, c->stream));
+  ST_CUDA(cudaStreamSynchronize(c->stream));
+  int64_t total = 0;
+  for (int64_t x : ns) total += x;
   *n_samples = total;
   return ST_OK;
 }

@@ -182,7 +182,8 @@ int launch_gather_phase(const double* Sy, const double* Sz, const int32_t* turns
 // host), dt, and the test-noise amplitudes and frequencies; per particle, the
 // aggregators of the last window, field-major: s1[(k * 3 + c) * n + i].
 constexpr int kSpecFreqs = 17;
-constexpr int kSpecBlock = 128;  // four particles (warps) per block
+constexpr int kSpecBlock = 64;   // two warps per block
+constexpr int kSpecGroup = 8;    // particles per warp
 struct SpecSet {
   double freq[kSpecFreqs], two_cos[kSpecFreqs], sin_a[kSpecFreqs];
   double fdt;
@@ -197,6 +198,10 @@ struct SpecArgs {
 int floquet_frequencies(const st_options& o, double freq[kSpecFreqs], double* dt);
 int build_spec_set(const st_options& o, SpecSet* q);
 int launch_spectrum(const RunArgs& a, int window, double next_t, const SpecArgs& sp, void* stream);
+int spectrum_prepare();
+int launch_spec_gather(const double* src, double* dst, int64_t n, void* stream);
+int launch_covariance(const SpecArgs& sp, int64_t n, int64_t first, int64_t n_set, const double* cos_sin, double* out,
+                      void* stream);
 
 // Host-side launch helpers implemented in st_kernels.cu.  Return a cudaError_t
 // cast to int (0 = success).
