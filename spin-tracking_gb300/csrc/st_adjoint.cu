@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(kAdjBlock) k_adj_backward(RunArgs a, TapeArgs 
   const unsigned FULL = 0xffffffffu;
   const bool pulse = t.pulse_grads != 0;
   const int64_t pages = t.pool_pages;
-  bool active = false, done = false;
+  bool active = false, done = (int)(threadIdx.x & 31) >= a.spread;
   int64_t i = 0;
   const SetParams* P = a.sets;
   Seg g;

@@ -382,6 +382,7 @@ st::RunArgs make_args(st_ctx* c, int w_begin, int w_end, void* snap) {
   a.any_gas = 0;
   a.any_ext = ctx_any_ext(c) ? 1 : 0;
   a.any_rk45 = ctx_any_rk45(c) ? 1 : 0;
+  a.spread = st::spread_lanes(c->n, c->sm_count);
   a.ahead = c->ahead;
   a.ahead_q = 0;
   for (const auto& P : c->sets_h) a.any_gas |= P.gas ? 1 : 0;
@@ -429,12 +430,12 @@ int arm_deadline(st_ctx* c, st::RunArgs& a) {
 // fastest.
 int autotune(st_ctx* c);
 
-// Blocks of a persistent launch: the resident ones, no more than the work items fill.
-int persistent_blocks(const st_ctx* c, int variant, int per_sm) {
-  const int64_t block = std::max(1, st::persistent_variant_block(variant));
-  const int64_t lanes_per_item = st::persistent_variant_family(variant) == 3 ? 4 : 1;  // three of every 3.2 lanes
-  const int64_t need = (c->n * lanes_per_item + block - 1) / block;
-  return (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)c->sm_count * per_sm, need));
+// Blocks of a persistent launch for n work items: the resident ones, no more than the items
+// fill at `spread` lanes per warp (three lanes per particle: ten particles per warp).
+int persistent_blocks(int64_t n, int sm_count, int variant, int per_sm) {
+  const int64_t warps = std::max(1, st::persistent_variant_block(variant) / 32);
+  const int64_t per_block = warps * (st::persistent_variant_family(variant) == 3 ? 10 : st::spread_lanes(n, sm_count));
+  return (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)sm_count * per_sm, (n + per_block - 1) / per_block));
 }
 
 // Scratch of the trajectory-ahead kernel (its lanes' rings), kept with the context.  A larger one takes the place of the old: run graphs that hold its
@@ -456,8 +457,8 @@ int ensure_ahead(st_ctx* c, size_t need) {
 // at its highest occupancy, so that a change of configuration keeps the graphs.
 int ensure_ahead_variant(st_ctx* c) {
   auto bytes = [&](int v, int per_sm) {
-    return st::ahead_scratch_bytes(st::persistent_variant_ring(v),
-                                   (int64_t)persistent_blocks(c, v, per_sm) * st::persistent_variant_block(v));
+    const int64_t warps = (int64_t)persistent_blocks(c->n, c->sm_count, v, per_sm) * st::persistent_variant_block(v) / 32;
+    return st::ahead_scratch_bytes(st::persistent_variant_ring(v), warps * st::spread_lanes(c->n, c->sm_count));
   };
   size_t need = bytes(c->lc.variant, c->lc.blocks_per_sm);
   if (need <= c->ahead_bytes) return ST_OK;
@@ -473,7 +474,7 @@ int run_persistent(st_ctx* c, int w_begin, int w_end, void* snap) {
   ST_TRY(ensure_ahead_variant(c));
   st::RunArgs a = make_args(c, w_begin, w_end, snap);
   ST_TRY(arm_deadline(c, a));
-  const int blocks = persistent_blocks(c, c->lc.variant, c->lc.blocks_per_sm);
+  const int blocks = persistent_blocks(c->n, c->sm_count, c->lc.variant, c->lc.blocks_per_sm);
   int e = st::launch_persistent(a, c->lc.variant, blocks, c->lc.block_threads, c->stream);
   if (e) return fail(ST_ERR_CUDA, std::string("persistent launch: ") + cudaGetErrorString((cudaError_t)e));
   return ST_OK;
@@ -1079,10 +1080,12 @@ int adj_reset_replay_tape(st_ctx* c) { return adj_reset_tape(c, c->tape); }
 
 int adj_tape_launch(st_ctx* c, const st::RunArgs& a, const st::TapeArgs& t) {
   const int per_sm = std::max(1, st::tape_record_max_blocks_per_sm(ctx_any_ext(c) ? 1 : 0));
-  const int64_t block = st::tape_record_block();
-  const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)c->sm_count * per_sm, (a.nitems + block - 1) / block));
-  ST_TRY(ensure_ahead(c, st::ahead_scratch_bytes(st::tape_record_ring(), blocks * block)));
   st::RunArgs r = a;
+  r.spread = st::spread_lanes(a.nitems, c->sm_count);
+  const int64_t per_block = st::tape_record_block() / 32 * (int64_t)r.spread;
+  const int blocks =
+      (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)c->sm_count * per_sm, (a.nitems + per_block - 1) / per_block));
+  ST_TRY(ensure_ahead(c, st::ahead_scratch_bytes(st::tape_record_ring(), blocks * per_block)));
   r.ahead = c->ahead;
   int e = st::launch_tape_record(r, t, blocks, c->stream);
   if (e) return fail(ST_ERR_CUDA, std::string("adjoint tape launch: ") + cudaGetErrorString((cudaError_t)e));
@@ -1093,7 +1096,12 @@ int adj_backward_launch(st_ctx* c, const st::RunArgs& a, const st::TapeArgs& t) 
   ST_CUDA(cudaMemsetAsync(c->status_d, 0, sizeof(st::RunStatus), c->stream));
   const int magnus = ctx_any_ext(c) ? 1 : 0;  // the record pass admits types 0 or 2, one per context
   const int per_sm = std::max(1, st::adj_backward_max_blocks_per_sm(magnus));
-  int e = st::launch_adj_backward(a, t, c->sm_count * per_sm, magnus, c->stream);
+  st::RunArgs r = a;
+  r.spread = st::spread_lanes(a.nitems, c->sm_count);
+  const int64_t per_block = st::adj_backward_block() / 32 * (int64_t)r.spread;
+  const int blocks =
+      (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)c->sm_count * per_sm, (a.nitems + per_block - 1) / per_block));
+  int e = st::launch_adj_backward(r, t, blocks, magnus, c->stream);
   if (e) return fail(ST_ERR_CUDA, std::string("adjoint backward launch: ") + cudaGetErrorString((cudaError_t)e));
   long long rep[st::kTapeErrorSlots] = {};
   ST_CUDA(cudaMemcpyAsync(rep, c->tape_error, sizeof(rep), cudaMemcpyDeviceToHost, c->stream));
@@ -1871,10 +1879,14 @@ int autotune(st_ctx* c) {
   // the variant): on every workload measured, fewer resident blocks lost.
   for (int v = 0; v < nv; ++v) {
     if (st::persistent_max_blocks_per_sm(v, ext) <= 0) continue;  // not built for this kind of run
-    // The warp-specialised and three-lane variants were slower on every
-    // workload measured, and a short sample can favour them: only an explicit
-    // st_set_launch_config selects them.
-    if (st::persistent_variant_family(v) >= 2) continue;
+    // The warp-specialised variants hide the trajectory behind the spin where a
+    // run is as long as its slowest particle: 1,000 particles x 0.5 s without
+    // gas, 46.6 ms against 55.8; at 20,000 they lose, 10.7 against 7.6.  They are
+    // candidates while the particles do not fill two warps per SM, the sample
+    // is then the run itself.  The three-lane variants were slower on every
+    // workload measured: only an explicit st_set_launch_config selects them.
+    const int family = st::persistent_variant_family(v);
+    if (family == 3 || (family == 2 && st::spread_lanes(s->n, s->sm_count) == 32)) continue;
     const int maxb = std::max(1, st::persistent_max_blocks_per_sm(v, ext));
     {
       st_launch_config cfg{0, maxb, v};

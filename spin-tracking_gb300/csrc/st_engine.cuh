@@ -146,11 +146,12 @@ __device__ __forceinline__ bool window_nested(PState& p, const SetParams& P, dou
 // EXT: also integrator types 2-5.
 template <int BLOCK, bool EXT>
 __global__ void __launch_bounds__(BLOCK) k_plain(RunArgs a, int window, double next_t) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const int64_t i = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * a.spread + lane;
   unsigned long long n_dop = 0, n_rk = 0, n_ext = 0, n_seg = 0;
   bool hit = false;
   const unsigned long long dl = run_deadline(a);
-  if (i < a.s.n) {
+  if (lane < a.spread && i < a.s.n) {
     const SetParams& P = a.sets[a.s.set[i]];
     double tf = next_t;
     bool run = true;
@@ -182,7 +183,7 @@ enum LaneMode { M_FETCH = 0, M_EVENT = 1, M_SEG = 2, M_WEND = 3, M_DONE = 4 };
 
 template <int BLOCK, int MINB, bool EXT>
 __global__ void __launch_bounds__(BLOCK, MINB) k_persistent(RunArgs a) {
-  int mode = M_FETCH;
+  int mode = (int)(threadIdx.x & 31) < a.spread ? M_FETCH : M_DONE;
   int64_t i = 0;
   const SetParams* P = a.sets;
   PState p;
@@ -538,13 +539,16 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batched(RunArgs a, int starve, 
                    reinterpret_cast<fx::Limb*>(stages + 12 * sizeof(fx::Limb2) * BLOCK) + threadIdx.x, BLOCK};
   const unsigned FULL = 0xffffffffu;
   const int QCAP = a.ahead_q;
-  char* const mine = a.ahead + ((size_t)blockIdx.x * BLOCK + threadIdx.x) * ahead_lane_bytes(QCAP);
+  const int lane = threadIdx.x & 31;
+  // (lanes without particles share the last one's scratch, and only ever read it)
+  char* const mine = a.ahead + ((((size_t)blockIdx.x * BLOCK + threadIdx.x) >> 5) * a.spread + min(lane, a.spread - 1)) *
+                                   ahead_lane_bytes(QCAP);
   TrajState* const slots = reinterpret_cast<TrajState*>(mine);  // [0]: between phases, [1 + k]: window ends
   SegRec* const ring = reinterpret_cast<SegRec*>(slots + 1 + kAheadSlots);
   // ---- trajectory side
   int64_t ti = 0;
   int tw = 0, twl = 0;
-  bool t_run = false, t_done = false, t_wend = false, t_stop = false;
+  bool t_run = false, t_done = lane >= a.spread, t_wend = false, t_stop = false;
   // ---- ring and window slots (records and slots in use)
   int qhead = 0, qcount = 0, whead = 0, wcount = 0;
   // ---- spin side
@@ -647,7 +651,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batched(RunArgs a, int starve, 
         const unsigned mm = __ballot_sync(FULL, more);
         const bool leave = mm == 0u || (__popc(mm) < keep && !__any_sync(FULL, more && qcount == 0));
         if (defer_m != 0u && (__popc(defer_m) >= defer_k || pm == 0u || leave)) {
-          deferred_events_warp<GAS>(tp, *tP, dd, defer_m, threadIdx.x & 31);
+          deferred_events_warp<GAS>(tp, *tP, dd, defer_m, lane);
           continue;
         }
         if (leave) break;
@@ -665,7 +669,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batched(RunArgs a, int starve, 
           break;
         }
       }
-      slots[0] = traj_of(tp);
+      if (lane < a.spread) slots[0] = traj_of(tp);
       if (hit) break;
     }
     // ================================================================ spin phase

@@ -91,6 +91,19 @@ struct RunStatus {
   int pad;                         // set by a kernel that detected an internal logic error
 };
 
+// Lanes of a warp that take particles when n of them share a GPU with `sms` SMs: few
+// particles are spread over the SMs, two warps each, before warps fill up.  A warp's time
+// is its lanes' divergent paths one after another: 100 particles took 26.6 ms in 4 full
+// warps and take 13.0 in 100 warps of one lane (two 25 ms windows with gas, plain kernel);
+// a 4 x 4 frequency grid of 24 particles a cell 95.5 and 65.  With four warps per SM the
+// FP64-bound steppers lose to the idle lanes (4 x 4,096 particles: 104 ms against 92), with
+// one the fixed-point step waits for itself (1,000 particles, flat kernel: 81 ms against 78).
+inline int spread_lanes(int64_t n, int sms) {
+  const int64_t warps = (int64_t)sms * 2;
+  const int64_t l = (n + warps - 1) / (warps > 0 ? warps : 1);
+  return l < 1 ? 1 : (l > 32 ? 32 : (int)l);
+}
+
 struct RunArgs {
   const SetParams* sets;
   int nsets;
@@ -106,6 +119,7 @@ struct RunArgs {
   int any_gas;                    // some set has gas collisions (else gas-free kernels may run)
   int any_ext;                    // some set integrates with type 2-5 (the EXT kernels must run)
   int any_rk45;                   // some set integrates with RK45 (type 1)
+  int spread;                     // particles are dealt to the first `spread` lanes of each warp (spread_lanes)
   char* ahead;                    // trajectory-ahead kernel: scratch of ahead_lane_bytes(ahead_q) per launched lane
   int ahead_q;                    // its ring depth (records per lane)
 };

@@ -155,7 +155,7 @@ int launch_init(const RunArgs& a, int block, void* stream) {
 
 template <int B>
 static int plain_launch(const RunArgs& a, int window, double next_t, void* stream) {
-  k_plain<B, false><<<grid_for(a.s.n, B), B, 0, (cudaStream_t)stream>>>(a, window, next_t);
+  k_plain<B, false><<<grid_for((a.s.n + a.spread - 1) / a.spread * 32, B), B, 0, (cudaStream_t)stream>>>(a, window, next_t);
   return (int)cudaGetLastError();
 }
 
@@ -347,7 +347,8 @@ int launch_persistent(const RunArgs& a, int v, int blocks, int block, void* stre
   cudaError_t e = ensure_smem(v, gas, kind);
   if (e != cudaSuccess) return (int)e;
   RunArgs args = a;
-  int t0 = x.starve, t1 = x.keep, dk = x.defer;
+  // the thresholds count lanes of a full warp
+  int t0 = (x.starve * a.spread + 31) / 32, t1 = (x.keep * a.spread + 31) / 32, dk = (x.defer * a.spread + 31) / 32;
   if (x.family == 1) args.ahead_q = x.qcap;
   TapeArgs none{};
   void* params_flat[] = {&args};
@@ -395,7 +396,7 @@ int launch_tape_record(const RunArgs& a, const TapeArgs& t, int blocks, void* st
   if (e != cudaSuccess) return (int)e;
   RunArgs args = a;
   TapeArgs tape = t;
-  int t0 = 4, t1 = 8, dk = 12;
+  int t0 = (4 * a.spread + 31) / 32, t1 = (8 * a.spread + 31) / 32, dk = (12 * a.spread + 31) / 32;
   args.ahead_q = kTapeQcap;
   void* params[] = {&args, &t0, &t1, &dk, &tape};
   return (int)cudaLaunchKernel(tape_fn(gas, ext), dim3(blocks), dim3(kTapeBlock), params, tape_smem(),

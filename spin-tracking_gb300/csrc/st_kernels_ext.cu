@@ -33,7 +33,8 @@ const void* tape_fn_ext() {
 
 template <int B>
 static int plain_launch_ext(const RunArgs& a, int window, double next_t, void* stream) {
-  k_plain<B, true><<<(unsigned)((a.s.n + B - 1) / B), B, 0, (cudaStream_t)stream>>>(a, window, next_t);
+  const int64_t threads = (a.s.n + a.spread - 1) / a.spread * 32;
+  k_plain<B, true><<<(unsigned)((threads + B - 1) / B), B, 0, (cudaStream_t)stream>>>(a, window, next_t);
   return (int)cudaGetLastError();
 }
 

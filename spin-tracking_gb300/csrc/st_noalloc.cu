@@ -216,6 +216,7 @@ extern "C" int st_run_noalloc(const st_options* sets, int nsets, void* state, si
     if (e != cudaSuccess) return set_last_error(ST_ERR_CUDA, cudaGetErrorString(e));
     // flat_b128_m2 (the flattened persistent kernel) at its full occupancy; the
     // occupancy query and the shared-memory attribute allocate nothing
+    a.spread = spread_lanes(n, sms);
     const int per_sm = persistent_max_blocks_per_sm(kNoAllocVariant, a.any_ext | (a.any_rk45 << 1));
     if (per_sm < 1) return set_last_error(ST_ERR_CUDA, "st_run_noalloc: the persistent kernel cannot be resident");
     int le = launch_init(a, 256, st_);
