@@ -1,4 +1,4 @@
-// DOP853 step arithmetic in 64-bit fixed point on the integer pipes.
+// DOP853 and Magnus step arithmetic in 64-bit fixed point on the integer pipes.
 //
 // GB300 issues one FP64 warp instruction per 64 or more cycles on each SM
 // sub-partition (measured: 76 cycles per DFMA, DADD, DMUL or DSETP), while a
@@ -569,15 +569,33 @@ __device__ __forceinline__ u64 root16(u64 a, u64 b, int i) {
   return r;
 }
 
-// One attempted DOP853 step of size h at tau = tx (t = x) over a scaled
-// segment: new spin in S (on any outcome the caller decides whether to keep
-// it: Sn), the error's verdict in out.  False: outside the fixed-point range.
-template <class V, class KS>
-__device__ __forceinline__ bool dop_step(const V& view, KS& ks, const SegScale& q, const i64* o0, const i64* o1, const i64* o2,
-                                         i64 ga, u64 wm, int we, double x, double tx, double h, const StepTol& tol,
-                                         const i64* S, i64* Sn, StepOut& out) {
-  using namespace dop;
-  constexpr int N = V::N;
+// h Omega over a step, as 2^ez (w(c)) with the norm of w in [1/4, 1/2): at the node
+// c (0 <= c <= 1) w = 4 w0 + c w1 + c^2 w2, and on z the pulse's 2 hg cos(2 pi (phi0 + c dphi)).
+template <int N>
+struct StepField {
+  i64 w0[N];
+  Limb w1[N], w2[N], hg, dphi;
+  u64 phi0;
+  int ez;
+  bool pulse;
+  // without the pulse; the halves of the node and of its square
+  __device__ __forceinline__ i64 at(int k, Limb c, Limb c2) const {
+    Acc o;
+    o.hh = madw(c.h, w1[k].h, w0[k]);
+    o.mid = madw(c.h, w1[k].l, kHalfLimb >> 1);
+    o.mid = madw(c.l, w1[k].h, o.mid);
+    mac(o, c2, w2[k]);
+    return q63(o, 1);
+  }
+  __device__ __forceinline__ i64 pulse_at(Limb c) const {
+    return mulq(hg, limb(half_cos_turns(phi0 + (u64)mulq(c, dphi, 1)) + 16), 1);
+  }
+};
+// False: the step leaves the segment, reaches 2^max_ez / 2 rad or passes a quarter
+// of a pulse's turn.
+template <int N>
+__device__ __forceinline__ bool step_field(const SegScale& q, const i64* o0, const i64* o1, const i64* o2, i64 ga, u64 wm,
+                                           int we, double x, double tx, double h, int max_ez, StepField<N>& f) {
   // ---- the step in segment units
   if ((i64)f64_bits(h) <= 0 || (i64)f64_bits(tx) < 0) return false;  // (a NaN is out of range below)
   const int eh = bexp(h) - 1021;  // h = hm 2^eh, hm in [1/4, 1/2)
@@ -589,36 +607,48 @@ __device__ __forceinline__ bool dop_step(const V& view, KS& ks, const SegScale& 
   // ---- h Omega = 2^ez omega, |omega| in [1/4, 1/2)
   const bool small = (float)(uint32_t)(hm >> 32) * q.on < 0x1.ff8p-4f * 0x1p31f;
   const i64 hs = small ? hm << 1 : hm;
-  const int ez = eh + q.oe - 1 - (small ? 1 : 0);
-  if (ez > 1) return false;  // the step turns the spin by up to 1 rad or more
-  const int r = 1 - ez > 63 ? 63 : 1 - ez;
+  f.ez = eh + q.oe - 1 - (small ? 1 : 0);
+  if (f.ez > max_ez) return false;
   const Limb hsl = limb(hs), hml = limb(hm), ul = limb(u);
   const int s63 = sh > 63 ? 63 : sh;
   const i64 g1 = mulq(hsl, hml, 1) >> s63;  // hs eta
   const Limb g1l = limb(g1);
   const i64 g2 = mulq(g1l, hml, 1) >> s63;  // hs eta^2
   const Limb g2l = limb(g2);
-  i64 w0[N];
-  Limb w1[N], w2[N];
 #pragma unroll
   for (int c = 0; c < N; ++c) {
     const Limb o2l = limb(o2[c]);
     const i64 t1 = mulq(ul, o2l);
-    w0[c] = mulq(hsl, limb(o0[c] + mulq(ul, limb(o1[c] + t1))), -1);  // a quarter of it
-    w1[c] = limb(mulq(g1l, limb(o1[c] + shl(t1, 1)), 1));
-    w2[c] = limb(mulq(g2l, o2l, 1));
+    f.w0[c] = mulq(hsl, limb(o0[c] + mulq(ul, limb(o1[c] + t1))), -1);  // a quarter of it
+    f.w1[c] = limb(mulq(g1l, limb(o1[c] + shl(t1, 1)), 1));
+    f.w2[c] = limb(mulq(g2l, o2l, 1));
   }
-  const bool pulse = ga != 0;
-  Limb hgl{0, 0}, dphi{0, 0};
-  u64 phi0 = 0;
-  if (pulse) {
-    hgl = limb(mulq(hsl, limb(ga), 1));
+  f.pulse = ga != 0;
+  f.hg = f.dphi = {0, 0};
+  f.phi0 = 0;
+  if (f.pulse) {
+    f.hg = limb(mulq(hsl, limb(ga), 1));
     const u64 dp = turns_of(h, wm, we);
     if (dp >= 0x4000000000000000ull || bexp(h) - 1022 + we > 0) return false;  // a quarter turn or more
-    dphi = limb((i64)dp);
+    f.dphi = limb((i64)dp);
     const u64 p = turns_of(fabs(x), wm, we);
-    phi0 = x < 0.0 ? 0ull - p : p;
+    f.phi0 = x < 0.0 ? 0ull - p : p;
   }
+  return true;
+}
+
+// One attempted DOP853 step of size h at tau = tx (t = x) over a scaled
+// segment: new spin in S (on any outcome the caller decides whether to keep
+// it: Sn), the error's verdict in out.  False: outside the fixed-point range.
+template <class V, class KS>
+__device__ __forceinline__ bool dop_step(const V& view, KS& ks, const SegScale& q, const i64* o0, const i64* o1, const i64* o2,
+                                         i64 ga, u64 wm, int we, double x, double tx, double h, const StepTol& tol,
+                                         const i64* S, i64* Sn, StepOut& out) {
+  using namespace dop;
+  constexpr int N = V::N;
+  StepField<N> f;
+  if (!step_field(q, o0, o1, o2, ga, wm, we, x, tx, h, 1, f)) return false;  // (1: up to 1 rad)
+  const int ez = f.ez, r = 1 - ez > 63 ? 63 : 1 - ez;
   // ---- stages: kappa_s = Y_s x omega_s, Y_s = S + 2^ez sum a_sj kappa_j
   i64 Sr[N];
 #pragma unroll
@@ -657,14 +687,8 @@ __device__ __forceinline__ bool dop_step(const V& view, KS& ks, const SegScale& 
       // |2 sum a kappa| < 1/2: neither the shift below nor Y can overflow
       bad |= ((unsigned)(int)(a[c].hh >> 32) + (1u << (28 - p))) & ~((1u << (29 - p)) - 1u);
       Y[c] = limb(Sr[c] + (q63(a[c], 1 + p) >> r));
-      Acc o;
-      o.hh = madw(row.c.h, w1[c].h, w0[c]);
-      o.mid = madw(row.c.h, w1[c].l, kHalfLimb >> 1);
-      o.mid = madw(row.c.l, w1[c].h, o.mid);
-      mac(o, row.c2, w2[c]);
-      i64 w = q63(o, 1);
-      if (pulse && view.is_z(c))
-        w += mulq(hgl, limb(half_cos_turns(phi0 + (u64)mulq(row.c, dphi, 1)) + 16), 1);
+      i64 w = f.at(c, row.c, row.c2);
+      if (f.pulse && view.is_z(c)) w += f.pulse_at(row.c);
       W[c] = limb(w);
     }
     view.cross(Y, W, a);
@@ -776,6 +800,144 @@ __device__ __forceinline__ bool dop_step(const V& view, KS& ks, const SegScale& 
   const int zr = clz64(rr);  // rr / 2^64 = r / 2, to the nearest double
   out.root8 = bits_f64(((u64)(1022 + 1 - zr - j) << 52) + ((rr << zr) >> 11) + (((rr << zr) >> 10) & 1) - kOne);
   return true;
+}
+
+// ---------------------------------------------------------------- Magnus step
+// The 16 exponents' weights of the five node fields in the order they are applied
+// (11 of CFET8, rows 1..5 with the nodes reversed, then rows 6..1; 5 of CFET6,
+// rows 1 and 2 reversed, then rows 3..1).  A row's magnitudes sum to less than 1.45.
+namespace cfx {
+constexpr double g[6][5] = {{cfet::G11, cfet::G12, cfet::G13, cfet::G14, cfet::G15},
+                            {cfet::G21, cfet::G22, cfet::G23, cfet::G24, cfet::G25},
+                            {cfet::G31, cfet::G32, cfet::G33, cfet::G34, cfet::G35},
+                            {cfet::G41, cfet::G42, cfet::G43, cfet::G44, cfet::G45},
+                            {cfet::G51, cfet::G52, cfet::G53, cfet::G54, cfet::G55},
+                            {cfet::G61, cfet::G62, cfet::G63, cfet::G64, cfet::G65}};
+constexpr double h[3][5] = {{cfet::H11, cfet::H12, cfet::H13, cfet::H14, cfet::H15},
+                            {cfet::H21, cfet::H22, cfet::H23, cfet::H24, cfet::H25},
+                            {cfet::H31, cfet::H32, cfet::H33, cfet::H34, cfet::H35}};
+constexpr double x[5] = {cfet::X1, cfet::X2, cfet::X3, cfet::X4, cfet::X5};
+constexpr double weight(int n, int j) {
+  return n < 5 ? g[n][4 - j] : n < 11 ? g[10 - n][j] : n < 13 ? h[n - 11][4 - j] : h[15 - n][j];
+}
+}  // namespace cfx
+#define ST_W(n) \
+  {coef(cfx::weight(n, 0), 0), coef(cfx::weight(n, 1), 0), coef(cfx::weight(n, 2), 0), coef(cfx::weight(n, 3), 0), \
+   coef(cfx::weight(n, 4), 0)}
+static __constant__ Limb kMagnusCoef[16][5] = {ST_W(0), ST_W(1), ST_W(2),  ST_W(3),  ST_W(4),  ST_W(5),  ST_W(6),  ST_W(7),
+                                               ST_W(8), ST_W(9), ST_W(10), ST_W(11), ST_W(12), ST_W(13), ST_W(14), ST_W(15)};
+#undef ST_W
+#define ST_X(j) {coef(cfx::x[j], 1), coef(cfx::x[j] * cfx::x[j], 1)}
+static __constant__ Limb kMagnusNode[5][2] = {ST_X(0), ST_X(1), ST_X(2), ST_X(3), ST_X(4)};
+#undef ST_X
+// 1 / (2k + 3)! and 1 / (2k + 2)! as Q63: sin b / b = 1 - z (1/3! - z/5! ...), cos b = 1 - z (1/2! - z/4! ...), z = b^2
+static __constant__ i64 kHalfAngle[8][2] = {
+    {1537228672809129301ll, 4611686018427387904ll}, {76861433640456465ll, 384307168202282325ll},
+    {1830034134296583ll, 12810238940076078ll}, {25417140754119ll, 228754266787073ll},
+    {231064915947ll, 2541714075412ll}, {1481185359ll, 19255409662ll},
+    {7053264ll, 105798954ll}, {25931ll, 440829ll}};
+
+// One Magnus step (CFET8 with its CFET6 companion) of size h at tau = tx (t = x) over a
+// scaled segment: the proposal in y8, its difference from the companion's in e.  Each of
+// the 16 exponents k turns the spin by v' = v + S (w (v x k) + S/2 (v x k) x k) with
+// b = |k|/2, S = sin b / b, w = cos b: both are even series in b, so neither a square
+// root nor a division is needed; for steps above 1 rad the series run at b 2^-m
+// and are doubled m times.  In FP64 a rotation is some 100 instructions of 76 cycles,
+// its sincos more than half of them; here it is about 400 of 2 to 4.
+// False: out of range (above 4 rad, off the segment, no field): the caller takes FP64.
+__device__ __forceinline__ bool magnus_step(const SegScale& q, const i64* o0, const i64* o1, const i64* o2, i64 ga, u64 wm,
+                                            int we, double x, double tx, double h, const i64* S, i64* y8, i64* e) {
+  const Lane3 view;
+  Limb W[5][3];
+  int ez;
+  {
+    StepField<3> f;
+    if (!step_field(q, o0, o1, o2, ga, wm, we, x, tx, h, 3, f)) return false;
+    ez = f.ez;
+#pragma unroll
+    for (int i = 0; i < 5; ++i)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        i64 w = f.at(c, kMagnusNode[i][0], kMagnusNode[i][1]);
+        if (c == 2 && f.pulse) w += f.pulse_at(kMagnusNode[i][0]);
+        W[i][c] = limb(w);
+      }
+  }
+  constexpr i64 kHalf = 1ll << 62;
+  const int ps = ez < -60 ? 62 : (ez < 1 ? 1 - ez : 0);
+  i64 y[3] = {S[0], S[1], S[2]};
+  bool zero = false;
+#pragma unroll 1
+  for (int n = 0; n < 16; ++n) {
+    if (n == 11) {  // CFET8 done: CFET6 from S
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        y8[c] = y[c];
+        y[c] = S[c];
+      }
+    }
+    const Limb* cf = kMagnusCoef[n];
+    Limb k[3], v[3];
+    Acc t[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      Acc a = mac0(cf[0], W[0][c], kHalfLimb);
+#pragma unroll
+      for (int j = 1; j < 5; ++j) mac(a, cf[j], W[j][c]);
+      k[c] = limb(q63(a));
+      v[c] = limb(y[c] + 16);
+    }
+    Acc a = mac0(k[0], k[0]);
+    mac(a, k[1], k[1]);
+    mac(a, k[2], k[2]);
+    const i64 k2 = q63(a);
+    zero |= k2 == 0;
+    // z = |kappa|^2 4^(ez - 1) 4^-doublings <= 1/4
+    const int lead = clz64((u64)k2), dbl = 2 * ez + 2 - lead, doublings = dbl > 0 ? dbl >> 1 : 0;
+    const int zs = 2 - 2 * ez + 2 * doublings;
+    const i64 zw = zs >= 0 ? k2 >> (zs > 62 ? 62 : zs) : shl(k2, -zs);
+    const Limb z = limb(zw + 16);
+    // z < 2^-n: the first term left out is below 2^-65
+    const int nz = clz64((u64)zw) - 1;
+    const int terms = nz >= 20 ? 2 : (nz >= 13 ? 3 : (nz >= 9 ? 4 : (nz >= 7 ? 5 : (nz >= 5 ? 6 : 8))));
+    i64 sb = kHalfAngle[terms - 1][0], cb = kHalfAngle[terms - 1][1];
+#pragma unroll 1
+    for (int i = terms - 2; i >= 0; --i) {
+      sb = kHalfAngle[i][0] - mulq(z, limb(sb));
+      cb = kHalfAngle[i][1] - mulq(z, limb(cb));
+    }
+    i64 s2 = kHalf - q63(mac0(z, limb(sb)), -1), w2 = kHalf - q63(mac0(z, limb(cb)), -1);  // S / 2, w / 2
+#pragma unroll 1
+    for (int i = 0; i < doublings; ++i) {
+      const Limb sl = limb(s2 + 16), wl = limb(w2 + 16);
+      s2 = q63(mac0(sl, wl), 1);
+      w2 = (i64)((u64)q63(mac0(wl, wl), 2) - (u64)kHalf);
+    }
+    const Limb sl = limb(s2 + 16);
+    const Limb fs = limb(mulq(sl, limb(w2 + 16), 1)), fp = limb(mulq(sl, sl, 1));  // S w / 2, S^2 / 2
+    // tau = 2^ts v x kappa, as large as |v| < 0.251 and |kappa| < 2^((1 - lead) / 2) let it be
+    // (and b times that)
+    const int tb = ez - (lead >> 1);
+    const int ts = (lead < 30 ? 2 + ((lead > 2 ? lead - 2 : 0) >> 1) : 16) - (tb > 0 ? tb : 0);
+    const int us = ts - ez > 62 ? 62 : ts - ez;
+    const i64 half = us > 0 ? (1ll << us) >> 1 : 0;
+    view.cross(v, k, t);
+    Limb tau[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) tau[c] = limb(q63(t[c], ts) - (16 << ts) + 16);  // (the limb's half was shifted with the product)
+    view.cross(tau, k, t);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const i64 p = q63(t[c]) - 16;  // 2^(ez - 1) tau x kappa
+      Acc d = mac0(fs, tau[c]);
+      mac(d, fp, limb((ez >= 1 ? shl(p, ez - 1) : p >> ps) + 16));
+      const i64 u = q63(d, 1);
+      y[c] += us < 0 ? shl(u, -us) : (u + half) >> us;
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) e[c] = y8[c] - y[c];
+  return !zero;
 }
 
 }  // namespace fx
