@@ -234,6 +234,83 @@ __device__ __forceinline__ void magnus_step_adjoint(const Seg& g, const SetParam
 #undef ST_VN
 }
 
+// One DOP853 step back in FP64 for a segment that may be in fixed point; a call, not
+// inlined: the fixed-point step takes all but a few.
+template <int BLOCK>
+static __device__ __noinline__ void dop_adjoint_slow(const Seg& g, const SetParams& P, double x, double h, const double y[3],
+                                                     double lam[3], Moments& M, bool pulse, double* sm) {
+  Seg t = g;
+  if (t.fx) seg_unscale(t);
+  dop_step_adjoint<BLOCK>(t, P, x, h, y, lam, M, pulse, sm);
+}
+
+// Stage array of the fixed-point form: 36 words at a stride.
+struct StageWords {
+  fx::Limb* p;
+  int stride;
+  __device__ __forceinline__ void load(int s, fx::Limb k[3]) const {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) k[c] = p[(s * 3 + c) * stride];
+  }
+  __device__ __forceinline__ void store(int s, const fx::Limb k[3]) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) p[(s * 3 + c) * stride] = k[c];
+  }
+};
+
+// One DOP853 step back, in fixed point where the step fits.  What bounded it in FP64: the
+// pipe, 850 instructions of 76 cycles a step; in fixed point the latency of two warps per
+// sub-partition and the slowest particle of each warp.  32,768 particles x 0.1 s: backward pass
+// 50 to 58 ms in FP64, 28 to 31 in fixed point.
+template <int BLOCK>
+__device__ __forceinline__ void dop_adjoint_step(const Seg& g, const SetParams& P, double x, double h, const double y[3],
+                                                 double lam[3], Moments& M, bool pulse, double* sm) {
+#if ST_GRAD_IS_LINEAR && ST_PULSE_IS_Z_COS
+  int se, le;
+  if (g.fx && fx::spin_scale(y, se) && fx::spin_scale(lam, le) && le > -800 && le < 800 && se + le > -800 && se + le < 800) {
+    const fx::i64 o0[3] = {as_i64(g.o0x), as_i64(g.o0y), as_i64(g.o0z)};
+    const fx::i64 o1[3] = {as_i64(g.o1x), as_i64(g.o1y), as_i64(g.o1z)};
+    const fx::i64 o2[3] = {as_i64(g.o2x), as_i64(g.o2y), as_i64(g.o2z)};
+    fx::i64 S[3], L[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      S[c] = fx::to_q63(y[c], se);
+      L[c] = fx::to_q63(lam[c], le);
+    }
+    // both stage arrays in this thread's own 72 words: other lanes may be in the FP64 form
+    StageWords ks{reinterpret_cast<fx::Limb*>(sm), BLOCK}, ys{reinterpret_cast<fx::Limb*>(sm) + 36 * BLOCK, BLOCK};
+    fx::AdjMoments m;
+    const double tx = x - g.t0;
+    if (fx::dop_adjoint(ks, ys, g.sc, o0, o1, o2, as_i64(g.gpa), P.wturn_m, P.wturn_e, x, tx, h, pulse, S, L, m)) {
+      const int E = se + le + m.exp;
+      const double hh = h * h;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        lam[c] = fx::from_q63(L[c], le);
+        // sums over the stages at tau = tx + c h
+        const double z0 = h * fx::from_q63(m.z0[c], E), z1 = hh * fx::from_q63(m.z1[c], E), z2 = hh * fx::from_q63(m.z2[c], E);
+        M.z0[c] += z0;
+        M.z1[c] += fma(tx, z0, z1);
+        M.z2[c] += fma(tx, fma(tx, z0, 2.0 * z1), h * z2);
+      }
+      if (pulse) {  // the phases are those of |w|
+        const double sz = h * fx::from_q63(m.sz, E + 1), sc = hh * fx::from_q63(m.scz, E + 1);
+        M.ga = fma(P.gamma * h, fx::from_q63(m.cz, E + 1), M.ga);
+        M.gw = fma(P.w < 0.0 ? P.gamma * P.a : -P.gamma * P.a, fma(x, sz, sc), M.gw);
+      }
+      return;
+    }
+  }
+#endif
+  const Seg t = g;  // (addresses go to the call: the caller's stay in registers)
+  double yt[3] = {y[0], y[1], y[2]}, lt[3] = {lam[0], lam[1], lam[2]};
+  Moments Mt = M;
+  dop_adjoint_slow<BLOCK>(t, P, x, h, yt, lt, Mt, pulse, sm);
+  M = Mt;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) lam[c] = lt[c];
+}
+
 // Contract a segment's moments into dL/dtheta (theta order of the file header);
 // gth is strided by `stride` (shared memory, one column per thread).
 __device__ __forceinline__ void contract(const SetParams& P, const double p0[3], const double v0[3], const Moments& M,
@@ -282,6 +359,7 @@ __device__ __forceinline__ void tape_load_seg(const TapeArgs& t, const SetParams
   double o0[3], o1[3];
   seg_field(P, r[1], r[2], r[3], r[4], r[5], r[6], o0, o1);
   seg_begin(g, P, r[0], r[0], o0, o1);
+  g.fx = false;
 }
 
 // Lane state machine: fetch a particle from the work order (divergent, once
@@ -294,7 +372,7 @@ __device__ __forceinline__ void tape_load_seg(const TapeArgs& t, const SetParams
 // MAGNUS: the tape holds Magnus CFET8 steps (integratorType 2) instead of DOP853 ones.
 template <bool MAGNUS>
 __global__ void __launch_bounds__(kAdjBlock) k_adj_backward(RunArgs a, TapeArgs t) {
-  __shared__ double stage_all[2 * 12 * 3 * kAdjBlock];  // stage states, then stage fields
+  __shared__ double stage_all[2 * 12 * 3 * kAdjBlock];  // a column per thread: FP64 stage states and fields, or fixed-point states and derivatives
   __shared__ double gsm_all[kNumTheta * kAdjBlock];
   double* stg = stage_all + threadIdx.x;
   double* gth = gsm_all + threadIdx.x;  // gradient accumulators, stride kAdjBlock
@@ -305,6 +383,7 @@ __global__ void __launch_bounds__(kAdjBlock) k_adj_backward(RunArgs a, TapeArgs 
   int64_t i = 0;
   const SetParams* P = a.sets;
   Seg g;
+  bool fresh = false;  // g is as loaded, not scaled to fixed point yet (DOP853)
   Moments M;
   double lam[3] = {0.0, 0.0, 0.0};
   int sp = -1, si = 0, gp = -1, gi = 0;
@@ -337,6 +416,7 @@ __global__ void __launch_bounds__(kAdjBlock) k_adj_backward(RunArgs a, TapeArgs 
       }
       P = &a.sets[a.s.set[i]];
       tape_load_seg(t, *P, gp, gi, g);
+      fresh = true;
 #pragma unroll
       for (int q = 0; q < kNumTheta; ++q) gth[q * kAdjBlock] = t.grad[i * kNumTheta + q];
 #pragma unroll
@@ -355,7 +435,17 @@ __global__ void __launch_bounds__(kAdjBlock) k_adj_backward(RunArgs a, TapeArgs 
     if (MAGNUS)
       magnus_step_adjoint<kAdjBlock>(g, *P, x, h, y, lam, M, pulse, stg);
     else
-      dop_step_adjoint<kAdjBlock>(g, *P, x, h, y, lam, M, pulse, stg);
+    {
+      if (fresh) {  // the segment's last step ends with it
+        SegPoly q;
+        q.o0[0] = g.o0x; q.o0[1] = g.o0y; q.o0[2] = g.o0z;
+        q.o1[0] = g.o1x; q.o1[1] = g.o1y; q.o1[2] = g.o1z;
+        seg_scale(q, *P, x + h - g.t0);
+        seg_open(g, *P, q, g.t0, g.t0);
+        fresh = false;
+      }
+      dop_adjoint_step<kAdjBlock>(g, *P, x, h, y, lam, M, pulse, stg);
+    }
     ++walked_s;
     bool finish = false;
     int bad = 0;
@@ -395,6 +485,7 @@ __global__ void __launch_bounds__(kAdjBlock) k_adj_backward(RunArgs a, TapeArgs 
         bad = 4;  // a segment left without steps
       } else {
         tape_load_seg(t, *P, gp, gi, g);
+        fresh = true;
       }
     } else if (sp < 0 || sp >= pages) {
       finish = true;

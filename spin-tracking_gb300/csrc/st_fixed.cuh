@@ -637,18 +637,15 @@ __device__ __forceinline__ bool step_field(const SegScale& q, const i64* o0, con
   return true;
 }
 
-// One attempted DOP853 step of size h at tau = tx (t = x) over a scaled
-// segment: new spin in S (on any outcome the caller decides whether to keep
-// it: Sn), the error's verdict in out.  False: outside the fixed-point range.
-template <class V, class KS>
-__device__ __forceinline__ bool dop_step(const V& view, KS& ks, const SegScale& q, const i64* o0, const i64* o1, const i64* o2,
-                                         i64 ga, u64 wm, int we, double x, double tx, double h, const StepTol& tol,
-                                         const i64* S, i64* Sn, StepOut& out) {
-  using namespace dop;
+// ys of dop_stages where the stage states are not kept.
+struct StageNone {
+  __device__ __forceinline__ void store(int, const Limb*) {}
+};
+// The stages of a step: kappa_1..kappa_12 in ks, the states Y in ys; not zero: a sum
+// left its range.
+template <class V, class KS, class YS>
+__device__ __forceinline__ unsigned dop_stages(const V& view, KS& ks, YS& ys, const StepField<V::N>& f, const i64* S, int r) {
   constexpr int N = V::N;
-  StepField<N> f;
-  if (!step_field(q, o0, o1, o2, ga, wm, we, x, tx, h, 1, f)) return false;  // (1: up to 1 rad)
-  const int ez = f.ez, r = 1 - ez > 63 ? 63 : 1 - ez;
   // ---- stages: kappa_s = Y_s x omega_s, Y_s = S + 2^ez sum a_sj kappa_j
   i64 Sr[N];
 #pragma unroll
@@ -695,7 +692,26 @@ __device__ __forceinline__ bool dop_step(const V& view, KS& ks, const SegScale& 
 #pragma unroll
     for (int c = 0; c < N; ++c) k[c] = limb(q63(a[c]));
     ks.store(s, k);
+    ys.store(s, Y);
   }
+  return bad;
+}
+
+// One attempted DOP853 step of size h at tau = tx (t = x) over a scaled
+// segment: new spin in S (on any outcome the caller decides whether to keep
+// it: Sn), the error's verdict in out.  False: outside the fixed-point range.
+template <class V, class KS>
+__device__ __forceinline__ bool dop_step(const V& view, KS& ks, const SegScale& q, const i64* o0, const i64* o1, const i64* o2,
+                                         i64 ga, u64 wm, int we, double x, double tx, double h, const StepTol& tol,
+                                         const i64* S, i64* Sn, StepOut& out) {
+  using namespace dop;
+  constexpr int N = V::N;
+  StepField<N> f;
+  if (!step_field(q, o0, o1, o2, ga, wm, we, x, tx, h, 1, f)) return false;  // (1: up to 1 rad)
+  const int ez = f.ez, r = 1 - ez > 63 ? 63 : 1 - ez;
+  StageNone none;
+  const unsigned stages_bad = dop_stages(view, ks, none, f, S, r);
+  unsigned bad = stages_bad;
   // ---- 8th-order sum, new spin, the two error rows
   Acc sb[N], s3[N], s5[N];
 #pragma unroll
@@ -799,6 +815,156 @@ __device__ __forceinline__ bool dop_step(const V& view, KS& ks, const SegScale& 
   const u64 rr = root16(A, b, i);
   const int zr = clz64(rr);  // rr / 2^64 = r / 2, to the nearest double
   out.root8 = bits_f64(((u64)(1022 + 1 - zr - j) << 52) + ((rr << zr) >> 11) + (((rr << zr) >> 10) & 1) - kOne);
+  return true;
+}
+
+// ---------------------------------------------------------------- adjoint step
+// Column s of the tableau, from stage s's side: the stages r = s + 1 .. s + n that read
+// kappa_s (their a_rs from kAdjCoef[off], over 2^7 for r >= 9 and 2^2 below) and b_s / 2^3.
+namespace adjcol {
+__device__ __forceinline__ constexpr int last_reader(int s) { return s == 2 ? 3 : (s == 3 ? 5 : 12); }
+__device__ __forceinline__ constexpr double col(int s, int r) {
+  return dopst::a(r, s == 1 ? 0 : (r == 3 ? 1 : (r <= 5 ? s - 2 : s - 3)));
+}
+}  // namespace adjcol
+struct AdjRow {
+  int off, n;
+  Limb b;
+};
+#define ST_ROW(s, off) {off, adjcol::last_reader(s) - (s), coef(dopst::b(s), 3)}
+static __constant__ AdjRow kAdjRows[12] = {ST_ROW(1, 0),  ST_ROW(2, 11),  ST_ROW(3, 12),  ST_ROW(4, 14),
+                                           ST_ROW(5, 22), ST_ROW(6, 29),  ST_ROW(7, 35),  ST_ROW(8, 40),
+                                           ST_ROW(9, 44), ST_ROW(10, 47), ST_ROW(11, 49), ST_ROW(12, 50)};
+#undef ST_ROW
+#define ST_A(s, r) coef(adjcol::col(s, r), (r) >= 9 ? 7 : 2)
+static __constant__ Limb kAdjCoef[51] = {
+    ST_A(1, 2), ST_A(1, 3), ST_A(1, 4), ST_A(1, 5), ST_A(1, 6), ST_A(1, 7), ST_A(1, 8), ST_A(1, 9),
+    ST_A(1, 10), ST_A(1, 11), ST_A(1, 12), ST_A(2, 3), ST_A(3, 4), ST_A(3, 5), ST_A(4, 5), ST_A(4, 6),
+    ST_A(4, 7), ST_A(4, 8), ST_A(4, 9), ST_A(4, 10), ST_A(4, 11), ST_A(4, 12), ST_A(5, 6), ST_A(5, 7),
+    ST_A(5, 8), ST_A(5, 9), ST_A(5, 10), ST_A(5, 11), ST_A(5, 12), ST_A(6, 7), ST_A(6, 8), ST_A(6, 9),
+    ST_A(6, 10), ST_A(6, 11), ST_A(6, 12), ST_A(7, 8), ST_A(7, 9), ST_A(7, 10), ST_A(7, 11), ST_A(7, 12),
+    ST_A(8, 9), ST_A(8, 10), ST_A(8, 11), ST_A(8, 12), ST_A(9, 10), ST_A(9, 11), ST_A(9, 12), ST_A(10, 11),
+    ST_A(10, 12), ST_A(11, 12), {0, 0}};
+#undef ST_A
+
+// What a step adds to the gradient moments, times 2^(exp + scales of spin and adjoint) / h:
+// the sums over the stages of z, c z, c^2 z with z = (dL/dk_s / h) x Y_s at the node c, and with
+// the pulse's phase of cos z_z, sin z_z, c sin z_z (halved).
+struct AdjMoments {
+  i64 z0[3], z1[3], z2[3], cz, sz, scz;
+  int exp;
+};
+
+// Backward through one DOP853 step of size h at tau = tx from the spin S: the adjoint lam (a
+// scaled vector like S) of the step's result becomes that of S.  With kh_s = (dL/dk_s) / h
+//   kh_s = b_s lam + sum_{r > s} a_rs yb_r,  yb_s = h Omega_s x kh_s,  dL/dS = lam + sum_s yb_s;
+// kh is kept as kh 2^-K: sum |a_rs| |yb_r| + |b_s| stays under 17, 10, 7.5 |lam| (|lam| <= 1/4)
+// for steps below 1/4, 1/8, 1/16 rad; above that the growing K costs more bits than FP64
+// loses.  For s >= 9 it stays under 0.6, and
+// the large coefficients of the tableau multiply these: they have a K of their own, -1.
+// The stages' 12 states Y go to ys, kappa and then yb to ks.  In FP64 a step takes some 850
+// instructions of 76 cycles.  False: out of range, the caller takes FP64.
+template <class KS>
+__device__ __forceinline__ bool dop_adjoint(KS& ks, KS& ys, const SegScale& q, const i64* o0, const i64* o1, const i64* o2,
+                                            i64 ga, u64 wm, int we, double x, double tx, double h, bool pulse_grads,
+                                            const i64* S, i64* lam, AdjMoments& m) {
+  const Lane3 view;
+  StepField<3> f;
+  if (!step_field(q, o0, o1, o2, ga, wm, we, x, tx, h, -1, f)) return false;  // (-1: up to 1/4 rad)
+  if (pulse_grads && !f.pulse) return false;
+  const int ez = f.ez, r = 1 - ez > 63 ? 63 : 1 - ez;
+  if (dop_stages(view, ks, ys, f, S, r) != 0) return false;
+  const int K = ez < -3 ? 1 : 4 + ez;
+  Limb ll[3];
+  i64 ln[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    ll[c] = limb(lam[c] + 16);
+    ln[c] = lam[c];
+    m.z0[c] = m.z1[c] = m.z2[c] = 0;
+  }
+  m.cz = m.sz = m.scz = 0;
+  m.exp = K + 3;
+#pragma unroll 1
+  for (int s = 11; s >= 0; --s) {
+    const AdjRow& row = kAdjRows[s];
+    const Limb nc = kStageRows[s].c, nc2 = kStageRows[s].c2;
+    const bool late = s >= 8;
+    Acc a[3];
+    i64 kq[3];
+    // the stages r >= 9, then those below
+#pragma unroll
+    for (int c = 0; c < 3; ++c) a[c] = {0, 0};
+    int j = row.n;
+#pragma unroll 1
+    for (const int j0 = late ? 0 : 7 - s; j > j0;) {
+      Limb yb[3];
+      --j;
+      const Limb g = kAdjCoef[row.off + j];
+      ks.load(s + 1 + j, yb);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) mac(a[c], g, yb[c]);
+    }
+    const int ls = late ? 6 + ez : 5 + ez - K;  // (at most 7)
+    const int bs = late ? 0 : K - 1;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const i64 t = late ? q63(mac0(row.b, ll[c]), 4) : q63(mac0(row.b, ll[c]), 2) >> bs;
+      kq[c] = t + (ls >= 0 ? q63(a[c], ls) : q63(a[c]) >> (ls < -63 ? 63 : -ls));
+      a[c] = {0, 0};
+    }
+#pragma unroll 1
+    while (j > 0) {
+      Limb yb[3];
+      --j;
+      const Limb g = kAdjCoef[row.off + j];
+      ks.load(s + 1 + j, yb);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) mac(a[c], g, yb[c]);
+    }
+    Limb kl[3], W[3], Y[3];
+    i64 hc = 0, hs = 0;
+    if (f.pulse) {
+      const u64 phi = f.phi0 + (u64)mulq(nc, f.dphi, 1);
+      hc = half_cos_turns(phi);
+      if (pulse_grads) hs = half_cos_turns(phi - 0x4000000000000000ull);
+    }
+    ys.load(s, Y);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      kl[c] = limb(kq[c] + (ez >= -1 ? q63(a[c], 1 + ez) : q63(a[c]) >> (ez < -64 ? 63 : -1 - ez)) + 16);
+      i64 w = f.at(c, nc, nc2);
+      if (c == 2 && f.pulse) w += mulq(f.hg, limb(hc + 16), 1);
+      W[c] = limb(w);
+    }
+    view.cross(W, kl, a);  // half of yb 2^-(K + ez)
+    const int us = ez - 1 + (late ? -1 : K), zs = late ? K + 5 : 4;
+    Limb yb[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const i64 y2 = q63(a[c], 1) - 32;
+      yb[c] = limb(y2 + 16);
+      ln[c] += us >= 0 ? shl(y2, us) : y2 >> (us < -63 ? 63 : -us);
+    }
+    ks.store(s, yb);
+    view.cross(kl, Y, a);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const i64 z = q63(a[c], 1) - 32;  // |kq| < 0.95, |Y| < 0.27
+      const Limb zl = limb(z + 16);
+      m.z0[c] += z >> zs;
+      m.z1[c] += q63(mac0(nc, zl), 1) >> zs;
+      m.z2[c] += q63(mac0(nc2, zl), 1) >> zs;
+      if (c == 2 && pulse_grads) {
+        m.cz += q63(mac0(limb(hc + 16), zl)) >> zs;
+        const i64 t = q63(mac0(limb(hs + 16), zl));
+        m.sz += t >> zs;
+        m.scz += q63(mac0(nc, limb(t + 16)), 1) >> zs;
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) lam[c] = ln[c];
   return true;
 }
 
