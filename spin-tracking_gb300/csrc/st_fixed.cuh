@@ -1,4 +1,4 @@
-// DOP853 and Magnus step arithmetic in 64-bit fixed point on the integer pipes.
+// DOP853, Magnus and quaternion step arithmetic in 64-bit fixed point on the integer pipes.
 //
 // GB300 issues one FP64 warp instruction per 64 or more cycles on each SM
 // sub-partition (measured: 76 cycles per DFMA, DADD, DMUL or DSETP), while a
@@ -1003,17 +1003,73 @@ static __constant__ i64 kHalfAngle[8][2] = {
     {231064915947ll, 2541714075412ll}, {1481185359ll, 19255409662ll},
     {7053264ll, 105798954ll}, {25931ll, 440829ll}};
 
+// One rotation: y by 2^ez |kappa| about -kappa, |kappa| < 0.73, |y| < 0.251.  With k = 2^ez kappa
+// and b = |k|/2, v' = v + S (w (v x k) + S/2 (v x k) x k), S = sin b / b and w = cos b: both are
+// even series in b, so neither a square root nor a division is needed; above 1 rad the series
+// run at b 2^-m and are doubled m times.  In FP64 a rotation is some 100 instructions of 76 cycles,
+// its sincos more than half of them; here it is about 400 of 2 to 4.  False: kappa is zero.
+__device__ __forceinline__ bool rotate(int ez, const Limb* k, i64* y) {
+  const Lane3 view;
+  constexpr i64 kHalf = 1ll << 62;
+  const int ps = ez < -60 ? 62 : (ez < 1 ? 1 - ez : 0);
+  Acc t[3];
+  Limb v[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) v[c] = limb(y[c] + 16);
+  Acc a = mac0(k[0], k[0]);
+  mac(a, k[1], k[1]);
+  mac(a, k[2], k[2]);
+  const i64 k2 = q63(a);
+  // z = |kappa|^2 4^(ez - 1) 4^-doublings <= 1/4
+  const int lead = clz64((u64)k2), dbl = 2 * ez + 2 - lead, doublings = dbl > 0 ? dbl >> 1 : 0;
+  const int zs = 2 - 2 * ez + 2 * doublings;
+  const i64 zw = zs >= 0 ? k2 >> (zs > 62 ? 62 : zs) : shl(k2, -zs);
+  const Limb z = limb(zw + 16);
+  // z < 2^-n: the first term left out is below 2^-65
+  const int nz = clz64((u64)zw) - 1;
+  const int terms = nz >= 20 ? 2 : (nz >= 13 ? 3 : (nz >= 9 ? 4 : (nz >= 7 ? 5 : (nz >= 5 ? 6 : 8))));
+  i64 sb = kHalfAngle[terms - 1][0], cb = kHalfAngle[terms - 1][1];
+#pragma unroll 1
+  for (int i = terms - 2; i >= 0; --i) {
+    sb = kHalfAngle[i][0] - mulq(z, limb(sb));
+    cb = kHalfAngle[i][1] - mulq(z, limb(cb));
+  }
+  i64 s2 = kHalf - q63(mac0(z, limb(sb)), -1), w2 = kHalf - q63(mac0(z, limb(cb)), -1);  // S / 2, w / 2
+#pragma unroll 1
+  for (int i = 0; i < doublings; ++i) {
+    const Limb sl = limb(s2 + 16), wl = limb(w2 + 16);
+    s2 = q63(mac0(sl, wl), 1);
+    w2 = (i64)((u64)q63(mac0(wl, wl), 2) - (u64)kHalf);
+  }
+  const Limb sl = limb(s2 + 16);
+  const Limb fs = limb(mulq(sl, limb(w2 + 16), 1)), fp = limb(mulq(sl, sl, 1));  // S w / 2, S^2 / 2
+  // tau = 2^ts v x kappa, as large as |v| < 0.251 and |kappa| < 2^((1 - lead) / 2) let it be
+  // (and b times that)
+  const int tb = ez - (lead >> 1);
+  const int ts = (lead < 30 ? 2 + ((lead > 2 ? lead - 2 : 0) >> 1) : 16) - (tb > 0 ? tb : 0);
+  const int us = ts - ez > 62 ? 62 : ts - ez;
+  const i64 half = us > 0 ? (1ll << us) >> 1 : 0;
+  view.cross(v, k, t);
+  Limb tau[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) tau[c] = limb(q63(t[c], ts) - (16 << ts) + 16);  // (the limb's half was shifted with the product)
+  view.cross(tau, k, t);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const i64 p = q63(t[c]) - 16;  // 2^(ez - 1) tau x kappa
+    Acc d = mac0(fs, tau[c]);
+    mac(d, fp, limb((ez >= 1 ? shl(p, ez - 1) : p >> ps) + 16));
+    const i64 u = q63(d, 1);
+    y[c] += us < 0 ? shl(u, -us) : (u + half) >> us;
+  }
+  return k2 != 0;
+}
+
 // One Magnus step (CFET8 with its CFET6 companion) of size h at tau = tx (t = x) over a
-// scaled segment: the proposal in y8, its difference from the companion's in e.  Each of
-// the 16 exponents k turns the spin by v' = v + S (w (v x k) + S/2 (v x k) x k) with
-// b = |k|/2, S = sin b / b, w = cos b: both are even series in b, so neither a square
-// root nor a division is needed; for steps above 1 rad the series run at b 2^-m
-// and are doubled m times.  In FP64 a rotation is some 100 instructions of 76 cycles,
-// its sincos more than half of them; here it is about 400 of 2 to 4.
+// scaled segment: the proposal in y8, its difference from the companion's in e.
 // False: out of range (above 4 rad, off the segment, no field): the caller takes FP64.
 __device__ __forceinline__ bool magnus_step(const SegScale& q, const i64* o0, const i64* o1, const i64* o2, i64 ga, u64 wm,
                                             int we, double x, double tx, double h, const i64* S, i64* y8, i64* e) {
-  const Lane3 view;
   Limb W[5][3];
   int ez;
   {
@@ -1029,8 +1085,6 @@ __device__ __forceinline__ bool magnus_step(const SegScale& q, const i64* o0, co
         W[i][c] = limb(w);
       }
   }
-  constexpr i64 kHalf = 1ll << 62;
-  const int ps = ez < -60 ? 62 : (ez < 1 ? 1 - ez : 0);
   i64 y[3] = {S[0], S[1], S[2]};
   bool zero = false;
 #pragma unroll 1
@@ -1043,67 +1097,71 @@ __device__ __forceinline__ bool magnus_step(const SegScale& q, const i64* o0, co
       }
     }
     const Limb* cf = kMagnusCoef[n];
-    Limb k[3], v[3];
-    Acc t[3];
+    Limb k[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       Acc a = mac0(cf[0], W[0][c], kHalfLimb);
 #pragma unroll
       for (int j = 1; j < 5; ++j) mac(a, cf[j], W[j][c]);
       k[c] = limb(q63(a));
-      v[c] = limb(y[c] + 16);
     }
-    Acc a = mac0(k[0], k[0]);
-    mac(a, k[1], k[1]);
-    mac(a, k[2], k[2]);
-    const i64 k2 = q63(a);
-    zero |= k2 == 0;
-    // z = |kappa|^2 4^(ez - 1) 4^-doublings <= 1/4
-    const int lead = clz64((u64)k2), dbl = 2 * ez + 2 - lead, doublings = dbl > 0 ? dbl >> 1 : 0;
-    const int zs = 2 - 2 * ez + 2 * doublings;
-    const i64 zw = zs >= 0 ? k2 >> (zs > 62 ? 62 : zs) : shl(k2, -zs);
-    const Limb z = limb(zw + 16);
-    // z < 2^-n: the first term left out is below 2^-65
-    const int nz = clz64((u64)zw) - 1;
-    const int terms = nz >= 20 ? 2 : (nz >= 13 ? 3 : (nz >= 9 ? 4 : (nz >= 7 ? 5 : (nz >= 5 ? 6 : 8))));
-    i64 sb = kHalfAngle[terms - 1][0], cb = kHalfAngle[terms - 1][1];
-#pragma unroll 1
-    for (int i = terms - 2; i >= 0; --i) {
-      sb = kHalfAngle[i][0] - mulq(z, limb(sb));
-      cb = kHalfAngle[i][1] - mulq(z, limb(cb));
-    }
-    i64 s2 = kHalf - q63(mac0(z, limb(sb)), -1), w2 = kHalf - q63(mac0(z, limb(cb)), -1);  // S / 2, w / 2
-#pragma unroll 1
-    for (int i = 0; i < doublings; ++i) {
-      const Limb sl = limb(s2 + 16), wl = limb(w2 + 16);
-      s2 = q63(mac0(sl, wl), 1);
-      w2 = (i64)((u64)q63(mac0(wl, wl), 2) - (u64)kHalf);
-    }
-    const Limb sl = limb(s2 + 16);
-    const Limb fs = limb(mulq(sl, limb(w2 + 16), 1)), fp = limb(mulq(sl, sl, 1));  // S w / 2, S^2 / 2
-    // tau = 2^ts v x kappa, as large as |v| < 0.251 and |kappa| < 2^((1 - lead) / 2) let it be
-    // (and b times that)
-    const int tb = ez - (lead >> 1);
-    const int ts = (lead < 30 ? 2 + ((lead > 2 ? lead - 2 : 0) >> 1) : 16) - (tb > 0 ? tb : 0);
-    const int us = ts - ez > 62 ? 62 : ts - ez;
-    const i64 half = us > 0 ? (1ll << us) >> 1 : 0;
-    view.cross(v, k, t);
-    Limb tau[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) tau[c] = limb(q63(t[c], ts) - (16 << ts) + 16);  // (the limb's half was shifted with the product)
-    view.cross(tau, k, t);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const i64 p = q63(t[c]) - 16;  // 2^(ez - 1) tau x kappa
-      Acc d = mac0(fs, tau[c]);
-      mac(d, fp, limb((ez >= 1 ? shl(p, ez - 1) : p >> ps) + 16));
-      const i64 u = q63(d, 1);
-      y[c] += us < 0 ? shl(u, -us) : (u + half) >> us;
-    }
+    zero |= !rotate(ez, k, y);
   }
 #pragma unroll
   for (int c = 0; c < 3; ++c) e[c] = y8[c] - y[c];
   return !zero;
+}
+
+// The quaternion steppers' rotations in the order they are applied, each at a node (the halves of
+// it and of its square) by a weight: RK45's proposal (5), its comparison (4); RKF45's 5, whose
+// first four are the comparison.
+struct QuatRow {
+  Limb c, c2, w;
+};
+#define ST_Q(node, w) {coef(node, 1), coef((node) * (node), 1), coef(w, 0)}
+static __constant__ QuatRow kQuatRows[14] = {
+    ST_Q(0.0, rk45::CH1),      ST_Q(rk45::A3, rk45::CH3),   ST_Q(rk45::A4, rk45::CH4),   ST_Q(rk45::A5, rk45::CH5),
+    ST_Q(rk45::A6, rk45::CH6), ST_Q(0.0, rk45::C1),         ST_Q(rk45::A3, rk45::C3),    ST_Q(rk45::A4, rk45::C4),
+    ST_Q(rk45::A5, rk45::C5),  ST_Q(0.0, rkf45::C1),        ST_Q(rkf45::A3, rkf45::C3),  ST_Q(rkf45::A4, rkf45::C4),
+    ST_Q(rkf45::A5, rkf45::C5), ST_Q(rkf45::A6, rkf45::C6)};
+#undef ST_Q
+
+// One step of RK45 (F: RKF45) with quaternions: the rotations turn the spin one after another,
+// which is what the product of their quaternions does.  Proposal in w, its difference from the
+// comparison in e.  False: out of range, as magnus_step.
+template <bool F>
+__device__ __forceinline__ bool quat_step(const SegScale& q, const i64* o0, const i64* o1, const i64* o2, i64 ga, u64 wm, int we,
+                                          double x, double tx, double h, const i64* S, i64* w, i64* e) {
+  StepField<3> f;
+  if (!step_field(q, o0, o1, o2, ga, wm, we, x, tx, h, 3, f)) return false;
+  i64 y[3] = {S[0], S[1], S[2]}, y0[3] = {S[0], S[1], S[2]};
+  bool ok = true;
+  constexpr int kFirst = F ? 9 : 0, kLast = F ? 14 : 9, kSwap = F ? 13 : 5;
+#pragma unroll 1
+  for (int n = kFirst; n < kLast; ++n) {
+    if (n == kSwap) {  // RK45: proposal done, comparison from S; RKF45: comparison done
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        y0[c] = y[c];
+        if (!F) y[c] = S[c];
+      }
+    }
+    const QuatRow& row = kQuatRows[n];
+    Limb k[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      i64 o = f.at(c, row.c, row.c2);
+      if (c == 2 && f.pulse) o += f.pulse_at(row.c);
+      k[c] = limb(mulq(row.w, limb(o)));
+    }
+    ok &= rotate(f.ez, k, y);
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    w[c] = F ? y[c] : y0[c];
+    e[c] = F ? y[c] - y0[c] : y0[c] - y[c];
+  }
+  return ok;
 }
 
 }  // namespace fx

@@ -12,8 +12,8 @@
 // lane serves CW particle slots (slot lane + 32 c of the block): every pass it
 // takes the slot of its CW whose ring holds the fewest records and runs one
 // trajectory event for it, so producer lanes are busy whenever any of their
-// slots has room, and the integer-heavy trajectory code overlaps the
-// consumers' FP64 stream on the same SM.
+// slots has room, and the trajectory overlaps the consumers' steps on the same
+// SM (worth it for few particles: 1,000 x 0.5 s, 46.6 ms against 55.8 for the trajectory-ahead kernel).
 //
 // A slot's trajectory state lives in shared memory.  The consumer writes it at
 // a particle's fetch and reads it at window ends; the producer owns it in
