@@ -632,13 +632,12 @@ def run_ours(args, world, rank, local):
             "work_per_launch": {"dop_attempts": counters["dop_attempts"], "segments": counters["segments"],
                                 "flops": flops, "kernel_ms": kernel_s * 1e3}}
     # DRAM bytes of one launch, from an ncu capture of dram__bytes_read.sum + dram__bytes_write.sum
-    # (one pass) of this kernel on this workload at its full size, 1,048,576 particles and two
-    # windows: 279.85 MB read (the state, once) + 453.40 MB written (the state and a snapshot block
-    # at each window end), 699 B per particle per two windows; other sizes scale by particles and
-    # windows (every particle's state and snapshot cross DRAM once per window end).
-    roof["traffic"] = 733.3e6 * (n / 1048576.0) * (nwin / 2.0)
-    roof["traffic_source"] = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of this kernel on the full "
-                              "workload (1,048,576 particles, 2 windows: 733.3 MB), scaled to this launch")
+    # (one pass) of this kernel on 1,048,576 particles x 0.1 s: 25.2 GB read + 19.5 GB written for
+    # 156.7 M segments, 286 B each: the segment records' way through the rings, which together
+    # exceed L2.  Other sizes scale by segments.
+    roof["traffic"] = 286.0 * counters["segments"]
+    roof["traffic_source"] = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of this kernel on 1,048,576 "
+                              "particles x 0.1 s (44.8 GB, 286 B per segment), scaled by segments")
 
     # ---- plain one-thread-per-particle kernel on the same workload (1 step)
     plain = None

@@ -317,8 +317,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_persistent(RunArgs a) {
 // two phases alternated every other attempt and half the time went into
 // instruction supply (1,048,576 particles x 0.1 s: 398 ms with the trajectory
 // in FP64, 463 ms with its faster but larger integer code).  A ring of 64 records is
-// about 190 attempts; its 5 KB per lane live in L2 and cost ~160 bytes of traffic per
-// segment.
+// about 190 attempts.  The rings of a full grid (5 KB a lane, 10 with 128 records) exceed L2:
+// 286 bytes of DRAM traffic per segment, 142 GB/s, 2% of the copy bandwidth.
 //
 // The trajectory side crosses window ends and goes on to its next particle, so
 // rings never block there: at a window end it saves its state in one of
