@@ -876,7 +876,7 @@ __device__ __forceinline__ double as_f64(fx::i64 m) { return __longlong_as_doubl
 __device__ __forceinline__ fx::i64 as_i64(double x) { return __double_as_longlong(x); }
 
 // The field of a segment as the trajectory side hands it to the spin side:
-// the polynomial's o0 and o1, for DOP853, Magnus and quaternion sets scaled to fixed point where they
+// the polynomial's o0 and o1, for DOP853 and quaternion sets scaled to fixed point where they
 // have a scale there (fx; then o0 and o1 hold Q63 words).
 struct SegPoly {
   double o0[3], o1[3], o2[3];
@@ -888,7 +888,7 @@ __device__ __forceinline__ void seg_scale(SegPoly& q, const SetParams& P, double
   q.fx = false;
 #if ST_GRAD_IS_LINEAR && ST_PULSE_IS_Z_COS
   const double gpa = P.gamma * P.a;
-  if (((P.integrator == 0 && P.tol_ratio >= 0.0) || P.integrator == 2 || P.integrator == 3 || P.integrator == 5) && (gpa == 0.0 || isfinite(P.w)))
+  if (((P.integrator == 0 && P.tol_ratio >= 0.0) || P.integrator == 3 || P.integrator == 5) && (gpa == 0.0 || isfinite(P.w)))
     q.fx = fx::field_scale(q.o0, q.o1, P.o2c, gpa, T, q.sc);
   if (q.fx) {
     const int e0 = q.sc.oe, e1 = e0 - q.sc.te, e2 = e1 - q.sc.te;
@@ -1666,24 +1666,22 @@ __device__ __forceinline__ void rkf45_stages(Seg& g, const SetParams& P, double 
 
 // The same in FP64 for a segment that may be in fixed point; a call, not inlined: the
 // fixed-point step takes all but a few.
-static __device__ __noinline__ void rotation_slow(const Seg& g, const SetParams& P, double tx, double h, double Sx, double Sy,
+static __device__ __noinline__ void quat_slow(const Seg& g, const SetParams& P, double tx, double h, double Sx, double Sy,
                                                   double Sz, double w[3], double e[3]) {
   Seg t = g;
   if (t.fx) seg_unscale(t);
-  if (P.integrator == 2)
-    magnus_stages(t, P, tx, h, Sx, Sy, Sz, w, e);
-  else if (P.integrator == 3)
+  if (P.integrator == 3)
     quat_stages<false>(t, P, tx, h, Sx, Sy, Sz, w, e);
   else
     quat_stages<true>(t, P, tx, h, Sx, Sy, Sz, w, e);
 }
 
-// The proposal and error vector of a Magnus or quaternion step: in fixed point where it fits.  In
-// FP64 an attempt's 16 rotations are some 100 FP64 instructions of 76 cycles each.  65,536
-// particles x 0.1 s: 51.9 ms with them, 28.1 in fixed point, 13.5 without the step.  A
-// quaternion RKF45 attempt took 700 FP64 instructions; RK45, RKF45 and both quaternion forms,
-// 4,096 particles each: 92 ms, 44 with the quaternion forms in fixed point.
-__device__ __forceinline__ void rotation_step(const Seg& g, const SetParams& P, double tx, double h, double Sx, double Sy,
+// The proposal and error vector of a quaternion step: in fixed point where it fits.  In FP64 an
+// attempt of the quaternion RKF45 takes 700 FP64 instructions of 76 cycles: RK45, RKF45 and both
+// quaternion forms, 4,096 particles each, 92 ms, 44 with the quaternion forms in fixed point.
+// (The Magnus stepper stays in FP64: its error estimate is rounding noise on smooth fields, so
+// its steps of a radian and more, and the turns counted at their ends, hang on the noise's bits.)
+__device__ __forceinline__ void quat_step(const Seg& g, const SetParams& P, double tx, double h, double Sx, double Sy,
                                               double Sz, double w[3], double e[3]) {
 #if ST_GRAD_IS_LINEAR && ST_PULSE_IS_Z_COS
   if (g.fx) {
@@ -1697,9 +1695,8 @@ __device__ __forceinline__ void rotation_step(const Seg& g, const SetParams& P, 
 #pragma unroll
       for (int c = 0; c < 3; ++c) q[c] = fx::to_q63(S[c], se);
       const fx::i64 ga = as_i64(g.gpa);
-      const bool ok = P.integrator == 2   ? fx::magnus_step(g.sc, o0, o1, o2, ga, P.wturn_m, P.wturn_e, g.x, tx, h, q, y, d)
-                      : P.integrator == 3 ? fx::quat_step<false>(g.sc, o0, o1, o2, ga, P.wturn_m, P.wturn_e, g.x, tx, h, q, y, d)
-                                          : fx::quat_step<true>(g.sc, o0, o1, o2, ga, P.wturn_m, P.wturn_e, g.x, tx, h, q, y, d);
+      const bool ok = P.integrator == 3 ? fx::quat_step<false>(g.sc, o0, o1, o2, ga, P.wturn_m, P.wturn_e, g.x, tx, h, q, y, d)
+                                        : fx::quat_step<true>(g.sc, o0, o1, o2, ga, P.wturn_m, P.wturn_e, g.x, tx, h, q, y, d);
       if (ok) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -1713,7 +1710,7 @@ __device__ __forceinline__ void rotation_step(const Seg& g, const SetParams& P, 
 #endif
   const Seg t = g;  // (their addresses go to the call: g, w and e stay in registers)
   double ws[3], es[3];
-  rotation_slow(t, P, tx, h, Sx, Sy, Sz, ws, es);
+  quat_slow(t, P, tx, h, Sx, Sy, Sz, ws, es);
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     w[c] = ws[c];
@@ -1750,8 +1747,10 @@ __device__ __forceinline__ int ext_attempt(Seg& g, const SetParams& P, double& S
   }
   const double tx = g.x - g.t0;
   double w[3], e[3];
-  if (P.integrator != 4)
-    rotation_step(g, P, tx, h, Sx, Sy, Sz, w, e);
+  if (P.integrator == 2)
+    magnus_stages(g, P, tx, h, Sx, Sy, Sz, w, e);
+  else if (P.integrator != 4)
+    quat_step(g, P, tx, h, Sx, Sy, Sz, w, e);
   else
     rkf45_stages(g, P, tx, h, Sx, Sy, Sz, w, e);
   double error = sfp::sqrt_rn(fma(e[2], e[2], fma(e[1], e[1], e[0] * e[0])));

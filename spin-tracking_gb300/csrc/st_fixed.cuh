@@ -1,4 +1,4 @@
-// DOP853, Magnus and quaternion step arithmetic in 64-bit fixed point on the integer pipes.
+// DOP853 and quaternion step arithmetic in 64-bit fixed point on the integer pipes.
 //
 // GB300 issues one FP64 warp instruction per 64 or more cycles on each SM
 // sub-partition (measured: 76 cycles per DFMA, DADD, DMUL or DSETP), while a
@@ -968,34 +968,7 @@ __device__ __forceinline__ bool dop_adjoint(KS& ks, KS& ys, const SegScale& q, c
   return true;
 }
 
-// ---------------------------------------------------------------- Magnus step
-// The 16 exponents' weights of the five node fields in the order they are applied
-// (11 of CFET8, rows 1..5 with the nodes reversed, then rows 6..1; 5 of CFET6,
-// rows 1 and 2 reversed, then rows 3..1).  A row's magnitudes sum to less than 1.45.
-namespace cfx {
-constexpr double g[6][5] = {{cfet::G11, cfet::G12, cfet::G13, cfet::G14, cfet::G15},
-                            {cfet::G21, cfet::G22, cfet::G23, cfet::G24, cfet::G25},
-                            {cfet::G31, cfet::G32, cfet::G33, cfet::G34, cfet::G35},
-                            {cfet::G41, cfet::G42, cfet::G43, cfet::G44, cfet::G45},
-                            {cfet::G51, cfet::G52, cfet::G53, cfet::G54, cfet::G55},
-                            {cfet::G61, cfet::G62, cfet::G63, cfet::G64, cfet::G65}};
-constexpr double h[3][5] = {{cfet::H11, cfet::H12, cfet::H13, cfet::H14, cfet::H15},
-                            {cfet::H21, cfet::H22, cfet::H23, cfet::H24, cfet::H25},
-                            {cfet::H31, cfet::H32, cfet::H33, cfet::H34, cfet::H35}};
-constexpr double x[5] = {cfet::X1, cfet::X2, cfet::X3, cfet::X4, cfet::X5};
-constexpr double weight(int n, int j) {
-  return n < 5 ? g[n][4 - j] : n < 11 ? g[10 - n][j] : n < 13 ? h[n - 11][4 - j] : h[15 - n][j];
-}
-}  // namespace cfx
-#define ST_W(n) \
-  {coef(cfx::weight(n, 0), 0), coef(cfx::weight(n, 1), 0), coef(cfx::weight(n, 2), 0), coef(cfx::weight(n, 3), 0), \
-   coef(cfx::weight(n, 4), 0)}
-static __constant__ Limb kMagnusCoef[16][5] = {ST_W(0), ST_W(1), ST_W(2),  ST_W(3),  ST_W(4),  ST_W(5),  ST_W(6),  ST_W(7),
-                                               ST_W(8), ST_W(9), ST_W(10), ST_W(11), ST_W(12), ST_W(13), ST_W(14), ST_W(15)};
-#undef ST_W
-#define ST_X(j) {coef(cfx::x[j], 1), coef(cfx::x[j] * cfx::x[j], 1)}
-static __constant__ Limb kMagnusNode[5][2] = {ST_X(0), ST_X(1), ST_X(2), ST_X(3), ST_X(4)};
-#undef ST_X
+// ---------------------------------------------------------------- rotations
 // 1 / (2k + 3)! and 1 / (2k + 2)! as Q63: sin b / b = 1 - z (1/3! - z/5! ...), cos b = 1 - z (1/2! - z/4! ...), z = b^2
 static __constant__ i64 kHalfAngle[8][2] = {
     {1537228672809129301ll, 4611686018427387904ll}, {76861433640456465ll, 384307168202282325ll},
@@ -1065,52 +1038,6 @@ __device__ __forceinline__ bool rotate(int ez, const Limb* k, i64* y) {
   return k2 != 0;
 }
 
-// One Magnus step (CFET8 with its CFET6 companion) of size h at tau = tx (t = x) over a
-// scaled segment: the proposal in y8, its difference from the companion's in e.
-// False: out of range (above 4 rad, off the segment, no field): the caller takes FP64.
-__device__ __forceinline__ bool magnus_step(const SegScale& q, const i64* o0, const i64* o1, const i64* o2, i64 ga, u64 wm,
-                                            int we, double x, double tx, double h, const i64* S, i64* y8, i64* e) {
-  Limb W[5][3];
-  int ez;
-  {
-    StepField<3> f;
-    if (!step_field(q, o0, o1, o2, ga, wm, we, x, tx, h, 3, f)) return false;
-    ez = f.ez;
-#pragma unroll
-    for (int i = 0; i < 5; ++i)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        i64 w = f.at(c, kMagnusNode[i][0], kMagnusNode[i][1]);
-        if (c == 2 && f.pulse) w += f.pulse_at(kMagnusNode[i][0]);
-        W[i][c] = limb(w);
-      }
-  }
-  i64 y[3] = {S[0], S[1], S[2]};
-  bool zero = false;
-#pragma unroll 1
-  for (int n = 0; n < 16; ++n) {
-    if (n == 11) {  // CFET8 done: CFET6 from S
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        y8[c] = y[c];
-        y[c] = S[c];
-      }
-    }
-    const Limb* cf = kMagnusCoef[n];
-    Limb k[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      Acc a = mac0(cf[0], W[0][c], kHalfLimb);
-#pragma unroll
-      for (int j = 1; j < 5; ++j) mac(a, cf[j], W[j][c]);
-      k[c] = limb(q63(a));
-    }
-    zero |= !rotate(ez, k, y);
-  }
-#pragma unroll
-  for (int c = 0; c < 3; ++c) e[c] = y8[c] - y[c];
-  return !zero;
-}
 
 // The quaternion steppers' rotations in the order they are applied, each at a node (the halves of
 // it and of its square) by a weight: RK45's proposal (5), its comparison (4); RKF45's 5, whose
@@ -1128,7 +1055,7 @@ static __constant__ QuatRow kQuatRows[14] = {
 
 // One step of RK45 (F: RKF45) with quaternions: the rotations turn the spin one after another,
 // which is what the product of their quaternions does.  Proposal in w, its difference from the
-// comparison in e.  False: out of range, as magnus_step.
+// comparison in e.  False: out of range (above 4 rad, off the segment, no field): the caller takes FP64.
 template <bool F>
 __device__ __forceinline__ bool quat_step(const SegScale& q, const i64* o0, const i64* o1, const i64* o2, i64 ga, u64 wm, int we,
                                           double x, double tx, double h, const i64* S, i64* w, i64* e) {
