@@ -154,11 +154,8 @@ __device__ __forceinline__ bool lt(double a, double b) { return key(a) < key(b) 
 __device__ __forceinline__ bool le(double a, double b) { return key(a) <= key(b) && !is_nan(a) && !is_nan(b); }
 __device__ __forceinline__ bool eq(double a, double b) { return key(a) == key(b) && !is_nan(a) && !is_nan(b); }
 __device__ __forceinline__ bool negative(double x) { return f64_bits(x) > kSign && !is_nan(x); }  // x < 0
-// |a| > b for b >= 0 that is a number
-__device__ __forceinline__ bool abs_gt(double a, double b) {
-  const u64 m = f64_bits(a) & ~kSign;
-  return m > f64_bits(b) && m <= 0x7ff0000000000000ull;
-}
+// |a| > b (any b: a limit below zero is exceeded by every number)
+__device__ __forceinline__ bool abs_gt(double a, double b) { return lt(b, bits_f64(f64_bits(a) & ~kSign)); }
 
 }  // namespace sfp
 }  // namespace st
