@@ -240,7 +240,7 @@ template <int BLOCK>
 static __device__ __noinline__ void dop_adjoint_slow(const Seg& g, const SetParams& P, double x, double h, const double y[3],
                                                      double lam[3], Moments& M, bool pulse, double* sm) {
   Seg t = g;
-  if (t.fx) seg_unscale(t);
+  if (t.fx) seg_unscale(t, P);
   dop_step_adjoint<BLOCK>(t, P, x, h, y, lam, M, pulse, sm);
 }
 
@@ -266,39 +266,57 @@ template <int BLOCK>
 __device__ __forceinline__ void dop_adjoint_step(const Seg& g, const SetParams& P, double x, double h, const double y[3],
                                                  double lam[3], Moments& M, bool pulse, double* sm) {
 #if ST_GRAD_IS_LINEAR && ST_PULSE_IS_Z_COS
-  int se, le;
-  if (g.fx && fx::spin_scale(y, se) && fx::spin_scale(lam, le) && le > -800 && le < 800 && se + le > -800 && se + le < 800) {
-    const fx::i64 o0[3] = {as_i64(g.o0x), as_i64(g.o0y), as_i64(g.o0z)};
-    const fx::i64 o1[3] = {as_i64(g.o1x), as_i64(g.o1y), as_i64(g.o1z)};
-    const fx::i64 o2[3] = {as_i64(g.o2x), as_i64(g.o2y), as_i64(g.o2z)};
-    fx::i64 S[3], L[3];
+  if (g.fx) {
+    double yw[3] = {y[0], y[1], y[2]}, lw[3] = {lam[0], lam[1], lam[2]};
+    turn_by(yw[0], yw[1], yw[2], P.axis);
+    turn_by(lw[0], lw[1], lw[2], P.axis);
+    fx::SegScale sc = g.sc;
+    sc.pz = P.pz;
+    int le, gl;
+    if (fx::spin_scale(yw, sc.se) && fx::adjoint_scale(lw, sc.ok, le, gl) && le > -800 && le < 800 && sc.se + le > -800 &&
+        sc.se + le < 800) {
+      const fx::i64 o0[3] = {as_i64(g.o0x), as_i64(g.o0y), as_i64(g.o0z)};
+      const fx::i64 o1[3] = {as_i64(g.o1x), as_i64(g.o1y), as_i64(g.o1z)};
+      const fx::i64 o2[3] = {as_i64(g.o2x), as_i64(g.o2y), as_i64(g.o2z)};
+      fx::i64 S[3], L[3];
+      sc.sk = fx::spin_grade(yw, sc.se, sc.ok);
+      fx::spin_words(yw, sc.se, sc.sk, S);
+      fx::spin_words(lw, le, gl, L);
+      // both stage arrays in this thread's own 72 words: other lanes may be in the FP64 form
+      StageWords ks{reinterpret_cast<fx::Limb*>(sm), BLOCK}, ys{reinterpret_cast<fx::Limb*>(sm) + 36 * BLOCK, BLOCK};
+      fx::AdjMoments m;
+      const double tx = x - g.t0;
+      if (fx::dop_adjoint(ks, ys, sc, o0, o1, o2, as_i64(g.gpa), P.wturn_m, P.wturn_e, x, tx, h, pulse, S, L, m, gl)) {
+        const fx::Grade gr{gl};
+        const int E = sc.se + le + m.exp;
+        const double hh = h * h;
+        double z0[3], z1[3], z2[3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      S[c] = fx::to_q63(y[c], se);
-      L[c] = fx::to_q63(lam[c], le);
-    }
-    // both stage arrays in this thread's own 72 words: other lanes may be in the FP64 form
-    StageWords ks{reinterpret_cast<fx::Limb*>(sm), BLOCK}, ys{reinterpret_cast<fx::Limb*>(sm) + 36 * BLOCK, BLOCK};
-    fx::AdjMoments m;
-    const double tx = x - g.t0;
-    if (fx::dop_adjoint(ks, ys, g.sc, o0, o1, o2, as_i64(g.gpa), P.wturn_m, P.wturn_e, x, tx, h, pulse, S, L, m)) {
-      const int E = se + le + m.exp;
-      const double hh = h * h;
+        for (int c = 0; c < 3; ++c) {
+          lam[c] = fx::from_q63(L[c], le - (c == 0 ? gr.e0() : gr.e1()));
+          // sums over the stages at tau = tx + c h
+          z0[c] = h * fx::from_q63(m.z0[c], E - m.e[c]);
+          z1[c] = hh * fx::from_q63(m.z1[c], E - m.e[c]);
+          z2[c] = hh * fx::from_q63(m.z2[c], E - m.e[c]);
+        }
+        unturn(lam[0], lam[1], lam[2], P.axis);
+        unturn(z0[0], z0[1], z0[2], P.axis);
+        unturn(z1[0], z1[1], z1[2], P.axis);
+        unturn(z2[0], z2[1], z2[2], P.axis);
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        lam[c] = fx::from_q63(L[c], le);
-        // sums over the stages at tau = tx + c h
-        const double z0 = h * fx::from_q63(m.z0[c], E), z1 = hh * fx::from_q63(m.z1[c], E), z2 = hh * fx::from_q63(m.z2[c], E);
-        M.z0[c] += z0;
-        M.z1[c] += fma(tx, z0, z1);
-        M.z2[c] += fma(tx, fma(tx, z0, 2.0 * z1), h * z2);
+        for (int c = 0; c < 3; ++c) {
+          M.z0[c] += z0[c];
+          M.z1[c] += fma(tx, z0[c], z1[c]);
+          M.z2[c] += fma(tx, fma(tx, z0[c], 2.0 * z1[c]), h * z2[c]);
+        }
+        if (pulse) {  // the phases are those of |w|
+          const int Ez = E + 1 - (P.pz == 0 ? m.e[0] : m.e[1]);
+          const double sz = h * fx::from_q63(m.sz, Ez), scz = hh * fx::from_q63(m.scz, Ez);
+          M.ga = fma(P.gamma * h, fx::from_q63(m.cz, Ez), M.ga);
+          M.gw = fma(P.w < 0.0 ? P.gamma * P.a : -P.gamma * P.a, fma(x, sz, scz), M.gw);
+        }
+        return;
       }
-      if (pulse) {  // the phases are those of |w|
-        const double sz = h * fx::from_q63(m.sz, E + 1), sc = hh * fx::from_q63(m.scz, E + 1);
-        M.ga = fma(P.gamma * h, fx::from_q63(m.cz, E + 1), M.ga);
-        M.gw = fma(P.w < 0.0 ? P.gamma * P.a : -P.gamma * P.a, fma(x, sz, sc), M.gw);
-      }
-      return;
     }
   }
 #endif

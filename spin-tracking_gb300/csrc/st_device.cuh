@@ -825,6 +825,9 @@ __device__ inline void prepare_set(SetParams& P) {
     }
   }
   P.gB0[0] = gm * P.B0x; P.gB0[1] = gm * P.B0y; P.gB0[2] = gm * P.B0z;
+  P.axis = fabs(P.gB0[1]) > fabs(P.gB0[0]) ? 1 : 0;
+  if (fabs(P.gB0[2]) > fabs(P.gB0[P.axis])) P.axis = 2;
+  P.pz = (5 - P.axis) % 3;
   const Vec3 ex = {1.0, 0.0, 0.0}, ey = {0.0, 1.0, 0.0}, ez = {0.0, 0.0, 1.0};
   const Vec3 c0 = st_grad(ex, P), c1 = st_grad(ey, P), c2 = st_grad(ez, P);
   P.gGc[0][0] = gm * c0.x; P.gGc[0][1] = gm * c0.y; P.gGc[0][2] = gm * c0.z;
@@ -838,6 +841,7 @@ __device__ inline void prepare_set(SetParams& P) {
 #else
   P.o2c[0] = P.o2c[1] = P.o2c[2] = 0.0;  // the hook is evaluated at every stage instead
 #endif
+  for (int c = 0; c < 3; ++c) P.o2w[c] = P.o2c[(c + P.axis) % 3];
 }
 
 // Coefficients o0, o1 of the field polynomial of a segment starting at (p0, v0).
@@ -875,9 +879,23 @@ __device__ __forceinline__ void seg_begin(Seg& g, const SetParams& P, double t0,
 __device__ __forceinline__ double as_f64(fx::i64 m) { return __longlong_as_double(m); }
 __device__ __forceinline__ fx::i64 as_i64(double x) { return __double_as_longlong(x); }
 
+// Components turned n places (0 to 2): x becomes component n.  Words have the set's axis first
+// (n = P.axis); back with unturn.
+template <class T>
+__device__ __forceinline__ void turn_by(T& x, T& y, T& z, int n) {
+#pragma unroll 1
+  for (; n > 0; --n) {
+    const T t = x;
+    x = y;
+    y = z;
+    z = t;
+  }
+}
+__device__ __forceinline__ void unturn(double& x, double& y, double& z, int axis) { turn_by(x, y, z, axis == 0 ? 0 : 3 - axis); }
+
 // The field of a segment as the trajectory side hands it to the spin side:
 // the polynomial's o0 and o1, for DOP853 and quaternion sets scaled to fixed point where they
-// have a scale there (fx; then o0 and o1 hold Q63 words).
+// have a scale there (fx; then o0, o1 and o2 hold Q63 words, the set's axis first).
 struct SegPoly {
   double o0[3], o1[3], o2[3];
   fx::SegScale sc;
@@ -889,14 +907,23 @@ __device__ __forceinline__ void seg_scale(SegPoly& q, const SetParams& P, double
 #if ST_GRAD_IS_LINEAR && ST_PULSE_IS_Z_COS
   const double gpa = P.gamma * P.a;
   if (((P.integrator == 0 && P.tol_ratio >= 0.0) || P.integrator == 3 || P.integrator == 5) && (gpa == 0.0 || isfinite(P.w)))
-    q.fx = fx::field_scale(q.o0, q.o1, P.o2c, gpa, T, q.sc);
+  {
+    turn_by(q.o0[0], q.o0[1], q.o0[2], P.axis);
+    turn_by(q.o1[0], q.o1[1], q.o1[2], P.axis);
+    q.sc.pz = P.pz;
+    q.fx = fx::field_scale(q.o0, q.o1, P.o2w, gpa, T, q.sc, true);
+    if (!q.fx) {
+      unturn(q.o0[0], q.o0[1], q.o0[2], P.axis);
+      unturn(q.o1[0], q.o1[1], q.o1[2], P.axis);
+    }
+  }
   if (q.fx) {
-    const int e0 = q.sc.oe, e1 = e0 - q.sc.te, e2 = e1 - q.sc.te;
 #pragma unroll 1  // rolled: less code
     for (int c = 0; c < 3; ++c) {
+      const int e0 = q.sc.oe - (c == 0 ? 0 : q.sc.ok), e1 = e0 - q.sc.te, e2 = e1 - q.sc.te;
       q.o0[c] = as_f64(fx::to_q63(q.o0[c], e0));
       q.o1[c] = as_f64(fx::to_q63(q.o1[c], e1));
-      q.o2[c] = as_f64(fx::to_q63(P.o2c[c], e2));
+      q.o2[c] = as_f64(fx::to_q63(P.o2w[c], e2));
     }
   }
 #endif
@@ -910,12 +937,13 @@ __device__ __forceinline__ void seg_poly(SegPoly& q, const SetParams& P, const S
 __device__ __forceinline__ void seg_open(Seg& g, const SetParams& P, const SegPoly& q, double t0, double t_end) {
   seg_begin(g, P, t0, t_end, q.o0, q.o1);
   g.fx = q.fx;
-  const int se = g.sc.se;  // the spin's own scale goes on
+  const int se = g.sc.se, sk = g.sc.sk;  // the spin's own scale and grade go on
   g.sc = q.sc;
   g.sc.se = se;
+  g.sc.sk = sk;
   if (q.fx) {
     g.o2x = q.o2[0]; g.o2y = q.o2[1]; g.o2z = q.o2[2];
-    g.gpa = as_f64(fx::to_q63(g.gpa, q.sc.oe));
+    g.gpa = as_f64(fx::to_q63(g.gpa, q.sc.oe - (P.pz == 0 ? 0 : q.sc.ok)));
   }
 }
 
@@ -1015,32 +1043,64 @@ __device__ __forceinline__ void homega_at(const HPoly& q, const Seg& g, const Se
 
 // ------------------------------------------------------------ DOP853
 // A fixed-point segment's field back in doubles.
-__device__ __forceinline__ void seg_unscale(Seg& g) {
-  const int e0 = g.sc.oe, e1 = e0 - g.sc.te, e2 = e1 - g.sc.te;
-  g.o0x = fx::from_q63(as_i64(g.o0x), e0); g.o0y = fx::from_q63(as_i64(g.o0y), e0); g.o0z = fx::from_q63(as_i64(g.o0z), e0);
-  g.o1x = fx::from_q63(as_i64(g.o1x), e1); g.o1y = fx::from_q63(as_i64(g.o1y), e1); g.o1z = fx::from_q63(as_i64(g.o1z), e1);
-  g.o2x = fx::from_q63(as_i64(g.o2x), e2); g.o2y = fx::from_q63(as_i64(g.o2y), e2); g.o2z = fx::from_q63(as_i64(g.o2z), e2);
-  g.gpa = fx::from_q63(as_i64(g.gpa), e0);
+__device__ __forceinline__ void seg_unscale(Seg& g, const SetParams& P) {
+  const int e0 = g.sc.oe, e1 = e0 - g.sc.te, e2 = e1 - g.sc.te, ok = g.sc.ok;
+  g.o0x = fx::from_q63(as_i64(g.o0x), e0);
+  g.o0y = fx::from_q63(as_i64(g.o0y), e0 - ok);
+  g.o0z = fx::from_q63(as_i64(g.o0z), e0 - ok);
+  g.o1x = fx::from_q63(as_i64(g.o1x), e1);
+  g.o1y = fx::from_q63(as_i64(g.o1y), e1 - ok);
+  g.o1z = fx::from_q63(as_i64(g.o1z), e1 - ok);
+  g.o2x = fx::from_q63(as_i64(g.o2x), e2);
+  g.o2y = fx::from_q63(as_i64(g.o2y), e2 - ok);
+  g.o2z = fx::from_q63(as_i64(g.o2z), e2 - ok);
+  unturn(g.o0x, g.o0y, g.o0z, P.axis);
+  unturn(g.o1x, g.o1y, g.o1z, P.axis);
+  unturn(g.o2x, g.o2y, g.o2z, P.axis);
+  g.gpa = fx::from_q63(as_i64(g.gpa), e0 - (P.pz == 0 ? 0 : ok));
   g.fx = false;
 }
 
 // The spin of a fixed-point segment in progress as doubles.
-__device__ __forceinline__ void dop_spin(const Seg& g, double& Sx, double& Sy, double& Sz) {
-  Sx = fx::from_q63(as_i64(g.kx), g.sc.se);
-  Sy = fx::from_q63(as_i64(g.ky), g.sc.se);
-  Sz = fx::from_q63(as_i64(g.kz), g.sc.se);
+__device__ __forceinline__ void dop_spin(const Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz) {
+  const fx::Grade k{g.sc.sk};
+  Sx = fx::from_q63(as_i64(g.kx), g.sc.se - k.e0());
+  Sy = fx::from_q63(as_i64(g.ky), g.sc.se - k.e1());
+  Sz = fx::from_q63(as_i64(g.kz), g.sc.se - k.e1());
+  unturn(Sx, Sy, Sz, P.axis);
 }
 
 // A spin in fixed point stays there from segment to segment (g.carry): it becomes
 // doubles again at a window end, or where a segment runs in FP64.
-__device__ __forceinline__ void spin_settle(Seg& g, double& Sx, double& Sy, double& Sz) {
-  if (g.carry) dop_spin(g, Sx, Sy, Sz);
+__device__ __forceinline__ void spin_settle(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz) {
+  if (g.carry) dop_spin(g, P, Sx, Sy, Sz);
   g.carry = false;
+}
+
+// A spin as words: ok false where it has no scale, the tolerances do not fit, or a word
+// would lose its sign (-0, or less than half a unit: turns count signs).
+struct SpinWords {
+  fx::i64 w[3];
+  int se, sk;
+  bool ok;
+};
+static __device__ __noinline__ SpinWords spin_words_of(const SetParams& P, int field_grade, double Sx, double Sy, double Sz) {
+  SpinWords r;
+  turn_by(Sx, Sy, Sz, P.axis);
+  const double S[3] = {Sx, Sy, Sz};
+  r.ok = fx::spin_scale(S, r.se) && fx::ratio_fits(P.tol_ratio, r.se);
+  if (r.ok) {
+    r.sk = fx::spin_grade(S, r.se, field_grade);
+    fx::spin_words(S, r.se, r.sk, r.w);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) r.ok &= r.w[c] != 0 || !signbit(S[c]);
+  }
+  return r;
 }
 
 // The derivative at the start of an FP64 segment, taking the segment out of fixed point first.
 static __device__ __noinline__ void dop_begin_f64(Seg& g, const SetParams& P, double Sx, double Sy, double Sz) {
-  if (g.fx) seg_unscale(g);
+  if (g.fx) seg_unscale(g, P);
   feval(g, P, 0.0, Sx, Sy, Sz, g.kx, g.ky, g.kz);
 }
 
@@ -1053,16 +1113,18 @@ __device__ __forceinline__ void dop_begin(Seg& g, const SetParams& P, double& Sx
   g.reject = false;
   g.last = false;
   if (g.fx && !g.carry) {
-    const double S[3] = {Sx, Sy, Sz};
-    if (fx::spin_scale(S, g.sc.se) && fx::ratio_fits(P.tol_ratio, g.sc.se)) {
-      g.kx = as_f64(fx::to_q63(Sx, g.sc.se));
-      g.ky = as_f64(fx::to_q63(Sy, g.sc.se));
-      g.kz = as_f64(fx::to_q63(Sz, g.sc.se));
+    const SpinWords r = spin_words_of(P, g.sc.ok, Sx, Sy, Sz);
+    if (r.ok) {
+      g.kx = as_f64(r.w[0]);
+      g.ky = as_f64(r.w[1]);
+      g.kz = as_f64(r.w[2]);
+      g.sc.se = r.se;
+      g.sc.sk = r.sk;
       g.carry = true;
     }
   }
   if (!(g.fx && g.carry)) {
-    spin_settle(g, Sx, Sy, Sz);
+    spin_settle(g, P, Sx, Sy, Sz);
     Seg t = g;  // the call takes its address: g itself stays in registers
     dop_begin_f64(t, P, Sx, Sy, Sz);
     g = t;
@@ -1218,8 +1280,8 @@ static __device__ __noinline__ int dop_attempt_slow(Seg& g, const SetParams& P, 
   if (!g.fx) return dop_attempt_f64(g, P, Sx, Sy, Sz);
   Seg t = g;
   double x, y, z;
-  dop_spin(g, x, y, z);
-  seg_unscale(t);
+  dop_spin(g, P, x, y, z);
+  seg_unscale(t, P);
   feval(t, P, t.x - t.t0, x, y, z, t.kx, t.ky, t.kz);
   const int r = dop_attempt_f64(t, P, x, y, z);
   if (t.acc) {
@@ -1262,13 +1324,19 @@ __device__ __forceinline__ int dop_attempt_v(const V& view, KS& ks, Seg& g, cons
   fx::StepOut out;
   bool fixed = g.fx;
   if (fixed) {
-    fx::i64 o0[V::N], o1[V::N], o2[V::N], S[V::N];
+    fx::i64 o0[V::N], o1[V::N], o2[V::N], S[V::N], K[3] = {as_i64(g.kx), as_i64(g.ky), as_i64(g.kz)};
+    fx::regrade(K, g.sc.sk, g.sc.ok);
+    g.kx = as_f64(K[0]);
+    g.ky = as_f64(K[1]);
+    g.kz = as_f64(K[2]);
     view.pick(as_i64(g.o0x), as_i64(g.o0y), as_i64(g.o0z), o0);
     view.pick(as_i64(g.o1x), as_i64(g.o1y), as_i64(g.o1z), o1);
     view.pick(as_i64(g.o2x), as_i64(g.o2y), as_i64(g.o2z), o2);
-    view.pick(as_i64(g.kx), as_i64(g.ky), as_i64(g.kz), S);
+    view.pick(K[0], K[1], K[2], S);
     const fx::StepTol tol = {P.rtol, P.tol_ratio};
-    fixed = fx::dop_step(view, ks, g.sc, o0, o1, o2, as_i64(g.gpa), (fx::u64)P.wturn_m, P.wturn_e, g.x, g.x - g.t0, h,
+    fx::SegScale sc = g.sc;
+    sc.pz = P.pz;
+    fixed = fx::dop_step(view, ks, sc, o0, o1, o2, as_i64(g.gpa), (fx::u64)P.wturn_m, P.wturn_e, g.x, g.x - g.t0, h,
                          tol, S, Sn, out);
   }
   if (!fixed) {  // rare: on copies, so that g itself stays in registers
@@ -1294,8 +1362,18 @@ __device__ __forceinline__ int dop_attempt_v(const V& view, KS& ks, Seg& g, cons
     g.hu = h;
     fx::i64 N3[3];
     view.gather(Sn, N3);
-    const fx::i64 y0 = as_i64(g.ky), z0 = as_i64(g.kz);
-    if (y0 < 0 && N3[1] < 0 && (z0 < 0) != (N3[2] < 0)) g.turns += z0 < 0 ? -1 : 1;  // count_turn
+    // count_turn; y is word 1 - axis, z word 2 - axis, modulo 3
+    int y0 = (int)(as_i64(g.ky) >> 32), z0 = (int)(as_i64(g.kz) >> 32), y1 = (int)(N3[1] >> 32), z1 = (int)(N3[2] >> 32);
+    if (P.axis != 0) {
+      const int x0 = (int)(as_i64(g.kx) >> 32), x1 = (int)(N3[0] >> 32);
+      const bool one = P.axis == 1;
+      const int u0 = one ? y0 : x0, u1 = one ? y1 : x1;
+      y0 = one ? x0 : z0;
+      y1 = one ? x1 : z1;
+      z0 = u0;
+      z1 = u1;
+    }
+    if ((y0 & y1 & (z0 ^ z1)) < 0) g.turns += z0 < 0 ? -1 : 1;
     g.kx = as_f64(N3[0]);
     g.ky = as_f64(N3[1]);
     g.kz = as_f64(N3[2]);
@@ -1669,7 +1747,7 @@ __device__ __forceinline__ void rkf45_stages(Seg& g, const SetParams& P, double 
 static __device__ __noinline__ void quat_slow(const Seg& g, const SetParams& P, double tx, double h, double Sx, double Sy,
                                                   double Sz, double w[3], double e[3]) {
   Seg t = g;
-  if (t.fx) seg_unscale(t);
+  if (t.fx) seg_unscale(t, P);
   if (P.integrator == 3)
     quat_stages<false>(t, P, tx, h, Sx, Sy, Sz, w, e);
   else
@@ -1685,24 +1763,30 @@ __device__ __forceinline__ void quat_step(const Seg& g, const SetParams& P, doub
                                               double Sz, double w[3], double e[3]) {
 #if ST_GRAD_IS_LINEAR && ST_PULSE_IS_Z_COS
   if (g.fx) {
-    const double S[3] = {Sx, Sy, Sz};
+    double S[3] = {Sx, Sy, Sz};
+    turn_by(S[0], S[1], S[2], P.axis);
     const fx::i64 o0[3] = {as_i64(g.o0x), as_i64(g.o0y), as_i64(g.o0z)};
     const fx::i64 o1[3] = {as_i64(g.o1x), as_i64(g.o1y), as_i64(g.o1z)};
     const fx::i64 o2[3] = {as_i64(g.o2x), as_i64(g.o2y), as_i64(g.o2z)};
-    int se;
-    if (fx::spin_scale(S, se)) {
+    fx::SegScale sc = g.sc;
+    sc.pz = P.pz;
+    if (fx::spin_scale(S, sc.se)) {
       fx::i64 q[3], y[3], d[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) q[c] = fx::to_q63(S[c], se);
+      sc.sk = fx::spin_grade(S, sc.se, sc.ok);
+      fx::spin_words(S, sc.se, sc.sk, q);
       const fx::i64 ga = as_i64(g.gpa);
-      const bool ok = P.integrator == 3 ? fx::quat_step<false>(g.sc, o0, o1, o2, ga, P.wturn_m, P.wturn_e, g.x, tx, h, q, y, d)
-                                        : fx::quat_step<true>(g.sc, o0, o1, o2, ga, P.wturn_m, P.wturn_e, g.x, tx, h, q, y, d);
+      const bool ok = P.integrator == 3 ? fx::quat_step<false>(sc, o0, o1, o2, ga, P.wturn_m, P.wturn_e, g.x, tx, h, q, y, d)
+                                        : fx::quat_step<true>(sc, o0, o1, o2, ga, P.wturn_m, P.wturn_e, g.x, tx, h, q, y, d);
       if (ok) {
+        const fx::Grade k{sc.sk};
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          w[c] = fx::from_q63(y[c], se);
-          e[c] = fx::from_q63(d[c], se);
+          const int E = sc.se - (c == 0 ? k.e0() : k.e1());
+          w[c] = fx::from_q63(y[c], E);
+          e[c] = fx::from_q63(d[c], E);
         }
+        unturn(w[0], w[1], w[2], P.axis);
+        unturn(e[0], e[1], e[2], P.axis);
         return;
       }
     }

@@ -136,7 +136,7 @@ __device__ __forceinline__ bool window_nested(PState& p, const SetParams& P, dou
     p.n_steps += 1;
     if (((++guard) & 255u) == 0u && past_deadline(dl)) return false;
   }
-  spin_settle(g, p.Sx, p.Sy, p.Sz);
+  spin_settle(g, P, p.Sx, p.Sy, p.Sz);
   return true;
 }
 
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_persistent(RunArgs a) {
         }
       }
       if (mode == M_WEND) {
-        spin_settle(g, p.Sx, p.Sy, p.Sz);
+        spin_settle(g, *P, p.Sx, p.Sy, p.Sz);
         write_snap(a, i, w, p);
         ++w;
         store_state(a.s, i, p);  // every window end is a resumable checkpoint
@@ -334,7 +334,7 @@ struct alignas(16) SegRec {
   double p0[3], v0[3];
 #endif
   int on, scale;  // the fixed-point field scale (SegScale), packed
-  int flags, pad;
+  int flags, grade;    // (grade: the field's, SegScale::ok)
 };
 // SegRec::flags: window end reached, particle stopped, bounce, gas collision, field in fixed
 // point, start of a new particle (its index in t0); bits 8-15 sanity failure code.
@@ -472,12 +472,13 @@ __device__ __forceinline__ DeviceState state_slot(const DeviceState& b, int64_t 
 
 // A record's field scale in two words.
 __device__ __forceinline__ int pack_exps(const fx::SegScale& s) { return (int)((unsigned)s.oe << 16) | (s.te & 0xffff); }
-__device__ __forceinline__ fx::SegScale unpack_scale(int on, int exps) {
+__device__ __forceinline__ fx::SegScale unpack_scale(int on, int exps, int grade) {
   fx::SegScale s;
   s.on = fx::bits_f32((uint32_t)on);
   s.oe = exps >> 16;
   s.te = (int)(short)(exps & 0xffff);
   s.se = 0;
+  s.ok = grade;
   return s;
 }
 
@@ -508,6 +509,7 @@ __device__ __forceinline__ int produce_record(PState& tp, const SetParams& P, do
     if (q.fx) {
       r->on = (int)fx::f32_bits(q.sc.on);
       r->scale = pack_exps(q.sc);
+      r->grade = q.sc.ok;
       flags |= R_FX;
     }
   }
@@ -733,7 +735,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batched(RunArgs a, int starve, 
           } else if (spin_on<EXT>(P->integrator)) {
             SegPoly q;
             q.fx = (flags & R_FX) != 0;
-            q.sc = unpack_scale(r->on, r->scale);
+            q.sc = unpack_scale(r->on, r->scale, r->grade);
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
               q.o0[c] = r->o0[c];
@@ -768,7 +770,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batched(RunArgs a, int starve, 
           } else {
             out = load_state(a.s, i);  // stopped: the trajectory fields stay (or become NaN)
           }
-          spin_settle(g, Sx, Sy, Sz);
+          spin_settle(g, *P, Sx, Sy, Sz);
           out.Sx = Sx; out.Sy = Sy; out.Sz = Sz;
           out.h = ph;
           out.turns = turns;
@@ -810,7 +812,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batched(RunArgs a, int starve, 
         int r;
         if (P->integrator == 0) {
           double y0x = Sx, y0y = Sy, y0z = Sz;
-          if (TAPE && g.fx) dop_spin(g, y0x, y0y, y0z);
+          if (TAPE && g.fx) dop_spin(g, *P, y0x, y0y, y0z);
           const double x0 = g.x;
           r = dop_attempt_v(fx::Lane3(), ks, g, *P, Sx, Sy, Sz);
           ++n_dop;

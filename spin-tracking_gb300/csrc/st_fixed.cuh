@@ -19,6 +19,17 @@
 // size, and the first one while the sum of the products' magnitudes stays
 // below 2.
 //
+// A block's power of two is that of its norm, so a component that is small beside the
+// norm would have fewer bits than a double.  In the usual geometry components
+// are small: fields lie along one axis but for 1e-4 or less of them, spins (and
+// adjoints) along that axis or across it.  The words are therefore turned so that
+// component 0 is the axis, and graded: the field's components 1 and 2 are kept times
+// 2^ok, a spin's times 2^sk where it lies along the axis (sk > 0), its component 0 times
+// 2^-sk where it lies across (sk < 0), with |sk| <= ok.  Of the terms of a cross product,
+// those that stay small have the grade of the component they go to, and the others
+// need one shift (Grade).  Ungraded, a spin within 1e-5 of its axis lost its
+// transverse part at 5e-17 of the norm per step of 0.13 rad, where FP64 loses 6e-21.
+//
 // The stages run as one rolled loop over tables in constant memory, with the
 // stage derivatives in shared (or local) memory: the hot code has to stay
 // within the ~16 KB of instructions that a sub-partition holds close by.
@@ -142,6 +153,7 @@ typedef unsigned long long u64;
 
 #ifdef __CUDA_ARCH__
 __device__ __forceinline__ int clz64(u64 x) { return __clzll((long long)x); }
+__device__ __forceinline__ int clz32(unsigned x) { return __clz((int)x); }
 __device__ __forceinline__ float lg2f_approx(float x) {
   float r;
   asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -181,6 +193,7 @@ __device__ __forceinline__ u64 f64_bits(double x) { return (u64)__double_as_long
 __device__ __forceinline__ double bits_f64(u64 b) { return __longlong_as_double((long long)b); }
 #else
 inline int clz64(u64 x) { return x ? __builtin_clzll(x) : 64; }
+inline int clz32(unsigned x) { return x ? __builtin_clz(x) : 32; }
 inline float lg2f_approx(float x) { return log2f(x); }
 inline float ex2f_approx(float x) { return exp2f(x); }
 inline float rcpf_approx(float x) { return 1.0f / x; }
@@ -212,6 +225,7 @@ inline uint32_t rcp_hi(double x) { return (uint32_t)(f64_bits(1.0 / x * seed_err
 #endif
 
 __device__ __forceinline__ i64 shl(i64 a, int k) { return (i64)((u64)a << k); }
+__device__ __forceinline__ i64 add(i64 a, i64 b) { return (i64)((u64)a + (u64)b); }  // modulo 2^64
 
 // ---------------------------------------------------------------- conversions
 // Biased exponent of x (0: zero or subnormal, 0x7ff: infinite or NaN).
@@ -237,12 +251,18 @@ __device__ __forceinline__ double from_q63(i64 m, int E) {
   return m == 0 ? 0.0 : bits_f64(b + ((u64)(i64)(E - 63) << 52));
 }
 
+// m 2^-n, rounded.
+__device__ __forceinline__ i64 rsh(i64 m, int n) { return (m + ((i64)((1ull << n) >> 1))) >> n; }
+// |m| or one less, for its leading zeros
+__device__ __forceinline__ unsigned mag(int m) { return (unsigned)(m ^ (m >> 31)); }
+
 // ---------------------------------------------------------------- products
 struct Limb {
   int h, l;
 };
-// m to 58 fractional bits, rounded down (callers add 16 units first to round to nearest).
+// m to 58 fractional bits, rounded down (callers add 16 units first to round to nearest), and back.
 __device__ __forceinline__ Limb limb(i64 m) { return {(int)(m >> 32), (int)((unsigned)m >> 5)}; }
+__device__ __forceinline__ i64 unlimb(Limb a) { return (i64)((u64)(unsigned)a.h << 32 | (unsigned)a.l << 5); }
 __device__ __forceinline__ Limb neg(Limb a) { return {-a.h, -a.l}; }
 
 struct Acc {
@@ -267,11 +287,24 @@ __device__ __forceinline__ i64 q63(const Acc& a, int k = 0) { return shl(a.hh, 1
 __device__ __forceinline__ i64 mulq(Limb x, Limb y, int k = 0) {
   return q63(mac0(x, y, kHalfLimb), k);
 }
+// x m with all of m's bits, as Q63 times 2^k.
+__device__ __forceinline__ i64 mulw63(Limb x, i64 m, int k) {
+  Acc a = mac0(x, limb(m));
+  a.mid += (madw(x.h, (int)m & 31, 16) >> 5) + (1 << (25 - k));
+  return q63(a, k);
+}
 // A tableau entry times 2^-p as limbs (folds to immediates).
 __device__ __forceinline__ constexpr Limb coef(double a, int p) {
   const double s = a * (double)(1ull << (58 - p));
   const i64 q = (i64)(s + (s < 0.0 ? -0.5 : 0.5));
   const i64 h = (q + (1ll << 26)) >> 27;
+  return {(int)h, (int)(q - (i64)((u64)h << 27))};
+}
+// Half of c^2 as limbs, 2^-5 <= c <= 1 (or 0): squared as an integer, since c^2 rounded to a double
+// would cost the second moments of the adjoint up to 5e-16.
+__device__ __forceinline__ constexpr Limb coef_sq(double c) {
+  const u64 m = (u64)(c * (double)(1ull << 58)), a = m >> 29, b = m & 0x1fffffffull;
+  const i64 q = (i64)((a * a + ((2 * a * b + (b * b >> 29)) >> 29) + 1) >> 1), h = (q + (1ll << 26)) >> 27;
   return {(int)h, (int)(q - (i64)((u64)h << 27))};
 }
 // High 64 bits of the product of two 64-bit fractions, at most 3 units low.
@@ -316,7 +349,7 @@ struct Lane3 {
     for (int c = 0; c < 3; ++c) all[c] = v[c];
   }
   __device__ __forceinline__ bool any(bool b) const { return b; }
-  __device__ __forceinline__ bool is_z(int c) const { return c == 2; }
+  __device__ __forceinline__ int comp(int c) const { return c; }
   __device__ __forceinline__ void pick(i64 x, i64 y, i64 z, i64 v[3]) const {
     v[0] = x;
     v[1] = y;
@@ -429,7 +462,28 @@ __device__ __forceinline__ u64 turns_of(double t, u64 wm, int we) {
 struct SegScale {
   int oe, te, se;
   float on;
+  int ok = 0, sk = 0;  // grades of the field and the spin
+  int pz = 2;          // component of the words along z (the pulse)
 };
+
+// What a spin's (or adjoint's) grade g does in a step: components 0, and 1 and 2, are kept
+// times 2^e0, 2^e1.
+struct Grade {
+  int g;
+  __device__ __forceinline__ int e0() const { return g < 0 ? -g : 0; }
+  __device__ __forceinline__ int e1() const { return g > 0 ? g : 0; }
+  // A derivative's component 0 is kept times 2^(e0 + up()): the spin adds it that much further down.
+  __device__ __forceinline__ int up() const { return 2 * e1(); }
+  // In the derivative's components 1 and 2, component 0 stands this much further down.
+  __device__ __forceinline__ int down() const { return 2 * e0(); }
+};
+// The grade, up to ok, that brings the smaller side's words (leading zeros a along
+// the axis, b across) up to [1/8, 1/4), where the larger side's are.
+__device__ __forceinline__ int grade_of(int a, int b, int ok) {
+  int n = (a > b ? a : b) - 3;
+  n = n < 0 ? 0 : (n > ok ? ok : n);
+  return b > a ? n : -n;
+}
 
 // 31-bit magnitude of x 2^-E (|x| < 2^E), for norms.
 __device__ __forceinline__ uint32_t mag31(double x, int E) {
@@ -453,10 +507,38 @@ __device__ __forceinline__ bool spin_scale(const double S[3], int& se) {
   return true;
 }
 
-// Scale of the field over a segment of length T: false when a coefficient is
-// infinite or NaN, T is not positive, or an exponent leaves the usual range.
+// Grade of a spin of scale se (its components in the order of the words), up to ok.
+__device__ __forceinline__ int spin_grade(const double S[3], int se, int ok) {
+  const int top = se + 1023;  // less the biased exponent: the word's leading zeros
+  return grade_of(top - bexp(S[0]), top - imax(bexp(S[1]), bexp(S[2])), ok);
+}
+__device__ __forceinline__ void spin_words(const double S[3], int se, int sk, i64 w[3]) {
+  const Grade g{sk};
+  w[0] = to_q63(S[0], se - g.e0());
+  w[1] = to_q63(S[1], se - g.e1());
+  w[2] = to_q63(S[2], se - g.e1());
+}
+// The words of a spin of grade sk at the grade that fits them best, up to ok (or nearer to it
+// where their high halves are zero).
+__device__ __forceinline__ void regrade(i64 w[3], int& sk, int ok) {
+  const Grade g{sk};
+  const int h0 = (int)(w[0] >> 32), h1 = (int)(w[1] >> 32), h2 = (int)(w[2] >> 32);
+  const int n = grade_of(clz32(mag(h0)) + g.e0(), clz32(mag(h1) | mag(h2)) + g.e1(), ok);
+  if (n == sk) return;
+  sk = n;
+  const int d0 = g.e0() - Grade{n}.e0(), d1 = g.e1() - Grade{n}.e1();
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const int d = c == 0 ? d0 : d1;
+    w[c] = d >= 0 ? rsh(w[c], d) : shl(w[c], -d);
+  }
+}
+
+// Scale of the field over a segment of length T, and with `grade` its grade (else 0):
+// false when a coefficient is infinite or NaN, T is not positive, or an exponent
+// leaves the usual range.  ga is on component q.pz.
 __device__ __forceinline__ bool field_scale(const double o0[3], const double o1[3], const double o2[3], double ga,
-                                            double T, SegScale& q) {
+                                            double T, SegScale& q, bool grade = false) {
   if (!(T > 0.0)) return false;
   const int t = bexp(T) - 1021;  // T < 2^(te - 1)
   int e0 = bexp(ga), e1 = 0, e2 = 0;
@@ -473,12 +555,13 @@ __device__ __forceinline__ bool field_scale(const double o0[3], const double o1[
   if (e < 64) e = 64;  // no field to speak of: every coefficient rounds to zero
   if (e > 1900) return false;
   const int E = e - 1023 + 3;  // each term below 1/4, the sum of a component's below 1
-  u64 n2 = 0;
+  u64 n2 = 0, axis2 = 0;
 #pragma unroll 1
   for (int c = 0; c < 3; ++c) {
     const u64 m = (u64)mag31(o0[c], E) + mag31(o1[c], E - t) + 2ull * mag31(o2[c], E - 2 * t) +
-                  (c == 2 ? mag31(ga, E) : 0u) + 4u;  // units of 2^-31, rounded up
+                  (c == q.pz ? mag31(ga, E) : 0u) + 4u;  // units of 2^-31, rounded up
     n2 += (m * m) >> 2;
+    if (c == 0) axis2 = n2;
   }
   const float n = sqrtf((float)n2) * 0x1p-30f;  // norm of 2^-E Omega, below 1.8
   const uint32_t nb = f32_bits(n);
@@ -486,6 +569,9 @@ __device__ __forceinline__ bool field_scale(const double o0[3], const double o1[
   q.oe = E + ne;
   q.te = t;
   q.on = bits_f32(nb - ((uint32_t)ne << 23)) * 1.00001f;
+  q.ok = 0;
+  if (grade)  // the words across grow no larger than the norm: all to sqrt 2 times it at most
+    q.ok = imax((int)(f32_bits((float)n2) - f32_bits((float)(n2 - axis2))) >> 24, 0);  // (at most 28: the sums are 4 units or more)
   return true;
 }
 
@@ -497,8 +583,8 @@ struct StepTol {
 // Whether a spin of scale se can be stepped with this ratio.  A component near
 // zero is weighted by atol alone, while its error estimate carries the rounding
 // of the whole spin (2^-58 of its norm): up to norm / ratio = 16 the estimate was
-// better than the FP64 step's on every case tried, at 64 it spoiled the growth of
-// tiny steps (14 of 20,000).
+// better than the FP64 step's in the median (spins of any direction, and along and across the
+// field's axis), at 64 it spoiled the growth of tiny steps (14 of 20,000).
 __device__ __forceinline__ bool ratio_fits(double ratio, int se) {
   const int e = bexp(ratio) - 1023;  // ratio >= 2^e
   return ratio > 0.0 && e >= se - 6 && e < se + 40;
@@ -521,7 +607,7 @@ struct StageRow {
   Limb c, c2;
 };
 #define ST_ROW(s, off) {off, dopst::cnt(s), (s) == 3 ? 1 : ((s) <= 5 ? 2 : 3), stage_p(s), \
-                        coef(dopst::c(s), 1), coef(dopst::c(s) * dopst::c(s), 1)}
+                        coef(dopst::c(s), 1), coef_sq(dopst::c(s))}
 static __constant__ StageRow kStageRows[12] = {ST_ROW(1, 0),  ST_ROW(2, 0),  ST_ROW(3, 1),  ST_ROW(4, 3),
                                                ST_ROW(5, 5),  ST_ROW(6, 8),  ST_ROW(7, 11), ST_ROW(8, 15),
                                                ST_ROW(9, 20), ST_ROW(10, 26), ST_ROW(11, 33), ST_ROW(12, 41)};
@@ -576,7 +662,7 @@ struct StepField {
   i64 w0[N];
   Limb w1[N], w2[N], hg, dphi;
   u64 phi0;
-  int ez;
+  int ez, pz;
   bool pulse;
   // without the pulse; the halves of the node and of its square
   __device__ __forceinline__ i64 at(int k, Limb c, Limb c2) const {
@@ -587,15 +673,23 @@ struct StepField {
     mac(o, c2, w2[k]);
     return q63(o, 1);
   }
+  template <class V>
+  __device__ __forceinline__ void add_pulse(const V& view, i64 p, i64* w) const {
+#pragma unroll
+    for (int c = 0; c < N; ++c)
+      if (view.comp(c) == pz) w[c] += p;
+  }
   __device__ __forceinline__ i64 pulse_at(Limb c) const {
     return mulq(hg, limb(half_cos_turns(phi0 + (u64)mulq(c, dphi, 1)) + 16), 1);
   }
 };
-// False: the step leaves the segment, reaches 2^max_ez / 2 rad or passes a quarter
-// of a pulse's turn.
-template <int N>
-__device__ __forceinline__ bool step_field(const SegScale& q, const i64* o0, const i64* o1, const i64* o2, i64 ga, u64 wm,
-                                           int we, double x, double tx, double h, int max_ez, StepField<N>& f) {
+// Components 1 and 2 come out at the grade ok - kw.  False: the step leaves the
+// segment, reaches 2^max_ez / 2 rad or passes a quarter of a pulse's turn.
+template <class V>
+__device__ __forceinline__ bool step_field(const V& view, const SegScale& q, int kw, const i64* o0, const i64* o1,
+                                           const i64* o2, i64 ga, u64 wm, int we, double x, double tx, double h, int max_ez,
+                                           StepField<V::N>& f) {
+  constexpr int N = V::N;
   // ---- the step in segment units
   if ((i64)f64_bits(h) <= 0 || (i64)f64_bits(tx) < 0) return false;  // (a NaN is out of range below)
   const int eh = bexp(h) - 1021;  // h = hm 2^eh, hm in [1/4, 1/2)
@@ -619,15 +713,17 @@ __device__ __forceinline__ bool step_field(const SegScale& q, const i64* o0, con
   for (int c = 0; c < N; ++c) {
     const Limb o2l = limb(o2[c]);
     const i64 t1 = mulq(ul, o2l);
-    f.w0[c] = mulq(hsl, limb(o0[c] + mulq(ul, limb(o1[c] + t1))), -1);  // a quarter of it
-    f.w1[c] = limb(mulq(g1l, limb(o1[c] + shl(t1, 1)), 1));
-    f.w2[c] = limb(mulq(g2l, o2l, 1));
+    const int d = view.comp(c) == 0 ? 0 : kw;
+    f.w0[c] = mulq(hsl, limb(o0[c] + mulq(ul, limb(o1[c] + t1))), -1) >> d;  // a quarter of it
+    f.w1[c] = limb(mulq(g1l, limb(o1[c] + shl(t1, 1)), 1) >> d);
+    f.w2[c] = limb(mulq(g2l, o2l, 1) >> d);
   }
   f.pulse = ga != 0;
+  f.pz = q.pz;
   f.hg = f.dphi = {0, 0};
   f.phi0 = 0;
   if (f.pulse) {
-    f.hg = limb(mulq(hsl, limb(ga), 1));
+    f.hg = limb(mulq(hsl, limb(ga), 1) >> (q.pz == 0 ? 0 : kw));
     const u64 dp = turns_of(h, wm, we);
     if (dp >= 0x4000000000000000ull || bexp(h) - 1022 + we > 0) return false;  // a quarter turn or more
     f.dphi = limb((i64)dp);
@@ -641,11 +737,13 @@ __device__ __forceinline__ bool step_field(const SegScale& q, const i64* o0, con
 struct StageNone {
   __device__ __forceinline__ void store(int, const Limb*) {}
 };
-// The stages of a step: kappa_1..kappa_12 in ks, the states Y in ys; not zero: a sum
-// left its range.
+// The stages of a step from a spin of grade g, the field at the grade |g|: kappa_1..
+// kappa_12 in ks, the states Y in ys; not zero: a sum left its range.
 template <class V, class KS, class YS>
-__device__ __forceinline__ unsigned dop_stages(const V& view, KS& ks, YS& ys, const StepField<V::N>& f, const i64* S, int r) {
+__device__ __forceinline__ unsigned dop_stages(const V& view, KS& ks, YS& ys, const StepField<V::N>& f, const i64* S, int r,
+                                               Grade g) {
   constexpr int N = V::N;
+  const int r0 = r + g.up() > 63 ? 63 : r + g.up();
   // ---- stages: kappa_s = Y_s x omega_s, Y_s = S + 2^ez sum a_sj kappa_j
   i64 Sr[N];
 #pragma unroll
@@ -677,22 +775,26 @@ __device__ __forceinline__ unsigned dop_stages(const V& view, KS& ks, YS& ys, co
 #pragma unroll
       for (int c = 0; c < N; ++c) mac(a[c], f, k[c]);
     }
-    Limb Y[N], W[N];
+    Limb Yg[N], Y[N], W[N];
+    const i64 pulse = f.pulse ? f.pulse_at(row.c) : 0;  // (one copy of its code)
 #pragma unroll
     for (int c = 0; c < N; ++c) {
       const int p = row.p;
+      const bool axis = view.comp(c) == 0;
       // |2 sum a kappa| < 1/2: neither the shift below nor Y can overflow
       bad |= ((unsigned)(int)(a[c].hh >> 32) + (1u << (28 - p))) & ~((1u << (29 - p)) - 1u);
-      Y[c] = limb(Sr[c] + (q63(a[c], 1 + p) >> r));
+      const i64 y = Sr[c] + (q63(a[c], 1 + p) >> (axis ? r0 : r));
+      Yg[c] = limb(y);
+      Y[c] = limb(axis ? y >> g.down() : y);
       i64 w = f.at(c, row.c, row.c2);
-      if (f.pulse && view.is_z(c)) w += f.pulse_at(row.c);
+      if (view.comp(c) == f.pz) w += pulse;
       W[c] = limb(w);
     }
     view.cross(Y, W, a);
 #pragma unroll
     for (int c = 0; c < N; ++c) k[c] = limb(q63(a[c]));
     ks.store(s, k);
-    ys.store(s, Y);
+    ys.store(s, Yg);
   }
   return bad;
 }
@@ -706,11 +808,13 @@ __device__ __forceinline__ bool dop_step(const V& view, KS& ks, const SegScale& 
                                          const i64* S, i64* Sn, StepOut& out) {
   using namespace dop;
   constexpr int N = V::N;
+  const Grade g{q.sk};
+  const int k = g.e0() + g.e1();
   StepField<N> f;
-  if (!step_field(q, o0, o1, o2, ga, wm, we, x, tx, h, 1, f)) return false;  // (1: up to 1 rad)
-  const int ez = f.ez, r = 1 - ez > 63 ? 63 : 1 - ez;
+  if (!step_field(view, q, q.ok - k, o0, o1, o2, ga, wm, we, x, tx, h, 1, f)) return false;  // (1: up to 1 rad)
+  const int ez = f.ez, r = 1 - ez > 63 ? 63 : 1 - ez, r0 = r + g.up() > 63 ? 63 : r + g.up();
   StageNone none;
-  const unsigned stages_bad = dop_stages(view, ks, none, f, S, r);
+  const unsigned stages_bad = dop_stages(view, ks, none, f, S, r, g);
   unsigned bad = stages_bad;
   // ---- 8th-order sum, new spin, the two error rows
   Acc sb[N], s3[N], s5[N];
@@ -739,18 +843,17 @@ __device__ __forceinline__ bool dop_step(const V& view, KS& ks, const SegScale& 
     }
   }
   i64 e3[N], e5[N], big[N];
-  const i64 half = (i64)((1ull << r) >> 1);
 #pragma unroll
   for (int c = 0; c < N; ++c) {
     bad |= ((unsigned)(int)(sb[c].hh >> 32) + (1u << 24)) & ~((1u << 25) - 1u);
-    Sn[c] = S[c] + ((q63(sb[c], 5) + half) >> r);
+    Sn[c] = S[c] + rsh(q63(sb[c], 5), view.comp(c) == 0 ? r0 : r);
     e3[c] = q63(s3[c]);  // 2^-4 of the row
     e5[c] = q63(s5[c]);  // 2^-3 of the row
     const i64 m0 = S[c] < 0 ? -S[c] : S[c], m1 = Sn[c] < 0 ? -Sn[c] : Sn[c];
     big[c] = m0 > m1 ? m0 : m1;
   }
   if (view.any(bad != 0)) return false;
-  // ---- err^2 = 2^2(ez - sa) N5^2 / (3 rtol^2 (N5 + N3 / 100)), N = sum (e_c / G_c)^2 with
+  // ---- err^2 = 2^2(ee - sa) N5^2 / (3 rtol^2 (N5 + N3 / 100)), N = sum (e_c / G_c)^2 with
   // G_c = |S_c| + atol / rtol in units of 2^(se + sa); one component after another in a
   // rolled loop, their words in the stage array
   i64 E5[3], E3[3], Mx[3];
@@ -758,6 +861,13 @@ __device__ __forceinline__ bool dop_step(const V& view, KS& ks, const SegScale& 
   view.gather(e3, E3);
   view.gather(big, Mx);
   if (((u64)(Mx[0] | Mx[1] | Mx[2]) >> 62) != 0) return false;  // a spin twice its norm: a step far too long
+  // the spin at grade 0, the errors times 2^e1: component 0's were kept times 2^k more
+  Mx[0] >>= g.e0();
+  Mx[1] >>= g.e1();
+  Mx[2] >>= g.e1();
+  E5[0] >>= k;
+  E3[0] >>= k;
+  const int ee = ez - g.e1();
   u64 all5 = 0, all3 = 0;
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
@@ -808,10 +918,10 @@ __device__ __forceinline__ bool dop_step(const V& view, KS& ks, const SegScale& 
   const u64 A = umul(n5, n5);                  // in [1/4, 1)
   const u64 B = umul(umul(rt, rt), t);         // times 3 / 16: in [2^-7, 1/4)
   const u64 b = (B >> 3) + (B >> 4);
-  // X = err^2 = 2^k A / b, A >= b
-  const int k = 2 * (ez - sa) + 24 - 2 * l5 - 2 * z5 - et + zt - 2 * (bexp(tol.rtol) - 1022) - 4;
-  out.accept = k <= 0 && (k < -10 || (A >> -k) <= b);
-  const int i = k & 15, j = k >> 4;  // k = 16 j + i
+  // X = err^2 = 2^kx A / b, A >= b
+  const int kx = 2 * (ee - sa) + 24 - 2 * l5 - 2 * z5 - et + zt - 2 * (bexp(tol.rtol) - 1022) - 4;
+  out.accept = kx <= 0 && (kx < -10 || (A >> -kx) <= b);
+  const int i = kx & 15, j = kx >> 4;  // kx = 16 j + i
   const u64 rr = root16(A, b, i);
   const int zr = clz64(rr);  // rr / 2^64 = r / 2, to the nearest double
   out.root8 = bits_f64(((u64)(1022 + 1 - zr - j) << 52) + ((rr << zr) >> 11) + (((rr << zr) >> 10) & 1) - kOne);
@@ -853,7 +963,18 @@ static __constant__ Limb kAdjCoef[51] = {
 struct AdjMoments {
   i64 z0[3], z1[3], z2[3], cz, sz, scz;
   int exp;
+  int e[3] = {0, 0, 0};  // less these, by component (the pulse's: component pz's)
 };
+
+// Scale and grade of an adjoint: as a spin's, but graded, its words' norm may be sqrt 3 times
+// that of the vector and the field's sqrt 2 times, so its scale is one bit up (dop_adjoint's bounds).
+__device__ __forceinline__ bool adjoint_scale(const double l[3], int ok, int& le, int& gl) {
+  if (!spin_scale(l, le)) return false;
+  gl = spin_grade(l, le, ok);
+  if (gl >= -1 && gl <= 1) gl = 0;  // (a grade of 1 would gain nothing)
+  le += gl != 0 ? 1 : 0;
+  return true;
+}
 
 // Backward through one DOP853 step of size h at tau = tx from the spin S: the adjoint lam (a
 // scaled vector like S) of the step's result becomes that of S.  With kh_s = (dL/dk_s) / h
@@ -862,19 +983,26 @@ struct AdjMoments {
 // for steps below 1/4, 1/8, 1/16 rad; above that the growing K costs more bits than FP64
 // loses.  For s >= 9 it stays under 0.6, and
 // the large coefficients of the tableau multiply these: they have a K of their own, -1.
+// The adjoint has a grade gl of its own (adjoint_scale).
 // The stages' 12 states Y go to ys, kappa and then yb to ks.  In FP64 a step takes some 850
 // instructions of 76 cycles.  False: out of range, the caller takes FP64.
 template <class KS>
 __device__ __forceinline__ bool dop_adjoint(KS& ks, KS& ys, const SegScale& q, const i64* o0, const i64* o1, const i64* o2,
                                             i64 ga, u64 wm, int we, double x, double tx, double h, bool pulse_grads,
-                                            const i64* S, i64* lam, AdjMoments& m) {
+                                            const i64* S, i64* lam, AdjMoments& m, int gl = 0) {
   const Lane3 view;
+  const Grade gs{q.sk}, g{gl};
   StepField<3> f;
-  if (!step_field(q, o0, o1, o2, ga, wm, we, x, tx, h, -1, f)) return false;  // (-1: up to 1/4 rad)
+  if (!step_field(view, q, q.ok - gs.e0() - gs.e1(), o0, o1, o2, ga, wm, we, x, tx, h, -1, f)) return false;  // (-1: up to 1/4 rad)
   if (pulse_grads && !f.pulse) return false;
   const int ez = f.ez, r = 1 - ez > 63 ? 63 : 1 - ez;
-  if (dop_stages(view, ks, ys, f, S, r) != 0) return false;
+  if (dop_stages(view, ks, ys, f, S, r, gs) != 0) return false;
+  if (gl != q.sk) step_field(view, q, q.ok - g.e0() - g.e1(), o0, o1, o2, ga, wm, we, x, tx, h, -1, f);
   const int K = ez < -3 ? 1 : 4 + ez;
+  // z = kh x Y: in components 1 and 2, Y_0 and kh_0 meet the other's components 1 and 2
+  const int zd = (g.e1() + gs.e0()) - (g.e0() + gs.e1()), zy = zd > 0 ? zd : 0, zk = zd < 0 ? -zd : 0;
+  m.e[0] = g.e1() + gs.e1();
+  m.e[1] = m.e[2] = g.e1() + gs.e0() - zy;
   Limb ll[3];
   i64 ln[3];
 #pragma unroll
@@ -884,7 +1012,9 @@ __device__ __forceinline__ bool dop_adjoint(KS& ks, KS& ys, const SegScale& q, c
     m.z0[c] = m.z1[c] = m.z2[c] = 0;
   }
   m.cz = m.sz = m.scz = 0;
-  m.exp = K + 3;
+  // A stage's z may pass the words' range (sum |kh| |Y| up to 6), the sums do not: they are
+  // mean values of lam x Y over the step, below 0.1.  So the sums run modulo 2^64, without shifts down.
+  m.exp = -2;
 #pragma unroll 1
   for (int s = 11; s >= 0; --s) {
     const AdjRow& row = kAdjRows[s];
@@ -910,7 +1040,8 @@ __device__ __forceinline__ bool dop_adjoint(KS& ks, KS& ys, const SegScale& q, c
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const i64 t = late ? q63(mac0(row.b, ll[c]), 4) : q63(mac0(row.b, ll[c]), 2) >> bs;
-      kq[c] = t + (ls >= 0 ? q63(a[c], ls) : q63(a[c]) >> (ls < -63 ? 63 : -ls));
+      const int lc = c == 0 ? ls - g.up() : ls;
+      kq[c] = t + (lc >= 0 ? q63(a[c], lc) : q63(a[c]) >> (lc < -63 ? 63 : -lc));
       a[c] = {0, 0};
     }
 #pragma unroll 1
@@ -922,45 +1053,53 @@ __device__ __forceinline__ bool dop_adjoint(KS& ks, KS& ys, const SegScale& q, c
 #pragma unroll
       for (int c = 0; c < 3; ++c) mac(a[c], g, yb[c]);
     }
-    Limb kl[3], W[3], Y[3];
-    i64 hc = 0, hs = 0;
+    Limb kl[3], kc[3], W[3], Y[3];
+    i64 hc = 0, hs = 0, pulse = 0;
     if (f.pulse) {
       const u64 phi = f.phi0 + (u64)mulq(nc, f.dphi, 1);
       hc = half_cos_turns(phi);
+      pulse = mulq(f.hg, limb(hc + 16), 1);
       if (pulse_grads) hs = half_cos_turns(phi - 0x4000000000000000ull);
     }
     ys.load(s, Y);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      kl[c] = limb(kq[c] + (ez >= -1 ? q63(a[c], 1 + ez) : q63(a[c]) >> (ez < -64 ? 63 : -1 - ez)) + 16);
+      const int ec = 1 + (c == 0 ? ez - g.up() : ez);
+      const i64 kh = kq[c] + (ec >= 0 ? q63(a[c], ec) : q63(a[c]) >> (ec < -63 ? 63 : -ec));
+      kc[c] = limb((c == 0 ? kh >> g.down() : kh) + 16);
+      kl[c] = c == 0 ? limb((kh >> zk) + 16) : kc[c];
+      if (c == 0) Y[c] = limb((unlimb(Y[c]) >> zy) + (zy > 0 ? 16 : 0));
       i64 w = f.at(c, nc, nc2);
-      if (c == 2 && f.pulse) w += mulq(f.hg, limb(hc + 16), 1);
+      if (c == f.pz) w += pulse;
       W[c] = limb(w);
     }
-    view.cross(W, kl, a);  // half of yb 2^-(K + ez)
-    const int us = ez - 1 + (late ? -1 : K), zs = late ? K + 5 : 4;
+    view.cross(W, kc, a);  // half of yb 2^-(K + ez)
+    const int us = ez - 1 + (late ? -1 : K), zs = late ? 0 : K + 1;
     Limb yb[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const i64 y2 = q63(a[c], 1) - 32;
+      const int uc = c == 0 ? us - g.up() : us;
       yb[c] = limb(y2 + 16);
-      ln[c] += us >= 0 ? shl(y2, us) : y2 >> (us < -63 ? 63 : -us);
+      ln[c] += uc >= 0 ? shl(y2, uc) : rsh(y2, uc < -63 ? 63 : -uc);
     }
     ks.store(s, yb);
     view.cross(kl, Y, a);
+    i64 zz = 0;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      const i64 z = q63(a[c], 1) - 32;  // |kq| < 0.95, |Y| < 0.27
-      const Limb zl = limb(z + 16);
-      m.z0[c] += z >> zs;
-      m.z1[c] += q63(mac0(nc, zl), 1) >> zs;
-      m.z2[c] += q63(mac0(nc2, zl), 1) >> zs;
-      if (c == 2 && pulse_grads) {
-        m.cz += q63(mac0(limb(hc + 16), zl)) >> zs;
-        const i64 t = q63(mac0(limb(hs + 16), zl));
-        m.sz += t >> zs;
-        m.scz += q63(mac0(nc, limb(t + 16)), 1) >> zs;
-      }
+      a[c].mid -= kHalfLimb - (1 << 24);  // (half of the last bit in the place of half a limb)
+      const i64 z = q63(a[c], 1);         // |kq| < 0.95, |Y| < 0.44
+      m.z0[c] = add(m.z0[c], shl(z, zs));
+      m.z1[c] = add(m.z1[c], shl(mulw63(nc, z, 1), zs));
+      m.z2[c] = add(m.z2[c], shl(mulw63(nc2, z, 1), zs));
+      if (c == f.pz) zz = z;
+    }
+    if (pulse_grads) {
+      m.cz = add(m.cz, shl(mulw63(limb(hc + 16), zz, 0), zs));
+      const i64 t = mulw63(limb(hs + 16), zz, 0);
+      m.sz = add(m.sz, shl(t, zs));
+      m.scz = add(m.scz, shl(mulw63(nc, t, 1), zs));
     }
   }
 #pragma unroll
@@ -976,23 +1115,23 @@ static __constant__ i64 kHalfAngle[8][2] = {
     {231064915947ll, 2541714075412ll}, {1481185359ll, 19255409662ll},
     {7053264ll, 105798954ll}, {25931ll, 440829ll}};
 
-// One rotation: y by 2^ez |kappa| about -kappa, |kappa| < 0.73, |y| < 0.251.  With k = 2^ez kappa
+// One rotation: y (of grade g, kappa at the grade |g|) by 2^ez |kappa| about -kappa, |kappa| < 0.73, |y| < 0.251 (ungraded).  With k = 2^ez kappa
 // and b = |k|/2, v' = v + S (w (v x k) + S/2 (v x k) x k), S = sin b / b and w = cos b: both are
 // even series in b, so neither a square root nor a division is needed; above 1 rad the series
 // run at b 2^-m and are doubled m times.  In FP64 a rotation is some 100 instructions of 76 cycles,
 // its sincos more than half of them; here it is about 400 of 2 to 4.  False: kappa is zero.
-__device__ __forceinline__ bool rotate(int ez, const Limb* k, i64* y) {
+__device__ __forceinline__ bool rotate(int ez, const Limb* k, i64* y, Grade g) {
   const Lane3 view;
   constexpr i64 kHalf = 1ll << 62;
   const int ps = ez < -60 ? 62 : (ez < 1 ? 1 - ez : 0);
   Acc t[3];
   Limb v[3];
 #pragma unroll
-  for (int c = 0; c < 3; ++c) v[c] = limb(y[c] + 16);
-  Acc a = mac0(k[0], k[0]);
-  mac(a, k[1], k[1]);
+  for (int c = 0; c < 3; ++c) v[c] = limb((c == 0 ? y[c] >> g.down() : y[c]) + 16);
+  Acc a = mac0(k[1], k[1]);
   mac(a, k[2], k[2]);
-  const i64 k2 = q63(a);
+  const int kg = g.e0() + g.e1(), x2 = 2 * kg;
+  const i64 k2 = q63(mac0(k[0], k[0])) + (q63(a) >> x2);
   // z = |kappa|^2 4^(ez - 1) 4^-doublings <= 1/4
   const int lead = clz64((u64)k2), dbl = 2 * ez + 2 - lead, doublings = dbl > 0 ? dbl >> 1 : 0;
   const int zs = 2 - 2 * ez + 2 * doublings;
@@ -1019,21 +1158,33 @@ __device__ __forceinline__ bool rotate(int ez, const Limb* k, i64* y) {
   // tau = 2^ts v x kappa, as large as |v| < 0.251 and |kappa| < 2^((1 - lead) / 2) let it be
   // (and b times that)
   const int tb = ez - (lead >> 1);
-  const int ts = (lead < 30 ? 2 + ((lead > 2 ? lead - 2 : 0) >> 1) : 16) - (tb > 0 ? tb : 0);
+  // (graded, |v| < 0.44 and kappa's words up to 1.42 times as large)
+  const int ts = (lead < 30 ? 2 + ((lead > 2 ? lead - 2 : 0) >> 1) : 16) - (tb > 0 ? tb : 0) - (kg ? 1 : 0);
   const int us = ts - ez > 62 ? 62 : ts - ez;
   const i64 half = us > 0 ? (1ll << us) >> 1 : 0;
   view.cross(v, k, t);
-  Limb tau[3];
+  // tau's component 0 is kept times 2^(e0 + up()), and so is that of tau x kappa; in the others it
+  // stands 2^2k further down
+  Limb tau[3], tc[3];
 #pragma unroll
-  for (int c = 0; c < 3; ++c) tau[c] = limb(q63(t[c], ts) - (16 << ts) + 16);  // (the limb's half was shifted with the product)
-  view.cross(tau, k, t);
+  for (int c = 0; c < 3; ++c) {
+    const i64 x = ts >= 0 ? q63(t[c], ts) - (16 << ts) : (q63(t[c]) - 16) >> -ts;  // (the limb's half was shifted with the product)
+    tau[c] = limb(x + 16);
+    tc[c] = c == 0 ? limb((x >> x2) + 16) : tau[c];
+  }
+  view.cross(tc, k, t);
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     const i64 p = q63(t[c]) - 16;  // 2^(ez - 1) tau x kappa
     Acc d = mac0(fs, tau[c]);
     mac(d, fp, limb((ez >= 1 ? shl(p, ez - 1) : p >> ps) + 16));
     const i64 u = q63(d, 1);
-    y[c] += us < 0 ? shl(u, -us) : (u + half) >> us;
+    if (c == 0) {
+      const int u0 = us + g.up();
+      y[c] += u0 < 0 ? shl(u, -u0) : rsh(u, u0 > 62 ? 62 : u0);
+    } else {
+      y[c] += us < 0 ? shl(u, -us) : (u + half) >> us;
+    }
   }
   return k2 != 0;
 }
@@ -1045,7 +1196,7 @@ __device__ __forceinline__ bool rotate(int ez, const Limb* k, i64* y) {
 struct QuatRow {
   Limb c, c2, w;
 };
-#define ST_Q(node, w) {coef(node, 1), coef((node) * (node), 1), coef(w, 0)}
+#define ST_Q(node, w) {coef(node, 1), coef_sq(node), coef(w, 0)}
 static __constant__ QuatRow kQuatRows[14] = {
     ST_Q(0.0, rk45::CH1),      ST_Q(rk45::A3, rk45::CH3),   ST_Q(rk45::A4, rk45::CH4),   ST_Q(rk45::A5, rk45::CH5),
     ST_Q(rk45::A6, rk45::CH6), ST_Q(0.0, rk45::C1),         ST_Q(rk45::A3, rk45::C3),    ST_Q(rk45::A4, rk45::C4),
@@ -1059,8 +1210,9 @@ static __constant__ QuatRow kQuatRows[14] = {
 template <bool F>
 __device__ __forceinline__ bool quat_step(const SegScale& q, const i64* o0, const i64* o1, const i64* o2, i64 ga, u64 wm, int we,
                                           double x, double tx, double h, const i64* S, i64* w, i64* e) {
+  const Grade g{q.sk};
   StepField<3> f;
-  if (!step_field(q, o0, o1, o2, ga, wm, we, x, tx, h, 3, f)) return false;
+  if (!step_field(Lane3(), q, q.ok - g.e0() - g.e1(), o0, o1, o2, ga, wm, we, x, tx, h, 3, f)) return false;
   i64 y[3] = {S[0], S[1], S[2]}, y0[3] = {S[0], S[1], S[2]};
   bool ok = true;
   constexpr int kFirst = F ? 9 : 0, kLast = F ? 14 : 9, kSwap = F ? 13 : 5;
@@ -1075,13 +1227,13 @@ __device__ __forceinline__ bool quat_step(const SegScale& q, const i64* o0, cons
     }
     const QuatRow& row = kQuatRows[n];
     Limb k[3];
+    i64 o[3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      i64 o = f.at(c, row.c, row.c2);
-      if (c == 2 && f.pulse) o += f.pulse_at(row.c);
-      k[c] = limb(mulq(row.w, limb(o)));
-    }
-    ok &= rotate(f.ez, k, y);
+    for (int c = 0; c < 3; ++c) o[c] = f.at(c, row.c, row.c2);
+    if (f.pulse) f.add_pulse(Lane3(), f.pulse_at(row.c), o);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) k[c] = limb(mulq(row.w, limb(o[c])));
+    ok &= rotate(f.ez, k, y, g);
   }
 #pragma unroll
   for (int c = 0; c < 3; ++c) {

@@ -41,6 +41,8 @@ struct SetParams {
   double tol_ratio;               // atol / rtol, filled by launch_prepare_sets (-1: FP64 steps only)
   uint64_t wturn_m;               // |w| / (2 pi) = wturn_m 2^(wturn_e - 64), likewise
   int wturn_e;
+  int axis, pz;                   // component of B0 that leads, which fixed-point words have first; place of z in them
+  double o2w[3];                  // o2c in their order
   // ---- windows (src/simulation.cpp:43-49)
   double t0, tf, ioutInt;
   double yi_x, yi_y, yi_z;

@@ -325,7 +325,7 @@ __global__ void __launch_bounds__((CW + PW) * 32, MINB) k_split(RunArgs a) {
       } else if (mode == B_WEND) {
         // the window's last record is in: the producer has parked the slot,
         // whose trajectory fields are the state at the window end
-        spin_settle(g, tp.Sx, tp.Sy, tp.Sz);
+        spin_settle(g, *P, tp.Sx, tp.Sy, tp.Sz);
         PState out = tp;
         slot_load(m, j, out);
         out.Sx = tp.Sx; out.Sy = tp.Sy; out.Sz = tp.Sz;

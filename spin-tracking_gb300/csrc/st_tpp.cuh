@@ -36,7 +36,7 @@ struct Lane1 {
     for (int k = 0; k < 3; ++k) all[k] = __shfl_sync(mask, v[0], base + k);
   }
   __device__ __forceinline__ bool any(bool b) const { return __any_sync(mask, b) != 0; }
-  __device__ __forceinline__ bool is_z(int) const { return c == 2; }
+  __device__ __forceinline__ int comp(int) const { return c; }
   __device__ __forceinline__ void pick(fx::i64 x, fx::i64 y, fx::i64 z, fx::i64 v[1]) const {
     v[0] = c == 0 ? x : (c == 1 ? y : z);
   }
@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tpp3(RunArgs a) {
         }
       }
       if (mode == M_WEND) {
-        spin_settle(g, p.Sx, p.Sy, p.Sz);
+        spin_settle(g, *P, p.Sx, p.Sy, p.Sz);
         if (lead) {
           write_snap(a, i, w, p);
           store_state(a.s, i, p);  // every window end is a resumable checkpoint
