@@ -332,7 +332,10 @@ int persistent_max_blocks_per_sm(int v, int kind) {
   // the gas and gas-free instantiations have the same launch bounds; take the one with gas
   const void* fn = variant_fn(v, true, kind);
   if (!fn || !split_fits(v, fn)) return 0;  // not instantiated for this kind of run, or its split does not fit
-  if (ensure_smem(v, true, kind) != cudaSuccess) return 0;
+  if (ensure_smem(v, true, kind) != cudaSuccess) {  // more shared memory than a block can have: not offered
+    (void)cudaGetLastError();                        // (the next launch's check must not find it)
+    return 0;
+  }
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, kVariants[v].block, variant_smem(v));
   return nb;
 }

@@ -1,0 +1,60 @@
+"""A library built for edited field hooks (ST_GRAD_IS_LINEAR 0: every stage evaluates the gradient hook): with the hooks
+left as they are it follows the same physics, so counts are those of the default build and spins agree
+with it to 1e-9, for every integrator, in several contexts of one process."""
+from __future__ import annotations
+
+import shutil
+import subprocess
+import sys
+
+import pytest
+
+from conftest import REPO
+
+pytestmark = pytest.mark.gpu
+
+RUN = r"""
+import sys
+import numpy as np
+sys.path.insert(0, sys.argv[1])
+import spintrack as st
+from spintrack import build
+build.build()
+G = np.random.default_rng(8).normal(0.0, 1e-9, 9)
+out = {}
+for it, tf in ((0, 0.02), (1, 2e-5), (2, 0.02), (3, 2e-5), (4, 2e-5), (5, 2e-5)):
+    opt = st.derive(st.make_options(numParticles=33, dist="M", T=0.4, gas_coll=True, gravity=True, diffuse=0.1, Gx=G[0:3], Gy=G[3:6],
+                                    Gz=G[6:9], E=(0.0, 0.0, 75e5), B0=(3e-6, 0.0, 0.0), yi=(0.0, 0.0, 1.0), tf=tf, ioutInt=tf / 2,
+                                    seed=17, rtol=1e-10, atol=1e-10, integratorType=it, a=2e-6, w=6283.0, hmax=1e-4))
+    with st.Particles(opt) as p:
+        for kernel in (st.KERNEL_PLAIN, st.KERNEL_PERSISTENT):
+            p.init_particles()
+            p.run_windows(0, 2, kernel)
+            for f, v in p.output_data().items():
+                out[f"{it}_{kernel}_{f}"] = v
+np.savez(sys.argv[2], **out)
+"""
+
+
+def test_edited_hooks_build_and_run(gpu, tmp_path):
+    import numpy as np
+    script = tmp_path / "run.py"
+    script.write_text(RUN)
+    pkg = tmp_path / "spin-tracking_gb300"
+    shutil.copytree(REPO / "spin-tracking_gb300", pkg, ignore=shutil.ignore_patterns("_build", "__pycache__"))
+    shutil.copytree(REPO / "include", tmp_path / "include")
+    hooks = pkg / "csrc" / "st_fields.cuh"
+    text = hooks.read_text()
+    assert "#define ST_GRAD_IS_LINEAR 1" in text
+    hooks.write_text(text.replace("#define ST_GRAD_IS_LINEAR 1", "#define ST_GRAD_IS_LINEAR 0"))
+    got = []
+    for root in (REPO / "spin-tracking_gb300", pkg):
+        npz = tmp_path / f"{len(got)}.npz"
+        r = subprocess.run([sys.executable, str(script), str(root), str(npz)], capture_output=True, text=True)
+        assert r.returncode == 0, r.stderr[-2000:]
+        got.append(dict(np.load(npz)))
+    for k, v in got[0].items():
+        if k.endswith("_S"):
+            assert np.max(np.abs(v - got[1][k])) <= 1e-9, k
+        elif v.dtype.kind in "iu":
+            np.testing.assert_array_equal(v, got[1][k], err_msg=k)
