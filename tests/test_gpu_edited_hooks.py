@@ -55,6 +55,7 @@ def test_edited_hooks_build_and_run(gpu, tmp_path):
         got.append(dict(np.load(npz)))
     for k, v in got[0].items():
         if k.endswith("_S"):
-            assert np.max(np.abs(v - got[1][k])) <= 1e-9, k
+            np.testing.assert_array_equal(np.isnan(v), np.isnan(got[1][k]), err_msg=k)  # (RKF45 stops below hmin)
+            assert np.all(np.abs(v - got[1][k])[~np.isnan(v)] <= 1e-9), k
         elif v.dtype.kind in "iu":
             np.testing.assert_array_equal(v, got[1][k], err_msg=k)
