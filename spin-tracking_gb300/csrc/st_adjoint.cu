@@ -319,7 +319,6 @@ __device__ __forceinline__ void dop_adjoint_step(const Seg& g, const SetParams& 
       }
     }
   }
-#endif
   const Seg t = g;  // (addresses go to the call: the caller's stay in registers)
   double yt[3] = {y[0], y[1], y[2]}, lt[3] = {lam[0], lam[1], lam[2]};
   Moments Mt = M;
@@ -327,6 +326,9 @@ __device__ __forceinline__ void dop_adjoint_step(const Seg& g, const SetParams& 
   M = Mt;
 #pragma unroll
   for (int c = 0; c < 3; ++c) lam[c] = lt[c];
+#else
+  dop_step_adjoint<BLOCK>(g, P, x, h, y, lam, M, pulse, sm);
+#endif
 }
 
 // Contract a segment's moments into dL/dtheta (theta order of the file header);
@@ -458,8 +460,8 @@ __global__ void __launch_bounds__(kAdjBlock) k_adj_backward(RunArgs a, TapeArgs 
         SegPoly q;
         q.o0[0] = g.o0x; q.o0[1] = g.o0y; q.o0[2] = g.o0z;
         q.o1[0] = g.o1x; q.o1[1] = g.o1y; q.o1[2] = g.o1z;
-        seg_scale(q, *P, x + h - g.t0);
-        seg_open(g, *P, q, g.t0, g.t0);
+        seg_scale<kFixedPoint>(q, *P, x + h - g.t0);
+        seg_open<kFixedPoint>(g, *P, q, g.t0, g.t0);
         fresh = false;
       }
       dop_adjoint_step<kAdjBlock>(g, *P, x, h, y, lam, M, pulse, stg);

@@ -7,6 +7,7 @@
 #include <cctype>
 #include <cerrno>
 #include <chrono>
+#include <cfloat>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -95,6 +96,20 @@ bool to_bool(const std::string& s) {
 }
 
 // ---------------------------------------------------------------- params
+// atol / rtol where the fixed-point DOP853 step can weigh a spin like the set's yi with it
+// (ratio_fits and spin_scale of st_fixed.cuh), else -1: the set steps in FP64 alone.
+double fixed_point_ratio(const st_options& o) {
+  if (o.beta != 0.0 || !(o.rtol >= DBL_MIN) || !(o.atol >= 0.0)) return -1.0;
+  const double ratio = o.atol / o.rtol, m = std::max({std::fabs(o.yi.x), std::fabs(o.yi.y), std::fabs(o.yi.z)});
+  if (!(m >= DBL_MIN) || !std::isfinite(m) || !(ratio >= DBL_MIN) || !std::isfinite(ratio)) return -1.0;
+  int se = std::ilogb(m) + 2;
+  const double x = std::ldexp(o.yi.x, -se), y = std::ldexp(o.yi.y, -se), z = std::ldexp(o.yi.z, -se);
+  const double norm = std::sqrt(x * x + y * y + z * z);
+  se += norm > 0.5012 ? 2 : (norm > 0.2506 ? 1 : 0);
+  const int e = std::ilogb(ratio);
+  return e >= se - 6 && e < se + 40 ? ratio : -1.0;
+}
+
 int build_params(const st_options& o, int64_t first, SetParams* P) {
   if (o.numParticles < 0) return fail(ST_ERR_ARG, "numParticles must be >= 0");
   if (o.integratorType == 6 && !(o.w != 0.0 && std::isfinite(o.w)))
@@ -122,6 +137,7 @@ int build_params(const st_options& o, int64_t first, SetParams* P) {
   P->inv_c2 = 1.0 / st::kC2;
   P->rtol = o.rtol; P->atol = o.atol; P->hmin = o.hmin; P->hmax = o.hmax; P->h0 = o.h;
   P->safe = o.safe; P->fac1 = o.fac1; P->fac2 = o.fac2; P->beta = o.beta;
+  P->tol_ratio = fixed_point_ratio(o);
   P->facc1 = 1.0 / o.fac1;
   P->facc2 = 1.0 / o.fac2;
   P->expo1 = 1.0 / 8.0 - o.beta * 0.2;
@@ -328,7 +344,12 @@ bool ctx_any_ext(const st_ctx* c) {
     if (P.integrator >= 2 && P.integrator <= 5) return true;
   return false;
 }
-int ctx_kind(const st_ctx* c) { return (ctx_any_ext(c) ? 1 : 0) | (ctx_any_rk45(c) ? 2 : 0); }
+bool ctx_all_fp64(const st_ctx* c) {
+  for (const auto& P : c->sets_h)
+    if (st::set_steps_fixed(P)) return false;
+  return true;
+}
+int ctx_kind(const st_ctx* c) { return (ctx_any_ext(c) ? 1 : 0) | (ctx_any_rk45(c) ? 2 : 0) | (ctx_all_fp64(c) ? 4 : 0); }
 
 int order_group(int it) {
   switch (it) {
@@ -382,6 +403,7 @@ st::RunArgs make_args(st_ctx* c, int w_begin, int w_end, void* snap) {
   a.any_gas = 0;
   a.any_ext = ctx_any_ext(c) ? 1 : 0;
   a.any_rk45 = ctx_any_rk45(c) ? 1 : 0;
+  a.all_fp64 = ctx_all_fp64(c) ? 1 : 0;
   a.spread = st::spread_lanes(c->n, c->sm_count);
   a.ahead = c->ahead;
   a.ahead_q = 0;
@@ -934,12 +956,13 @@ int st_set_params(st_ctx* c, const st_options* sets, int nsets) {
     if (st::build_spec_set(sets[k], &q[k]) != 0) return fail(ST_ERR_ARG, "integratorType 6: no Floquet period");
   ST_CUDA(cudaSetDevice(c->device));
   // Captured run graphs hold the kernel instantiation chosen for the old sets
-  // (with or without gas collisions, integrator types 2-5) and the work order
+  // (with or without gas collisions or fixed-point steps, integrator types 2-5) and the work order
   // grouped by their integrators: when those change, drop both.  Values
   // alone (fields, tolerances, times) are read from the device table.
   bool kernels_change = false;
   for (int k = 0; k < nsets; ++k)
-    kernels_change |= P[k].gas != c->sets_h[k].gas || P[k].integrator != c->sets_h[k].integrator;
+    kernels_change |= P[k].gas != c->sets_h[k].gas || P[k].integrator != c->sets_h[k].integrator ||
+                      st::set_steps_fixed(P[k]) != st::set_steps_fixed(c->sets_h[k]);
   if (kernels_change) {
     ST_CUDA(cudaStreamSynchronize(c->stream));
     for (auto& g : c->graphs) cudaGraphExecDestroy(g.exec);
@@ -1079,7 +1102,7 @@ int adj_reset_tape(st_ctx* c, const st::TapeArgs& t) {
 int adj_reset_replay_tape(st_ctx* c) { return adj_reset_tape(c, c->tape); }
 
 int adj_tape_launch(st_ctx* c, const st::RunArgs& a, const st::TapeArgs& t) {
-  const int per_sm = std::max(1, st::tape_record_max_blocks_per_sm(ctx_any_ext(c) ? 1 : 0));
+  const int per_sm = std::max(1, st::tape_record_max_blocks_per_sm(ctx_kind(c)));
   st::RunArgs r = a;
   r.spread = st::spread_lanes(a.nitems, c->sm_count);
   const int64_t per_block = st::tape_record_block() / 32 * (int64_t)r.spread;

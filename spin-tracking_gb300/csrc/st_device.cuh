@@ -808,9 +808,7 @@ __device__ __forceinline__ int count_turn(double y0, double z0, double y1, doubl
 __device__ inline void prepare_set(SetParams& P) {
   const double gm = P.gamma;
   const double g_ = P.gravity ? kGravity : 0.0;
-  // atol / rtol for the fixed-point step controller (-1: out of its range), and
   // the pulse's turns per second |w| / 2 pi = wturn_m 2^(wturn_e - 64) to 64 bits
-  P.tol_ratio = P.beta == 0.0 && fx::bexp(P.rtol) > 0 && P.rtol > 0.0 && P.atol >= 0.0 ? P.atol / P.rtol : -1.0;
   P.wturn_m = 0;
   P.wturn_e = 0;
   if (P.w != 0.0 && isfinite(P.w)) {
@@ -902,9 +900,13 @@ struct SegPoly {
   bool fx;
 };
 // Scale a polynomial given in doubles over a segment of length T.
+// FX (here and below): an instantiation for runs with sets that step in fixed point; without it
+// every step is inlined in FP64 (the FP64 form as a call beside the fixed-point one takes 1.25 times
+// as long: 65,536 particles x 0.1 s with beta 0.04, 103 ms against 82).
+template <bool FX>
 __device__ __forceinline__ void seg_scale(SegPoly& q, const SetParams& P, double T) {
   q.fx = false;
-#if ST_GRAD_IS_LINEAR && ST_PULSE_IS_Z_COS
+  if (!FX) return;
   const double gpa = P.gamma * P.a;
   if (((P.integrator == 0 && P.tol_ratio >= 0.0) || P.integrator == 3 || P.integrator == 5) && (gpa == 0.0 || isfinite(P.w)))
   {
@@ -926,17 +928,19 @@ __device__ __forceinline__ void seg_scale(SegPoly& q, const SetParams& P, double
       q.o2[c] = as_f64(fx::to_q63(P.o2w[c], e2));
     }
   }
-#endif
 }
+template <bool FX>
 __device__ __forceinline__ void seg_poly(SegPoly& q, const SetParams& P, const SegStart& s0, double t_end) {
   seg_field(P, s0.px, s0.py, s0.pz, s0.vx, s0.vy, s0.vz, q.o0, q.o1);
-  seg_scale(q, P, t_end - s0.t);
+  seg_scale<FX>(q, P, t_end - s0.t);
 }
 
 // Fill the integrator's segment from the handed-over field.
+template <bool FX>
 __device__ __forceinline__ void seg_open(Seg& g, const SetParams& P, const SegPoly& q, double t0, double t_end) {
   seg_begin(g, P, t0, t_end, q.o0, q.o1);
-  g.fx = q.fx;
+  g.fx = FX && q.fx;
+  if (!FX) return;
   const int se = g.sc.se, sk = g.sc.sk;  // the spin's own scale and grade go on
   g.sc = q.sc;
   g.sc.se = se;
@@ -947,10 +951,11 @@ __device__ __forceinline__ void seg_open(Seg& g, const SetParams& P, const SegPo
   }
 }
 
+template <bool FX>
 __device__ __forceinline__ void seg_setup(Seg& g, const SetParams& P, const SegStart& s0, double t_end) {
   SegPoly q;
-  seg_poly(q, P, s0, t_end);
-  seg_open(g, P, q, s0.t, t_end);
+  seg_poly<FX>(q, P, s0, t_end);
+  seg_open<FX>(g, P, q, s0.t, t_end);
 #if !ST_GRAD_IS_LINEAR
   g.p0x = s0.px; g.p0y = s0.py; g.p0z = s0.pz;
   g.v0x = s0.vx; g.v0y = s0.vy; g.v0z = s0.vz;
@@ -1072,7 +1077,9 @@ __device__ __forceinline__ void dop_spin(const Seg& g, const SetParams& P, doubl
 
 // A spin in fixed point stays there from segment to segment (g.carry): it becomes
 // doubles again at a window end, or where a segment runs in FP64.
+template <bool FX>
 __device__ __forceinline__ void spin_settle(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz) {
+  if (!FX) return;
   if (g.carry) dop_spin(g, P, Sx, Sy, Sz);
   g.carry = false;
 }
@@ -1105,6 +1112,7 @@ static __device__ __noinline__ void dop_begin_f64(Seg& g, const SetParams& P, do
 }
 
 // Start a DOP853 call over the segment (src/integrator.cpp:102-119).
+template <bool FX>
 __device__ __forceinline__ void dop_begin(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz, double h) {
   g.h = h;
   g.facold = 1.0e-4;
@@ -1112,6 +1120,10 @@ __device__ __forceinline__ void dop_begin(Seg& g, const SetParams& P, double& Sx
   g.turns = 0;
   g.reject = false;
   g.last = false;
+  if (!FX) {
+    feval(g, P, 0.0, Sx, Sy, Sz, g.kx, g.ky, g.kz);
+    return;
+  }
   if (g.fx && !g.carry) {
     const SpinWords r = spin_words_of(P, g.sc.ok, Sx, Sy, Sz);
     if (r.ok) {
@@ -1124,7 +1136,7 @@ __device__ __forceinline__ void dop_begin(Seg& g, const SetParams& P, double& Sx
     }
   }
   if (!(g.fx && g.carry)) {
-    spin_settle(g, P, Sx, Sy, Sz);
+    spin_settle<FX>(g, P, Sx, Sy, Sz);
     Seg t = g;  // the call takes its address: g itself stays in registers
     dop_begin_f64(t, P, Sx, Sy, Sz);
     g = t;
@@ -1138,10 +1150,10 @@ struct StageF64 {
 };
 
 // One attempted DOP853 step (one pass of the loop at src/integrator.cpp:128-247)
-// in FP64.  A call, not inlined: the fixed-point step takes all but a few.  Returns 0 to continue, 1 when the segment's last
+// in FP64.  Returns 0 to continue, 1 when the segment's last
 // step was accepted (g.h then holds that step, as the reference returns it),
 // -1 after more than nmax attempts.
-static __device__ __noinline__ int dop_attempt_f64(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz) {
+__device__ __forceinline__ int dop_attempt_f64(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz) {
   using namespace dop;
   StageF64 ks;
   if (g.nstep > P.nmax) return -1;
@@ -1274,7 +1286,8 @@ static __device__ __noinline__ int dop_attempt_f64(Seg& g, const SetParams& P, d
 }
 
 
-// The FP64 attempt for any segment.  One in fixed point goes on in FP64 after an
+// The FP64 attempt for any segment, beside the fixed-point step, which takes all but a few (a
+// call, not inlined).  A segment in fixed point goes on in FP64 after an
 // accepted step; a rejected one changes its step size only.
 static __device__ __noinline__ int dop_attempt_slow(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz) {
   if (!g.fx) return dop_attempt_f64(g, P, Sx, Sy, Sz);
@@ -1308,9 +1321,10 @@ static __device__ __noinline__ int dop_attempt_slow(Seg& g, const SetParams& P, 
 // What bounds it: issue.  ~5,100 instructions, a third of them IMAD.WIDE (2.1
 // cycles each per SM sub-partition), most others 1-2 cycles, 11,300 cycles at two
 // warps, against ~510 FP64 instructions of 76 cycles before.
-template <class V, class KS>
+template <bool FX, class V, class KS>
 __device__ __forceinline__ int dop_attempt_v(const V& view, KS& ks, Seg& g, const SetParams& P, double& Sx, double& Sy,
                                              double& Sz) {
+  if (!FX) return dop_attempt_f64(g, P, Sx, Sy, Sz);
   if (g.nstep > P.nmax) return -1;
   double h = g.h;
   bool last = g.last;
@@ -1396,9 +1410,10 @@ __device__ __forceinline__ int dop_attempt_v(const V& view, KS& ks, Seg& g, cons
 }
 
 // One attempted DOP853 step on one lane, stage derivatives in local memory.
+template <bool FX>
 __device__ __forceinline__ int dop_attempt(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz) {
   fx::StageLocal<3> ks;
-  return dop_attempt_v(fx::Lane3(), ks, g, P, Sx, Sy, Sz);
+  return dop_attempt_v<FX>(fx::Lane3(), ks, g, P, Sx, Sy, Sz);
 }
 
 // ------------------------------------------------------------ RK45
@@ -1417,7 +1432,7 @@ __device__ __forceinline__ void rk45_begin(Seg& g, double h) {
 // state (zero on the first attempt of a call).  Returns 0 to continue, 1 when
 // the segment end was reached (g.h then holds the carried step), -1 when
 // h < hmin, -2 after more than nmax attempts.
-static __device__ __noinline__ int rk45_attempt_call(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz) {
+__device__ __forceinline__ int rk45_attempt_inl(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz) {
   using namespace rk45;
   g.nstep++;
   if (g.nstep > P.nmax) return -2;
@@ -1500,8 +1515,13 @@ static __device__ __noinline__ int rk45_attempt_call(Seg& g, const SetParams& P,
   return 0;
 }
 
-// The call on copies: the caller's segment and spin stay in registers.
+// Beside the fixed-point step a call on copies: the caller's segment and spin stay in registers.
+static __device__ __noinline__ int rk45_attempt_call(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz) {
+  return rk45_attempt_inl(g, P, Sx, Sy, Sz);
+}
+template <bool FX>
 __device__ __forceinline__ int rk45_attempt(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz) {
+  if (!FX) return rk45_attempt_inl(g, P, Sx, Sy, Sz);
   Seg t = g;
   double x = Sx, y = Sy, z = Sz;
   const int r = rk45_attempt_call(t, P, x, y, z);
@@ -1759,9 +1779,16 @@ static __device__ __noinline__ void quat_slow(const Seg& g, const SetParams& P, 
 // quaternion forms, 4,096 particles each, 92 ms, 44 with the quaternion forms in fixed point.
 // (The Magnus stepper stays in FP64: its error estimate is rounding noise on smooth fields, so
 // its steps of a radian and more, and the turns counted at their ends, hang on the noise's bits.)
+template <bool FX>
 __device__ __forceinline__ void quat_step(const Seg& g, const SetParams& P, double tx, double h, double Sx, double Sy,
                                               double Sz, double w[3], double e[3]) {
-#if ST_GRAD_IS_LINEAR && ST_PULSE_IS_Z_COS
+  if (!FX) {
+    if (P.integrator == 3)
+      quat_stages<false>(g, P, tx, h, Sx, Sy, Sz, w, e);
+    else
+      quat_stages<true>(g, P, tx, h, Sx, Sy, Sz, w, e);
+    return;
+  }
   if (g.fx) {
     double S[3] = {Sx, Sy, Sz};
     turn_by(S[0], S[1], S[2], P.axis);
@@ -1791,7 +1818,6 @@ __device__ __forceinline__ void quat_step(const Seg& g, const SetParams& P, doub
       }
     }
   }
-#endif
   const Seg t = g;  // (their addresses go to the call: g, w and e stay in registers)
   double ws[3], es[3];
   quat_slow(t, P, tx, h, Sx, Sy, Sz, ws, es);
@@ -1811,6 +1837,7 @@ __device__ __forceinline__ void ext_begin(Seg& g, double h) { rk45_begin(g, h); 
 // segment ends after nmax attempts, -2).  Returns 0 to continue, 1 at the
 // segment end (g.h then holds the carried step), -1 when h < hmin, -2 after
 // more than nmax attempts.
+template <bool FX>
 __device__ __forceinline__ int ext_attempt(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz) {
   g.nstep++;
   if (g.nstep > P.nmax) return -2;
@@ -1834,7 +1861,7 @@ __device__ __forceinline__ int ext_attempt(Seg& g, const SetParams& P, double& S
   if (P.integrator == 2)
     magnus_stages(g, P, tx, h, Sx, Sy, Sz, w, e);
   else if (P.integrator != 4)
-    quat_step(g, P, tx, h, Sx, Sy, Sz, w, e);
+    quat_step<FX>(g, P, tx, h, Sx, Sy, Sz, w, e);
   else
     rkf45_stages(g, P, tx, h, Sx, Sy, Sz, w, e);
   double error = sfp::sqrt_rn(fma(e[2], e[2], fma(e[1], e[1], e[0] * e[0])));

@@ -32,10 +32,10 @@ __device__ __forceinline__ bool spin_on(int it) {
 }
 
 // Start the integrator of the set's type over a segment.
-template <bool EXT>
+template <bool EXT, bool FX>
 __device__ __forceinline__ void spin_begin(Seg& g, const SetParams& P, double& Sx, double& Sy, double& Sz, double h) {
   if (P.integrator == 0)
-    dop_begin(g, P, Sx, Sy, Sz, h);
+    dop_begin<FX>(g, P, Sx, Sy, Sz, h);
   else if (!EXT || P.integrator == 1)
     rk45_begin(g, h);
   else
@@ -96,25 +96,25 @@ __device__ __forceinline__ bool window_nested(PState& p, const SetParams& P, dou
     if (p.fail == 0) {
       int res = 0;
       if (spin_on<EXT>(P.integrator)) {
-        seg_setup(g, P, s0, p.t);
+        seg_setup<kFixedPoint>(g, P, s0, p.t);
         if (P.integrator == 0) {
-          dop_begin(g, P, p.Sx, p.Sy, p.Sz, tempH);
+          dop_begin<kFixedPoint>(g, P, p.Sx, p.Sy, p.Sz, tempH);
           do {
-            res = dop_attempt(g, P, p.Sx, p.Sy, p.Sz);
+            res = dop_attempt<kFixedPoint>(g, P, p.Sx, p.Sy, p.Sz);
             ++n_dop;
             if (((++guard) & 1023u) == 0u && past_deadline(dl)) return false;
           } while (res == 0);
         } else if (!EXT || P.integrator == 1) {
           rk45_begin(g, tempH);
           do {
-            res = rk45_attempt(g, P, p.Sx, p.Sy, p.Sz);
+            res = rk45_attempt<kFixedPoint>(g, P, p.Sx, p.Sy, p.Sz);
             ++n_rk;
             if (((++guard) & 1023u) == 0u && past_deadline(dl)) return false;
           } while (res == 0);
         } else {
           ext_begin(g, tempH);
           do {
-            res = ext_attempt(g, P, p.Sx, p.Sy, p.Sz);
+            res = ext_attempt<kFixedPoint>(g, P, p.Sx, p.Sy, p.Sz);
             ++n_ext;
             if (((++guard) & 1023u) == 0u && past_deadline(dl)) return false;
           } while (res == 0);
@@ -136,7 +136,7 @@ __device__ __forceinline__ bool window_nested(PState& p, const SetParams& P, dou
     p.n_steps += 1;
     if (((++guard) & 255u) == 0u && past_deadline(dl)) return false;
   }
-  spin_settle(g, P, p.Sx, p.Sy, p.Sz);
+  spin_settle<kFixedPoint>(g, P, p.Sx, p.Sy, p.Sz);
   return true;
 }
 
@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(BLOCK) k_plain(RunArgs a, int window, double n
 // ------------------------------------------------------------------ persistent
 enum LaneMode { M_FETCH = 0, M_EVENT = 1, M_SEG = 2, M_WEND = 3, M_DONE = 4 };
 
-template <int BLOCK, int MINB, bool EXT>
+template <int BLOCK, int MINB, bool EXT, bool FX>
 __global__ void __launch_bounds__(BLOCK, MINB) k_persistent(RunArgs a) {
   int mode = (int)(threadIdx.x & 31) < a.spread ? M_FETCH : M_DONE;
   int64_t i = 0;
@@ -224,8 +224,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_persistent(RunArgs a) {
           finished = traj_event(p, *P, tf, s0);
           ++n_seg;
           if (p.fail == 0 && spin_on<EXT>(P->integrator)) {
-            seg_setup(g, *P, s0, p.t);
-            spin_begin<EXT>(g, *P, p.Sx, p.Sy, p.Sz, tempH);
+            seg_setup<FX>(g, *P, s0, p.t);
+            spin_begin<EXT, FX>(g, *P, p.Sx, p.Sy, p.Sz, tempH);
             mode = M_SEG;
           } else {
             if (p.fail == 0 && P->keep) p.h = tempH;
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_persistent(RunArgs a) {
         }
       }
       if (mode == M_WEND) {
-        spin_settle(g, *P, p.Sx, p.Sy, p.Sz);
+        spin_settle<FX>(g, *P, p.Sx, p.Sy, p.Sz);
         write_snap(a, i, w, p);
         ++w;
         store_state(a.s, i, p);  // every window end is a resumable checkpoint
@@ -263,13 +263,13 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_persistent(RunArgs a) {
     // Phase B (converged): one step attempt for every lane.
     int r;
     if (P->integrator == 0) {
-      r = dop_attempt(g, *P, p.Sx, p.Sy, p.Sz);
+      r = dop_attempt<FX>(g, *P, p.Sx, p.Sy, p.Sz);
       ++n_dop;
     } else if (!EXT || P->integrator == 1) {
-      r = rk45_attempt(g, *P, p.Sx, p.Sy, p.Sz);
+      r = rk45_attempt<FX>(g, *P, p.Sx, p.Sy, p.Sz);
       ++n_rk;
     } else {
-      r = ext_attempt(g, *P, p.Sx, p.Sy, p.Sz);
+      r = ext_attempt<FX>(g, *P, p.Sx, p.Sy, p.Sz);
       ++n_ext;
     }
     if (r != 0) {
@@ -483,7 +483,7 @@ __device__ __forceinline__ fx::SegScale unpack_scale(int on, int exps, int grade
 }
 
 // One trajectory event of a lane into ring record r.  Returns its flags.
-template <bool TAPE, bool GAS, bool EXT>
+template <bool TAPE, bool GAS, bool EXT, bool FX>
 __device__ __forceinline__ int produce_record(PState& tp, const SetParams& P, double tf, SegRec* r, EventDefer& dd,
                                               const TapeArgs& ta, TapeCursor& tc) {
   SegStart s0;
@@ -495,12 +495,12 @@ __device__ __forceinline__ int produce_record(PState& tp, const SetParams& P, do
   r->t1 = tp.t;
   if (spin_on<EXT>(P.integrator)) {
     SegPoly q;
-    seg_poly(q, P, s0, tp.t);
+    seg_poly<FX>(q, P, s0, tp.t);
 #pragma unroll 1
     for (int c = 0; c < 3; ++c) {
       r->o0[c] = q.o0[c];
       r->o1[c] = q.o1[c];
-      r->o2[c] = q.o2[c];
+      if (FX) r->o2[c] = q.o2[c];
     }
 #if !ST_GRAD_IS_LINEAR
     r->p0[0] = s0.px; r->p0[1] = s0.py; r->p0[2] = s0.pz;
@@ -531,8 +531,8 @@ enum BatchedMode { B_FETCH = 0, B_NEED = 1, B_SEG = 2, B_WEND = 3, B_DONE = 4 };
 // TAPE: also write the adjoint tape (steps and segments of every particle)
 // and state checkpoints at every ta.ckpt_every-th window end.
 // GAS = false: the instantiation for launches without gas collisions.
-// EXT: also integrator types 2-5.
-template <int BLOCK, int MINB, bool TAPE, bool GAS, bool EXT>
+// EXT: also integrator types 2-5.  FX: with fixed-point steps (seg_scale).
+template <int BLOCK, int MINB, bool TAPE, bool GAS, bool EXT, bool FX>
 __global__ void __launch_bounds__(BLOCK, MINB) k_batched(RunArgs a, int starve, int keep, int defer_k, TapeArgs ta) {
   extern __shared__ double st_smem[];
   // DOP853 stage derivatives
@@ -660,7 +660,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batched(RunArgs a, int starve, 
         if (prod) {
           int k = qhead + qcount;
           if (k >= QCAP) k -= QCAP;
-          const int flags = produce_record<TAPE, GAS, EXT>(tp, *tP, tf, ring + k, dd, ta, tcg);
+          const int flags = produce_record<TAPE, GAS, EXT, FX>(tp, *tP, tf, ring + k, dd, ta, tcg);
           ++qcount;
           ++n_seg;
           t_stop = (flags & R_STOP) != 0;
@@ -735,19 +735,19 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batched(RunArgs a, int starve, 
           } else if (spin_on<EXT>(P->integrator)) {
             SegPoly q;
             q.fx = (flags & R_FX) != 0;
-            q.sc = unpack_scale(r->on, r->scale, r->grade);
+            if (FX) q.sc = unpack_scale(r->on, r->scale, r->grade);
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
               q.o0[c] = r->o0[c];
               q.o1[c] = r->o1[c];
-              q.o2[c] = r->o2[c];
+              if (FX) q.o2[c] = r->o2[c];
             }
-            seg_open(g, *P, q, r->t0, r->t1);
+            seg_open<FX>(g, *P, q, r->t0, r->t1);
 #if !ST_GRAD_IS_LINEAR
             g.p0x = r->p0[0]; g.p0y = r->p0[1]; g.p0z = r->p0[2];
             g.v0x = r->v0[0]; g.v0y = r->v0[1]; g.v0z = r->v0[2];
 #endif
-            spin_begin<EXT>(g, *P, Sx, Sy, Sz, tempH);
+            spin_begin<EXT, FX>(g, *P, Sx, Sy, Sz, tempH);
             mode = B_SEG;
             break;
           } else {  // trajectory only: the segment completes at once
@@ -770,7 +770,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batched(RunArgs a, int starve, 
           } else {
             out = load_state(a.s, i);  // stopped: the trajectory fields stay (or become NaN)
           }
-          spin_settle(g, *P, Sx, Sy, Sz);
+          spin_settle<FX>(g, *P, Sx, Sy, Sz);
           out.Sx = Sx; out.Sy = Sy; out.Sz = Sz;
           out.h = ph;
           out.turns = turns;
@@ -812,17 +812,17 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batched(RunArgs a, int starve, 
         int r;
         if (P->integrator == 0) {
           double y0x = Sx, y0y = Sy, y0z = Sz;
-          if (TAPE && g.fx) dop_spin(g, *P, y0x, y0y, y0z);
+          if (TAPE && FX && g.fx) dop_spin(g, *P, y0x, y0y, y0z);
           const double x0 = g.x;
-          r = dop_attempt_v(fx::Lane3(), ks, g, *P, Sx, Sy, Sz);
+          r = dop_attempt_v<FX>(fx::Lane3(), ks, g, *P, Sx, Sy, Sz);
           ++n_dop;
           if (TAPE && g.acc) tape_step(ta, tcs, y0x, y0y, y0z, x0, g.hu);
         } else if (!EXT || P->integrator == 1) {
-          r = rk45_attempt(g, *P, Sx, Sy, Sz);
+          r = rk45_attempt<FX>(g, *P, Sx, Sy, Sz);
           ++n_rk;
         } else {
           const double y0x = Sx, y0y = Sy, y0z = Sz, x0 = g.x;
-          r = ext_attempt(g, *P, Sx, Sy, Sz);
+          r = ext_attempt<FX>(g, *P, Sx, Sy, Sz);
           ++n_ext;
           if (TAPE && g.acc) tape_step(ta, tcs, y0x, y0y, y0z, x0, g.hu);
         }
@@ -882,6 +882,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batched(RunArgs a, int starve, 
 // one configuration.
 constexpr int kTapeBlock = 64, kTapeQcap = 64;
 
+// Defined in st_kernels_fp64.cu: the kernel of persistent variant v, and the record pass, for runs in
+// which no set steps in fixed point.
+const void* variant_fn_fp64(int v, bool gas);
+const void* tape_fn_fp64(bool gas);
 // Defined in st_kernels_ext.cu: the kernel of persistent variant v with
 // integrator types 2-5, the record pass with them (gas-capable), and the plain
 // kernel's launch with them.

@@ -43,6 +43,9 @@
 
 namespace st {
 
+// Whether steps may run in fixed point in this build: their field is a polynomial plus the z cosine.
+constexpr bool kFixedPoint = ST_GRAD_IS_LINEAR && ST_PULSE_IS_Z_COS;
+
 struct Vec3 {
   double x, y, z;
 };

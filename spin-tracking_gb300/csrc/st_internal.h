@@ -38,8 +38,8 @@ struct SetParams {
   // ---- stepper (src/integrator.cpp:90-337)
   double rtol, atol, hmin, hmax, h0, safe, fac1, fac2, beta;
   double facc1, facc2, expo1, inv_safe;
-  double tol_ratio;               // atol / rtol, filled by launch_prepare_sets (-1: FP64 steps only)
-  uint64_t wturn_m;               // |w| / (2 pi) = wturn_m 2^(wturn_e - 64), likewise
+  double tol_ratio;               // atol / rtol (-1: FP64 steps only)
+  uint64_t wturn_m;               // |w| / (2 pi) = wturn_m 2^(wturn_e - 64), filled by launch_prepare_sets
   int wturn_e;
   int axis, pz;                   // component of B0 that leads, which fixed-point words have first; place of z in them
   double o2w[3];                  // o2c in their order
@@ -106,6 +106,11 @@ inline int spread_lanes(int64_t n, int sms) {
   return l < 1 ? 1 : (l > 32 ? 32 : (int)l);
 }
 
+// Whether a set's steps run in fixed point where they can.
+inline bool set_steps_fixed(const SetParams& P) {
+  return (P.integrator == 0 && P.tol_ratio >= 0.0) || P.integrator == 3 || P.integrator == 5;
+}
+
 struct RunArgs {
   const SetParams* sets;
   int nsets;
@@ -121,6 +126,7 @@ struct RunArgs {
   int any_gas;                    // some set has gas collisions (else gas-free kernels may run)
   int any_ext;                    // some set integrates with type 2-5 (the EXT kernels must run)
   int any_rk45;                   // some set integrates with RK45 (type 1)
+  int all_fp64;                   // no set steps in fixed point (set_steps_fixed; kernels of st_kernels_fp64.cu)
   int spread;                     // particles are dealt to the first `spread` lanes of each warp (spread_lanes)
   char* ahead;                    // trajectory-ahead kernel: scratch of ahead_lane_bytes(ahead_q) per launched lane
   int ahead_q;                    // its ring depth (records per lane)

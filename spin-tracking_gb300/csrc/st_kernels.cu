@@ -231,22 +231,22 @@ const char* persistent_variant_name(int v) { return (v >= 0 && v < kNumVariants)
 template <bool GAS>
 static const void* variant_fn_g(int v) {
   switch (v) {
-    case 0: return reinterpret_cast<const void*>(&k_persistent<128, 1, false>);
-    case 1: return reinterpret_cast<const void*>(&k_persistent<128, 2, false>);
-    case 2: return reinterpret_cast<const void*>(&k_persistent<128, 3, false>);
-    case 3: return reinterpret_cast<const void*>(&k_persistent<64, 4, false>);
-    case 4: return reinterpret_cast<const void*>(&k_persistent<256, 1, false>);
+    case 0: return reinterpret_cast<const void*>(&k_persistent<128, 1, false, kFixedPoint>);
+    case 1: return reinterpret_cast<const void*>(&k_persistent<128, 2, false, kFixedPoint>);
+    case 2: return reinterpret_cast<const void*>(&k_persistent<128, 3, false, kFixedPoint>);
+    case 3: return reinterpret_cast<const void*>(&k_persistent<64, 4, false, kFixedPoint>);
+    case 4: return reinterpret_cast<const void*>(&k_persistent<256, 1, false, kFixedPoint>);
     case 9:
     case 10:
     case 11:
     case 12:
-    case 20: return reinterpret_cast<const void*>(&k_batched<64, 6, false, GAS, false>);
-    case 13: return reinterpret_cast<const void*>(&k_batched<64, 8, false, GAS, false>);
-    case 19: return reinterpret_cast<const void*>(&k_batched<256, 1, false, GAS, false>);
-    case 14: return reinterpret_cast<const void*>(&k_split<3, 1, 2, 8, GAS, 0, 0>);
-    case 15: return reinterpret_cast<const void*>(&k_split<6, 2, 1, 8, GAS, 0, 0>);
+    case 20: return reinterpret_cast<const void*>(&k_batched<64, 6, false, GAS, false, kFixedPoint>);
+    case 13: return reinterpret_cast<const void*>(&k_batched<64, 8, false, GAS, false, kFixedPoint>);
+    case 19: return reinterpret_cast<const void*>(&k_batched<256, 1, false, GAS, false, kFixedPoint>);
+    case 14: return reinterpret_cast<const void*>(&k_split<3, 1, 2, 8, GAS, 0, 0, kFixedPoint>);
+    case 15: return reinterpret_cast<const void*>(&k_split<6, 2, 1, 8, GAS, 0, 0, kFixedPoint>);
 #if ST_TRAJ_CORRECTLY_ROUNDED
-    case 16: return reinterpret_cast<const void*>(&k_split<8, 4, 1, 8, GAS, 184, 136>);
+    case 16: return reinterpret_cast<const void*>(&k_split<8, 4, 1, 8, GAS, 184, 136, kFixedPoint>);
 #else
     case 16: return nullptr;  // ptxas 13.0 crashes on this instantiation with CUDA's inline log/sin/cos/acos
 #endif
@@ -257,13 +257,14 @@ static const void* variant_fn_g(int v) {
     case 17:
     case 18: return nullptr;  // the three-lane step assumes the default field hooks
 #endif
-    default: return reinterpret_cast<const void*>(&k_batched<64, 4, false, GAS, false>);  // 5 to 8
+    default: return reinterpret_cast<const void*>(&k_batched<64, 4, false, GAS, false, kFixedPoint>);  // 5 to 8
   }
 }
 // The kernel of variant v: with gas collisions or without, and with
 // integrator types 2-5 (whose instantiations handle gas and every type).
-// kind: bit 0 some set has type 2-5, bit 1 some set has RK45.
+// kind: bit 0 some set has type 2-5, bit 1 some set has RK45, bit 2 no set steps in fixed point.
 static const void* variant_fn(int v, bool gas, int kind) {
+  if (kFixedPoint && !(kind & 1) && (kind & 4)) return (kind & 2) && kVariants[v].family == 3 ? nullptr : variant_fn_fp64(v, gas);
   if (kind & 1) return kVariants[v].family >= 2 ? nullptr : variant_fn_ext(v);  // no k_split, k_tpp3 for types 2-5
   if ((kind & 2) && kVariants[v].family == 3) return nullptr;                  // k_tpp3 integrates DOP853 only
   return gas ? variant_fn_g<true>(v) : variant_fn_g<false>(v);
@@ -306,8 +307,8 @@ static int current_device() {
 // Opt the kernels that need more than 48 KiB of dynamic shared memory in, once per device.
 static cudaError_t ensure_smem(int v, bool gas, int kind) {
   const bool ext = (kind & 1) != 0;
-  static bool done[kAttrDevices][kNumVariants][3] = {};
-  const int k = ext ? 2 : (gas ? 1 : 0), d = current_device();
+  static bool done[kAttrDevices][kNumVariants][5] = {};
+  const int k = ext ? 2 : ((gas ? 1 : 0) + (kind & 4 ? 3 : 0)), d = current_device();
   if (d < kAttrDevices && done[d][v][k]) return cudaSuccess;
   const size_t sm = variant_smem(v);
   const void* fn = variant_fn(v, gas, kind);
@@ -323,6 +324,8 @@ int persistent_prepare(int v) {
   cudaError_t e = ensure_smem(v, true, 0);
   if (e == cudaSuccess) e = ensure_smem(v, false, 0);
   if (e == cudaSuccess) e = ensure_smem(v, true, 1);
+  if (e == cudaSuccess) e = ensure_smem(v, true, 4);
+  if (e == cudaSuccess) e = ensure_smem(v, false, 4);
   return (int)e;
 }
 
@@ -346,7 +349,7 @@ int launch_persistent(const RunArgs& a, int v, int blocks, int block, void* stre
   (void)block;
   const Variant& x = kVariants[v];
   const bool gas = a.any_gas != 0;
-  const int kind = (a.any_ext ? 1 : 0) | (a.any_rk45 ? 2 : 0);
+  const int kind = (a.any_ext ? 1 : 0) | (a.any_rk45 ? 2 : 0) | (a.all_fp64 ? 4 : 0);
   cudaError_t e = ensure_smem(v, gas, kind);
   if (e != cudaSuccess) return (int)e;
   RunArgs args = a;
@@ -366,43 +369,45 @@ int launch_persistent(const RunArgs& a, int v, int blocks, int block, void* stre
 
 // The record pass of the adjoint: the trajectory-ahead kernel with its tape on
 // (one configuration: kTapeBlock lanes, kTapeQcap-record rings); the EXT instantiation (st_kernels_ext.cu) records Magnus steps.
-static const void* tape_fn(bool gas, bool ext) {
+static const void* tape_fn(bool gas, bool ext, bool fp64) {
   if (ext) return tape_fn_ext();
-  return gas ? reinterpret_cast<const void*>(&k_batched<kTapeBlock, 4, true, true, false>)
-             : reinterpret_cast<const void*>(&k_batched<kTapeBlock, 4, true, false, false>);
+  if (kFixedPoint && fp64) return tape_fn_fp64(gas);
+  return gas ? reinterpret_cast<const void*>(&k_batched<kTapeBlock, 4, true, true, false, kFixedPoint>)
+             : reinterpret_cast<const void*>(&k_batched<kTapeBlock, 4, true, false, false, kFixedPoint>);
 }
 static size_t tape_smem() { return batched_smem(kTapeBlock); }
 
-static cudaError_t tape_ensure_smem(bool gas, bool ext) {
-  static bool done[kAttrDevices][3] = {};
-  const int k = ext ? 2 : (gas ? 1 : 0), d = current_device();
+static cudaError_t tape_ensure_smem(bool gas, bool ext, bool fp64) {
+  static bool done[kAttrDevices][5] = {};
+  const int k = ext ? 2 : ((gas ? 1 : 0) + (fp64 ? 3 : 0)), d = current_device();
   if (d < kAttrDevices && done[d][k]) return cudaSuccess;
   cudaError_t e =
-      cudaFuncSetAttribute(tape_fn(gas, ext), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tape_smem());
+      cudaFuncSetAttribute(tape_fn(gas, ext, fp64), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tape_smem());
   if (e == cudaSuccess && d < kAttrDevices) done[d][k] = true;
   return e;
 }
 
 int tape_record_block() { return kTapeBlock; }
 
-int tape_record_max_blocks_per_sm(int ext) {
+int tape_record_max_blocks_per_sm(int kind) {
   int nb = 0;
-  if (tape_ensure_smem(true, ext != 0) != cudaSuccess) return 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, tape_fn(true, ext != 0), kTapeBlock, tape_smem());
+  const bool ext = (kind & 1) != 0, fp64 = (kind & 4) != 0;
+  if (tape_ensure_smem(true, ext, fp64) != cudaSuccess) return 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, tape_fn(true, ext, fp64), kTapeBlock, tape_smem());
   return nb;
 }
 
 int launch_tape_record(const RunArgs& a, const TapeArgs& t, int blocks, void* stream) {
   if (a.nitems == 0) return 0;
-  const bool gas = a.any_gas != 0, ext = a.any_ext != 0;
-  cudaError_t e = tape_ensure_smem(gas, ext);
+  const bool gas = a.any_gas != 0, ext = a.any_ext != 0, fp64 = a.all_fp64 != 0;
+  cudaError_t e = tape_ensure_smem(gas, ext, fp64);
   if (e != cudaSuccess) return (int)e;
   RunArgs args = a;
   TapeArgs tape = t;
   int t0 = (4 * a.spread + 31) / 32, t1 = (8 * a.spread + 31) / 32, dk = (12 * a.spread + 31) / 32;
   args.ahead_q = kTapeQcap;
   void* params[] = {&args, &t0, &t1, &dk, &tape};
-  return (int)cudaLaunchKernel(tape_fn(gas, ext), dim3(blocks), dim3(kTapeBlock), params, tape_smem(),
+  return (int)cudaLaunchKernel(tape_fn(gas, ext, fp64), dim3(blocks), dim3(kTapeBlock), params, tape_smem(),
                                (cudaStream_t)stream);
 }
 

@@ -11,24 +11,24 @@ namespace st {
 
 const void* variant_fn_ext(int v) {
   switch (v) {
-    case 0: return reinterpret_cast<const void*>(&k_persistent<128, 1, true>);
-    case 1: return reinterpret_cast<const void*>(&k_persistent<128, 2, true>);
-    case 2: return reinterpret_cast<const void*>(&k_persistent<128, 3, true>);
-    case 3: return reinterpret_cast<const void*>(&k_persistent<64, 4, true>);
-    case 4: return reinterpret_cast<const void*>(&k_persistent<256, 1, true>);
+    case 0: return reinterpret_cast<const void*>(&k_persistent<128, 1, true, kFixedPoint>);
+    case 1: return reinterpret_cast<const void*>(&k_persistent<128, 2, true, kFixedPoint>);
+    case 2: return reinterpret_cast<const void*>(&k_persistent<128, 3, true, kFixedPoint>);
+    case 3: return reinterpret_cast<const void*>(&k_persistent<64, 4, true, kFixedPoint>);
+    case 4: return reinterpret_cast<const void*>(&k_persistent<256, 1, true, kFixedPoint>);
     case 9:
     case 10:
     case 11:
     case 12:
-    case 20: return reinterpret_cast<const void*>(&k_batched<64, 6, false, true, true>);
-    case 13: return reinterpret_cast<const void*>(&k_batched<64, 8, false, true, true>);
-    case 19: return reinterpret_cast<const void*>(&k_batched<256, 1, false, true, true>);
-    default: return reinterpret_cast<const void*>(&k_batched<64, 4, false, true, true>);  // 5 to 8
+    case 20: return reinterpret_cast<const void*>(&k_batched<64, 6, false, true, true, kFixedPoint>);
+    case 13: return reinterpret_cast<const void*>(&k_batched<64, 8, false, true, true, kFixedPoint>);
+    case 19: return reinterpret_cast<const void*>(&k_batched<256, 1, false, true, true, kFixedPoint>);
+    default: return reinterpret_cast<const void*>(&k_batched<64, 4, false, true, true, kFixedPoint>);  // 5 to 8
   }
 }
 
 const void* tape_fn_ext() {
-  return reinterpret_cast<const void*>(&k_batched<kTapeBlock, 4, true, true, true>);
+  return reinterpret_cast<const void*>(&k_batched<kTapeBlock, 4, true, true, true, kFixedPoint>);
 }
 
 template <int B>

@@ -205,9 +205,11 @@ extern "C" int st_run_noalloc(const st_options* sets, int nsets, void* state, si
   a.any_gas = 1;  // the caller's sets are not inspected on the host: the kernel with gas handles any set
   a.any_ext = 0;
   a.any_rk45 = 0;
+  a.all_fp64 = 1;
   for (int k = 0; k < nsets; ++k) {
     a.any_ext |= (sets[k].integratorType >= 2 && sets[k].integratorType <= 5) ? 1 : 0;
     a.any_rk45 |= sets[k].integratorType == 1 ? 1 : 0;
+    a.all_fp64 &= set_steps_fixed(table[k]) ? 0 : 1;
   }
   if (int pe = launch_prepare_sets(params, nsets, st_)) return set_last_error(ST_ERR_CUDA, cudaGetErrorString((cudaError_t)pe));
   if (n > 0) {
@@ -217,7 +219,7 @@ extern "C" int st_run_noalloc(const st_options* sets, int nsets, void* state, si
     // flat_b128_m2 (the flattened persistent kernel) at its full occupancy; the
     // occupancy query and the shared-memory attribute allocate nothing
     a.spread = spread_lanes(n, sms);
-    const int per_sm = persistent_max_blocks_per_sm(kNoAllocVariant, a.any_ext | (a.any_rk45 << 1));
+    const int per_sm = persistent_max_blocks_per_sm(kNoAllocVariant, a.any_ext | a.any_rk45 << 1 | a.all_fp64 << 2);
     if (per_sm < 1) return set_last_error(ST_ERR_CUDA, "st_run_noalloc: the persistent kernel cannot be resident");
     int le = launch_init(a, 256, st_);
     if (!le) le = launch_persistent(a, kNoAllocVariant, sms * per_sm, 0, st_);

@@ -154,7 +154,7 @@ __device__ __forceinline__ void split_produce(const SplitSmem& m, int j, int q, 
 // consumers' steps want more registers than the launch gives every thread, the
 // producers' trajectory events fewer); the host checks the shares against the
 // registers the block is launched with before any launch.
-template <int CW, int PW, int MINB, int QCAP, bool GAS, int CREG, int PREG>
+template <int CW, int PW, int MINB, int QCAP, bool GAS, int CREG, int PREG, bool FX>
 __global__ void __launch_bounds__((CW + PW) * 32, MINB) k_split(RunArgs a) {
   static_assert(CW % PW == 0, "every producer lane serves the same number of slots");
   static_assert(CREG == 0 || (CW % 4 == 0 && PW % 4 == 0), "register shares are per warpgroup");
@@ -309,13 +309,13 @@ __global__ void __launch_bounds__((CW + PW) * 32, MINB) k_split(RunArgs a) {
             q.o0[c] = o0[c];
             q.o1[c] = o1[c];
           }
-          seg_scale(q, *P, r1 - r0);
-          seg_open(g, *P, q, r0, r1);
+          seg_scale<FX>(q, *P, r1 - r0);
+          seg_open<FX>(g, *P, q, r0, r1);
 #if !ST_GRAD_IS_LINEAR
           g.p0x = pv[0]; g.p0y = pv[1]; g.p0z = pv[2];
           g.v0x = pv[3]; g.v0y = pv[4]; g.v0z = pv[5];
 #endif
-          spin_begin<false>(g, *P, tp.Sx, tp.Sy, tp.Sz, tempH);
+          spin_begin<false, FX>(g, *P, tp.Sx, tp.Sy, tp.Sz, tempH);
           mode = B_SEG;
           break;
         } else {  // trajectory only: the segment completes at once
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__((CW + PW) * 32, MINB) k_split(RunArgs a) {
       } else if (mode == B_WEND) {
         // the window's last record is in: the producer has parked the slot,
         // whose trajectory fields are the state at the window end
-        spin_settle(g, *P, tp.Sx, tp.Sy, tp.Sz);
+        spin_settle<FX>(g, *P, tp.Sx, tp.Sy, tp.Sz);
         PState out = tp;
         slot_load(m, j, out);
         out.Sx = tp.Sx; out.Sy = tp.Sy; out.Sz = tp.Sz;
@@ -369,10 +369,10 @@ __global__ void __launch_bounds__((CW + PW) * 32, MINB) k_split(RunArgs a) {
     if (mode == B_SEG) {
       int r;
       if (P->integrator == 0) {
-        r = dop_attempt(g, *P, tp.Sx, tp.Sy, tp.Sz);
+        r = dop_attempt<FX>(g, *P, tp.Sx, tp.Sy, tp.Sz);
         ++n_dop;
       } else {
-        r = rk45_attempt(g, *P, tp.Sx, tp.Sy, tp.Sz);
+        r = rk45_attempt<FX>(g, *P, tp.Sx, tp.Sy, tp.Sz);
         ++n_rk;
       }
       if (r != 0) {

@@ -92,8 +92,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tpp3(RunArgs a) {
           finished = traj_event(p, *P, tf, s0);
           if (lead) ++n_seg;
           if (p.fail == 0 && spin_on<false>(P->integrator)) {
-            seg_setup(g, *P, s0, p.t);
-            spin_begin<false>(g, *P, p.Sx, p.Sy, p.Sz, tempH);
+            seg_setup<true>(g, *P, s0, p.t);
+            spin_begin<false, true>(g, *P, p.Sx, p.Sy, p.Sz, tempH);
             mode = M_SEG;
           } else {
             if (p.fail == 0 && P->keep) p.h = tempH;
@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tpp3(RunArgs a) {
         }
       }
       if (mode == M_WEND) {
-        spin_settle(g, *P, p.Sx, p.Sy, p.Sz);
+        spin_settle<true>(g, *P, p.Sx, p.Sy, p.Sz);
         if (lead) {
           write_snap(a, i, w, p);
           store_state(a.s, i, p);  // every window end is a resumable checkpoint
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_tpp3(RunArgs a) {
     int r;
     if (P->integrator == 0) {
       fx::StageLocal<1> ks;
-      r = dop_attempt_v(G, ks, g, *P, p.Sx, p.Sy, p.Sz);
+      r = dop_attempt_v<true>(G, ks, g, *P, p.Sx, p.Sy, p.Sz);
       if (lead) ++n_dop;
     } else {
       // runs with RK45 sets do not get this kernel (the host leaves these
