@@ -16,6 +16,7 @@
 #include <string>
 #include <mutex>
 #include <thread>
+#include <tuple>
 #include <vector>
 
 #include "spintrack.h"
@@ -1838,12 +1839,18 @@ extern "C" int st_main_analysis(const st_options* opt_in, const char* out_path, 
 namespace {
 
 // Tuned configurations, keyed by the workload's shape, reused by every later
-// context of the process.
+// context of the process: what decides which kernels run and which candidates there are.  (Gas alone
+// turns the order round: 1,000 particles x 0.05 s, split_c3p1 against the best trajectory-ahead
+// variant 4.6 and 5.2 ms at 300 without gas, 31.9 and 11.5 at 1,000 with gas.)
 struct TuneKey {
-  int ntypes_mask;  // bit 0: a DOP853 set, bit 1: an RK45 set, bit 2: trajectory-only, bit 3 + t - 2: type t in 2-5
+  int types;   // bit 0: a DOP853 set, bit 1: an RK45 set, bit 2: trajectory-only, bit 3 + t - 2: type t in 2-5
+  int kind;    // ctx_kind, and bit 3 a set with gas, bit 4 a set with a pulse
   int log2n;
+  int spread;  // whether particles are spread over the SMs (then the split variants are candidates)
+  int length;  // binary exponent of the sample's simulated time
+  int sms;
   bool operator<(const TuneKey& o) const {
-    return ntypes_mask != o.ntypes_mask ? ntypes_mask < o.ntypes_mask : log2n < o.log2n;
+    return std::tie(types, kind, log2n, spread, length, sms) < std::tie(o.types, o.kind, o.log2n, o.spread, o.length, o.sms);
   }
 };
 // Process-wide choices, shared by contexts on any host thread.
@@ -1857,12 +1864,27 @@ std::mutex& tune_mutex() {
 }
 
 int autotune(st_ctx* c) {
-  TuneKey key{0, 0};
-  for (const auto& P : c->sets_h) {
-    const int it = P.integrator;
-    key.ntypes_mask |= it == 0 ? 1 : it == 1 ? 2 : (it >= 2 && it <= 5) ? (8 << (it - 2)) : 4;
-  }
+  // Simulated time that ranks the variants: 50 ms (~250 attempts per particle of DOP853 at rtol
+  // 1e-12), 50 us for sets of the fourth/fifth-order types (RK45, RKF45 and their quaternion forms), whose
+  // step at rtol 1e-12 is thousands of times shorter.  The run's own windows, so that short ones
+  // count as often as they come: 67,001 Magnus particles over three windows of 12 ms take 5.2 ms with
+  // the variant that three windows rank first, 7.2 with the one that a single window does.
+  // (64 windows at most.)
+  auto length_of = [](const st_options& o) {
+    const int it = o.integratorType;
+    return std::min({o.tf - o.t0, it == 1 || (it >= 3 && it <= 5) ? 5e-5 : 0.05, 64.0 * o.ioutInt});
+  };
   const int ext = ctx_kind(c);
+  TuneKey key{0, ext, 0, st::spread_lanes(c->n, c->sm_count) < 32, 0, c->sm_count};
+  double longest = 0.0;
+  for (size_t k = 0; k < c->sets_h.size(); ++k) {
+    const SetParams& P = c->sets_h[k];
+    const int it = P.integrator;
+    key.types |= it == 0 ? 1 : it == 1 ? 2 : (it >= 2 && it <= 5) ? (8 << (it - 2)) : 4;
+    key.kind |= (P.gas ? 8 : 0) | (P.a != 0.0 ? 16 : 0);
+    longest = std::max(longest, length_of(c->opts[k]));
+  }
+  key.length = longest > 0.0 ? std::ilogb(longest) : 0;
   while ((int64_t(1) << key.log2n) < c->n) ++key.log2n;
   {
     std::lock_guard<std::mutex> lock(tune_mutex());
@@ -1876,23 +1898,22 @@ int autotune(st_ctx* c) {
   const int nv = st::persistent_variant_count();
   // Sample: every set represented, about four particles per lane of the
   // widest candidate (one particle per lane would let the slowest particle
-  // decide and favour low occupancy), one short window on a scratch context,
-  // so each candidate runs for tens of milliseconds: the window is capped at
-  // 50 ms of simulated time for DOP853 sets (~250 attempts per particle at
-  // rtol 1e-12) and at 50 us for the fourth/fifth-order types (RK45, RKF45
-  // and their quaternion forms), whose step at rtol 1e-12 is thousands of
-  // times shorter.
+  // decide and favour low occupancy), that simulated time on a scratch context.
   std::vector<st_options> sample = c->opts;
   int widest = 1;
   for (int v = 0; v < nv; ++v)
     widest = std::max(widest, st::persistent_max_blocks_per_sm(v, ext) * st::persistent_variant_block(v));
   const int64_t want = std::max<int64_t>((int64_t)c->sm_count * widest * 4, 1);
   const double frac = std::min(1.0, (double)want / (double)std::max<int64_t>(c->n, 1));
+  int windows = 1;
   for (auto& o : sample) {
     o.numParticles = o.numParticles > 0 ? std::max(1, (int)std::ceil(o.numParticles * frac)) : 0;
-    const int it = o.integratorType;
-    o.ioutInt = std::min(o.ioutInt, (it == 1 || it == 3 || it == 4 || it == 5) ? 5e-5 : 0.05);
-    o.tf = o.t0 + o.ioutInt;
+    const double len = length_of(o);
+    if (len > 0.0) {
+      o.ioutInt = std::min(o.ioutInt, len);
+      o.tf = o.t0 + len * (1.0 + 1e-9);  // (the last window's end rounds either way)
+    }
+    windows = std::max(windows, st_num_windows(&o));
   }
   st_ctx* s = nullptr;
   ST_TRY(st_create_batch(sample.data(), (int)sample.size(), c->device, &s));
@@ -1902,24 +1923,25 @@ int autotune(st_ctx* c) {
   // the variant): on every workload measured, fewer resident blocks lost.
   for (int v = 0; v < nv; ++v) {
     if (st::persistent_max_blocks_per_sm(v, ext) <= 0) continue;  // not built for this kind of run
-    // The warp-specialised variants hide the trajectory behind the spin where a
-    // run is as long as its slowest particle: 1,000 particles x 0.5 s without
-    // gas, 46.6 ms against 55.8; at 20,000 they lose, 10.7 against 7.6.  They are
-    // candidates while the particles do not fill two warps per SM, the sample
-    // is then the run itself.  The three-lane variants were slower on every
-    // workload measured: only an explicit st_set_launch_config selects them.
+    // The warp-specialised variants hide the trajectory behind the spin where a run is as long as its
+    // slowest particle: 1,000 particles x 0.5 s without gas, 46.6 ms against 55.8; at 16,000 x 0.05 s they
+    // lose, 10.4 against 7.2.  They are candidates while particles are spread over the SMs.  The three-lane
+    // variants were slower on every workload measured, with idle lanes too (x 0.05 s, against the best other:
+    // 100 with gas 24.0 and 10.1 ms, 300 6.6 and 4.6, 1,000 6.6 and 5.7, 3,000 6.7 and 6.3): only an explicit
+    // st_set_launch_config selects them.
     const int family = st::persistent_variant_family(v);
-    if (family == 3 || (family == 2 && st::spread_lanes(s->n, s->sm_count) == 32)) continue;
+    if (family == 3 || (family == 2 && !key.spread)) continue;
     const int maxb = std::max(1, st::persistent_max_blocks_per_sm(v, ext));
     {
       st_launch_config cfg{0, maxb, v};
       st_set_launch_config(s, &cfg);
       double el = 1e300;
-      for (int rep = 0; rep < 2; ++rep) {  // first repetition warms the variant up
+      for (int rep = 0; rep < 2 || (rep < 4 && el < 5e-3); ++rep) {  // first repetition warms the variant up
         if (st_init(s) != ST_OK) break;
         const double t0 = now_s();
-        const int r = st_run_windows(s, ST_KERNEL_PERSISTENT, 0, 1, nullptr);
-        if (r == ST_OK) el = now_s() - t0;
+        const int r = st_run_windows(s, ST_KERNEL_PERSISTENT, 0, windows, nullptr);
+        if (r != ST_OK) break;
+        if (rep > 0) el = std::min(el, now_s() - t0);
       }
       if (el < best) {
         best = el;
