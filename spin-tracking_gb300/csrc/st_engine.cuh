@@ -552,7 +552,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batched(RunArgs a, int starve, 
   int tw = 0, twl = 0;
   bool t_run = false, t_done = lane >= a.spread, t_wend = false, t_stop = false;
   // ---- ring and window slots (records and slots in use)
-  int qhead = 0, qcount = 0, whead = 0, wcount = 0;
+  int qhead = 0, qcount = 0, whead = 0, wcount = 0, waiting = 0;  // waiting: particles in the ring
   // ---- spin side
   int mode = B_NEED;
   int64_t i = 0;
@@ -587,6 +587,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batched(RunArgs a, int starve, 
         tP = &a.sets[a.s.set[ti]];
         tf = ((double)tw + 1.0) * tP->ioutInt;
       }
+      // A ring may hold many particles of few segments.  A lane takes them all while plenty wait; of
+      // the last ones, only one beside the one that its spin side is on, so that no lane holds many
+      // while others go without.
+      const bool plenty = *((volatile unsigned long long*)&a.status->queue_head) +
+                              4ull * gridDim.x * (BLOCK / 32) * a.spread <=
+                          (unsigned long long)a.nitems;
       EventDefer dd;  // every field set: the warp's flush shuffles them from every lane
 #pragma unroll
       for (int k = 0; k < 7; ++k) dd.x[k] = 0.0;
@@ -614,7 +620,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batched(RunArgs a, int starve, 
           t_stop = false;
         }
         // the next particle
-        if (!t_run && !t_done && qcount < QCAP) {
+        if (!t_run && !t_done && qcount < QCAP && (plenty || waiting == 0)) {
           const unsigned long long item = atomicAdd(&a.status->queue_head, 1ull);
           if (item >= (unsigned long long)a.nitems) {
             t_done = true;
@@ -630,6 +636,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batched(RunArgs a, int starve, 
               ring[k].t0 = __longlong_as_double((long long)ti);
               ring[k].flags = R_FETCH;
               ++qcount;
+              ++waiting;
               tp = load_state(a.s, ti);
               t_run = !tp.stop;  // a particle that stopped before: the spin side carries it to the end
               tp.stop = false;
@@ -649,7 +656,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batched(RunArgs a, int starve, 
         const bool prod = t_run && !t_wend && !dd.pending && qcount < QCAP;
         const unsigned pm = __ballot_sync(FULL, prod);
         const unsigned defer_m = __ballot_sync(FULL, dd.pending);
-        const bool more = prod || (!t_run && !t_done && qcount < QCAP) || (t_wend && wcount < kAheadSlots);
+        const bool more = prod || (!t_run && !t_done && qcount < QCAP && (plenty || waiting == 0)) || (t_wend && wcount < kAheadSlots);
         const unsigned mm = __ballot_sync(FULL, more);
         const bool leave = mm == 0u || (__popc(mm) < keep && !__any_sync(FULL, more && qcount == 0));
         if (defer_m != 0u && (__popc(defer_m) >= defer_k || pm == 0u || leave)) {
@@ -696,6 +703,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batched(RunArgs a, int starve, 
           moved = true;
           const int flags = r->flags;
           if (flags & R_FETCH) {
+            --waiting;
             skip = false;
             i = (int64_t)__double_as_longlong(r->t0);
             P = &a.sets[a.s.set[i]];
