@@ -1845,12 +1845,12 @@ namespace {
 struct TuneKey {
   int types;   // bit 0: a DOP853 set, bit 1: an RK45 set, bit 2: trajectory-only, bit 3 + t - 2: type t in 2-5
   int kind;    // ctx_kind, and bit 3 a set with gas, bit 4 a set with a pulse
-  int log2n;
+  int count;   // particles: quarters of 256 lanes per SM up to eight times those, binary orders below and above
   int spread;  // whether particles are spread over the SMs (then the split variants are candidates)
-  int length;  // binary exponent of the sample's simulated time
+  int length;  // binary exponent of the run's simulated time, up to 50 ms
   int sms;
   bool operator<(const TuneKey& o) const {
-    return std::tie(types, kind, log2n, spread, length, sms) < std::tie(o.types, o.kind, o.log2n, o.spread, o.length, o.sms);
+    return std::tie(types, kind, count, spread, length, sms) < std::tie(o.types, o.kind, o.count, o.spread, o.length, o.sms);
   }
 };
 // Process-wide choices, shared by contexts on any host thread.
@@ -1863,17 +1863,9 @@ std::mutex& tune_mutex() {
   return m;
 }
 
+constexpr int kTuneProbe = 3;  // flat_b64_m4, which every kind of run has: measures how long the sample takes
+
 int autotune(st_ctx* c) {
-  // Simulated time that ranks the variants: 50 ms (~250 attempts per particle of DOP853 at rtol
-  // 1e-12), 50 us for sets of the fourth/fifth-order types (RK45, RKF45 and their quaternion forms), whose
-  // step at rtol 1e-12 is thousands of times shorter.  The run's own windows, so that short ones
-  // count as often as they come: 67,001 Magnus particles over three windows of 12 ms take 5.2 ms with
-  // the variant that three windows rank first, 7.2 with the one that a single window does.
-  // (64 windows at most.)
-  auto length_of = [](const st_options& o) {
-    const int it = o.integratorType;
-    return std::min({o.tf - o.t0, it == 1 || (it >= 3 && it <= 5) ? 5e-5 : 0.05, 64.0 * o.ioutInt});
-  };
   const int ext = ctx_kind(c);
   TuneKey key{0, ext, 0, st::spread_lanes(c->n, c->sm_count) < 32, 0, c->sm_count};
   double longest = 0.0;
@@ -1882,10 +1874,16 @@ int autotune(st_ctx* c) {
     const int it = P.integrator;
     key.types |= it == 0 ? 1 : it == 1 ? 2 : (it >= 2 && it <= 5) ? (8 << (it - 2)) : 4;
     key.kind |= (P.gas ? 8 : 0) | (P.a != 0.0 ? 16 : 0);
-    longest = std::max(longest, length_of(c->opts[k]));
+    longest = std::max(longest, std::min(P.tf - P.t0, 0.05));
   }
   key.length = longest > 0.0 ? std::ilogb(longest) : 0;
-  while ((int64_t(1) << key.log2n) < c->n) ++key.log2n;
+  // With a few particles per lane the number of rounds decides, and variants differ in lanes: 65,536 RKF45 particles
+  // with the choice of 50,000, 190 ms (six blocks per SM, a second round for a tenth of them), 118 with their own.
+  const int64_t quarter = std::max<int64_t>(1, (int64_t)c->sm_count * 64);
+  if (!key.spread && c->n < 32 * quarter)
+    key.count = 100 + (int)((c->n - 1) / quarter);
+  else
+    while ((int64_t(1) << key.count) < c->n) ++key.count;
   {
     std::lock_guard<std::mutex> lock(tune_mutex());
     auto it = tune_cache().find(key);
@@ -1898,25 +1896,64 @@ int autotune(st_ctx* c) {
   const int nv = st::persistent_variant_count();
   // Sample: every set represented, about four particles per lane of the
   // widest candidate (one particle per lane would let the slowest particle
-  // decide and favour low occupancy), that simulated time on a scratch context.
+  // decide and favour low occupancy), the same part of a round at the end as the run has (with
+  // six rounds and a half, full rounds alone rank variants 8% off), on a scratch context.
   std::vector<st_options> sample = c->opts;
   int widest = 1;
   for (int v = 0; v < nv; ++v)
     widest = std::max(widest, st::persistent_max_blocks_per_sm(v, ext) * st::persistent_variant_block(v));
-  const int64_t want = std::max<int64_t>((int64_t)c->sm_count * widest * 4, 1);
-  const double frac = std::min(1.0, (double)want / (double)std::max<int64_t>(c->n, 1));
+  const int64_t want = std::max<int64_t>((int64_t)c->sm_count * widest * 4, 1), round = 4 * quarter;
+  int64_t take = c->n;
+  if (take > want) take -= (take - want + round - 1) / round * round;
+  const double frac = (double)std::max<int64_t>(take, 1) / (double)std::max<int64_t>(c->n, 1);
+  for (auto& o : sample)
+    o.numParticles = o.numParticles > 0 ? std::max(1, (int)std::ceil(o.numParticles * std::min(frac, 1.0))) : 0;
+  // Its simulated time: the run's own windows (short ones count as often as they come: 67,001 Magnus particles over
+  // three windows of 12 ms take 5.2 ms with the variant that three windows rank first, 7.2 with the one that a single
+  // window does), at first up to 50 ms (~250 attempts per particle of DOP853 at rtol 1e-12) and 64
+  // windows, 50 us for the fourth/fifth-order types (RK45, RKF45 and their quaternion forms), whose step at rtol 1e-12
+  // is thousands of times shorter, then longer until a run of it takes 10 ms (RKF45 at rtol 1e-3: 50 us are 16 attempts).
   int windows = 1;
-  for (auto& o : sample) {
-    o.numParticles = o.numParticles > 0 ? std::max(1, (int)std::ceil(o.numParticles * frac)) : 0;
-    const double len = length_of(o);
-    if (len > 0.0) {
-      o.ioutInt = std::min(o.ioutInt, len);
-      o.tf = o.t0 + len * (1.0 + 1e-9);  // (the last window's end rounds either way)
+  auto set_length = [&](double grow) {  // false: no set got longer
+    bool longer = false;
+    windows = 1;
+    for (size_t k = 0; k < sample.size(); ++k) {
+      const st_options& full = c->opts[k];
+      st_options& o = sample[k];
+      const int it = full.integratorType;
+      const double all = full.tf - full.t0;
+      const double len = std::min(all, grow * std::min(it == 1 || (it >= 3 && it <= 5) ? 5e-5 : 0.05, 64.0 * full.ioutInt));
+      if (len > 0.0) {
+        o.ioutInt = std::min(full.ioutInt, len);
+        const double tf = o.t0 + len * (1.0 + 1e-9);  // (the last window's end rounds either way)
+        longer |= grow == 1.0 || tf > o.tf;
+        o.tf = tf;
+      }
+      windows = std::max(windows, st_num_windows(&o));
     }
-    windows = std::max(windows, st_num_windows(&o));
-  }
+    return longer;
+  };
+  set_length(1.0);
   st_ctx* s = nullptr;
   ST_TRY(st_create_batch(sample.data(), (int)sample.size(), c->device, &s));
+  auto time_of = [&](int v, int reps) {  // the first repetition warms the variant up
+    st_launch_config cfg{0, std::max(1, st::persistent_max_blocks_per_sm(v, ext)), v};
+    st_set_launch_config(s, &cfg);
+    double el = 1e300;
+    for (int rep = 0; rep < reps || (rep < 4 && el < 5e-3); ++rep) {
+      if (st_init(s) != ST_OK) break;
+      const double t0 = now_s();
+      if (st_run_windows(s, ST_KERNEL_PERSISTENT, 0, windows, nullptr) != ST_OK) break;
+      if (rep > 0) el = std::min(el, now_s() - t0);
+    }
+    return el;
+  };
+  for (double grow = 1.0;;) {
+    const double el = time_of(kTuneProbe, 2);
+    if (!(el < 1e-2)) break;
+    grow *= std::min(64.0, std::max(2.0, 2e-2 / el));
+    if (!set_length(grow) || st_set_params(s, sample.data(), (int)sample.size()) != ST_OK) break;
+  }
   double best = 1e300;
   st_launch_config best_cfg{0, 1, 1};
   // Each variant at its highest occupancy (its register budget is part of
@@ -1925,28 +1962,17 @@ int autotune(st_ctx* c) {
     if (st::persistent_max_blocks_per_sm(v, ext) <= 0) continue;  // not built for this kind of run
     // The warp-specialised variants hide the trajectory behind the spin where a run is as long as its
     // slowest particle: 1,000 particles x 0.5 s without gas, 46.6 ms against 55.8; at 16,000 x 0.05 s they
-    // lose, 10.4 against 7.2.  They are candidates while particles are spread over the SMs.  The three-lane
+    // lose, 10.4 against 7.2.  They are candidates while particles are spread over the SMs, and for RK45
+    // alone (65,536 particles x 50 us, 34.4 against 37.6).  The three-lane
     // variants were slower on every workload measured, with idle lanes too (x 0.05 s, against the best other:
     // 100 with gas 24.0 and 10.1 ms, 300 6.6 and 4.6, 1,000 6.6 and 5.7, 3,000 6.7 and 6.3): only an explicit
     // st_set_launch_config selects them.
     const int family = st::persistent_variant_family(v);
-    if (family == 3 || (family == 2 && !key.spread)) continue;
-    const int maxb = std::max(1, st::persistent_max_blocks_per_sm(v, ext));
-    {
-      st_launch_config cfg{0, maxb, v};
-      st_set_launch_config(s, &cfg);
-      double el = 1e300;
-      for (int rep = 0; rep < 2 || (rep < 4 && el < 5e-3); ++rep) {  // first repetition warms the variant up
-        if (st_init(s) != ST_OK) break;
-        const double t0 = now_s();
-        const int r = st_run_windows(s, ST_KERNEL_PERSISTENT, 0, windows, nullptr);
-        if (r != ST_OK) break;
-        if (rep > 0) el = std::min(el, now_s() - t0);
-      }
-      if (el < best) {
-        best = el;
-        best_cfg = cfg;
-      }
+    if (family == 3 || (family == 2 && !key.spread && key.types != 2)) continue;
+    const double el = time_of(v, 2);
+    if (el < best) {
+      best = el;
+      best_cfg = {0, std::max(1, st::persistent_max_blocks_per_sm(v, ext)), v};
     }
   }
   st_destroy(s);
