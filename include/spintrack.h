@@ -124,7 +124,11 @@ int st_run_until(st_ctx *ctx, double next_t);
  * own window count.  If snap != NULL, the state at the end of each window is
  * written to it: (w_end - w_begin) consecutive blocks, each laid out as
  * st_snapshot_bytes(ctx) bytes (see st_snapshot_field_offset).  snap is a
- * device pointer. */
+ * device pointer.  The trajectory-ahead variants ("ahead_*") keep rings of trajectory
+ * segments in device memory with the context: 112 bytes per record and 560 per lane for
+ * every launched lane, 301 MB for a full grid of 152 SMs with 64 records (161 MB with 32, 580
+ * with 128), less for few particles.  Where device memory does not hold them the run
+ * takes fewer blocks, with the same results. */
 int st_run_windows(st_ctx *ctx, int kernel, int w_begin, int w_end, void *snap);
 /* Bytes of one device snapshot block and the offset of field f within it
  * (f: 0 t, 1 pos_x, 2 pos_y, 3 pos_z, 4 v_x, 5 v_y, 6 v_z, 7 S_x, 8 S_y,
@@ -147,7 +151,8 @@ int st_synchronize(st_ctx *ctx);
 void *st_get_stream(st_ctx *ctx);
 /* Replace every set's parameters (same particle counts) without reallocating:
  * the device parameter table is re-uploaded; call st_init to restart.  Used
- * for parameter scans.  When gas collisions or an integrator type change, an
+ * for parameter scans.  When gas collisions, an integrator type or whether steps can run in
+ * fixed point (beta, atol against rtol) change, an
  * autotuned launch configuration (or a chosen one that has no kernel for the
  * new types) is dropped and tuned again at the next run.  No counterpart in the reference, which takes options
  * only at construction (include/particle.h:90). */
@@ -160,8 +165,8 @@ int st_get_launch_config(const st_ctx *ctx, st_launch_config *cfg);
 /* Number of persistent-kernel variants (valid st_launch_config.variant
  * values are 0 .. count-1) and the name of one, for external tuners.  The
  * autotuner offers the flattened ("flat_*") and trajectory-ahead ("ahead_*")
- * variants; the warp-specialised ("split_*") and three-lanes-per-particle
- * ("tpp3_*") ones run only when chosen here. */
+ * variants and, for few particles (up to 62 per SM) and for RK45 alone, the warp-specialised
+ * ("split_*") ones; the three-lanes-per-particle ("tpp3_*") ones run only when chosen here. */
 int st_launch_variant_count(void);
 const char *st_launch_variant_name(int variant);
 /* Device time budget for each following run call, in seconds (0 = none).

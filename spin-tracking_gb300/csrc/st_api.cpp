@@ -197,10 +197,12 @@ struct st_ctx {
     double deadline_s;
     cudaGraphExec_t exec;
     int launches;
+    char* ahead;  // the scratch its kernels use
   };
   std::vector<RunGraph> graphs;
   char* ahead = nullptr;     // trajectory-ahead kernel: scratch of its launched lanes (ensure_ahead)
-  size_t ahead_bytes = 0;
+  std::vector<char*> ahead_old;  // smaller ones that captured runs still use
+  size_t ahead_bytes = 0, ahead_refused = 0;  // (refused: the least that device memory did not hold)
   void* ens_buf = nullptr;   // ensemble statistics: control slots, block partials, histogram
   // integratorType 6 (every set of the context): the noise-spectrum aggregators
   bool spectrum = false;
@@ -461,43 +463,71 @@ int persistent_blocks(int64_t n, int sm_count, int variant, int per_sm) {
   return (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)sm_count * per_sm, (n + per_block - 1) / per_block));
 }
 
-// Scratch of the trajectory-ahead kernel (its lanes' rings), kept with the context.  A larger one takes the place of the old: run graphs that hold its
-// address go too.
-int ensure_ahead(st_ctx* c, size_t need) {
-  if (need <= c->ahead_bytes) return ST_OK;
-  ST_CUDA(cudaStreamSynchronize(c->stream));
+// Free the outgrown scratch that no captured run uses (between runs).
+void prune_ahead(st_ctx* c) {
+  auto unused = [&](char* p) {
+    for (const auto& g : c->graphs)
+      if (g.ahead == p) return false;
+    cudaFree(p);
+    return true;
+  };
+  c->ahead_old.erase(std::remove_if(c->ahead_old.begin(), c->ahead_old.end(), unused), c->ahead_old.end());
+}
+void drop_graphs(st_ctx* c) {
   for (auto& g : c->graphs) cudaGraphExecDestroy(g.exec);
   c->graphs.clear();
-  cudaFree(c->ahead);
+}
+
+// Scratch of the trajectory-ahead kernel (its lanes' rings), kept with the context: for *blocks blocks of
+// `lanes` lanes, or for as many as device memory holds (their lanes take the particles of the others). A
+// larger one takes the place of the old, which goes with the last captured run that uses it.
+int ensure_ahead(st_ctx* c, int ring, int64_t lanes, int* blocks) {
+  const size_t per = st::ahead_scratch_bytes(ring, lanes);
+  if (per == 0 || per * (size_t)*blocks <= c->ahead_bytes) return ST_OK;
+  const size_t held = c->ahead_bytes / per;
+  if (c->ahead_refused != 0 && per * (size_t)*blocks >= c->ahead_refused && held > 0) {
+    *blocks = (int)held;
+    return ST_OK;
+  }
+  ST_CUDA(cudaStreamSynchronize(c->stream));
+  if (c->ahead) c->ahead_old.push_back(c->ahead);
   c->ahead = nullptr;
   c->ahead_bytes = 0;
-  cudaError_t e = cudaMalloc(&c->ahead, need);
-  if (e != cudaSuccess) return fail(ST_ERR_NOMEM, std::string("trajectory rings: ") + cudaGetErrorString(e));
-  c->ahead_bytes = need;
-  return ST_OK;
+  prune_ahead(c);
+  if (cudaMalloc(&c->ahead, per * (size_t)*blocks) == cudaSuccess) {
+    c->ahead_bytes = per * (size_t)*blocks;
+    return ST_OK;
+  }
+  (void)cudaGetLastError();
+  drop_graphs(c);
+  prune_ahead(c);
+  for (int b = *blocks;; b = (b + 1) / 2) {
+    const cudaError_t e = cudaMalloc(&c->ahead, per * (size_t)b);
+    if (e == cudaSuccess) {
+      c->ahead_bytes = per * (size_t)b;
+      *blocks = b;
+      return ST_OK;
+    }
+    (void)cudaGetLastError();
+    c->ahead = nullptr;
+    c->ahead_refused = per * (size_t)b;
+    if (b == 1) return fail(ST_ERR_NOMEM, std::string("trajectory rings: ") + cudaGetErrorString(e));
+  }
 }
-// The same for the context's launch configuration, at once large enough for every variant
-// at its highest occupancy, so that a change of configuration keeps the graphs.
-int ensure_ahead_variant(st_ctx* c) {
-  auto bytes = [&](int v, int per_sm) {
-    const int64_t warps = (int64_t)persistent_blocks(c->n, c->sm_count, v, per_sm) * st::persistent_variant_block(v) / 32;
-    return st::ahead_scratch_bytes(st::persistent_variant_ring(v), warps * st::spread_lanes(c->n, c->sm_count));
-  };
-  size_t need = bytes(c->lc.variant, c->lc.blocks_per_sm);
-  if (need <= c->ahead_bytes) return ST_OK;
-  for (int v = 0; v < st::persistent_variant_count(); ++v)
-    if (st::persistent_variant_ring(v) > 0)
-      need = std::max(need, bytes(v, st::persistent_max_blocks_per_sm(v, ctx_kind(c))));
-  return ensure_ahead(c, need);
+// Blocks of the context's launch configuration, with scratch for them.
+int launch_blocks(st_ctx* c, int* blocks) {
+  *blocks = persistent_blocks(c->n, c->sm_count, c->lc.variant, c->lc.blocks_per_sm);
+  const int64_t lanes = (int64_t)st::persistent_variant_block(c->lc.variant) / 32 * st::spread_lanes(c->n, c->sm_count);
+  return ensure_ahead(c, st::persistent_variant_ring(c->lc.variant), lanes, blocks);
 }
 
 int run_persistent(st_ctx* c, int w_begin, int w_end, void* snap) {
   ST_TRY(ctx_build_order(c));
   if (c->lc.variant < 0 || c->lc.blocks_per_sm <= 0) ST_TRY(autotune(c));
-  ST_TRY(ensure_ahead_variant(c));
+  int blocks = 0;
+  ST_TRY(launch_blocks(c, &blocks));
   st::RunArgs a = make_args(c, w_begin, w_end, snap);
   ST_TRY(arm_deadline(c, a));
-  const int blocks = persistent_blocks(c->n, c->sm_count, c->lc.variant, c->lc.blocks_per_sm);
   int e = st::launch_persistent(a, c->lc.variant, blocks, c->lc.block_threads, c->stream);
   if (e) return fail(ST_ERR_CUDA, std::string("persistent launch: ") + cudaGetErrorString((cudaError_t)e));
   return ST_OK;
@@ -734,6 +764,7 @@ void st_destroy(st_ctx* c) {
   cudaFree(c->order_d);
   for (auto& g : c->graphs) cudaGraphExecDestroy(g.exec);
   cudaFree(c->ahead);
+  for (char* p : c->ahead_old) cudaFree(p);
   cudaFree(c->ens_buf);
   cudaFree(c->spec_sets_d);
   cudaFree(c->spec_pp);
@@ -822,7 +853,8 @@ int st_run_windows(st_ctx* c, int kernel, int w_begin, int w_end, void* snap) {
     if (c->lc.variant < 0 || c->lc.blocks_per_sm <= 0) ST_TRY(autotune(c));
     if (int e = st::persistent_prepare(c->lc.variant))
       return fail(ST_ERR_CUDA, std::string("kernel attributes: ") + cudaGetErrorString((cudaError_t)e));
-    ST_TRY(ensure_ahead_variant(c));
+    int blocks = 0;
+    ST_TRY(launch_blocks(c, &blocks));
   }
   c->fresh = false;
   c->adj_recorded = false;
@@ -857,7 +889,8 @@ int st_run_windows(st_ctx* c, int kernel, int w_begin, int w_end, void* snap) {
       cudaGraphExecDestroy(c->graphs.front().exec);
       c->graphs.erase(c->graphs.begin());
     }
-    c->graphs.push_back({kernel, w_begin, w_end, block, var, bps, snap, c->deadline_s, exec, launches});
+    c->graphs.push_back({kernel, w_begin, w_end, block, var, bps, snap, c->deadline_s, exec, launches, var < 0 ? nullptr : c->ahead});
+    prune_ahead(c);
     hit = c->graphs.size() - 1;
     captured = true;
   }
@@ -1107,9 +1140,9 @@ int adj_tape_launch(st_ctx* c, const st::RunArgs& a, const st::TapeArgs& t) {
   st::RunArgs r = a;
   r.spread = st::spread_lanes(a.nitems, c->sm_count);
   const int64_t per_block = st::tape_record_block() / 32 * (int64_t)r.spread;
-  const int blocks =
+  int blocks =
       (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)c->sm_count * per_sm, (a.nitems + per_block - 1) / per_block));
-  ST_TRY(ensure_ahead(c, st::ahead_scratch_bytes(st::tape_record_ring(), blocks * per_block)));
+  ST_TRY(ensure_ahead(c, st::tape_record_ring(), per_block, &blocks));
   r.ahead = c->ahead;
   int e = st::launch_tape_record(r, t, blocks, c->stream);
   if (e) return fail(ST_ERR_CUDA, std::string("adjoint tape launch: ") + cudaGetErrorString((cudaError_t)e));

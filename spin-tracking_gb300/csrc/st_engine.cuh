@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_persistent(RunArgs a) {
 // two phases alternated every other attempt and half the time went into
 // instruction supply (1,048,576 particles x 0.1 s: 398 ms with the trajectory
 // in FP64, 463 ms with its faster but larger integer code).  A ring of 64 records is
-// about 190 attempts.  The rings of a full grid (5 KB a lane, 10 with 128 records) exceed L2:
+// about 190 attempts.  The rings of a full grid (7.7 KB a lane, 14.9 with 128 records) exceed L2:
 // 286 bytes of DRAM traffic per segment, 142 GB/s, 2% of the copy bandwidth.
 //
 // The trajectory side crosses window ends and goes on to its next particle, so
@@ -336,6 +336,7 @@ struct alignas(16) SegRec {
   int on, scale;  // the fixed-point field scale (SegScale), packed
   int flags, grade;    // (grade: the field's, SegScale::ok)
 };
+static_assert(!ST_GRAD_IS_LINEAR || sizeof(SegRec) == 112, "the memory figures given for the rings");
 // SegRec::flags: window end reached, particle stopped, bounce, gas collision, field in fixed
 // point, start of a new particle (its index in t0); bits 8-15 sanity failure code.
 enum { R_FIN = 1, R_STOP = 2, R_WALL = 4, R_GAS = 8, R_FX = 16, R_FETCH = 32 };
