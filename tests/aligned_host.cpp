@@ -4,7 +4,7 @@
 // same inputs.  The steps' other forms are those of the three programs included.  Arguments:
 // form (0 DOP853, 1 its adjoint, 2 RK45 and 3 RKF45 with quaternions), count, seed, geometry of
 // the spin (0 any direction, 1 along, 2 across), of the adjoint, the small part, rotation angle,
-// axis, pulse (0, 1).  Prints the steps taken and refused, then component by component the
+// axis, pulse (0, 1), field (rad/s, 611.4 unless given).  Prints the steps taken and refused, then component by component the
 // error in fixed point and in FP64.
 #include <algorithm>
 #include <cmath>
@@ -54,6 +54,7 @@ int main(int argc, char** argv) {
   host_adj::g_state = std::strtoull(argv[3], nullptr, 10) * 2 + 1;
   const double small = std::atof(argv[6]), angle = std::atof(argv[7]);
   const bool pulse = std::atoi(argv[9]) != 0;
+  const double field = argc > 10 ? std::atof(argv[10]) : 611.4;
   for (int k = 0; k < 8; ++k) uniform();
   host_quat::g_stepper = form == 3;
   long taken = 0, refused = 0, wrong = 0;
@@ -69,18 +70,18 @@ int main(int argc, char** argv) {
     double l[3];
     for (int c = 0; c < 3; ++c) {
       const double size = c == axis ? 1e-3 : small;
-      q.o0[c] = 611.4 * (uniform() - 0.5) * size;
-      q.o1[c] = 3e3 * (uniform() - 0.5) * size;
-      q.o2[c] = 1e4 * (uniform() - 0.5) * size;
+      q.o0[c] = field * (uniform() - 0.5) * size;
+      q.o1[c] = 5.0 * field * (uniform() - 0.5) * size;
+      q.o2[c] = 16.0 * field * (uniform() - 0.5) * size;
     }
-    q.o0[axis] -= 611.4;
+    q.o0[axis] -= field;
     if (pulse) {
-      q.ga = -611.4 * small;
+      q.ga = -field * small;
       q.w = 6283.185307179586;
     }
     const double T = 7e-4 * (0.1 + uniform());
     q.t0 = uniform();
-    q.h = std::fmin(angle / 611.4 * (0.5 + uniform()), T * uniform());
+    q.h = std::fmin(angle / field * (0.5 + uniform()), T * uniform());
     const double x = q.t0 + (T - q.h) * uniform();
     q.tx = x - q.t0;
     draw(gS, small, axis, 1.0, q.S);

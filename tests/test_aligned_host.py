@@ -30,9 +30,9 @@ def aligned_host(tmp_path_factory):
     return exe
 
 
-def check(exe, form, spin, adjoint, small, angle, axis, pulse):
+def check(exe, form, spin, adjoint, small, angle, axis, pulse, field=611.4):
     out = subprocess.run([str(exe), str(form), "1500", "11", str(GEOMETRY[spin]), str(GEOMETRY[adjoint]), str(small), str(angle),
-                          str(axis), str(pulse)], check=True, capture_output=True, text=True).stdout.strip().splitlines()
+                          str(axis), str(pulse), str(field)], check=True, capture_output=True, text=True).stdout.strip().splitlines()
     head = out[0].split()
     assert int(head[1]) >= 1000 and int(head[5]) == 0, head
     if int(head[7]) >= 100:  # the medians of err^(-1/8)'s relative error
@@ -58,3 +58,12 @@ def test_steps(aligned_host, form, spin, small, axis, pulse):
 def test_step_adjoint(aligned_host, spin, adjoint, small, axis, pulse):
     for angle in (0.003, 0.05, 0.16):
         check(aligned_host, 1, spin, adjoint, small, angle, axis, pulse)
+
+
+@pytest.mark.parametrize("spin", sorted(GEOMETRY))
+@pytest.mark.parametrize("small", [0.3, 1e-3])
+@pytest.mark.parametrize("angle", [0.7, 1.0, 1.8, 2.6])
+@pytest.mark.parametrize("form", [2, 3], ids=["rk45q", "rkf45q"])
+def test_rotations_of_radians_in_a_pulse(aligned_host, form, angle, small, spin):
+    """In a strong field a step of radians is short against the pulse's quarter turn, so that it is taken."""
+    check(aligned_host, form, spin, "any", small, angle, 0, 1, field=3e5)
