@@ -371,9 +371,10 @@ def run_workload(args):
     line = {"workload": args.workload, "description": WORKLOADS[args.workload], "n_gpus": 1, "dtype": "f64",
             "data": "synthetic"}
 
-    def roofline(counters, secs, ext_type=None):
-        ach = workmodel.algorithmic_flops(counters, ext_type) / secs / 1e12
-        return {"bound": "fp64", "achieved": ach, "peak": peak.value, "unit": "TFLOP/s", "frac": ach / peak.value}
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+
+    def roofline(counters, secs, clk, ext_type=None):
+        return workmodel.roofline(counters, secs, peak.value, sms, clk["sm_mhz"] if clk else 2070.0, ext_type)
 
     if args.workload == "integrators":
         names = {0: "DOP853", 1: "RK45", 2: "Magnus CFET8", 3: "RK45 quaternion", 4: "RKF45", 5: "RKF45 quaternion"}
@@ -396,7 +397,7 @@ def run_workload(args):
                             "particles": npt, "value": npt * tf / secs, "ms_per_step": secs * 1e3, "attempts": att,
                             "attempts_per_s": att / secs, "segments": c["segments"],
                             "failed": int(np.count_nonzero(p.output_data()["fail"])),
-                            "roofline": roofline(c, secs, it if it >= 2 else None),
+                            "roofline": roofline(c, secs, clk, it if it >= 2 else None),
                             "launch_config": list(p.launch_config()), "clocks": clk})
         line.update({"metric": "particle*s simulated/s per integrator type", "unit": "particle*s/s",
                      "steps": args.steps, "warmup": 1, "per_type": per})
@@ -419,7 +420,7 @@ def run_workload(args):
             line.update({"metric": "particle*s simulated/s", "value": psec / secs, "unit": "particle*s/s",
                          "ms_per_step": secs * 1e3, "steps": args.steps, "warmup": 1, "particle_seconds": psec,
                          "counters": {k: c[k] for k in ("dop_attempts", "rk45_attempts", "segments")},
-                         "roofline": roofline(c, secs), "launch_config": list(p.launch_config()), "clocks": clk})
+                         "roofline": roofline(c, secs, clk), "launch_config": list(p.launch_config()), "clocks": clk})
             if args.workload == "sweep":
                 half = [sum(int(o.numParticles) * o.tf for o in sets[a:b]) for a, b in ((0, 2048), (2048, 4096))]
                 line["particle_seconds_dop853_rk45"] = half
@@ -623,14 +624,14 @@ def run_ours(args, world, rank, local):
     ms_per_step = elapsed / args.steps * 1e3
     value = n_total * sim * args.steps / elapsed
 
-    flops = workmodel.algorithmic_flops(counters)
-    achieved = flops / kernel_s * 1e-12
-    roof = {"bound": "fp64", "achieved": achieved, "peak": peak.value, "unit": "TFLOP/s",
-            "frac": achieved / peak.value if peak.value else None, "traffic": None,
-            "peak_source": "measured: DFMA issue-rate probe in this run (no FP64 entry in MEASURED_PEAKS.json; "
-                           "nominal GB300 FP64 1.25 TFLOP/s)",
-            "work_per_launch": {"dop_attempts": counters["dop_attempts"], "segments": counters["segments"],
-                                "flops": flops, "kernel_ms": kernel_s * 1e3}}
+    seen = clk.summary()
+    roof = workmodel.roofline(counters, kernel_s, peak.value, torch.cuda.get_device_properties(dev).multi_processor_count,
+                              seen["sm_mhz"] if seen else 2070.0)
+    if "fp64_equivalent" in roof:
+        roof["fp64_equivalent"]["peak_source"] = ("measured: DFMA issue-rate probe in this run (no FP64 entry in "
+                                                  "MEASURED_PEAKS.json; nominal GB300 FP64 1.25 TFLOP/s)")
+    roof["work_per_launch"] = {"dop_attempts": counters["dop_attempts"], "segments": counters["segments"],
+                               "flops": workmodel.algorithmic_flops(counters), "kernel_ms": kernel_s * 1e3}
     # DRAM bytes of one launch, from an ncu capture of dram__bytes_read.sum + dram__bytes_write.sum
     # (one pass) of this kernel on 1,048,576 particles x 0.1 s: 25.2 GB read + 19.5 GB written for
     # 156.7 M segments, 286 B each: the segment records' way through the rings, which together

@@ -1,6 +1,13 @@
-"""Algorithmic FP64 work of the hot path, for the roofline.
+"""Work of the hot path, for the roofline.
 
-Counts are of the engine's own arithmetic (st_device.cuh), FMA = 2 flops,
+DOP853 steps and the quaternion steppers' rotations run in fixed point on the integer
+pipes: what bounds them is instruction issue.  INSTR_PER_DOP_ATTEMPT is measured
+(profiles/k_batched_fixed_131k_full.md): warp instructions per attempt, one third of a
+segment's trajectory and the idle lanes' share included.
+
+The FP64 counts are of the FP64 form's arithmetic (st_device.cuh): the bound of the
+other steppers, and for fixed-point runs an equivalent, not work that they execute.
+FMA = 2 flops,
 add / mul / div / sqrt = 1, transcendentals (cos of the pulse, log, exp) not
 counted:
 
@@ -34,6 +41,7 @@ Integrator types 2-5 (ext_attempt; sincos of the rotations not counted):
     4 products (112), 2 rotations (82), error and controller (34)     361
 """
 FLOPS_PER_DOP_ATTEMPT = 785
+INSTR_PER_DOP_ATTEMPT = 298.4
 FLOPS_PER_RK45_ATTEMPT = 318
 FLOPS_PER_SEGMENT = 150
 FLOPS_PER_EXT_ATTEMPT = {2: 1191, 3: 497, 4: 318, 5: 361}
@@ -46,3 +54,21 @@ def algorithmic_flops(counters: dict, ext_type: int | None = None) -> float:
     ext = counters.get("ext_attempts", 0) * FLOPS_PER_EXT_ATTEMPT.get(ext_type, 0) if ext_type else 0
     return (counters["dop_attempts"] * FLOPS_PER_DOP_ATTEMPT + counters["rk45_attempts"] * FLOPS_PER_RK45_ATTEMPT
             + counters["segments"] * FLOPS_PER_SEGMENT + ext)
+
+
+def roofline(counters: dict, secs: float, fp64_peak: float, sms: int, sm_mhz: float, ext_type: int | None = None) -> dict:
+    """The bound of a run and the share of it that was reached.  Runs of DOP853 alone: warp instructions
+    issued against one per cycle and sub-partition.  The quaternion steppers (3, 5) and
+    mixed runs have no measured instruction count: FP64-equivalent rate alone.  RK45, Magnus and
+    RKF45 steps execute the counted FP64 work."""
+    tflops = algorithmic_flops(counters, ext_type) / secs / 1e12
+    fp64 = {"achieved": tflops, "peak": fp64_peak, "unit": "TFLOP/s", "frac": tflops / fp64_peak if fp64_peak else None}
+    dop, other = counters["dop_attempts"], counters["rk45_attempts"] + counters.get("ext_attempts", 0)
+    if dop and not other:
+        rate, peak = dop * INSTR_PER_DOP_ATTEMPT / secs / 1e9, sms * 4 * sm_mhz * 1e-3
+        return {"bound": "issue", "achieved": rate, "peak": peak, "unit": "G warp instructions/s", "frac": rate / peak,
+                "peak_source": "one instruction per cycle and sub-partition at the SM clock seen under load",
+                "fp64_equivalent": fp64}
+    if ext_type in (3, 5) or (dop and other):
+        return {"bound": "issue", "fp64_equivalent": fp64}
+    return {"bound": "fp64", **fp64}
