@@ -268,8 +268,9 @@ int st_adjoint_get_stats(const st_ctx *ctx, st_adjoint_stats *out);
 /* Unwrapped precession phase of every particle about x, accumulated on the
  * device over the whole run: atan2(Sz, Sy) + 2 pi * turns, where turns counts
  * the accepted steps that carried the spin's (y, z) projection across the
- * cut at +-pi (Sz changing sign with Sy < 0; a step at rtol 1e-12 turns the
- * spin by far less than pi).  Unlike phases taken from snapshots, it stays
+ * cut at +-pi (Sz changing sign with Sy < 0 at both ends of the step: DOP853 at
+ * rtol 1e-12 takes some 0.13 rad a step; a step of more than a quarter turn, which the Magnus
+ * stepper takes on long smooth segments, can miss a crossing).  Unlike phases taken from snapshots, it stays
  * continuous however long the window.  dst: device array, one double per
  * particle.  No counterpart in the reference (its scripts wrap phases). */
 int st_gather_phase(st_ctx *ctx, double *dst);

@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(kAdjBlock) k_adj_backward(RunArgs a, TapeArgs 
         SegPoly q;
         q.o0[0] = g.o0x; q.o0[1] = g.o0y; q.o0[2] = g.o0z;
         q.o1[0] = g.o1x; q.o1[1] = g.o1y; q.o1[2] = g.o1z;
-        seg_scale<kFixedPoint>(q, *P, x + h - g.t0);
+        seg_scale<kFixedPoint>(q, *P, x + h - g.t0, true);
         seg_open<kFixedPoint>(g, *P, q, g.t0, g.t0);
         fresh = false;
       }

@@ -98,17 +98,18 @@ bool to_bool(const std::string& s) {
 
 // ---------------------------------------------------------------- params
 // atol / rtol where the fixed-point DOP853 step can weigh a spin like the set's yi with it
-// (ratio_fits and spin_scale of st_fixed.cuh), else -1: the set steps in FP64 alone.
+// (ratio_fits and spin_scale of st_fixed.cuh), else the set steps in FP64 alone: -2 where that hangs on the
+// weights (the backward pass has none), -1 where the tolerances or beta are none of that form.
 double fixed_point_ratio(const st_options& o) {
   if (o.beta != 0.0 || !(o.rtol >= DBL_MIN) || !(o.atol >= 0.0)) return -1.0;
   const double ratio = o.atol / o.rtol, m = std::max({std::fabs(o.yi.x), std::fabs(o.yi.y), std::fabs(o.yi.z)});
-  if (!(m >= DBL_MIN) || !std::isfinite(m) || !(ratio >= DBL_MIN) || !std::isfinite(ratio)) return -1.0;
+  if (!(m >= DBL_MIN) || !std::isfinite(m) || !(ratio >= DBL_MIN) || !std::isfinite(ratio)) return -2.0;
   int se = std::ilogb(m) + 2;
   const double x = std::ldexp(o.yi.x, -se), y = std::ldexp(o.yi.y, -se), z = std::ldexp(o.yi.z, -se);
   const double norm = std::sqrt(x * x + y * y + z * z);
   se += norm > 0.5012 ? 2 : (norm > 0.2506 ? 1 : 0);
   const int e = std::ilogb(ratio);
-  return e >= se - 6 && e < se + 40 ? ratio : -1.0;
+  return e >= se - 6 && e < se + 40 ? ratio : -2.0;
 }
 
 int build_params(const st_options& o, int64_t first, SetParams* P) {

@@ -792,10 +792,12 @@ struct Seg {
 
 // Precession phase accumulation: the phase phi = atan2(Sz, Sy) about x jumps
 // by 2 pi where the spin's (y, z) projection crosses the cut at phi = +-pi
-// (Sy < 0, Sz changing sign).  An accepted step at rtol 1e-12 turns the spin
-// by far less than pi, so a crossing is a sign change of Sz with Sy < 0 at
-// both ends, counted +1 from phi near +pi to near -pi (phi increasing) and -1
-// back; atan2(Sz, Sy) + 2 pi * turns is then continuous along the run.
+// (Sy < 0, Sz changing sign).  While accepted steps turn the spin by less than a
+// quarter turn about x (DOP853 at rtol 1e-12: some 0.13 rad), a crossing is a sign
+// change of Sz with Sy < 0 at both ends; longer steps (Magnus passes a radian on long
+// smooth segments) and spins that cross near Sy = 0 can miss one.  Counted +1 from
+// phi near +pi to near -pi (phi increasing) and -1 back; atan2(Sz, Sy) + 2 pi * turns
+// is then continuous along the run.
 __device__ __forceinline__ int count_turn(double y0, double z0, double y1, double z1) {
   if (!(y0 < 0.0 && y1 < 0.0)) return 0;
   const bool s0 = signbit(z0), s1 = signbit(z1);
@@ -902,13 +904,13 @@ struct SegPoly {
 // Scale a polynomial given in doubles over a segment of length T.
 // FX (here and below): an instantiation for runs with sets that step in fixed point; without it
 // every step is inlined in FP64 (the FP64 form as a call beside the fixed-point one takes 1.25 times
-// as long: 65,536 particles x 0.1 s with beta 0.04, 103 ms against 82).
+// as long: 65,536 particles x 0.1 s with beta 0.04, 105 ms against 83).
 template <bool FX>
-__device__ __forceinline__ void seg_scale(SegPoly& q, const SetParams& P, double T) {
+__device__ __forceinline__ void seg_scale(SegPoly& q, const SetParams& P, double T, bool backward = false) {
   q.fx = false;
   if (!FX) return;
   const double gpa = P.gamma * P.a;
-  if (((P.integrator == 0 && P.tol_ratio >= 0.0) || P.integrator == 3 || P.integrator == 5) && (gpa == 0.0 || isfinite(P.w)))
+  if (((P.integrator == 0 && (P.tol_ratio >= 0.0 || (backward && P.tol_ratio == -2.0))) || P.integrator == 3 || P.integrator == 5) && (gpa == 0.0 || isfinite(P.w)))
   {
     turn_by(q.o0[0], q.o0[1], q.o0[2], P.axis);
     turn_by(q.o1[0], q.o1[1], q.o1[2], P.axis);
@@ -1318,9 +1320,10 @@ static __device__ __noinline__ int dop_attempt_slow(Seg& g, const SetParams& P, 
 // the segment is in fixed point Sx..Sz stay behind (spin_settle).
 // Returns as dop_attempt_f64.
 //
-// What bounds it: issue.  ~5,100 instructions, a third of them IMAD.WIDE (2.1
-// cycles each per SM sub-partition), most others 1-2 cycles, 11,300 cycles at two
-// warps, against ~510 FP64 instructions of 76 cycles before.
+// What bounds it: latency and supply of instructions at two warps per sub-partition (one
+// issued per 3.3 cycles; 298 warp instructions per attempt of a lane in the trajectory-ahead
+// kernel, the trajectory's and idle lanes' included), against ~510 FP64 instructions of 76 cycles
+// before: 1,048,576 particles x 0.1 s, 642 ms in FP64, 345 in fixed point.
 template <bool FX, class V, class KS>
 __device__ __forceinline__ int dop_attempt_v(const V& view, KS& ks, Seg& g, const SetParams& P, double& Sx, double& Sy,
                                              double& Sz) {

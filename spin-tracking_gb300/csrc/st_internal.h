@@ -38,7 +38,7 @@ struct SetParams {
   // ---- stepper (src/integrator.cpp:90-337)
   double rtol, atol, hmin, hmax, h0, safe, fac1, fac2, beta;
   double facc1, facc2, expo1, inv_safe;
-  double tol_ratio;               // atol / rtol (-1: FP64 steps only)
+  double tol_ratio;               // atol / rtol (-1: FP64 steps only, -2: forward)
   uint64_t wturn_m;               // |w| / (2 pi) = wturn_m 2^(wturn_e - 64), filled by launch_prepare_sets
   int wturn_e;
   int axis, pz;                   // component of B0 that leads, which fixed-point words have first; place of z in them
