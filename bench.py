@@ -374,7 +374,8 @@ def run_workload(args):
     sms = torch.cuda.get_device_properties(dev).multi_processor_count
 
     def roofline(counters, secs, clk, ext_type=None):
-        return workmodel.roofline(counters, secs, peak.value, sms, clk["sm_mhz"] if clk else 2070.0, ext_type)
+        return workmodel.roofline(counters, secs, peak.value, sms, clk["sm_mhz"] if clk else 2070.0, ext_type,
+                                  fp64=args.workload == "literal-gas")  # (segments far shorter than hmin)
 
     if args.workload == "integrators":
         names = {0: "DOP853", 1: "RK45", 2: "Magnus CFET8", 3: "RK45 quaternion", 4: "RKF45", 5: "RKF45 quaternion"}

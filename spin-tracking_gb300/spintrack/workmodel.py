@@ -56,19 +56,20 @@ def algorithmic_flops(counters: dict, ext_type: int | None = None) -> float:
             + counters["segments"] * FLOPS_PER_SEGMENT + ext)
 
 
-def roofline(counters: dict, secs: float, fp64_peak: float, sms: int, sm_mhz: float, ext_type: int | None = None) -> dict:
+def roofline(counters: dict, secs: float, fp64_peak: float, sms: int, sm_mhz: float, ext_type: int | None = None,
+             fp64: bool = False) -> dict:
     """The bound of a run and the share of it that was reached.  Runs of DOP853 alone: warp instructions
     issued against one per cycle and sub-partition.  The quaternion steppers (3, 5) and
     mixed runs have no measured instruction count: FP64-equivalent rate alone.  RK45, Magnus and
-    RKF45 steps execute the counted FP64 work."""
+    RKF45 steps execute the counted FP64 work, and so do DOP853 sets that step in FP64 alone (`fp64`)."""
     tflops = algorithmic_flops(counters, ext_type) / secs / 1e12
-    fp64 = {"achieved": tflops, "peak": fp64_peak, "unit": "TFLOP/s", "frac": tflops / fp64_peak if fp64_peak else None}
+    work = {"achieved": tflops, "peak": fp64_peak, "unit": "TFLOP/s", "frac": tflops / fp64_peak if fp64_peak else None}
     dop, other = counters["dop_attempts"], counters["rk45_attempts"] + counters.get("ext_attempts", 0)
-    if dop and not other:
+    if dop and not other and not fp64:
         rate, peak = dop * INSTR_PER_DOP_ATTEMPT / secs / 1e9, sms * 4 * sm_mhz * 1e-3
         return {"bound": "issue", "achieved": rate, "peak": peak, "unit": "G warp instructions/s", "frac": rate / peak,
                 "peak_source": "one instruction per cycle and sub-partition at the SM clock seen under load",
-                "fp64_equivalent": fp64}
+                "fp64_equivalent": work}
     if ext_type in (3, 5) or (dop and other):
-        return {"bound": "issue", "fp64_equivalent": fp64}
-    return {"bound": "fp64", **fp64}
+        return {"bound": "issue", "fp64_equivalent": work}
+    return {"bound": "fp64", **work}

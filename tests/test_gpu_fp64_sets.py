@@ -19,6 +19,7 @@ CASES = {
     "beta": dict(beta=0.04), "atol_small": dict(atol=1e-16), "atol_zero": dict(atol=0.0, rtol=1e-10, yi=(0.3, 0.4, 0.5)),
     "rk45": dict(integratorType=1, tf=2e-5, ioutInt=1e-5), "norm": dict(yi=(3000.0, 0.0, 4000.0), atol=1e-13),
     "trajectory_only": dict(integratorType=9),
+    "hmin_long": dict(hmin=3e-4), "hmin_past_collisions": dict(T=1.39, tf=2e-6, ioutInt=1e-6),
 }
 
 
