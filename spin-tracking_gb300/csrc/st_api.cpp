@@ -104,15 +104,27 @@ double segment_rate(const st_options& o) {
   return v / std::fabs(o.L.x) + v / std::fabs(o.L.y) + v / std::fabs(o.L.z) + (o.gas_coll ? 1.0 / o.tc : 0.0) + 1.0 / o.maxPosStep;
 }
 
+// Whether more than a few DOP853 steps reach the radian at which the fixed-point step ends: the step that the tolerance
+// allows (0.21 rad at 1e-12, its eighth root on) does, and so do more than 2% of the segments (exponential). Warps
+// whose lanes divide over both forms take both (100,000 particles x 0.05 s at 3 uT, ms: rtol 1e-7, fixed point
+// 18.5 and FP64 29.7, rtol 1e-6, 39.5 and 29.2; at 1 uT, 1e-6, 0.08% of the segments: 19.7 and 29.1).
+bool steps_of_radians(const st_options& o) {
+  const double omega = std::fabs(o.gamma) * (std::sqrt(o.B0.x * o.B0.x + o.B0.y * o.B0.y + o.B0.z * o.B0.z) + std::fabs(o.a));
+  const double norm = std::sqrt(o.yi.x * o.yi.x + o.yi.y * o.yi.y + o.yi.z * o.yi.z);
+  const double allowed = 0.21 * std::pow((o.rtol + o.atol / norm) * 1e12, 0.125);
+  const double angle = o.fixedStepSize ? omega * o.h : std::min(allowed, omega * o.hmax);
+  return angle > 0.95 && segment_rate(o) < 3.9 * omega;
+}
+
 // atol / rtol where the fixed-point DOP853 step can weigh a spin like the set's yi with it
 // (ratio_fits and spin_scale of st_fixed.cuh), else the set steps in FP64 alone: -2 where that hangs on the
-// weights (the backward pass has none) or on hmin, -1 where the tolerances or beta are none of that form.
+// weights (the backward pass has none), on hmin or on steps of a radian, -1 where the tolerances or beta are none of that form.
 // A segment shorter than hmin is overshot by a step of hmin and closed by one back, both in FP64; beyond an eighth
 // of the segments the warps' detours cost more than the fixed-point steps gain (65,536 particles x 600 collisions, ms:
 // mean free time 14, 10, 7, 5, 2, 0.5 hmin: 117, 134, 171, 217, 331, 424; in FP64 alone 135 to 150).
 double fixed_point_ratio(const st_options& o) {
   if (o.beta != 0.0 || !(o.rtol >= DBL_MIN) || !(o.atol >= 0.0)) return -1.0;
-  if (!(segment_rate(o) * o.hmin <= 0.125) && o.hmin > 0.0) return -2.0;
+  if ((!(segment_rate(o) * o.hmin <= 0.125) && o.hmin > 0.0) || steps_of_radians(o)) return -2.0;
   const double ratio = o.atol / o.rtol, m = std::max({std::fabs(o.yi.x), std::fabs(o.yi.y), std::fabs(o.yi.z)});
   if (!(m >= DBL_MIN) || !std::isfinite(m) || !(ratio >= DBL_MIN) || !std::isfinite(ratio)) return -2.0;
   int se = std::ilogb(m) + 2;

@@ -19,6 +19,7 @@ CASES = {
     "beta": dict(beta=0.04), "atol_small": dict(atol=1e-16), "atol_zero": dict(atol=0.0, rtol=1e-10, yi=(0.3, 0.4, 0.5)),
     "rk45": dict(integratorType=1, tf=2e-5, ioutInt=1e-5), "norm": dict(yi=(3000.0, 0.0, 4000.0), atol=1e-13),
     "trajectory_only": dict(integratorType=9),
+    "radians": dict(rtol=1e-5, atol=1e-5, gas_coll=False), "fixed_step_radians": dict(fixedStepSize=True, h=4e-3, nmax=20),
     "hmin_long": dict(hmin=3e-4), "hmin_past_collisions": dict(T=1.39, tf=2e-6, ioutInt=1e-6),
 }
 
@@ -47,7 +48,7 @@ def same(a, b, what):
 @pytest.mark.parametrize("gas", [False, True])
 @pytest.mark.parametrize("name", sorted(CASES))
 def test_every_variant_matches_plain(gpu, name, gas):
-    opt = options(gas_coll=gas, **CASES[name])
+    opt = options(**{"gas_coll": gas, **CASES[name]})
     ref = run(opt, st.KERNEL_PLAIN)
     ran = 0
     for v in range(_capi.load().st_launch_variant_count()):
