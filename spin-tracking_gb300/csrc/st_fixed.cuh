@@ -662,7 +662,7 @@ struct StepField {
   i64 w0[N];
   Limb w1[N], w2[N], hg, dphi;
   u64 phi0;
-  int ez, pz;
+  int ez, pz, dk;
   bool pulse;
   // without the pulse; the halves of the node and of its square
   __device__ __forceinline__ i64 at(int k, Limb c, Limb c2) const {
@@ -679,12 +679,14 @@ struct StepField {
     for (int c = 0; c < N; ++c)
       if (view.comp(c) == pz) w[c] += p;
   }
+  // the pulse's phase at a node, in turns
+  __device__ __forceinline__ u64 phase_at(Limb c) const { return phi0 + ((u64)mulq(c, dphi, 1) << dk); }
   __device__ __forceinline__ i64 pulse_at(Limb c) const {
-    return mulq(hg, limb(half_cos_turns(phi0 + (u64)mulq(c, dphi, 1)) + 16), 1);
+    return mulq(hg, limb(half_cos_turns(phase_at(c)) + 16), 1);
   }
 };
 // Components 1 and 2 come out at the grade ok - kw.  False: the step leaves the
-// segment, reaches 2^max_ez / 2 rad or passes a quarter of a pulse's turn.
+// segment, reaches 2^max_ez / 2 rad or passes 16 of the pulse's turns.
 template <class V>
 __device__ __forceinline__ bool step_field(const V& view, const SegScale& q, int kw, const i64* o0, const i64* o1,
                                            const i64* o2, i64 ga, u64 wm, int we, double x, double tx, double h, int max_ez,
@@ -722,11 +724,14 @@ __device__ __forceinline__ bool step_field(const V& view, const SegScale& q, int
   f.pz = q.pz;
   f.hg = f.dphi = {0, 0};
   f.phi0 = 0;
+  f.dk = 0;
   if (f.pulse) {
     f.hg = limb(mulq(hsl, limb(ga), 1) >> (q.pz == 0 ? 0 : kw));
-    const u64 dp = turns_of(h, wm, we);
-    if (dp >= 0x4000000000000000ull || bexp(h) - 1022 + we > 0) return false;  // a quarter turn or more
-    f.dphi = limb((i64)dp);
+    // the step's turns times 2^-dk, below a half
+    const int top = bexp(h) - 1022 + we;  // (below 2^top turns)
+    f.dk = top < -1 ? 0 : top + 2;
+    if (f.dk > 6) return false;  // 16 turns and more
+    f.dphi = limb((i64)turns_of(h, wm, we - f.dk));
     const u64 p = turns_of(fabs(x), wm, we);
     f.phi0 = x < 0.0 ? 0ull - p : p;
   }
@@ -1058,7 +1063,7 @@ __device__ __forceinline__ bool dop_adjoint(KS& ks, KS& ys, const SegScale& q, c
     Limb kl[3], kc[3], W[3], Y[3];
     i64 hc = 0, hs = 0, pulse = 0;
     if (f.pulse) {
-      const u64 phi = f.phi0 + (u64)mulq(nc, f.dphi, 1);
+      const u64 phi = f.phase_at(nc);
       hc = half_cos_turns(phi);
       pulse = mulq(f.hg, limb(hc + 16), 1);
       if (pulse_grads) hs = half_cos_turns(phi - 0x4000000000000000ull);

@@ -77,7 +77,7 @@ int main(int argc, char** argv) {
     q.o0[axis] -= field;
     if (pulse) {
       q.ga = -field * small;
-      q.w = 6283.185307179586;
+      q.w = argc > 11 ? std::atof(argv[11]) : 6283.185307179586;
     }
     const double T = 7e-4 * (0.1 + uniform());
     q.t0 = uniform();
