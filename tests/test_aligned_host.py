@@ -75,4 +75,4 @@ def test_rotations_of_radians_in_a_pulse(aligned_host, form, angle, small, spin)
 def test_turns_of_the_pulse_in_a_step(aligned_host, form, w, spin):
     """Steps of up to 16 turns of a weak fast pulse.  (The stages of DOP853 do not resolve it above a turn or so: its
     sums leave their range for most of them, which FP64 takes.)"""
-    check(aligned_host, form, spin, spin, 1e-2, 0.01, 0, 1, w=w, least=100 if w > 1e6 and form < 2 else 700)
+    check(aligned_host, form, spin, spin, 1e-2, 0.01, 0, 1, w=w, least=10 if w > 1e6 and form < 2 else 700)
