@@ -31,9 +31,9 @@
 //   STOPREQ -> BLOCKED  producer, acknowledging between two events
 //   any -> DONE         consumer, when it runs out of particles
 // Waits are bounded: a consumer lane starved of records for kSplitStallNs, or
-// a producer lane with work left that produced nothing for kSplitIdleNs, sets
-// RunStatus::pad and the kernel winds down; the host reports that run as an
-// error.  No block-wide barrier is taken after the start.
+// a producer lane with work left that produced nothing for kSplitIdleNs while none of its
+// consumers took a step, sets RunStatus::pad and the kernel winds down; the host
+// reports that run as an error.  No block-wide barrier is taken after the start.
 // Results equal k_batched's (and the plain kernel's) bit for bit: the producer
 // runs the same trajectory event (with diffuse reflections resolved at once,
 // as the plain kernel does) and the consumer the same step code.
@@ -50,7 +50,7 @@ constexpr unsigned long long kSplitIdleNs = 20000000000ull;  // a producer lane 
 // per-slot fields in shared memory (field-major over the block's slots)
 enum { SD_T = 0, SD_PX, SD_PY, SD_PZ, SD_VX, SD_VY, SD_VZ, SD_NG, SD_SPARE, SD_TF, SD_N };
 enum { SU_RX = 0, SU_RY, SU_RZ, SU_RW, SU_NCOLL, SU_NBOUNCE, SU_N };
-enum { SI_CTL = 0, SI_HEAD, SI_TAIL, SI_FAIL, SI_SET, SI_FLAGS, SI_N };
+enum { SI_CTL = 0, SI_HEAD, SI_TAIL, SI_FAIL, SI_SET, SI_FLAGS, SI_BEAT, SI_N };
 
 // Record fields, field-major: t_start, t_end, o0, o1 (+ p0, v0 when the grad hook is not linear).
 constexpr int kRecF = ST_GRAD_IS_LINEAR ? 8 : 14;
@@ -168,6 +168,7 @@ __global__ void __launch_bounds__((CW + PW) * 32, MINB) k_split(RunArgs a) {
     m.si[SI_CTL * NS + j] = kSplitIdle;
     m.si[SI_HEAD * NS + j] = 0;
     m.si[SI_TAIL * NS + j] = 0;
+    m.si[SI_BEAT * NS + j] = 0;
   }
   __syncthreads();
   bool stuck = false;
@@ -176,7 +177,7 @@ __global__ void __launch_bounds__((CW + PW) * 32, MINB) k_split(RunArgs a) {
     if (CREG > 0) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(PREG));
     const int pl = threadIdx.x - CW * 32;  // producer lane index
     unsigned long long n_seg = 0, idle_since = 0;
-    unsigned int tick = 0;
+    unsigned int tick = 0, beats = 0;
     while (true) {
       int best = -1, best_fill = QCAP, open = 0;
 #pragma unroll
@@ -205,9 +206,14 @@ __global__ void __launch_bounds__((CW + PW) * 32, MINB) k_split(RunArgs a) {
         ++n_seg;
         idle_since = 0;
       } else if (open > 0) {
+        // idle with full rings: no harm while its consumers take steps (one segment may take minutes)
+        unsigned int sum = 0;
+#pragma unroll
+        for (int c = 0; c < CW / PW; ++c) sum += (unsigned int)vload(&m.si[SI_BEAT * NS + pl + 32 * PW * c]);
         const unsigned long long now = globaltimer_ns();
-        if (idle_since == 0) idle_since = now;
+        if (idle_since == 0 || sum != beats) idle_since = now;
         else if (now - idle_since > kSplitIdleNs) stuck = true;
+        beats = sum;
         __nanosleep(64);
       }
       if (((++tick) & 63u) == 0u && __any_sync(FULL, stuck)) break;
@@ -404,6 +410,7 @@ __global__ void __launch_bounds__((CW + PW) * 32, MINB) k_split(RunArgs a) {
     } else {
       starved_since = 0;
     }
+    vstore(&m.si[SI_BEAT * NS + j], (int)tick);
     if (((++tick) & 255u) == 0u) {
       if (__any_sync(FULL, stuck)) break;
       if (__any_sync(FULL, past_deadline(dl))) {
