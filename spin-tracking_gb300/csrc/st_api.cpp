@@ -112,8 +112,8 @@ bool steps_of_radians(const st_options& o) {
   const double omega = std::fabs(o.gamma) * (std::sqrt(o.B0.x * o.B0.x + o.B0.y * o.B0.y + o.B0.z * o.B0.z) + std::fabs(o.a));
   const double norm = std::sqrt(o.yi.x * o.yi.x + o.yi.y * o.yi.y + o.yi.z * o.yi.z);
   const double allowed = 0.21 * std::pow((o.rtol + o.atol / norm) * 1e12, 0.125);
-  const double angle = o.fixedStepSize ? omega * o.h : std::min(allowed, omega * o.hmax);
-  return angle > 0.95 && segment_rate(o) < 3.9 * omega;
+  // (a fixed step becomes that of the segment's end and stays short)
+  return !o.fixedStepSize && std::min(allowed, omega * o.hmax) > 0.95 && segment_rate(o) < 3.9 * omega;
 }
 
 // atol / rtol where the fixed-point DOP853 step can weigh a spin like the set's yi with it
