@@ -95,7 +95,7 @@ def test_record_and_backward(gpu, gas):
 
 
 def test_split_waits_for_a_long_segment(gpu):
-    """One segment of ten million fixed steps keeps a consumer for longer than the producers' idle limit."""
-    opt = options(numParticles=3, tf=0.04, ioutInt=0.02, diffuse=0.1, gas_coll=False, fixedStepSize=True, h=2e-3, nmax=10000000, beta=1e-300)
+    """One segment of twenty million fixed steps keeps a consumer for longer than the producers' idle limit."""
+    opt = options(numParticles=3, tf=0.04, ioutInt=0.02, diffuse=0.1, gas_coll=False, fixedStepSize=True, h=2e-3, nmax=20000000, beta=1e-300)
     ref = run(opt, st.KERNEL_PERSISTENT, 3)
     same(run(opt, st.KERNEL_PERSISTENT, 14), ref, "split")
